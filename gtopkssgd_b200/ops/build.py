@@ -1,4 +1,5 @@
-"""In-tree build of libgtopk_b200.so (sm_100a only).
+"""In-tree build of libgtopk_b200.so (sm_100a only) and of the CPython module
+``_gtk_calls`` that calls its launch entry points.
 
 Every kernel file is plain CUDA with an ``extern "C"`` launcher, so nothing
 here needs the PyTorch headers and a full rebuild takes seconds.  The library
@@ -16,6 +17,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -23,6 +25,8 @@ CSRC = os.path.join(HERE, "csrc")
 LIB_NAME = "libgtopk_b200.so"
 LIB_PATH = os.path.join(HERE, LIB_NAME)
 DIGEST_PATH = LIB_PATH + ".digest"
+CALLS_SOURCE = os.path.join(CSRC, "py_calls.cpp")   # CPython module over the launch entry points
+CALLS_PATH = os.path.join(HERE, "_gtk_calls.so")
 OBJ_DIR = os.path.join(HERE, "build")
 
 ARCH_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a"]
@@ -38,7 +42,7 @@ def _nvcc() -> str:
 
 def sources() -> list[str]:
     names = sorted(f for f in os.listdir(CSRC) if f.endswith((".cu", ".cpp")))
-    return [os.path.join(CSRC, n) for n in names]
+    return [os.path.join(CSRC, n) for n in names if os.path.join(CSRC, n) != CALLS_SOURCE]
 
 
 def _digest() -> str:
@@ -48,12 +52,12 @@ def _digest() -> str:
             h.update(f.encode())
             with open(os.path.join(CSRC, f), "rb") as fh:
                 h.update(fh.read())
-    h.update(" ".join(ARCH_FLAGS + NVCC_FLAGS).encode())
+    h.update(" ".join(ARCH_FLAGS + NVCC_FLAGS + [sysconfig.get_config_var("SOABI") or ""]).encode())
     return h.hexdigest()
 
 
 def is_current() -> bool:
-    if not (os.path.exists(LIB_PATH) and os.path.exists(DIGEST_PATH)):
+    if not (os.path.exists(LIB_PATH) and os.path.exists(CALLS_PATH) and os.path.exists(DIGEST_PATH)):
         return False
     with open(DIGEST_PATH) as fh:
         return fh.read().strip() == _digest()
@@ -89,6 +93,13 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if res.returncode != 0:
         raise RuntimeError("link failed:\n%s\n%s" % (res.stdout, res.stderr))
     os.replace(tmp, LIB_PATH)
+    tmp = CALLS_PATH + ".tmp"
+    cmd = [nvcc, "-shared", "-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-I", CSRC, "-I", sysconfig.get_paths()["include"],
+           "-o", tmp, CALLS_SOURCE, "-L", HERE, "-l:" + LIB_NAME, "-Xlinker", "-rpath=$ORIGIN", "-cudart", "none"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("build of the call module failed:\n%s\n%s" % (res.stdout, res.stderr))
+    os.replace(tmp, CALLS_PATH)
     with open(DIGEST_PATH, "w") as fh:
         fh.write(_digest())
     return LIB_PATH

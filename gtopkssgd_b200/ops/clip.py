@@ -8,12 +8,10 @@ post-reduction ``clip_grad_norm_`` of the LSTM paths (gtopk_trainer.py:81-86).
 """
 from __future__ import annotations
 
-import ctypes as C
-
 import torch
 
 from . import lib as _lib
-from .select import current_stream_handle, pairs_to_tensors
+from .select import _ptr, current_stream_handle, pairs_to_tensors
 
 
 class ClipNorm:
@@ -31,9 +29,10 @@ class ClipNorm:
         if not self.is_cuda:
             self._cpu_sumsq += float(x.double().pow(2).sum())
             return
-        code = _lib.lib().gtk_k4_sumsq_dense(x.data_ptr(), x.numel(), self.state.data_ptr(),
-                                             current_stream_handle(self.device))
-        _lib.check(code, "gtk_k4_sumsq_dense")
+        code = _lib.calls().gtk_k4_sumsq_dense(x.data_ptr(), x.numel(), self.state.data_ptr(),
+                                               current_stream_handle(self.device))
+        if code:
+            _lib.check(code, "gtk_k4_sumsq_dense")
 
     def add_pairs(self, pairs: torch.Tensor, counts: torch.Tensor, nseg: int, seg_stride: int,
                   parity_word=None, parity_stride: int = 0) -> None:
@@ -44,11 +43,11 @@ class ClipNorm:
                 _, val = pairs_to_tensors(pairs[s * seg_stride:(s + 1) * seg_stride], int(counts[s]))
                 self._cpu_sumsq += float(val.double().pow(2).sum())
             return
-        code = _lib.lib().gtk_k4_sumsq_pairs(pairs.data_ptr(), counts.data_ptr(), nseg, seg_stride,
-                                             self.state.data_ptr(),
-                                             None if parity_word is None else parity_word.data_ptr(),
-                                             int(parity_stride), current_stream_handle(self.device))
-        _lib.check(code, "gtk_k4_sumsq_pairs")
+        code = _lib.calls().gtk_k4_sumsq_pairs(pairs.data_ptr(), counts.data_ptr(), nseg, seg_stride,
+                                               self.state.data_ptr(), _ptr(parity_word), parity_stride,
+                                               current_stream_handle(self.device))
+        if code:
+            _lib.check(code, "gtk_k4_sumsq_pairs")
 
     def finalize(self, max_norm: float, scale: float = 1.0) -> torch.Tensor:
         """coef <- min(1, max_norm / (scale*sqrt(sumsq) + 1e-6)); clears the
@@ -60,9 +59,10 @@ class ClipNorm:
             self.state.view(torch.float32)[2] = norm
             self._cpu_sumsq = 0.0
             return self.coef
-        code = _lib.lib().gtk_k4_finalize(self.state.data_ptr(), C.c_float(scale), C.c_float(max_norm),
-                                          self.coef.data_ptr(), current_stream_handle(self.device))
-        _lib.check(code, "gtk_k4_finalize")
+        code = _lib.calls().gtk_k4_finalize(self.state.data_ptr(), scale, max_norm, self.coef.data_ptr(),
+                                            current_stream_handle(self.device))
+        if code:
+            _lib.check(code, "gtk_k4_finalize")
         return self.coef
 
     def last_norm(self) -> float:

@@ -44,9 +44,32 @@ unsigned long long gtk_ctrl_bytes(void);
 unsigned long long gtk_k1state_bytes(void);
 const char* gtk_last_cuda_error(void);
 
+// ---- launches (each file documents its own) ----
 int gtk_k1_select(const float* g, float* r, const float* g_scale, long long d, unsigned int k,
                   void* cand, unsigned int cap, void* sel, void* state, void* ctrl,
                   float target_ratio, unsigned long long limit_ns, void* stream);
+int gtk_k2_exchange(const void* ranks_dev, unsigned int nranks, unsigned int rank_base, unsigned int P,
+                    unsigned int k, unsigned int kcap, unsigned int d, unsigned int nctas,
+                    unsigned long long limit_ns, int use_cluster, void* stream);
+int gtk_k2t_allgather(const void* ranks_dev, void* const* ctrl_dev, unsigned int nranks, unsigned int rank_base,
+                      unsigned int P, unsigned int k, unsigned int kcap, unsigned int work_cap, unsigned int d,
+                      int reselect, void* seg_counts, unsigned int nctas, unsigned long long limit_ns, void* stream);
+int gtk_k3_dense(float* p, float* buf, const float* g, const float* coef, float scale, long long d, float lr,
+                 const float* lr_ptr, float momentum, float dampening, float weight_decay, int nesterov,
+                 int first_step, void* stream);
+int gtk_k3_sparse(float* p, float* buf, const void* pairs, const unsigned int* counts, unsigned int nseg,
+                  unsigned int seg_stride, const float* coef, float scale, unsigned int d, float lr,
+                  const float* lr_ptr, float momentum, float dampening, float weight_decay, int nesterov,
+                  int first_step, int use_atomics, unsigned int* bad_index_count, const unsigned int* parity_word,
+                  unsigned int parity_stride, void* stream);
+int gtk_k3_scatter_dense(float* g, const void* pairs, const unsigned int* counts, unsigned int nseg,
+                         unsigned int seg_stride, float scale, long long d, int use_atomics,
+                         const unsigned int* parity_word, unsigned int parity_stride, void* stream);
+int gtk_k3_momentum_correct(float* v, float* g, float momentum, long long d, void* stream);
+int gtk_k4_sumsq_dense(const float* x, long long d, void* state, void* stream);
+int gtk_k4_sumsq_pairs(const void* pairs, const unsigned int* counts, unsigned int nseg, unsigned int seg_stride,
+                       void* state, const unsigned int* parity_word, unsigned int parity_stride, void* stream);
+int gtk_k4_finalize(void* state, float scale, float max_norm, float* coef_out, void* stream);
 
 #ifdef __cplusplus
 }

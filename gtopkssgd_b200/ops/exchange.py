@@ -244,13 +244,13 @@ def launch_gtopk(ranks: Sequence[ExchangeRank], desc: torch.Tensor, rank_base: i
     """Enqueue one gTop-k exchange.  ``ranks`` are the ranks served by this
     launch (one in production, all P when emulated); ``desc`` is their
     concatenated device descriptor array."""
-    L = _lib.lib()
     r0 = ranks[0]
     if nctas is None:
         nctas = default_nctas(k, len(ranks))
-    code = L.gtk_k2_exchange(desc.data_ptr(), len(ranks), rank_base, world, k, r0.kcap, r0.numel,
-                             nctas, int(limit_ms * 1e6), int(use_cluster), current_stream_handle(r0.resid.device))
-    _lib.check(code, "gtk_k2_exchange")
+    code = _lib.calls().gtk_k2_exchange(desc.data_ptr(), len(ranks), rank_base, world, k, r0.kcap, r0.numel, nctas,
+                                        int(limit_ms * 1e6), int(use_cluster), current_stream_handle(r0.resid.device))
+    if code:
+        _lib.check(code, "gtk_k2_exchange")
 
 
 def launch_allgather(ranks: Sequence[ExchangeRank], desc: torch.Tensor, seg_counts: torch.Tensor, rank_base: int,
@@ -259,15 +259,15 @@ def launch_allgather(ranks: Sequence[ExchangeRank], desc: torch.Tensor, seg_coun
     """Enqueue one Top-k all-gather ('topk'), optionally followed by the global
     re-selection ('topk2').  ``seg_counts`` is an int32 device tensor of
     len(ranks) * 16 words receiving the per-source counts."""
-    L = _lib.lib()
     r0 = ranks[0]
     if nctas is None:
         nctas = default_nctas(k * (world if reselect else 1) // 2 + 1, len(ranks))
     ctrls = (C.c_void_p * len(ranks))(*[C.c_void_p(r.ctrl.data_ptr()) for r in ranks])
-    code = L.gtk_k2t_allgather(desc.data_ptr(), ctrls, len(ranks), rank_base, world, k, r0.kcap, r0.work_cap,
-                               r0.numel, int(reselect), seg_counts.data_ptr(), nctas,
-                               int(limit_ms * 1e6), current_stream_handle(r0.resid.device))
-    _lib.check(code, "gtk_k2t_allgather")
+    code = _lib.calls().gtk_k2t_allgather(desc.data_ptr(), C.addressof(ctrls), len(ranks), rank_base, world, k, r0.kcap,
+                                          r0.work_cap, r0.numel, int(reselect), seg_counts.data_ptr(), nctas,
+                                          int(limit_ms * 1e6), current_stream_handle(r0.resid.device))
+    if code:
+        _lib.check(code, "gtk_k2t_allgather")
 
 
 def decode_k2_trace(tr: dict, rank: int, world: int) -> dict:

@@ -1,10 +1,12 @@
-"""ctypes binding of libgtopk_b200.so.
+"""Bindings of libgtopk_b200.so.
 
 The library exports a flat C ABI (raw device pointers + a CUDA stream handle),
-so no PyTorch C++ headers are involved.  ``lib()`` returns the loaded library
-with argument types declared; it builds the library first when it is missing
-or stale and a compiler is present.  On a machine with a GPU a missing library
-is an error, never a silent fallback.
+so no PyTorch C++ headers are involved.  ``lib()`` returns the library loaded
+with ctypes, argument types declared, for set-up and queries; ``calls()``
+returns the CPython module ``_gtk_calls`` with the launch entry points, whose
+argument conversion costs a tenth of ctypes'.  Both build the library first
+when it is missing or stale and a compiler is present.  On a machine with a GPU
+a missing library is an error, never a silent fallback.
 """
 from __future__ import annotations
 
@@ -16,6 +18,7 @@ from . import build as _build
 
 _lock = threading.Lock()
 _lib = None
+_calls = None
 
 GTK_OK = 0
 ERRORS = {-1: "bad argument", -2: "CUDA error", -3: "unsupported"}
@@ -48,7 +51,7 @@ class GtopkNativeError(RuntimeError):
 
 
 def _declare(lib):
-    vp, u32, u64, i64, f32, i32 = C.c_void_p, C.c_uint, C.c_ulonglong, C.c_longlong, C.c_float, C.c_int
+    vp, u32, u64, i64, i32 = C.c_void_p, C.c_uint, C.c_ulonglong, C.c_longlong, C.c_int
     lib.gtk_device_info.restype = vp
     lib.gtk_launch_count.restype = i64
     lib.gtk_reset_launch_count.restype = None
@@ -59,31 +62,10 @@ def _declare(lib):
     lib.gtk_k2rank_bytes.restype = u64
     lib.gtk_clipstate_bytes.restype = u64
     lib.gtk_last_cuda_error.restype = C.c_char_p
-    lib.gtk_k1_select.argtypes = [vp, vp, vp, i64, u32, vp, u32, vp, vp, vp, f32, u64, vp]
-    lib.gtk_k1_select.restype = i32
     lib.gtk_symm_layout.argtypes = [u32, i32, C.POINTER(u64)]
     lib.gtk_symm_layout.restype = None
     lib.gtk_k2rank_fill.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, u32, i32, u32, C.POINTER(vp)]
     lib.gtk_k2rank_fill.restype = i32
-    lib.gtk_k2_exchange.argtypes = [vp, u32, u32, u32, u32, u32, u32, u32, u64, i32, vp]
-    lib.gtk_k2_exchange.restype = i32
-    lib.gtk_k2t_allgather.argtypes = [vp, C.POINTER(vp), u32, u32, u32, u32, u32, u32, u32, i32, vp, u32, u64, vp]
-    lib.gtk_k2t_allgather.restype = i32
-    lib.gtk_k3_dense.argtypes = [vp, vp, vp, vp, f32, i64, f32, vp, f32, f32, f32, i32, i32, vp]
-    lib.gtk_k3_dense.restype = i32
-    lib.gtk_k3_sparse.argtypes = [vp, vp, vp, vp, u32, u32, vp, f32, u32, f32, vp, f32, f32, f32, i32, i32, i32, vp,
-                                  vp, u32, vp]
-    lib.gtk_k3_sparse.restype = i32
-    lib.gtk_k3_momentum_correct.argtypes = [vp, vp, f32, i64, vp]
-    lib.gtk_k3_momentum_correct.restype = i32
-    lib.gtk_k3_scatter_dense.argtypes = [vp, vp, vp, u32, u32, f32, i64, i32, vp, u32, vp]
-    lib.gtk_k3_scatter_dense.restype = i32
-    lib.gtk_k4_sumsq_dense.argtypes = [vp, i64, vp, vp]
-    lib.gtk_k4_sumsq_dense.restype = i32
-    lib.gtk_k4_sumsq_pairs.argtypes = [vp, vp, u32, u32, vp, vp, u32, vp]
-    lib.gtk_k4_sumsq_pairs.restype = i32
-    lib.gtk_k4_finalize.argtypes = [vp, f32, f32, vp, vp]
-    lib.gtk_k4_finalize.restype = i32
     lib.gtk_p2p_alloc.argtypes = [u64, C.POINTER(vp)]
     lib.gtk_p2p_alloc.restype = i32
     lib.gtk_p2p_free.argtypes = [vp]
@@ -127,6 +109,17 @@ def lib():
                         "libgtopk_b200.so is missing and could not be built: %s" % exc) from exc
         _lib = _declare(C.CDLL(path))
         return _lib
+
+
+def calls():
+    """The module with the launch entry points (same names and arguments as in C;
+    pointers as int or None)."""
+    global _calls
+    if _calls is None:
+        lib()  # builds both files when they are stale
+        from . import _gtk_calls
+        _calls = _gtk_calls
+    return _calls
 
 
 def check(code: int, what: str) -> None:

@@ -9,7 +9,6 @@ through the PyTorch oracle.
 """
 from __future__ import annotations
 
-import ctypes as C
 from dataclasses import dataclass
 from typing import Optional
 
@@ -42,11 +41,11 @@ def sgd_dense(p: torch.Tensor, buf: Optional[torch.Tensor], h: SgdHyper, first_s
         grad = g * c if g is not None else torch.zeros_like(p)
         oracle.sgd_step(p, buf, grad, h.lr, h.momentum, h.dampening, h.weight_decay, h.nesterov, first_step)
         return
-    L = _lib.lib()
-    code = L.gtk_k3_dense(p.data_ptr(), _ptr(buf), _ptr(g), _ptr(coef), C.c_float(scale), d, C.c_float(h.lr),
-                          _ptr(lr_dev), C.c_float(h.momentum), C.c_float(h.dampening), C.c_float(h.weight_decay),
-                          int(h.nesterov), int(first_step), current_stream_handle(p.device))
-    _lib.check(code, "gtk_k3_dense")
+    code = _lib.calls().gtk_k3_dense(p.data_ptr(), _ptr(buf), _ptr(g), _ptr(coef), scale, d, h.lr, _ptr(lr_dev),
+                                     h.momentum, h.dampening, h.weight_decay, int(h.nesterov), int(first_step),
+                                     current_stream_handle(p.device))
+    if code:
+        _lib.check(code, "gtk_k3_dense")
 
 
 def sgd_sparse(p: torch.Tensor, buf: Optional[torch.Tensor], pairs: torch.Tensor, counts: torch.Tensor,
@@ -76,15 +75,15 @@ def sgd_sparse(p: torch.Tensor, buf: Optional[torch.Tensor], pairs: torch.Tensor
                 step = sv + h.momentum * sb if h.nesterov else sb
             p.index_add_(0, idx, step, alpha=-h.lr)
         return
-    L = _lib.lib()
     if bad_index_count is None:
         bad_index_count = _scratch_word(p.device)
-    code = L.gtk_k3_sparse(p.data_ptr(), _ptr(buf), pairs.data_ptr(), counts.data_ptr(), nseg, seg_stride,
-                           _ptr(coef), C.c_float(scale), d, C.c_float(h.lr), _ptr(lr_dev), C.c_float(h.momentum),
-                           C.c_float(h.dampening), C.c_float(h.weight_decay), int(h.nesterov), int(first_step),
-                           int(use_atomics), bad_index_count.data_ptr(), _ptr(parity_word), int(parity_stride),
-                           current_stream_handle(p.device))
-    _lib.check(code, "gtk_k3_sparse")
+    code = _lib.calls().gtk_k3_sparse(p.data_ptr(), _ptr(buf), pairs.data_ptr(), counts.data_ptr(), nseg, seg_stride,
+                                      _ptr(coef), scale, d, h.lr, _ptr(lr_dev), h.momentum, h.dampening,
+                                      h.weight_decay, int(h.nesterov), int(first_step), int(use_atomics),
+                                      bad_index_count.data_ptr(), _ptr(parity_word), parity_stride,
+                                      current_stream_handle(p.device))
+    if code:
+        _lib.check(code, "gtk_k3_sparse")
 
 
 def scatter_dense(g: torch.Tensor, pairs: torch.Tensor, counts: torch.Tensor, nseg: int, seg_stride: int,
@@ -101,21 +100,21 @@ def scatter_dense(g: torch.Tensor, pairs: torch.Tensor, counts: torch.Tensor, ns
             idx, val = pairs_to_tensors(pairs[s * seg_stride:(s + 1) * seg_stride], n)
             g.index_add_(0, idx, val * scale)
         return
-    L = _lib.lib()
-    code = L.gtk_k3_scatter_dense(g.data_ptr(), pairs.data_ptr(), counts.data_ptr(), nseg, seg_stride,
-                                  C.c_float(scale), g.numel(), int(use_atomics), _ptr(parity_word), int(parity_stride),
-                                  current_stream_handle(g.device))
-    _lib.check(code, "gtk_k3_scatter_dense")
+    code = _lib.calls().gtk_k3_scatter_dense(g.data_ptr(), pairs.data_ptr(), counts.data_ptr(), nseg, seg_stride, scale,
+                                             g.numel(), int(use_atomics), _ptr(parity_word), parity_stride,
+                                             current_stream_handle(g.device))
+    if code:
+        _lib.check(code, "gtk_k3_scatter_dense")
 
 
 _scratch = {}
 
 
 def _scratch_word(device: torch.device) -> torch.Tensor:
-    key = (device.type, device.index)
-    if key not in _scratch:
-        _scratch[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _scratch[key]
+    word = _scratch.get(device)
+    if word is None:
+        word = _scratch[device] = torch.zeros(1, dtype=torch.int32, device=device)
+    return word
 
 
 def momentum_correct(v: torch.Tensor, g: torch.Tensor, momentum: float) -> None:
@@ -126,7 +125,7 @@ def momentum_correct(v: torch.Tensor, g: torch.Tensor, momentum: float) -> None:
         v.mul_(momentum).add_(g)
         g.copy_(v)
         return
-    L = _lib.lib()
-    code = L.gtk_k3_momentum_correct(v.data_ptr(), g.data_ptr(), C.c_float(momentum), g.numel(),
-                                     current_stream_handle(g.device))
-    _lib.check(code, "gtk_k3_momentum_correct")
+    code = _lib.calls().gtk_k3_momentum_correct(v.data_ptr(), g.data_ptr(), momentum, g.numel(),
+                                                current_stream_handle(g.device))
+    if code:
+        _lib.check(code, "gtk_k3_momentum_correct")
