@@ -15,6 +15,7 @@
 // where f = 1 on the first step and 1 - dampening afterwards.  Both parts add up
 // to the reference's update because it is affine in the gradient.
 #include "common.cuh"
+#include "launch.cuh"
 #include "host_api.h"
 
 namespace gtk {
@@ -42,8 +43,9 @@ struct SgdHyper {
 
 template <bool HAS_G, bool HAS_BUF>
 __global__ void __launch_bounds__(kK3Threads, 2)
-k3_dense(float* __restrict__ p, float* __restrict__ buf, const float* __restrict__ g,
-         const float* __restrict__ coef_ptr, float scale, long long d, SgdHyper h) {
+k3_dense(float* p, float* buf, const float* g,
+         const float* coef_ptr, float scale, long long d, SgdHyper h) {
+  pdl_begin(p, buf, g, coef_ptr, h.lr_ptr);
   if (h.lr_ptr) h.lr = *h.lr_ptr;
   const float coef = (HAS_G && coef_ptr) ? (*coef_ptr) * scale : scale;
   const float f = h.first_step ? 1.0f : 1.0f - h.dampening;
@@ -95,40 +97,62 @@ k3_dense(float* __restrict__ p, float* __restrict__ buf, const float* __restrict
   }
 }
 
-// Sparse part.  `pairs` holds nseg segments of seg_stride pairs; segment s has
-// counts[s] live pairs.  use_atomics: indices may repeat across segments.
+// Sparse part.  `pairs` holds nseg segments of seg_stride pairs; segment s (one row of the grid) has
+// counts[s] live pairs.  use_atomics: indices may repeat across segments.  Bound by the latency of scattered
+// 4-byte accesses, so a thread has kSparseBatch entries' loads in flight before the first store.
+constexpr int kSparseBatch = 4;
 __global__ void __launch_bounds__(256)
-k3_sparse(float* __restrict__ p, float* __restrict__ buf, const Pair* __restrict__ pairs,
-          const unsigned int* __restrict__ counts, unsigned int nseg, unsigned int seg_stride,
-          const float* __restrict__ coef_ptr, float scale, unsigned int d, SgdHyper h,
-          int use_atomics, unsigned int* __restrict__ bad_index_count,
-          const unsigned int* __restrict__ parity_word, unsigned int parity_stride) {
+k3_sparse(float* p, float* buf, const Pair* pairs,
+          const unsigned int* counts, unsigned int seg_stride,
+          const float* coef_ptr, float scale, unsigned int d, SgdHyper h,
+          int use_atomics, unsigned int* bad_index_count,
+          const unsigned int* parity_word, unsigned int parity_stride) {
+  pdl_begin(p, buf, pairs, counts, coef_ptr, parity_word, h.lr_ptr);
   if (h.lr_ptr) h.lr = *h.lr_ptr;
   pairs = parity_base(pairs, parity_word, parity_stride);
   const float coef = coef_ptr ? (*coef_ptr) * scale : scale;
   const float f = h.first_step ? 1.0f : 1.0f - h.dampening;
   const bool has_buf = buf != nullptr && h.momentum != 0.f;
+  const Pair* seg = pairs + (size_t)blockIdx.y * seg_stride;
+  unsigned int n = counts[blockIdx.y];
+  if (n > seg_stride) n = seg_stride;
   const unsigned int stride = gridDim.x * blockDim.x;
-  for (unsigned int s = 0; s < nseg; ++s) {
-    unsigned int n = counts[s];
-    if (n > seg_stride) n = seg_stride;
-    const Pair* seg = pairs + (size_t)s * seg_stride;
-    for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-      const Pair e = seg[i];
-      if ((unsigned int)e.idx >= d) {
+  for (unsigned int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kSparseBatch * stride) {
+    Pair e[kSparseBatch];
+    float pv[kSparseBatch], bv[kSparseBatch];
+#pragma unroll
+    for (int u = 0; u < kSparseBatch; ++u) {
+      const unsigned int i = i0 + (unsigned int)u * stride;
+      e[u].idx = -1;
+      if (i >= n) continue;
+      e[u] = seg[i];
+      if ((unsigned int)e[u].idx >= d) {
         atomicAdd(bad_index_count, 1u);
-        continue;
+        e[u].idx = -1;
       }
-      const float sv = e.val * coef;
+    }
+    if (!use_atomics) {
+#pragma unroll
+      for (int u = 0; u < kSparseBatch; ++u) {
+        pv[u] = bv[u] = 0.f;
+        if (e[u].idx < 0) continue;
+        pv[u] = p[e[u].idx];
+        if (has_buf) bv[u] = buf[e[u].idx];
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kSparseBatch; ++u) {
+      if (e[u].idx < 0) continue;
+      const float sv = e[u].val * coef;
       float step = sv;
       if (has_buf) {
         const float sb = f * sv;
-        if (use_atomics) atomicAdd(&buf[e.idx], sb);
-        else buf[e.idx] += sb;
+        if (use_atomics) atomicAdd(&buf[e[u].idx], sb);
+        else buf[e[u].idx] = bv[u] + sb;
         step = h.nesterov ? fmaf(h.momentum, sb, sv) : sb;
       }
-      if (use_atomics) atomicAdd(&p[e.idx], -h.lr * step);
-      else p[e.idx] = fmaf(-h.lr, step, p[e.idx]);
+      if (use_atomics) atomicAdd(&p[e[u].idx], -h.lr * step);
+      else p[e[u].idx] = fmaf(-h.lr, step, pv[u]);
     }
   }
 }
@@ -136,22 +160,20 @@ k3_sparse(float* __restrict__ p, float* __restrict__ buf, const Pair* __restrict
 // Optional: build the dense averaged gradient (for callers that want to look at
 // p.grad after synchronize()).  g must have been zeroed by the caller.
 __global__ void __launch_bounds__(256)
-k3_scatter_dense(float* __restrict__ g, const Pair* __restrict__ pairs,
-                 const unsigned int* __restrict__ counts, unsigned int nseg,
-                 unsigned int seg_stride, float scale, unsigned int d, int use_atomics,
-                 const unsigned int* __restrict__ parity_word, unsigned int parity_stride) {
+k3_scatter_dense(float* g, const Pair* pairs,
+                 const unsigned int* counts, unsigned int seg_stride, float scale, unsigned int d, int use_atomics,
+                 const unsigned int* parity_word, unsigned int parity_stride) {
+  pdl_begin(g, pairs, counts, parity_word);
   pairs = parity_base(pairs, parity_word, parity_stride);
+  const Pair* seg = pairs + (size_t)blockIdx.y * seg_stride;
+  unsigned int n = counts[blockIdx.y];
+  if (n > seg_stride) n = seg_stride;
   const unsigned int stride = gridDim.x * blockDim.x;
-  for (unsigned int s = 0; s < nseg; ++s) {
-    unsigned int n = counts[s];
-    if (n > seg_stride) n = seg_stride;
-    const Pair* seg = pairs + (size_t)s * seg_stride;
-    for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-      const Pair e = seg[i];
-      if ((unsigned int)e.idx >= d) continue;
-      if (use_atomics) atomicAdd(&g[e.idx], e.val * scale);
-      else g[e.idx] = e.val * scale;
-    }
+  for (unsigned int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const Pair e = seg[i];
+    if ((unsigned int)e.idx >= d) continue;
+    if (use_atomics) atomicAdd(&g[e.idx], e.val * scale);
+    else g[e.idx] = e.val * scale;
   }
 }
 
@@ -159,7 +181,8 @@ k3_scatter_dense(float* __restrict__ g, const Pair* __restrict__ pairs,
 // velocity, not the raw gradient, is what gets sparsified.  v = m*v + g; g = v, over a whole merged
 // group in one pass (the reference does it per parameter tensor inside the gradient hook).
 __global__ void __launch_bounds__(kK3Threads, 2)
-k3_momentum_correct(float* __restrict__ v, float* __restrict__ g, float m, long long d) {
+k3_momentum_correct(float* v, float* g, float m, long long d) {
+  pdl_begin(v, g);
   const unsigned int mis = (unsigned int)((reinterpret_cast<uintptr_t>(g) >> 2) & 3u);
   long long head = mis ? (4 - mis) : 0;
   if (head > d) head = d;
@@ -213,12 +236,13 @@ extern "C" int gtk_k3_dense(float* p, float* buf, const float* g, const float* c
     return GTK_ERR_ARG;
   SgdHyper h{lr_ptr, lr, momentum, dampening, weight_decay, nesterov, first_step};
   const int grid = dense_grid(d);
-  if (has_g && has_buf) k3_dense<true, true><<<grid, kK3Threads, 0, stream>>>(p, buf, g, coef, scale, d, h);
-  else if (has_g) k3_dense<true, false><<<grid, kK3Threads, 0, stream>>>(p, p, g, coef, scale, d, h);
-  else if (has_buf) k3_dense<false, true><<<grid, kK3Threads, 0, stream>>>(p, buf, p, coef, scale, d, h);
-  else k3_dense<false, false><<<grid, kK3Threads, 0, stream>>>(p, p, p, coef, scale, d, h);
+  cudaError_t e;
+  if (has_g && has_buf) e = launch_pdl(k3_dense<true, true>, grid, kK3Threads, stream, p, buf, g, coef, scale, d, h);
+  else if (has_g) e = launch_pdl(k3_dense<true, false>, grid, kK3Threads, stream, p, p, g, coef, scale, d, h);
+  else if (has_buf) e = launch_pdl(k3_dense<false, true>, grid, kK3Threads, stream, p, buf, p, coef, scale, d, h);
+  else e = launch_pdl(k3_dense<false, false>, grid, kK3Threads, stream, p, p, p, coef, scale, d, h);
   gtk_count_launch(1);
-  return cudaGetLastError() == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
+  return e == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
 }
 
 extern "C" int gtk_k3_sparse(float* p, float* buf, const void* pairs, const unsigned int* counts,
@@ -233,11 +257,10 @@ extern "C" int gtk_k3_sparse(float* p, float* buf, const void* pairs, const unsi
   SgdHyper h{lr_ptr, lr, momentum, dampening, weight_decay, nesterov, first_step};
   unsigned int blocks = (seg_stride + 255u) / 256u;
   if (blocks > 1184u) blocks = 1184u;
-  k3_sparse<<<blocks, 256, 0, stream>>>(p, buf, (const Pair*)pairs, counts, nseg, seg_stride, coef,
-                                        scale, d, h, use_atomics, bad_index_count, parity_word,
-                                        parity_stride);
+  const cudaError_t e = launch_pdl(k3_sparse, dim3(blocks, nseg), 256, stream, p, buf, (const Pair*)pairs, counts,
+                                   seg_stride, coef, scale, d, h, use_atomics, bad_index_count, parity_word, parity_stride);
   gtk_count_launch(1);
-  return cudaGetLastError() == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
+  return e == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
 }
 
 extern "C" int gtk_k3_scatter_dense(float* g, const void* pairs, const unsigned int* counts,
@@ -246,20 +269,20 @@ extern "C" int gtk_k3_scatter_dense(float* g, const void* pairs, const unsigned 
                                     unsigned int parity_stride, void* stream_) {
   cudaStream_t stream = (cudaStream_t)stream_;
   if (cudaMemsetAsync(g, 0, (size_t)d * sizeof(float), stream) != cudaSuccess) return GTK_ERR_CUDA;
+  if (nseg == 0 || seg_stride == 0) return GTK_OK;
   unsigned int blocks = (seg_stride + 255u) / 256u;
   if (blocks > 1184u) blocks = 1184u;
-  k3_scatter_dense<<<blocks, 256, 0, stream>>>(g, (const Pair*)pairs, counts, nseg, seg_stride,
-                                               scale, (unsigned int)d, use_atomics, parity_word,
-                                               parity_stride);
+  const cudaError_t e = launch_pdl(k3_scatter_dense, dim3(blocks, nseg), 256, stream, g, (const Pair*)pairs, counts,
+                                   seg_stride, scale, (unsigned int)d, use_atomics, parity_word, parity_stride);
   gtk_count_launch(1);
-  return cudaGetLastError() == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
+  return e == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
 }
 
 extern "C" int gtk_k3_momentum_correct(float* v, float* g, float momentum, long long d, void* stream_) {
   cudaStream_t stream = (cudaStream_t)stream_;
   if (d <= 0 || !v || !g) return GTK_ERR_ARG;
   if ((reinterpret_cast<uintptr_t>(v) & 15u) != (reinterpret_cast<uintptr_t>(g) & 15u)) return GTK_ERR_ARG;
-  k3_momentum_correct<<<dense_grid(d), kK3Threads, 0, stream>>>(v, g, momentum, d);
+  const cudaError_t e = launch_pdl(k3_momentum_correct, dense_grid(d), kK3Threads, stream, v, g, momentum, d);
   gtk_count_launch(1);
-  return cudaGetLastError() == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
+  return e == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
 }

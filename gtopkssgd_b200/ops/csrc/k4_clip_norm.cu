@@ -8,6 +8,7 @@
 //     coef = min(1, max_norm / (scale * sqrt(sumsq) + 1e-6))
 // and the consumers (K1 stream pass, K3) read coef from device memory.
 #include "common.cuh"
+#include "launch.cuh"
 #include "host_api.h"
 
 namespace gtk {
@@ -33,7 +34,8 @@ __device__ __forceinline__ void block_accumulate(double local, double* acc) {
 }
 
 __global__ void __launch_bounds__(kK4Threads)
-k4_sumsq_dense(const float* __restrict__ x, long long d, ClipState* st) {
+k4_sumsq_dense(const float* x, long long d, ClipState* st) {
+  pdl_begin(x, st);
   const unsigned int mis = (unsigned int)((reinterpret_cast<uintptr_t>(x) >> 2) & 3u);
   long long head = mis ? (4 - mis) : 0;
   if (head > d) head = d;
@@ -71,9 +73,10 @@ k4_sumsq_dense(const float* __restrict__ x, long long d, ClipState* st) {
 }
 
 __global__ void __launch_bounds__(kK4Threads)
-k4_sumsq_pairs(const Pair* __restrict__ pairs, const unsigned int* __restrict__ counts,
+k4_sumsq_pairs(const Pair* pairs, const unsigned int* counts,
                unsigned int nseg, unsigned int seg_stride, ClipState* st,
-               const unsigned int* __restrict__ parity_word, unsigned int parity_stride) {
+               const unsigned int* parity_word, unsigned int parity_stride) {
+  pdl_begin(pairs, counts, parity_word, st);
   if (parity_word) pairs += (size_t)((*parity_word - 1u) & 1u) * parity_stride;
   double total = 0.0;
   const unsigned int stride = gridDim.x * kK4Threads;
@@ -90,6 +93,7 @@ k4_sumsq_pairs(const Pair* __restrict__ pairs, const unsigned int* __restrict__ 
 }
 
 __global__ void k4_finalize(ClipState* st, float scale, float max_norm, float* coef_out) {
+  pdl_begin(st);
   if (threadIdx.x == 0 && blockIdx.x == 0) {
     const float norm = scale * (float)sqrt(st->sumsq);
     float coef = max_norm / (norm + 1e-6f);
@@ -115,9 +119,9 @@ extern "C" int gtk_k4_sumsq_dense(const float* x, long long d, void* state, void
   long long need = (d / 4 + 4ll * kK4Threads - 1) / (4ll * kK4Threads);
   long long grid = (long long)sms * 4;
   if (need < grid) grid = need > 0 ? need : 1;
-  k4_sumsq_dense<<<(int)grid, kK4Threads, 0, stream>>>(x, d, (ClipState*)state);
+  const cudaError_t e = launch_pdl(k4_sumsq_dense, (int)grid, kK4Threads, stream, x, d, (ClipState*)state);
   gtk_count_launch(1);
-  return cudaGetLastError() == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
+  return e == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
 }
 
 extern "C" int gtk_k4_sumsq_pairs(const void* pairs, const unsigned int* counts, unsigned int nseg,
@@ -128,16 +132,16 @@ extern "C" int gtk_k4_sumsq_pairs(const void* pairs, const unsigned int* counts,
   if (nseg == 0 || seg_stride == 0) return GTK_ERR_ARG;
   unsigned int blocks = (seg_stride + kK4Threads - 1) / kK4Threads;
   if (blocks > 592u) blocks = 592u;
-  k4_sumsq_pairs<<<blocks, kK4Threads, 0, stream>>>((const Pair*)pairs, counts, nseg, seg_stride,
-                                                    (ClipState*)state, parity_word, parity_stride);
+  const cudaError_t e = launch_pdl(k4_sumsq_pairs, blocks, kK4Threads, stream, (const Pair*)pairs, counts, nseg, seg_stride,
+                                   (ClipState*)state, parity_word, parity_stride);
   gtk_count_launch(1);
-  return cudaGetLastError() == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
+  return e == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
 }
 
 extern "C" int gtk_k4_finalize(void* state, float scale, float max_norm, float* coef_out,
                                void* stream_) {
   cudaStream_t stream = (cudaStream_t)stream_;
-  k4_finalize<<<1, 32, 0, stream>>>((ClipState*)state, scale, max_norm, coef_out);
+  const cudaError_t e = launch_pdl(k4_finalize, 1, 32, stream, (ClipState*)state, scale, max_norm, coef_out);
   gtk_count_launch(1);
-  return cudaGetLastError() == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
+  return e == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
 }
