@@ -44,7 +44,9 @@ struct Ctrl {
   unsigned int cursor[kMaxRounds + 2];        // one output cursor per round
   unsigned int tie[kMaxRounds + 2];           // one tie counter per round
   unsigned int live[kMaxRounds + 2];
-  unsigned int pad[64 - 16 - 3 * (kMaxRounds + 2)];
+  unsigned int ticket[8];                     // K1: work handed out per phase, and work completed
+  unsigned int done[8];
+  unsigned int pad[64 - 16 - 3 * (kMaxRounds + 2) - 16];
   unsigned long long trace[kTraceSlots];      // %globaltimer stamps of CTA 0 at phase boundaries
   // Radix histograms, one set of four rows per tree round (K2) or per use (K1: sets 0-2, rows 0-2).
   // K2 rows: 0 = first digit; 1 and 2[0..1023] = second digit of the entries whose first digit is one

@@ -17,7 +17,7 @@ enum {
   GTK_ERR_UNSUPPORTED = -3,
 };
 
-// Persistent per-group selection state (device memory, 32 bytes).
+// Persistent per-group selection state (device memory, 64 bytes, zero except tau = +inf at first).
 typedef struct K1State {
   float tau;                 // candidate threshold of the next stream pass (+inf: none yet)
   unsigned int n_sel;        // pairs written by the last select
@@ -26,7 +26,11 @@ typedef struct K1State {
   unsigned int n_fallbacks;  // running count of exact dense passes
   unsigned int n_calls;      // running count of calls
   float kth_mag;             // exact k-th magnitude of the last call
-  unsigned int reserved;
+  unsigned int stream_calls; // calls whose stream pass has begun
+  unsigned int aimed;        // candidates that tau was aimed at (0: tau is no prediction)
+  float slack;               // decaying maximum of |log(candidates found / aimed)|
+  float alpha;               // smoothed tail exponent (0: not measured yet)
+  unsigned int reserved[5];
 } K1State;
 
 typedef struct DeviceInfo {

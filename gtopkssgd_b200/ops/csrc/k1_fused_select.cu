@@ -1,103 +1,157 @@
-// K1: fused residual add + magnitude top-k selection + residual write-back,
-// one cooperative kernel.
+// K1: fused residual add + magnitude top-k selection + residual write-back, two
+// kernels behind one call.
 //
 // Replaces the op sequence of the reference's TopKCompressor.compress
 // (compression.py:32-57: add_, abs, topk, gather, mask fill/scatter, mul, sub_)
 // and the gather of the selected values (allreducer.py:543).
 //
-// Phase 1 (all CTAs)  one streaming pass over g and r (read 8d bytes, write 4d):
+// k1_stream  one pass over g and r (read 8d bytes, write 4d):
 //     acc = g*scale + r; entries with |acc| >= tau become candidates (appended to
-//     a bounded list, r <- 0, first radix digit counted), all others r <- acc.
-//     tau is a device-resident prediction from the previous call.
+//     a bounded list, r <- 0), all others r <- acc.  tau is a device-resident
+//     prediction from the previous call.
 //     Non-finite entries (+-Inf, NaN) count as the largest magnitudes on both paths,
 //     NaN above Inf, as torch.topk(|acc|) ranks them: they are selected, never left
 //     in the residual.
-// grid barrier
-// Phase 2  normal mode (k <= C <= cap candidates): the first C/1024 CTAs run the
-//     remaining two radix passes over the candidates, compact the k winners,
-//     return the rejected candidates to r and re-predict tau from the measured
-//     tail slope; the other CTAs leave.
+// k1_pick    normal mode (k <= C <= cap candidates): finds the k-th magnitude
+//     among the candidates, compacts the k winners, returns the rejected
+//     candidates to r and re-predicts tau from the measured tail slope.
 //     exact mode (C < k or the list overflowed; always on the first call, when
-//     tau is +inf): all CTAs restore r = acc from the stored candidates, then run
-//     a 3-pass radix select over all d entries of r and one collect pass.
+//     tau is +inf): restores r = acc from the stored candidates, then runs a
+//     3-pass radix select over all d entries of r and one collect pass.
 // The dense sparsified gradient of the reference is never materialised; the
 // output is k (int32 index, fp32 value) pairs in no particular order.
 //
+// Why two kernels: as one cooperative kernel the two halves met in a grid barrier
+// (1.3 us plus the wait for the slowest CTA), and a cooperative launch cannot
+// overlap with its predecessor (launch.cuh).  The boundary between the two costs
+// about as much as the barrier did, and both now start in the shadow of the
+// kernel before them.
+//
+// No CTA waits for one that may not have started: within k1_pick work is handed
+// out by tickets, and a CTA only waits for tickets that running CTAs hold.  So no
+// co-residency is needed, whatever else runs on the device.
+//
 // No host-side clearing: the caller provides two control blocks; call i uses
-// block (i & 1) and zeroes the other one for call i + 1 (i is K1State::n_calls,
-// read on the device, so the launch can be replayed from a CUDA graph).
+// block (i & 1) and the stream pass zeroes the other one for call i + 1 (i is
+// K1State::n_calls, read on the device, so the launches can be replayed from a
+// CUDA graph).  k1_stream reads only n_calls and k1_pick only stream_calls, each
+// written by the other kernel, so a late CTA never sees its call's own update.
 #include <atomic>
 #include <cstddef>
+#include <cooperative_groups.h>
 #include "select_common.cuh"
 #include "host_api.h"
+#include "launch.cuh"
 
 namespace gtk {
 
-constexpr int kK1Threads = kSelThreads;    // 512
-constexpr int kK1Vec = 4;                  // float4 loads of g and of r in flight per thread
+constexpr int kK1Threads = 512;            // k1_stream
 constexpr int kWarpStage = 128;            // pairs staged per warp
 constexpr int kWarpFlushAt = kWarpStage - 32;
-// From this many float4 per array on (48 M elements) the stream pass hands work out dynamically; below
-// it the static split is faster (measured: +3.6 % at 138 M and +1.5 % at 64 M, but -4 % at 25.6 M).
-constexpr long long kDynamicMinVec = 12ll * 1000 * 1000;
+// From this many float4 per array on (20 M elements) the stream pass hands work out dynamically; below it the
+// static split is as fast or faster (whole call: 59.0 against 60.3 us at 25.6 M, but 30.6 against 30.0 at 14.7 M).
+constexpr long long kDynamicMinVec = 5ll * 1000 * 1000;
+constexpr unsigned int kShards = 16;       // ticket counters of the dynamic stream pass
+// Up to kPickSmall candidates one CTA selects among them, up to kPickCluster one cluster of 8 CTAs, both from
+// registers; above, all CTAs share them out by tickets.  Measured at the borders (k1_pick alone): one CTA
+// 2.9 us at 2.6 K candidates and 2 us more than the cluster at 10 K; the cluster 9.3 us at 50 K as the tickets
+// at 100 K (whose phases cost 2 to 3 us of dependent global atomics and polls), but 27 us at 200 K, where 8
+// SMs are too few for the scattered write-back.
+constexpr unsigned int kPickSmall = 4096;
+constexpr unsigned int kPickCluster = 65536;
+constexpr int kPickThreads = 1024;
+constexpr int kPickCtas = 8;               // CTAs per cluster
+constexpr int kBins = kHistBins;           // 2048
 
-constexpr int kPredDigits = 3;  // second-digit histograms are kept for the predicted first digit and its neighbours
+// Bins of the first selection level: (key - lo) >> shift, the last bin open to the top.  lo is the candidate
+// threshold and shift puts the previous call's k-th magnitude into bins 256..511, so that the new one lies in
+// a bin of its own width even when the tail is steep (bits of the key itself would put almost all candidates
+// into two or three bins, whose counters then serialise the whole CTA).
+struct Bands {
+  uint32_t lo;
+  unsigned int shift;
+  __device__ __forceinline__ unsigned int bin(uint32_t key) const {  // key >= lo
+    const unsigned int b = (key - lo) >> shift;
+    return b < (unsigned int)kBins ? b : (unsigned int)kBins - 1u;
+  }
+};
+__device__ __forceinline__ Bands first_bands(float tau, float kth) {
+  const uint32_t lo = mag_key(tau), hi = mag_key(kth);
+  const uint32_t w = hi > lo ? hi - lo : 1u;
+  const int top = 31 - __clz(w);
+  return Bands{lo, top > 8 ? (unsigned int)(top - 8) : 0u};
+}
+
 struct StreamShared {
   Pair wstage[kK1Threads / 32][kWarpStage];  // per-warp candidate staging
-  unsigned int hist[kHistBins];              // first radix digit of this CTA's candidates
-  unsigned int hist1[kPredDigits][1024];     // second digit of the candidates whose first digit is pred-1, pred, pred+1
+  unsigned int warp_n[kK1Threads / 32];
+  unsigned int base;
+  unsigned int hist[kBins];                  // this CTA's candidates (counted only when k is large)
 };
-constexpr size_t kK1SmemBytes =
-    sizeof(StreamShared) > sizeof(SelectShared) ? sizeof(StreamShared) : sizeof(SelectShared);
-// bytes of a control block that K1 dirties: header, trace, three histogram sets
-// (set 0: candidate select, set 1: exact mode, set 2: second-digit histograms built by the stream pass)
-constexpr size_t kK1ClearBytes = offsetof(Ctrl, hist) + 3 * sizeof(((Ctrl*)0)->hist[0]);
+// bytes of a control block that K1 dirties: header, trace, three rows of one histogram set
+// (candidate levels in set 0, exact mode in set 1)
+constexpr size_t kK1ClearBytes = offsetof(Ctrl, hist) + 2 * sizeof(((Ctrl*)0)->hist[0]);
 
-__device__ __forceinline__ void warp_flush(Pair* wbuf, unsigned int& wcnt, Pair* cand,
-                                           unsigned int cap, unsigned int* counter, float* r) {
+// The warp's staged candidates to list positions base...; what does not fit stays in the residual.
+__device__ __forceinline__ void warp_store(const Pair* wbuf, unsigned int n, unsigned int base, Pair* cand,
+                                           unsigned int cap, float* r) {
+  for (unsigned int i = lane_id(); i < n; i += 32) {
+    const Pair p = wbuf[i];
+    if (base + i < cap) st_pair(&cand[base + i], p);
+    else r[p.idx] = p.val;
+  }
+}
+__device__ __forceinline__ void warp_flush(Pair* wbuf, unsigned int& wcnt, Pair* cand, unsigned int cap,
+                                           unsigned int* counter, float* r) {
   __syncwarp();
   unsigned int base = 0;
   if (lane_id() == 0) base = atomicAdd(counter, wcnt);
   base = __shfl_sync(0xffffffffu, base, 0);
-  for (unsigned int i = lane_id(); i < wcnt; i += 32) {
-    const Pair p = wbuf[i];
-    if (base + i < cap) {
-      st_pair(&cand[base + i], p);
-    } else {
-      r[p.idx] = p.val;  // list is full: the entry stays in the residual
-    }
-  }
+  warp_store(wbuf, wcnt, base, cand, cap, r);
   wcnt = 0;
   __syncwarp();
 }
 
-// Counts one candidate: its first radix digit always, its second digit when the
-// first one is within one of `pred` (the first digit of the previous call's k-th
-// magnitude), so that the candidate select can usually skip its first sweep.
-__device__ __forceinline__ void count_candidate(StreamShared& ss, float a, unsigned int pred) {
-  const uint32_t key = mag_key(a);
-  const unsigned int fd = key >> 20;
-  atomicAdd(&ss.hist[fd], 1u);
-  const unsigned int off = fd - pred + 1u;  // wraps for fd < pred - 1: then off >= kPredDigits
-  if (off < (unsigned int)kPredDigits) atomicAdd(&ss.hist1[off][(key >> 10) & 1023u], 1u);
+// What a thread of the stream pass carries along.
+struct StreamCtx {
+  float* r;
+  Pair* cand;
+  unsigned int cap;
+  unsigned int* counter;
+  float scale;
+  uint32_t tau_key;
+  Bands bands;
+  Pair* wbuf;
+  unsigned int wcnt;
+};
+
+// Appends the lanes' candidates (warp-uniform call).
+template <bool HIST>
+__device__ __forceinline__ void take_candidates(StreamShared& ss, StreamCtx& c, bool is, long long idx, float a) {
+  const unsigned int m = __ballot_sync(0xffffffffu, is);
+  if (!m) return;
+  if (is) {
+    Pair p;
+    p.idx = (int32_t)idx;
+    p.val = a;
+    c.wbuf[c.wcnt + __popc(m & lanemask_lt())] = p;
+    if (HIST) atomicAdd(&ss.hist[c.bands.bin(mag_key(a))], 1u);
+  }
+  c.wcnt += __popc(m);
+  if (c.wcnt > (unsigned int)kWarpFlushAt) warp_flush(c.wbuf, c.wcnt, c.cand, c.cap, c.counter, c.r);
 }
 
-// One tile of the stream pass: kK1Vec float4 of g and of r per thread, STRIDE
+// One tile of the stream pass: U float4 of g and of r per thread, STRIDE
 // float4 apart (the CTA's 512 threads or one warp's 32 lanes work side by side).
-template <int STRIDE>
-__device__ __forceinline__ void stream_tile(long long v0, long long nvec, long long head,
-                                            const float4* __restrict__ g4, float4* __restrict__ r4,
-                                            float scale, float tau, unsigned int pred, StreamShared& ss,
-                                            Pair* wbuf,
-                                            unsigned int& wcnt, Pair* __restrict__ cand, unsigned int cap,
-                                            unsigned int* counter, float* __restrict__ r) {
+template <int STRIDE, int U, bool HIST>
+__device__ __forceinline__ void stream_tile(long long v0, long long nvec, long long head, const float4* g4, float4* r4,
+                                            StreamShared& ss, StreamCtx& c) {
   // Candidates are decided on the bit pattern of |acc|, which orders like the magnitude for finite
   // values and puts +-Inf and NaN on top: a non-finite entry is a candidate on this path exactly as it
   // is the largest key on the exact path (torch.topk(|acc|) in compression.py:43 also ranks NaN first).
-  const uint32_t tau_key = __float_as_uint(tau);
-  float4 gv[kK1Vec], rv[kK1Vec];
+  float4 gv[U], rv[U];
 #pragma unroll
-  for (int u = 0; u < kK1Vec; ++u) {
+  for (int u = 0; u < U; ++u) {
     const long long v = v0 + (long long)u * STRIDE;
     if (v < nvec) {
       gv[u] = __ldcs(&g4[v]);
@@ -108,56 +162,57 @@ __device__ __forceinline__ void stream_tile(long long v0, long long nvec, long l
     }
   }
 #pragma unroll
-  for (int u = 0; u < kK1Vec; ++u) {
+  for (int u = 0; u < U; ++u) {
     const long long v = v0 + (long long)u * STRIDE;
     const bool inb = v < nvec;
     float a[4];
-    a[0] = fmaf(gv[u].x, scale, rv[u].x);
-    a[1] = fmaf(gv[u].y, scale, rv[u].y);
-    a[2] = fmaf(gv[u].z, scale, rv[u].z);
-    a[3] = fmaf(gv[u].w, scale, rv[u].w);
-    bool c[4];
+    a[0] = fmaf(gv[u].x, c.scale, rv[u].x);
+    a[1] = fmaf(gv[u].y, c.scale, rv[u].y);
+    a[2] = fmaf(gv[u].z, c.scale, rv[u].z);
+    a[3] = fmaf(gv[u].w, c.scale, rv[u].w);
+    bool is[4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) c[e] = inb && (mag_key(a[e]) >= tau_key);
+    for (int e = 0; e < 4; ++e) is[e] = inb && (mag_key(a[e]) >= c.tau_key);
     if (inb) {
       float4 o;
-      o.x = c[0] ? 0.f : a[0];
-      o.y = c[1] ? 0.f : a[1];
-      o.z = c[2] ? 0.f : a[2];
-      o.w = c[3] ? 0.f : a[3];
+      o.x = is[0] ? 0.f : a[0];
+      o.y = is[1] ? 0.f : a[1];
+      o.z = is[2] ? 0.f : a[2];
+      o.w = is[3] ? 0.f : a[3];
       r4[v] = o;
     }
-    const unsigned int any = __ballot_sync(0xffffffffu, c[0] | c[1] | c[2] | c[3]);
-    if (any) {
+    if (__any_sync(0xffffffffu, is[0] | is[1] | is[2] | is[3])) {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const unsigned int m = __ballot_sync(0xffffffffu, c[e]);
-        if (m) {
-          if (c[e]) {
-            Pair p;
-            p.idx = (int32_t)(head + (v << 2) + e);
-            p.val = a[e];
-            wbuf[wcnt + __popc(m & lanemask_lt())] = p;
-            count_candidate(ss, a[e], pred);
-          }
-          wcnt += __popc(m);
-          if (wcnt > (unsigned int)kWarpFlushAt) warp_flush(wbuf, wcnt, cand, cap, counter, r);
-        }
-      }
+      for (int e = 0; e < 4; ++e) take_candidates<HIST>(ss, c, is[e], head + (v << 2) + e, a[e]);
     }
   }
 }
 
-__device__ __forceinline__ void stream_phase(StreamShared& ss, const float* __restrict__ g,
-                                             float* __restrict__ r, float scale, float tau,
-                                             Pair* __restrict__ cand, unsigned int cap, Ctrl* ctrl,
-                                             long long d, unsigned int pred) {
-  for (int i = threadIdx.x; i < kHistBins; i += kK1Threads) ss.hist[i] = 0u;
-  for (int i = threadIdx.x; i < kPredDigits * 1024; i += kK1Threads) (&ss.hist1[0][0])[i] = 0u;
-  __syncthreads();
-  Pair* wbuf = ss.wstage[threadIdx.x >> 5];
-  unsigned int wcnt = 0;
-  unsigned int* counter = &ctrl->n_out;
+template <bool HIST, bool DYNAMIC>
+__global__ void __launch_bounds__(kK1Threads, 2)
+k1_stream(const float* g, float* r, const float* g_scale, long long d, Pair* cand, unsigned int cap, K1State* st,
+          Ctrl* ctrl_pair) {
+  constexpr int U = DYNAMIC ? 4 : 2;  // float4 loads of g and of r in flight per thread
+  __shared__ StreamShared ss;
+  if (HIST)
+    for (int i = threadIdx.x; i < kBins; i += kK1Threads) ss.hist[i] = 0u;
+  pdl_begin(g, r, g_scale, st, ctrl_pair);
+  const unsigned int calls = st->n_calls;
+  const float tau = st->tau;
+  Ctrl* ctrl = ctrl_pair + (calls & 1u);
+  if (blockIdx.x == 0 && threadIdx.x == 0) st->stream_calls = calls + 1u;
+  trace_stamp(ctrl, 0);
+  StreamCtx c;
+  c.r = r;
+  c.cand = cand;
+  c.cap = cap;
+  c.counter = &ctrl->n_out;
+  c.scale = g_scale ? *g_scale : 1.0f;
+  c.tau_key = __float_as_uint(tau);
+  c.bands = first_bands(tau, st->kth_mag);
+  c.wbuf = ss.wstage[threadIdx.x >> 5];
+  c.wcnt = 0;
+  if (HIST) __syncthreads();
 
   // Leading scalars up to the first 16-byte boundary (g and r share the offset).
   const unsigned int mis = (unsigned int)((reinterpret_cast<uintptr_t>(r) >> 2) & 3u);
@@ -168,211 +223,650 @@ __device__ __forceinline__ void stream_phase(StreamShared& ss, const float* __re
   const float4* g4 = reinterpret_cast<const float4*>(g + head);
   float4* r4 = reinterpret_cast<float4*>(r + head);
 
-  constexpr long long kTileVec = (long long)kK1Threads * kK1Vec;
-  constexpr long long kWarpTileVec = 32ll * kK1Vec;
-  if (nvec < kDynamicMinVec) {
+  if (!DYNAMIC) {
     // Static split: CTA b takes tiles b, b + grid, ...; every load instruction of the CTA covers 8 KB.
     // (One contiguous, equally sized range per CTA was tried: its ragged last tile costs almost a full
     // tile's latency in every CTA, and the call got 3 % slower at d = 25.6 M.)
+    constexpr long long kTileVec = (long long)kK1Threads * U;
     const long long ntiles = (nvec + kTileVec - 1) / kTileVec;
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-      stream_tile<kK1Threads>(tile * kTileVec + threadIdx.x, nvec, head, g4, r4, scale, tau, pred, ss, wbuf, wcnt,
-                              cand, cap, counter, r);
+      stream_tile<kK1Threads, U, HIST>(tile * kTileVec + threadIdx.x, nvec, head, g4, r4, ss, c);
   } else {
-    // Large vectors: SMs do not all see the same memory bandwidth, and with the static split the grid
-    // barrier waited up to 13 us (d = 64 M) for the slowest CTA.  Here work is handed out per warp in
-    // chunks of kChunkTiles warp-tiles (32 lanes x kK1Vec float4): the first chunk of a warp is fixed,
-    // further chunks come from a ticket counter that is read one chunk ahead, so the atomic's latency
-    // hides behind the loads.
-    constexpr long long kChunkTiles = 4;
-    const long long nchunks = (nvec + kWarpTileVec * kChunkTiles - 1) / (kWarpTileVec * kChunkTiles);
-    const unsigned int nwarps_grid = gridDim.x * (kK1Threads / 32);
-    unsigned int* ticket = &ctrl->scratch[1];
-    long long chunk = (long long)blockIdx.x * (kK1Threads / 32) + (threadIdx.x >> 5);
-    while (chunk < nchunks) {
+    // Large vectors: SMs do not all see the same memory bandwidth, and with the static split the slowest
+    // CTA ended up to 13 us (d = 64 M) after the first.  Here work is handed out per warp in tiles of 32 lanes
+    // x U float4: the first tile of a warp is fixed, further ones come from a ticket counter that is read one
+    // tile ahead, so the atomic's latency hides behind the loads.  kShards counters, each for every kShards-th
+    // warp and tile: one counter cannot serve a ticket per ns, and longer chunks (four tiles, 17 us each at
+    // the end) let the last warp finish 8 us after the first.
+    constexpr long long kWarpTileVec = 32ll * U;
+    const long long ntiles = (nvec + kWarpTileVec - 1) / kWarpTileVec;
+    const unsigned int warp = blockIdx.x * (kK1Threads / 32) + (threadIdx.x >> 5);
+    const unsigned int shard = warp % kShards;
+    const unsigned int warps = (gridDim.x * (kK1Threads / 32) - shard + kShards - 1u) / kShards;  // of this shard
+    unsigned int* ticket = &ctrl->hist[1][3][shard * 32u];  // 128 bytes apart; this row is not used otherwise
+    long long turn = warp / kShards;
+    for (long long tile = warp; tile < ntiles; tile = turn * kShards + shard) {
       unsigned int nxt = 0;
-      if (lane_id() == 0) nxt = atomicAdd(ticket, 1u);  // consumed after this chunk
-      for (long long wt = 0; wt < kChunkTiles; ++wt) {
-        const long long base = (chunk * kChunkTiles + wt) * kWarpTileVec;
-        if (base >= nvec) break;  // warp-uniform
-        stream_tile<32>(base + lane_id(), nvec, head, g4, r4, scale, tau, pred, ss, wbuf, wcnt, cand, cap, counter,
-                        r);
-      }
-      nxt = __shfl_sync(0xffffffffu, nxt, 0);
-      chunk = (long long)nwarps_grid + nxt;
+      if (lane_id() == 0) nxt = atomicAdd(ticket, 1u);  // consumed after this tile
+      stream_tile<32, U, HIST>(tile * kWarpTileVec + lane_id(), nvec, head, g4, r4, ss, c);
+      turn = (long long)warps + __shfl_sync(0xffffffffu, nxt, 0);
     }
   }
   // Scalar head and tail (at most 3 + 3 entries), one warp of CTA 0.
-  const uint32_t tau_key = __float_as_uint(tau);
   if (blockIdx.x == 0 && threadIdx.x < 32) {
     const long long nscalar = head + (d - tail0);
-    for (long long base = 0; base < nscalar; base += 32) {
-      const long long j = base + lane_id();
-      bool c = false;
-      float a = 0.f;
-      long long i = 0;
-      if (j < nscalar) {
-        i = j < head ? j : tail0 + (j - head);
-        a = fmaf(g[i], scale, r[i]);
-        c = mag_key(a) >= tau_key;
-        r[i] = c ? 0.f : a;
-      }
-      const unsigned int m = __ballot_sync(0xffffffffu, c);
-      if (m) {
-        if (c) {
-          Pair p;
-          p.idx = (int32_t)i;
-          p.val = a;
-          wbuf[wcnt + __popc(m & lanemask_lt())] = p;
-          count_candidate(ss, a, pred);
-        }
-        wcnt += __popc(m);
-        if (wcnt > (unsigned int)kWarpFlushAt) warp_flush(wbuf, wcnt, cand, cap, counter, r);
-      }
+    bool is = false;
+    float a = 0.f;
+    long long i = 0;
+    const long long j = lane_id();
+    if (j < nscalar) {
+      i = j < head ? j : tail0 + (j - head);
+      a = fmaf(g[i], c.scale, r[i]);
+      is = mag_key(a) >= c.tau_key;
+      r[i] = is ? 0.f : a;
     }
+    take_candidates<HIST>(ss, c, is, i, a);
   }
-  if (wcnt) warp_flush(wbuf, wcnt, cand, cap, counter, r);
-  // publish this CTA's part of the first-pass histogram
-  __syncthreads();
-  for (int i = threadIdx.x; i < kHistBins; i += kK1Threads) {
-    const unsigned int c = ss.hist[i];
-    if (c) atomicAdd(&ctrl->hist[0][0][i], c);
-  }
-  for (int i = threadIdx.x; i < kPredDigits * 1024; i += kK1Threads) {
-    const unsigned int c = ss.hist1[i >> 10][i & 1023];
-    if (c) atomicAdd(&ctrl->hist[2][i >> 10][i & 1023], c);
-  }
-}
-
-// Re-predict tau so that the next stream pass yields about target_ratio * k
-// candidates, assuming a power-law tail count(t) = k * (t / t_k)^(-alpha) whose
-// exponent is measured from (C candidates at tau_used, k entries at t_k).
-__device__ __forceinline__ float predict_tau(float t_k, float tau_used, unsigned int C,
-                                             unsigned int k, float target_ratio) {
-  float alpha = 8.0f;
-  const float ratio = (float)C / (float)(k ? k : 1u);
-  if (tau_used > 0.f && tau_used < t_k * 0.999f && ratio > 1.05f && isfinite(tau_used)) {
-    alpha = logf(ratio) / logf(t_k / tau_used);
-    alpha = fminf(fmaxf(alpha, 2.0f), 64.0f);
-  }
-  const float next = t_k * expf(-logf(target_ratio) / alpha);
-  return next > 0.f ? next : 0.f;
-}
-
-__global__ void __launch_bounds__(kK1Threads, 2)
-k1_fused(const float* __restrict__ g, float* __restrict__ r, const float* __restrict__ g_scale,
-         long long d, Pair* __restrict__ cand, unsigned int cap, Pair* __restrict__ sel,
-         unsigned int k, K1State* st, Ctrl* ctrl_pair, float target_ratio,
-         unsigned long long limit_ns) {
-  __shared__ __align__(16) unsigned char smem_raw[kK1SmemBytes];
-  // Every CTA reads the call parity before the grid barrier; it is advanced after it.
-  const unsigned int calls = st->n_calls;
-  Ctrl* ctrl = ctrl_pair + (calls & 1u);
-  {  // prepare the other control block for the next call
+  // The other control block, for the next call (its last user ended before this kernel began).
+  {
     uint4* other = reinterpret_cast<uint4*>(ctrl_pair + ((calls & 1u) ^ 1u));
     const size_t nvec16 = kK1ClearBytes / 16;
-    for (size_t i = (size_t)blockIdx.x * kK1Threads + threadIdx.x; i < nvec16;
-         i += (size_t)gridDim.x * kK1Threads)
+    for (size_t i = (size_t)blockIdx.x * kK1Threads + threadIdx.x; i < nvec16; i += (size_t)gridDim.x * kK1Threads)
       other[i] = make_uint4(0u, 0u, 0u, 0u);
   }
-  const float tau_used = st->tau;
-  const float scale = g_scale ? *g_scale : 1.0f;
-  trace_stamp(ctrl, 0);
-  const unsigned int pred = mag_key(st->kth_mag) >> 20;  // first digit of the previous call's k-th magnitude
-  stream_phase(*reinterpret_cast<StreamShared*>(smem_raw), g, r, scale, tau_used, cand, cap, ctrl, d, pred);
+  // One list reservation for what the CTA's warps still hold: a reservation per warp queues thousands of
+  // atomics on one address just when all CTAs finish.
+  const int w = threadIdx.x >> 5;
+  if (lane_id() == 0) ss.warp_n[w] = c.wcnt;
+  __syncthreads();
+  unsigned int before = 0, total = 0;
+#pragma unroll
+  for (int q = 0; q < kK1Threads / 32; ++q) {
+    const unsigned int n = ss.warp_n[q];
+    if (q < w) before += n;
+    total += n;
+  }
+  if (total) {
+    if (threadIdx.x == 0) ss.base = atomicAdd(c.counter, total);
+    __syncthreads();
+    warp_store(c.wbuf, c.wcnt, ss.base + before, cand, cap, r);
+  }
+  if (HIST) {  // publish this CTA's part of the first level
+    for (int i = threadIdx.x; i < kBins; i += kK1Threads) {
+      const unsigned int n = ss.hist[i];
+      if (n) atomicAdd(&ctrl->hist[0][0][i], n);
+    }
+  }
+  trace_stamp(ctrl, 1);  // CTA 0 finished its share
+}
 
-  trace_stamp(ctrl, 1);  // CTA 0 finished its share of the stream
-  RankBarrier bar_all{ctrl, gridDim.x, 0u, limit_ns};
-  if (!bar_all.sync(90)) return;
-  trace_stamp(ctrl, 2);  // every CTA did
-  if (blockIdx.x == 0 && threadIdx.x == 0) st->n_calls = calls + 1u;
+// ---------------------------------------------------------------------------
+// k1_pick
+// ---------------------------------------------------------------------------
+struct PickShared {
+  unsigned int hist[kBins];
+  unsigned int share[2][kBins / kPickCtas]; // cluster: the sums of bins b = rank (mod 8), for alternating levels
+  unsigned int warp_tot[kPickThreads / 32];
+  unsigned int warp_n[2][kPickThreads / 32];
+  unsigned int base[2];
+  unsigned int res_bin, res_krem;
+  unsigned int chunk;
+  unsigned int tie;
+  unsigned int cta_n[kPickCtas];
+  int ok;
+};
 
-  SelectShared& s = *reinterpret_cast<SelectShared*>(smem_raw);
-  const unsigned int count = __ldcg(&ctrl->n_out);
+// The keys that still matter: lo <= key <= hi, in bins of 2^shift.  An open level clamps everything
+// above its last bin into it.
+struct Level {
+  uint32_t lo, hi;
+  unsigned int shift;
+  bool open;
+  __device__ __forceinline__ bool has(uint32_t key) const { return key - lo <= hi - lo; }
+  __device__ __forceinline__ unsigned int bin(uint32_t key) const {
+    const unsigned int b = (key - lo) >> shift;
+    return b < (unsigned int)kBins ? b : (unsigned int)kBins - 1u;
+  }
+  // The level inside bin b; false when the bin is a single key (then lo is that key).
+  __device__ __forceinline__ bool narrow(unsigned int b) {
+    lo += b << shift;
+    if (!(open && b == (unsigned int)kBins - 1u)) {
+      if (shift == 0u) return false;
+      hi = lo + ((1u << shift) - 1u);
+    }
+    const uint32_t width = hi - lo;  // an open top is as wide as the keys go
+    const int bits = 32 - __clz(width);
+    shift = bits > 11 ? (unsigned int)(bits - 11) : 0u;
+    open = false;
+    return true;
+  }
+};
+
+// Finds the bin B with count(bins > B) < k_rem <= count(bins >= B): res_bin, and k_rem minus the count
+// above it: res_krem.  c: the complete counts of bins 2t and 2t + 1.
+__device__ __forceinline__ void find_bin(PickShared& s, uint2 c, unsigned int k_rem) {
+  const int t = threadIdx.x, w = t >> 5;
+  const unsigned int mine = c.x + c.y;
+  unsigned int suf = mine;  // inclusive suffix sum over the warp (higher lane = higher bins)
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned int v = __shfl_down_sync(0xffffffffu, suf, o);
+    if ((int)lane_id() + o < 32) suf += v;
+  }
+  if (lane_id() == 0) s.warp_tot[w] = suf;
+  __syncthreads();
+  const unsigned int v = s.warp_tot[lane_id()];
+  const unsigned int above = __reduce_add_sync(0xffffffffu, (int)lane_id() > w ? v : 0u) + (suf - mine);
+  if (above < k_rem && k_rem <= above + mine) {
+    const bool upper = k_rem <= above + c.y;
+    s.res_bin = 2u * t + (upper ? 1u : 0u);
+    s.res_krem = k_rem - above - (upper ? 0u : c.y);
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ uint2 global_counts(const unsigned int* ghist) {
+  return __ldcg(reinterpret_cast<const uint2*>(ghist) + threadIdx.x);
+}
+__device__ __forceinline__ uint2* my_bins(PickShared& s) {
+  return reinterpret_cast<uint2*>(s.hist) + threadIdx.x;
+}
+__device__ __forceinline__ void publish_hist(PickShared& s, unsigned int* ghist) {
+  const uint2 c = *my_bins(s);
+  if (c.x) atomicAdd(&ghist[2 * threadIdx.x], c.x);
+  if (c.y) atomicAdd(&ghist[2 * threadIdx.x + 1], c.y);
+}
+
+// Output position of the first of this thread's n entries.  cursor: global list cursor, or nullptr when
+// this CTA writes the whole list.  turn alternates between consecutive calls.
+__device__ __forceinline__ unsigned int place(PickShared& s, unsigned int n, unsigned int* cursor, unsigned int turn) {
+  const int w = threadIdx.x >> 5;
+  unsigned int pre = n;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned int v = __shfl_up_sync(0xffffffffu, pre, o);
+    if ((int)lane_id() >= o) pre += v;
+  }
+  if (lane_id() == 31) s.warp_n[turn & 1u][w] = pre;
+  __syncthreads();
+  const unsigned int v = s.warp_n[turn & 1u][lane_id()];
+  const unsigned int before = __reduce_add_sync(0xffffffffu, (int)lane_id() < w ? v : 0u);
+  unsigned int base = 0;
+  if (cursor) {
+    const unsigned int total = __reduce_add_sync(0xffffffffu, v);
+    if (threadIdx.x == 0) s.base[turn & 1u] = total ? atomicAdd(cursor, total) : 0u;
+    __syncthreads();
+    base = s.base[turn & 1u];
+  }
+  return base + before + pre - n;
+}
+
+// One entry against the threshold; called by whole warps.  Entries equal to it take tickets, the first
+// `quota` of which are selected.
+__device__ __forceinline__ bool passes(bool live, uint32_t key, uint32_t th, unsigned int quota, unsigned int* tie) {
+  const bool equal = live && key == th;
+  bool win = live && key > th;
+  const unsigned int m = __ballot_sync(0xffffffffu, equal);
+  if (m) {
+    unsigned int base = 0;
+    if (lane_id() == (unsigned int)(__ffs(m) - 1)) base = atomicAdd(tie, (unsigned int)__popc(m));
+    base = __shfl_sync(0xffffffffu, base, __ffs(m) - 1);
+    if (equal) win = base + __popc(m & lanemask_lt()) < quota;
+  }
+  return win;
+}
+
+// Calls f(chunk) for every chunk this CTA gets of phase ph; returns how many.
+template <typename F>
+__device__ __forceinline__ unsigned int for_chunks(PickShared& s, Ctrl* ctrl, int ph, unsigned int nchunks, F f) {
+  unsigned int mine = 0, next = 0;
+  if (threadIdx.x == 0) next = atomicAdd(&ctrl->ticket[ph], 1u);
+  for (;;) {
+    __syncthreads();
+    if (threadIdx.x == 0) s.chunk = next;
+    __syncthreads();
+    const unsigned int chunk = s.chunk;
+    if (chunk >= nchunks) return mine;
+    if (threadIdx.x == 0) next = atomicAdd(&ctrl->ticket[ph], 1u);  // arrives while this chunk is worked on
+    f(chunk);
+    ++mine;
+  }
+}
+// Reports this CTA's chunks of phase ph as done (all threads' work before it included); true in thread 0
+// of the CTA that completes the phase.
+__device__ __forceinline__ bool report(Ctrl* ctrl, int ph, unsigned int mine, unsigned int nchunks) {
+  __syncthreads();
+  if (threadIdx.x != 0 || mine == 0u) return false;
+  __threadfence();
+  return atomicAdd(&ctrl->done[ph], mine) + mine == nchunks;
+}
+// Waits until the phase is complete.  All its tickets are taken by running CTAs when a CTA gets here.
+__device__ __forceinline__ bool wait_phase(PickShared& s, Ctrl* ctrl, int ph, unsigned int nchunks,
+                                           uint64_t limit_ns, uint32_t where) {
+  if (threadIdx.x == 0) {
+    int ok = 1;
+    const uint64_t t0 = globaltimer_ns();
+    unsigned int spins = 0;
+    while (ld_acquire_gpu_u32(&ctrl->done[ph]) < nchunks) {
+      if (aborted(ctrl)) { ok = 0; break; }
+      if ((++spins & 63u) == 0u && globaltimer_ns() - t0 > limit_ns) {
+        record_error(ctrl, ST_TIMEOUT_BARRIER, where);
+        ok = 0;
+        break;
+      }
+    }
+    s.ok = ok;
+  }
+  __syncthreads();
+  return s.ok != 0;
+}
+
+// State for the next call: tau such that its stream pass finds about ratio * k candidates, from a
+// power-law tail count(t) = k * (t / t_k)^(-alpha) whose exponent is measured from (C candidates at the tau
+// used, k entries at t_k) and smoothed.  Every candidate beyond k costs an append, a count and a scattered
+// write back, a shortfall costs an exact pass.  So ratio adapts to how well the predictions have
+// hit lately (|log(found / aimed)|, decaying maximum) and to the sampling noise of a small k, at most
+// target_ratio.
+// `was` is the state as the kernel found it.
+__device__ __forceinline__ void finish_state(K1State* st, const K1State& was, uint32_t key_k, unsigned int n_sel,
+                                             unsigned int k, unsigned int count, unsigned int C, bool exact,
+                                             float target_ratio) {
+  const float t_k = __uint_as_float(key_k), tau = was.tau;
+  float alpha = was.alpha, slack = was.slack;
+  const unsigned int aimed = was.aimed;
+  const float ratio_found = (float)C / (float)k;
+  if (!exact && tau > 0.f && tau < t_k * 0.9999f && ratio_found > 1.02f && isfinite(t_k)) {
+    float m = logf(ratio_found) / logf(t_k / tau);
+    m = fminf(fmaxf(m, 2.0f), 1024.0f);
+    alpha = alpha > 0.f ? 0.5f * (alpha + m) : m;
+  }
+  slack *= 0.9f;
+  if (exact) {
+    slack = 1.f;
+  } else if (aimed) {
+    slack = fmaxf(slack, fabsf(logf((float)C / (float)aimed)));
+  }
+  const float ratio = fminf(target_ratio, expf(0.1f + 4.f * rsqrtf((float)k) + 3.f * slack));
+  const float next = t_k * expf(-logf(ratio) / (alpha > 0.f ? alpha : 8.0f));
+  st->tau = next > 0.f ? next : 0.f;
+  st->aimed = (unsigned int)(ratio * (float)k);
+  st->alpha = alpha;
+  st->slack = slack;
+  st->n_sel = n_sel;
+  st->n_cand = count;
+  st->fallback = exact ? 1u : 0u;
+  if (exact) st->n_fallbacks = was.n_fallbacks + 1u;
+  st->kth_mag = t_k;
+  st->n_calls = was.stream_calls;
+}
+
+constexpr int kSmallRegs = kPickSmall / kPickThreads;  // candidates per thread in registers: one CTA
+constexpr int kClusterRegs = kPickCluster / (kPickCtas * kPickThreads);  // and the cluster
+constexpr unsigned int kPickChunk = 4u * kPickThreads; // candidates per ticket above
+constexpr int kExactVec = 4;                           // float4 of r per thread and ticket in exact mode
+constexpr unsigned int kExactChunk = kExactVec * 4u * kPickThreads;
+
+// k <= C <= kPickSmall: one CTA, candidates in registers, nothing but the list itself in global memory.
+// Latency-bound (about 1 000 to 4 000 entries): what counts is the number of dependent steps.
+__device__ __forceinline__ uint32_t pick_small(PickShared& s, float* r, const Pair* cand, Pair* sel, unsigned int k,
+                                               unsigned int C, Level lv, Pair ahead) {
+  Pair c[kSmallRegs];
+  c[0] = ahead;
+#pragma unroll
+  for (int j = 1; j < kSmallRegs; ++j) {
+    const unsigned int i = (unsigned int)j * kPickThreads + threadIdx.x;
+    c[j].idx = 0;
+    c[j].val = 0.f;
+    if (i < C) c[j] = ld_pair_cg(&cand[i]);
+  }
+  auto live = [&](int j) { return (unsigned int)j * kPickThreads + threadIdx.x < C; };
+  unsigned int k_rem = k;
+  for (;;) {
+    *my_bins(s) = make_uint2(0u, 0u);
+    if (threadIdx.x == 0) s.tie = 0u;
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kSmallRegs; ++j)
+      if (live(j) && lv.has(mag_key(c[j].val))) atomicAdd(&s.hist[lv.bin(mag_key(c[j].val))], 1u);
+    __syncthreads();
+    find_bin(s, *my_bins(s), k_rem);
+    k_rem = s.res_krem;
+    if (!lv.narrow(s.res_bin)) break;
+  }
+  const uint32_t th = lv.lo;
+  unsigned int won = 0, n = 0;
+#pragma unroll
+  for (int j = 0; j < kSmallRegs; ++j) {
+    if ((unsigned int)j * kPickThreads >= C) break;
+    if (passes(live(j), mag_key(c[j].val), th, k_rem, &s.tie)) {
+      won |= 1u << j;
+      ++n;
+    }
+  }
+  unsigned int pos = place(s, n, nullptr, 0u);
+#pragma unroll
+  for (int j = 0; j < kSmallRegs; ++j) {
+    if (!live(j)) break;
+    if (won & (1u << j)) st_pair(&sel[pos++], c[j]);
+    else r[c[j].idx] = c[j].val;
+  }
+  return th;
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// kPickSmall < C <= kPickCluster: the same with 8 CTAs that meet in the hardware barrier (0.2 us) and add
+// up their counts over distributed shared memory.  Every CTA of the first cluster calls this.
+__device__ __forceinline__ uint32_t pick_cluster(PickShared& s, float* r, const Pair* cand, Pair* sel, unsigned int k,
+                                                 unsigned int C, Level lv) {
+  namespace cg = cooperative_groups;
+  const cg::cluster_group cluster = cg::this_cluster();
+  const unsigned int rank = cluster.block_rank();
+  constexpr unsigned int kStride = (unsigned int)kPickCtas * kPickThreads;
+  static_assert(kClusterRegs * kStride == kPickCluster, "every candidate has a register");
+  const unsigned int lane0 = rank * kPickThreads + threadIdx.x;
+  const unsigned int trips = (C + kStride - 1u) / kStride;
+  Pair c[kClusterRegs];
+#pragma unroll
+  for (int j = 0; j < kClusterRegs; ++j) {
+    const unsigned int i = (unsigned int)j * kStride + lane0;
+    c[j].idx = -1;
+    c[j].val = 0.f;
+    if (i < C) c[j] = ld_pair_cg(&cand[i]);
+  }
+  unsigned int k_rem = k;
+  int buf = 0;
+  for (;;) {
+    *my_bins(s) = make_uint2(0u, 0u);
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < kClusterRegs; ++j) {
+      if ((unsigned int)j >= trips) break;
+      const uint32_t key = mag_key(c[j].val);
+      if (c[j].idx >= 0 && lv.has(key)) atomicAdd(&s.hist[lv.bin(key)], 1u);
+    }
+    __syncthreads();
+    // Bin b is summed up in CTA b mod 8.  (Reading all eight histograms in every CTA moves 64 KB per SM over
+    // the cluster network: 2 us per level.)  The next level's share is cleared here, which everybody is past
+    // reading since the barrier before.
+    const uint2 part = *my_bins(s);
+    const unsigned int b0 = 2u * threadIdx.x;
+    if (part.x) atomicAdd(cluster.map_shared_rank(&s.share[buf][b0 / kPickCtas], b0 % kPickCtas), part.x);
+    if (part.y) atomicAdd(cluster.map_shared_rank(&s.share[buf][b0 / kPickCtas], b0 % kPickCtas + 1u), part.y);
+    if (threadIdx.x < (unsigned int)(kBins / kPickCtas)) s.share[buf ^ 1][threadIdx.x] = 0u;
+    cluster_barrier();
+    uint2 sum;
+    sum.x = *cluster.map_shared_rank(&s.share[buf][b0 / kPickCtas], b0 % kPickCtas);
+    sum.y = *cluster.map_shared_rank(&s.share[buf][b0 / kPickCtas], b0 % kPickCtas + 1u);
+    find_bin(s, sum, k_rem);
+    k_rem = s.res_krem;
+    if (!lv.narrow(s.res_bin)) break;
+    buf ^= 1;
+  }
+  const uint32_t th = lv.lo;
+  unsigned int* const tie = cluster.map_shared_rank(&s.tie, 0);
+  unsigned int won = 0, n = 0;
+#pragma unroll
+  for (int j = 0; j < kClusterRegs; ++j) {
+    if ((unsigned int)j >= trips) break;
+    if (passes(c[j].idx >= 0, mag_key(c[j].val), th, k_rem, tie)) {
+      won |= 1u << j;
+      ++n;
+    }
+  }
+  unsigned int pos = place(s, n, nullptr, 0u);
+  // the CTA's total to everybody (nobody reads another CTA's memory after this barrier, so CTAs may leave)
+  if (threadIdx.x == kPickThreads - 1) s.base[0] = pos + n;
+  __syncthreads();
+  if (threadIdx.x < (unsigned int)kPickCtas) *cluster.map_shared_rank(&s.cta_n[rank], threadIdx.x) = s.base[0];
+  cluster_barrier();
+  for (unsigned int q = 0; q < rank; ++q) pos += s.cta_n[q];
+#pragma unroll
+  for (int j = 0; j < kClusterRegs; ++j) {
+    if (c[j].idx < 0) break;
+    if (won & (1u << j)) st_pair(&sel[pos++], c[j]);
+    else r[c[j].idx] = c[j].val;
+  }
+  return th;
+}
+
+__global__ void __cluster_dims__(kPickCtas, 1, 1) __launch_bounds__(kPickThreads, 1)
+k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Pair* sel, unsigned int k, K1State* st,
+        Ctrl* ctrl_pair, int counted, float target_ratio, unsigned long long limit_ns) {
+  __shared__ __align__(16) PickShared s;
+  // what the cluster's CTAs add to in one another, ready before the stream pass has ended
+  if (threadIdx.x == 0) s.tie = 0u;
+  if (threadIdx.x < (unsigned int)(kBins / kPickCtas)) s.share[0][threadIdx.x] = 0u;
+  cluster_barrier();
+  pdl_begin(r, cand, st, ctrl_pair);
+  // one round of loads: the call's parity, both blocks' counts, and (unseen) the first candidates
+  K1State was;
+  was.stream_calls = st->stream_calls;
+  was.tau = st->tau;
+  was.kth_mag = st->kth_mag;
+  was.alpha = st->alpha;
+  was.slack = st->slack;
+  was.aimed = st->aimed;
+  was.n_fallbacks = st->n_fallbacks;
+  const unsigned int calls = was.stream_calls - 1u;
+  const unsigned int n_out[2] = {__ldcg(&ctrl_pair[0].n_out), __ldcg(&ctrl_pair[1].n_out)};
+  Pair ahead;
+  ahead.idx = 0;
+  ahead.val = 0.f;
+  if (blockIdx.x == 0 && threadIdx.x < cap) ahead = ld_pair_cg(&cand[threadIdx.x]);
+  Ctrl* const ctrl = ctrl_pair + (calls & 1u);
+  const unsigned int count = n_out[calls & 1u];
   const unsigned int C = count < cap ? count : cap;
   const bool exact_mode = (count > cap) || (C < k);
-  Threshold th;
-  auto none = [](Pair, unsigned int) {};
+  trace_stamp(ctrl, 2);
+  const Bands bands = first_bands(was.tau, was.kth_mag);
+  Level lv{bands.lo, 0x7fffffffu, bands.shift, true};
+  uint32_t th = 0u;
 
+  if (!exact_mode && C <= kPickCluster) {
+    if (C <= kPickSmall) {
+      if (blockIdx.x != 0) return;
+      th = pick_small(s, r, cand, sel, k, C, lv, ahead);
+    } else {
+      if (blockIdx.x >= (unsigned int)kPickCtas) return;
+      th = pick_cluster(s, r, cand, sel, k, C, lv);
+      if (blockIdx.x != 0) return;
+    }
+    trace_stamp(ctrl, 4);
+    if (threadIdx.x == 0) finish_state(st, was, th, k, k, count, C, false, target_ratio);
+    return;
+  }
+
+  int ph = 0;
+  unsigned int k_rem = k;
   if (!exact_mode) {
-    unsigned int nct = (C + 1023u) / 1024u;  // one or two candidates per thread and pass
-    if (nct < 1u) nct = 1u;
-    if (nct > gridDim.x) nct = gridDim.x;
-    if (blockIdx.x >= nct) return;
-    RankBarrier bar{ctrl, nct, 0u, limit_ns, &ctrl->scratch[0]};
-    auto key_at = [&](unsigned int i) -> uint32_t { return mag_key(ld_pair_cg(&cand[i]).val); };
-    if (!radix_select_kth(s, bar, blockIdx.x, nct, C, k, ctrl->hist[0], key_at, &th, 100, true, ctrl->hist[2],
-                          pred - 1u, kPredDigits))
-      return;
-    trace_stamp(ctrl, 3);  // k-th magnitude known
-    StagedAppender app{&s, sel, &ctrl->cursor[0], k, ctrl};
-    app.begin();
-    const unsigned int stride = nct * kSelThreads;
-    const unsigned int trips = (C + stride - 1) / stride;
-    for (unsigned int t = 0; t < trips; ++t) {
-      const unsigned int i = t * stride + blockIdx.x * kSelThreads + threadIdx.x;
-      if (i < C) {
-        const Pair e = ld_pair_cg(&cand[i]);
-        if (passes_threshold(mag_key(e.val), th, &ctrl->tie[0])) {
-          app.put(e);
-        } else {
-          r[e.idx] = e.val;
+    // The candidates in chunks: the first level was counted by the stream pass (counted) or is counted here,
+    // the rest (one level of single keys, as a rule) and the compaction take a phase each.
+    const unsigned int nchunks = (C + kPickChunk - 1u) / kPickChunk;
+    unsigned int* level_hist = ctrl->hist[0][0];
+    bool have = counted != 0;
+    int row = 0;
+    for (;;) {
+      if (!have) {
+        *my_bins(s) = make_uint2(0u, 0u);
+        const unsigned int mine = for_chunks(s, ctrl, ph, nchunks, [&](unsigned int chunk) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const unsigned int i = chunk * kPickChunk + (unsigned int)j * kPickThreads + threadIdx.x;
+            if (i >= C) break;
+            const uint32_t key = mag_key(ld_pair_cg(&cand[i]).val);
+            if (lv.has(key)) atomicAdd(&s.hist[lv.bin(key)], 1u);
+          }
+        });
+        if (mine == 0u) return;  // those that hold chunks finish the call
+        publish_hist(s, level_hist);
+        report(ctrl, ph, mine, nchunks);
+        if (!wait_phase(s, ctrl, ph, nchunks, limit_ns, 100 + ph)) return;
+        ++ph;
+      }
+      have = false;
+      find_bin(s, global_counts(level_hist), k_rem);
+      k_rem = s.res_krem;
+      if (!lv.narrow(s.res_bin)) break;
+      level_hist = ctrl->hist[0][++row];
+      __syncthreads();
+    }
+    th = lv.lo;
+    if (threadIdx.x == 0) ctrl->trace[3] = globaltimer_ns();  // k-th magnitude known
+    unsigned int turn = 0;
+    const unsigned int mine = for_chunks(s, ctrl, ph, nchunks, [&](unsigned int chunk) {
+      Pair c[4];
+      unsigned int won = 0, n = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const unsigned int i = chunk * kPickChunk + (unsigned int)j * kPickThreads + threadIdx.x;
+        c[j].idx = -1;
+        c[j].val = 0.f;
+        if (i < C) c[j] = ld_pair_cg(&cand[i]);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (passes(c[j].idx >= 0, mag_key(c[j].val), th, k_rem, &ctrl->tie[0])) {
+          won |= 1u << j;
+          ++n;
         }
       }
-      app.end_tile(none);
-    }
-    app.flush(none);
-    trace_stamp(ctrl, 4);  // CTA 0 compacted its share
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      const float t_k = __uint_as_float(th.key);
-      st->n_sel = k;
-      st->n_cand = count;
-      st->fallback = 0u;
-      st->kth_mag = t_k;
-      st->tau = predict_tau(t_k, tau_used, C, k, target_ratio);
+      unsigned int pos = place(s, n, &ctrl->cursor[0], turn++);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (c[j].idx < 0) break;
+        if (won & (1u << j)) {
+          if (pos < k) st_pair(&sel[pos], c[j]);
+          ++pos;
+        } else {
+          r[c[j].idx] = c[j].val;
+        }
+      }
+    });
+    if (report(ctrl, ph, mine, nchunks)) {
+      finish_state(st, was, th, k, k, count, C, false, target_ratio);
+      ctrl->trace[4] = globaltimer_ns();  // all winners compacted
     }
     return;
   }
 
-  // Exact mode: every CTA of the grid takes part.
-  const unsigned int nct = gridDim.x;
-  const unsigned int stride = nct * kSelThreads;
-  for (unsigned int i = blockIdx.x * kSelThreads + threadIdx.x; i < C; i += stride) {
-    const Pair e = ld_pair_cg(&cand[i]);
-    r[e.idx] = e.val;
+  // ---- exact mode
+  if (C) {  // the stream pass took these out of the residual
+    const unsigned int nchunks = (C + kPickChunk - 1u) / kPickChunk;
+    const unsigned int mine = for_chunks(s, ctrl, ph, nchunks, [&](unsigned int chunk) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const unsigned int i = chunk * kPickChunk + (unsigned int)j * kPickThreads + threadIdx.x;
+        if (i >= C) break;
+        const Pair e = ld_pair_cg(&cand[i]);
+        r[e.idx] = e.val;
+      }
+    });
+    report(ctrl, ph, mine, nchunks);  // (a CTA without a chunk of this short phase stays for the sweeps)
+    if (!wait_phase(s, ctrl, ph, nchunks, limit_ns, 110)) return;
+    ++ph;
   }
-  if (!bar_all.sync(110)) return;
-  const unsigned int n = (unsigned int)d;
-  auto key_at = [&](unsigned int i) -> uint32_t { return mag_key(__ldcg(&r[i])); };
-  if (!radix_select_kth(s, bar_all, blockIdx.x, nct, n, k, ctrl->hist[1], key_at, &th, 120)) return;
-  StagedAppender app{&s, sel, &ctrl->cursor[1], k, ctrl};
-  app.begin();
-  const unsigned int trips = (n + stride - 1) / stride;
-  for (unsigned int t = 0; t < trips; ++t) {
-    const unsigned int i = t * stride + blockIdx.x * kSelThreads + threadIdx.x;
-    if (i < n) {
-      const float v = __ldcg(&r[i]);
-      if (passes_threshold(mag_key(v), th, &ctrl->tie[1])) {
-        Pair e;
-        e.idx = (int32_t)i;
-        e.val = v;
-        app.put(e);
-        r[i] = 0.f;
+  const unsigned int mis = (unsigned int)((reinterpret_cast<uintptr_t>(r) >> 2) & 3u);
+  long long head = mis ? (4 - mis) : 0;
+  if (head > d) head = d;
+  const unsigned int nvec = (unsigned int)((d - head) >> 2);
+  const float4* r4 = reinterpret_cast<const float4*>(r + head);
+  const unsigned int nscalar = (unsigned int)(d - ((long long)nvec << 2));   // head and tail, at most 6
+  const unsigned int nchunks = (unsigned int)((d + kExactChunk - 1) / kExactChunk);
+  // this thread's float4 u of a chunk (out of range: ok = false), and chunk 0's scalar
+  auto vec_at = [&](unsigned int chunk, int u) { return chunk * (kExactChunk / 4u) + (unsigned int)u * kPickThreads + threadIdx.x; };
+  auto scalar_at = [&](unsigned int chunk) -> long long {
+    if (chunk != 0u || threadIdx.x >= nscalar) return -1;
+    const long long j = threadIdx.x;
+    return j < head ? j : head + ((long long)nvec << 2) + (j - head);
+  };
+  unsigned int quota = 0xffffffffu;  // d <= k: everything is selected
+  if (d > (long long)k) {
+    lv = Level{0u, 0x7fffffffu, 20u, false};
+    int row = 0;
+    for (;;) {
+      *my_bins(s) = make_uint2(0u, 0u);
+      const unsigned int mine = for_chunks(s, ctrl, ph, nchunks, [&](unsigned int chunk) {
+        float4 x[kExactVec];
+#pragma unroll
+        for (int u = 0; u < kExactVec; ++u) {
+          const unsigned int v = vec_at(chunk, u);
+          if (v < nvec) x[u] = __ldcg(&r4[v]);
+        }
+        auto count_key = [&](float a) {
+          if (lv.has(mag_key(a))) atomicAdd(&s.hist[lv.bin(mag_key(a))], 1u);
+        };
+#pragma unroll
+        for (int u = 0; u < kExactVec; ++u) {
+          if (vec_at(chunk, u) >= nvec) break;
+          count_key(x[u].x);
+          count_key(x[u].y);
+          count_key(x[u].z);
+          count_key(x[u].w);
+        }
+        const long long i = scalar_at(chunk);
+        if (i >= 0) count_key(__ldcg(&r[i]));
+      });
+      if (mine == 0u) return;  // those that hold chunks finish the call
+      publish_hist(s, ctrl->hist[1][row]);
+      report(ctrl, ph, mine, nchunks);
+      if (!wait_phase(s, ctrl, ph, nchunks, limit_ns, 120 + ph)) return;
+      ++ph;
+      find_bin(s, global_counts(ctrl->hist[1][row]), k_rem);
+      k_rem = s.res_krem;
+      if (!lv.narrow(s.res_bin)) break;
+      ++row;
+      __syncthreads();
+    }
+    th = lv.lo;
+    quota = k_rem;
+  }
+  unsigned int turn = 0;
+  const unsigned int mine = for_chunks(s, ctrl, ph, nchunks, [&](unsigned int chunk) {
+    float x[4 * kExactVec + 1];
+    unsigned int won = 0, n = 0;
+#pragma unroll
+    for (int u = 0; u < kExactVec; ++u) {
+      const unsigned int v = vec_at(chunk, u);
+      float4 y = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (v < nvec) y = __ldcg(&r4[v]);
+      x[4 * u] = y.x;
+      x[4 * u + 1] = y.y;
+      x[4 * u + 2] = y.z;
+      x[4 * u + 3] = y.w;
+    }
+    const long long is = scalar_at(chunk);
+    x[4 * kExactVec] = is >= 0 ? __ldcg(&r[is]) : 0.f;
+#pragma unroll
+    for (int e = 0; e <= 4 * kExactVec; ++e) {
+      const bool live = e < 4 * kExactVec ? vec_at(chunk, e >> 2) < nvec : is >= 0;
+      if (passes(live, mag_key(x[e]), th, quota, &ctrl->tie[1])) {
+        won |= 1u << e;
+        ++n;
       }
     }
-    app.end_tile(none);
+    unsigned int pos = place(s, n, &ctrl->cursor[1], turn++);
+    if (n == 0u) return;
+#pragma unroll
+    for (int e = 0; e <= 4 * kExactVec; ++e) {
+      if (!(won & (1u << e))) continue;
+      const long long i = e < 4 * kExactVec ? head + 4ll * vec_at(chunk, e >> 2) + (e & 3) : is;
+      Pair p;
+      p.idx = (int32_t)i;
+      p.val = x[e];
+      if (pos < k) st_pair(&sel[pos], p);
+      ++pos;
+      r[i] = 0.f;
+    }
+  });
+  if (report(ctrl, ph, mine, nchunks)) {
+    const unsigned int n_sel = d < (long long)k ? (unsigned int)d : k;
+    finish_state(st, was, th, n_sel, k, count, C, true, target_ratio);
+    ctrl->trace[5] = globaltimer_ns();
   }
-  app.flush(none);
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    const float t_k = th.select_all ? 0.f : __uint_as_float(th.key);
-    st->n_sel = th.select_all ? s.res_total : k;
-    st->n_cand = count;
-    st->fallback = 1u;
-    st->n_fallbacks += 1u;
-    st->kth_mag = t_k;
-    st->tau = predict_tau(t_k, 0.f, 0u, k, target_ratio);
-  }
-  trace_stamp(ctrl, 5);  // exact mode: CTA 0 collected its share
 }
 
 }  // namespace gtk
@@ -382,36 +876,33 @@ using namespace gtk;
 extern "C" unsigned long long gtk_ctrl_bytes(void) { return sizeof(Ctrl); }
 
 namespace {
-// Co-resident CTAs of k1_fused on the current device (cached).
-int k1_max_grid() {
-  static std::atomic<int> cached[64];  // per device: GPUs of one process need not be alike
-  const DeviceInfo* di = gtk_device_info();
-  if (!di || di->device < 0 || di->device >= 64) return 0;
-  const int have = cached[di->device].load(std::memory_order_relaxed);
-  if (have) return have;
-  int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k1_fused, kK1Threads, 0) != cudaSuccess ||
-      occ < 1)
-    return 0;
-  if (occ > 2) occ = 2;
-  cached[di->device].store(di->sms * occ, std::memory_order_relaxed);
-  return di->sms * occ;
-}
-
 int k1_launch(const float* g, float* r, const float* g_scale, long long d, unsigned int k,
               Pair* cand, unsigned int cap, Pair* sel, K1State* st, Ctrl* ctrl_pair,
               float target_ratio, unsigned long long limit_ns, cudaStream_t stream) {
-  const int max_grid = k1_max_grid();
-  if (max_grid < 1) return GTK_ERR_CUDA;
-  const long long tile = (long long)kK1Threads * kK1Vec;
-  const long long ntiles = ((d / 4) + tile - 1) / tile;
-  long long want = (cap + 1023u) / 1024u;  // CTAs the candidate select can use
-  if (ntiles > want) want = ntiles;
-  int grid = want < max_grid ? (int)(want > 0 ? want : 1) : max_grid;
-  void* args[] = {&g, &r, &g_scale, &d, &cand, &cap, &sel, &k, &st, &ctrl_pair, &target_ratio, &limit_ns};
-  const cudaError_t e = cudaLaunchCooperativeKernel((void*)k1_fused, dim3(grid), dim3(kK1Threads),
-                                                    args, 0, stream);
-  gtk_count_launch(1);
+  const DeviceInfo* di = gtk_device_info();
+  if (!di) return GTK_ERR_CUDA;
+  // Two float4 of each array per thread and tile in the static split (four: 2 % slower, a coarser last round),
+  // four in the dynamic one (two: 2 % slower at 138 M).
+  const long long full = 2ll * di->sms;
+  const long long nvec = d / 4;
+  const bool dynamic = nvec >= kDynamicMinVec;
+  const long long tile = (long long)kK1Threads * (dynamic ? 4 : 2);
+  long long grid = (nvec + tile - 1) / tile;
+  grid = grid < 1 ? 1 : (grid > full ? full : grid);
+  // The first level is counted on the fly where the candidates will be shared out by tickets; below, the CTAs
+  // that pick count faster than the stream pass publishes.
+  const int counted = k > kPickCluster / 2 ? 1 : 0;
+  auto stream_fn = dynamic ? (counted ? k1_stream<true, true> : k1_stream<false, true>)
+                           : (counted ? k1_stream<true, false> : k1_stream<false, false>);
+  cudaError_t e = launch_pdl(stream_fn, (int)grid, kK1Threads, stream, g, r, g_scale, d, cand, cap, st, ctrl_pair);
+  if (e != cudaSuccess) return GTK_ERR_CUDA;
+  // k1_pick: as many clusters as exact mode can use
+  long long pick = (d + kExactChunk - 1) / kExactChunk;
+  if (pick > di->sms) pick = di->sms;
+  pick = (pick + kPickCtas - 1) / kPickCtas * kPickCtas;
+  e = launch_pdl(k1_pick, (int)pick, kPickThreads, stream, r, d, cand, cap, sel, k, st, ctrl_pair, counted, target_ratio,
+                 limit_ns);
+  gtk_count_launch(2);
   return e == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
 }
 }  // namespace
@@ -433,7 +924,7 @@ extern "C" int gtk_k1_select(const float* g, float* r, const float* g_scale, lon
 // ---------------------------------------------------------------------------
 // Allocation-free variant (declared and documented in k1_select_noalloc.h).
 // The scratch that gtk_k1_select takes from its caller lives here in a static
-// device array; the kernel is the one above, unchanged.
+// device array; the kernels are the ones above, unchanged.
 // ---------------------------------------------------------------------------
 #include <mutex>
 #include "k1_select_noalloc.h"
@@ -460,6 +951,8 @@ __global__ void k1_noalloc_reset_state(K1State* st) {
     st->n_cand = 0u;
     st->fallback = 0u;
     st->kth_mag = 0.f;
+    st->aimed = 0u;
+    st->alpha = 0.f;
   }
 }
 

@@ -48,11 +48,11 @@ class TopkSelector:
         self.cap = int(max(self.max_k, min(self.numel, max(cap_factor * self.max_k, 4096))))
         self.is_cuda = self.device.type == "cuda"
         self.sel = torch.zeros((self.max_k, 2), dtype=torch.int32, device=self.device)
-        self.state = torch.zeros(8, dtype=torch.int32, device=self.device)
+        self.state = torch.zeros(16, dtype=torch.int32, device=self.device)
         self.reset_threshold()
         if self.is_cuda:
             L = _lib.lib()
-            assert L.gtk_k1state_bytes() == 32
+            assert L.gtk_k1state_bytes() == 64
             self.cand = torch.empty((self.cap, 2), dtype=torch.int32, device=self.device)
             # two control blocks: call i uses block i & 1 and clears the other one for call i + 1
             self.ctrl_words = int(L.gtk_ctrl_bytes()) // 4
