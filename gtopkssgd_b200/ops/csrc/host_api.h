@@ -52,6 +52,9 @@ const char* gtk_last_cuda_error(void);
 int gtk_k1_select(const float* g, float* r, const float* g_scale, long long d, unsigned int k,
                   void* cand, unsigned int cap, void* sel, void* state, void* ctrl,
                   float target_ratio, unsigned long long limit_ns, void* stream);
+int gtk_k1_compress(float* g, float* r, long long d, unsigned int k, void* cand, unsigned int cap, void* sel,
+                    void* state, void* ctrl, float target_ratio, unsigned long long limit_ns, long long* idx_out,
+                    float* val_out, void* stream);
 int gtk_k2_exchange(const void* ranks_dev, unsigned int nranks, unsigned int rank_base, unsigned int P,
                     unsigned int k, unsigned int kcap, unsigned int d, unsigned int nctas,
                     unsigned long long limit_ns, int use_cluster, void* stream);

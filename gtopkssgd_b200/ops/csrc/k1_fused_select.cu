@@ -18,8 +18,10 @@
 //     exact mode (C < k or the list overflowed; always on the first call, when
 //     tau is +inf): restores r = acc from the stored candidates, then runs a
 //     3-pass radix select over all d entries of r and one collect pass.
-// The dense sparsified gradient of the reference is never materialised; the
-// output is k (int32 index, fp32 value) pairs in no particular order.
+// The output is k (int32 index, fp32 value) pairs in no particular order.  The dense
+// sparsified gradient of the reference is not materialised, except by gtk_k1_compress,
+// where the stream pass leaves zeros in g and k1_pick puts the winners back, next to
+// their int64 indices and values as separate lists.
 //
 // Why two kernels: as one cooperative kernel the two halves met in a grid barrier
 // (1.3 us plus the wait for the slowest CTA), and a cooperative launch cannot
@@ -38,6 +40,7 @@
 // written by the other kernel, so a late CTA never sees its call's own update.
 #include <atomic>
 #include <cstddef>
+#include <type_traits>
 #include <cooperative_groups.h>
 #include "select_common.cuh"
 #include "host_api.h"
@@ -143,8 +146,8 @@ __device__ __forceinline__ void take_candidates(StreamShared& ss, StreamCtx& c, 
 
 // One tile of the stream pass: U float4 of g and of r per thread, STRIDE
 // float4 apart (the CTA's 512 threads or one warp's 32 lanes work side by side).
-template <int STRIDE, int U, bool HIST>
-__device__ __forceinline__ void stream_tile(long long v0, long long nvec, long long head, const float4* g4, float4* r4,
+template <int STRIDE, int U, bool HIST, bool ZERO>
+__device__ __forceinline__ void stream_tile(long long v0, long long nvec, long long head, float4* g4, float4* r4,
                                             StreamShared& ss, StreamCtx& c) {
   // Candidates are decided on the bit pattern of |acc|, which orders like the magnitude for finite
   // values and puts +-Inf and NaN on top: a non-finite entry is a candidate on this path exactly as it
@@ -180,6 +183,7 @@ __device__ __forceinline__ void stream_tile(long long v0, long long nvec, long l
       o.z = is[2] ? 0.f : a[2];
       o.w = is[3] ? 0.f : a[3];
       r4[v] = o;
+      if (ZERO) g4[v] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (__any_sync(0xffffffffu, is[0] | is[1] | is[2] | is[3])) {
 #pragma unroll
@@ -188,9 +192,10 @@ __device__ __forceinline__ void stream_tile(long long v0, long long nvec, long l
   }
 }
 
-template <bool HIST, bool DYNAMIC>
+// ZERO: g <- 0 on the way (a constant in a template, so that the training path has no store to g).
+template <bool HIST, bool DYNAMIC, bool ZERO>
 __global__ void __launch_bounds__(kK1Threads, 2)
-k1_stream(const float* g, float* r, const float* g_scale, long long d, Pair* cand, unsigned int cap, K1State* st,
+k1_stream(float* g, float* r, const float* g_scale, long long d, Pair* cand, unsigned int cap, K1State* st,
           Ctrl* ctrl_pair) {
   constexpr int U = DYNAMIC ? 4 : 2;  // float4 loads of g and of r in flight per thread
   __shared__ StreamShared ss;
@@ -220,7 +225,7 @@ k1_stream(const float* g, float* r, const float* g_scale, long long d, Pair* can
   if (head > d) head = d;
   const long long nvec = (d - head) >> 2;
   const long long tail0 = head + (nvec << 2);
-  const float4* g4 = reinterpret_cast<const float4*>(g + head);
+  float4* g4 = reinterpret_cast<float4*>(g + head);
   float4* r4 = reinterpret_cast<float4*>(r + head);
 
   if (!DYNAMIC) {
@@ -230,7 +235,7 @@ k1_stream(const float* g, float* r, const float* g_scale, long long d, Pair* can
     constexpr long long kTileVec = (long long)kK1Threads * U;
     const long long ntiles = (nvec + kTileVec - 1) / kTileVec;
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-      stream_tile<kK1Threads, U, HIST>(tile * kTileVec + threadIdx.x, nvec, head, g4, r4, ss, c);
+      stream_tile<kK1Threads, U, HIST, ZERO>(tile * kTileVec + threadIdx.x, nvec, head, g4, r4, ss, c);
   } else {
     // Large vectors: SMs do not all see the same memory bandwidth, and with the static split the slowest
     // CTA ended up to 13 us (d = 64 M) after the first.  Here work is handed out per warp in tiles of 32 lanes
@@ -248,7 +253,7 @@ k1_stream(const float* g, float* r, const float* g_scale, long long d, Pair* can
     for (long long tile = warp; tile < ntiles; tile = turn * kShards + shard) {
       unsigned int nxt = 0;
       if (lane_id() == 0) nxt = atomicAdd(ticket, 1u);  // consumed after this tile
-      stream_tile<32, U, HIST>(tile * kWarpTileVec + lane_id(), nvec, head, g4, r4, ss, c);
+      stream_tile<32, U, HIST, ZERO>(tile * kWarpTileVec + lane_id(), nvec, head, g4, r4, ss, c);
       turn = (long long)warps + __shfl_sync(0xffffffffu, nxt, 0);
     }
   }
@@ -264,6 +269,7 @@ k1_stream(const float* g, float* r, const float* g_scale, long long d, Pair* can
       a = fmaf(g[i], c.scale, r[i]);
       is = mag_key(a) >= c.tau_key;
       r[i] = is ? 0.f : a;
+      if (ZERO) g[i] = 0.f;
     }
     take_candidates<HIST>(ss, c, is, i, a);
   }
@@ -303,6 +309,22 @@ k1_stream(const float* g, float* r, const float* g_scale, long long d, Pair* can
 // ---------------------------------------------------------------------------
 // k1_pick
 // ---------------------------------------------------------------------------
+// Where a winner goes: the pair list, and for gtk_k1_compress the other forms.
+struct Winners {
+  Pair* sel;
+  float* dense;        // nullptr: pairs only
+  long long* idx;
+  float* val;
+  __device__ __forceinline__ void put(unsigned int pos, Pair e) const {
+    st_pair(&sel[pos], e);
+    if (dense) {
+      dense[e.idx] = e.val;
+      idx[pos] = e.idx;
+      val[pos] = e.val;
+    }
+  }
+};
+
 struct PickShared {
   unsigned int hist[kBins];
   unsigned int share[2][kBins / kPickCtas]; // cluster: the sums of bins b = rank (mod 8), for alternating levels
@@ -508,8 +530,8 @@ constexpr unsigned int kExactChunk = kExactVec * 4u * kPickThreads;
 
 // k <= C <= kPickSmall: one CTA, candidates in registers, nothing but the list itself in global memory.
 // Latency-bound (about 1 000 to 4 000 entries): what counts is the number of dependent steps.
-__device__ __forceinline__ uint32_t pick_small(PickShared& s, float* r, const Pair* cand, Pair* sel, unsigned int k,
-                                               unsigned int C, Level lv, Pair ahead) {
+__device__ __forceinline__ uint32_t pick_small(PickShared& s, float* r, const Pair* cand, const Winners& out,
+                                               unsigned int k, unsigned int C, Level lv, Pair ahead) {
   Pair c[kSmallRegs];
   c[0] = ahead;
 #pragma unroll
@@ -547,7 +569,7 @@ __device__ __forceinline__ uint32_t pick_small(PickShared& s, float* r, const Pa
 #pragma unroll
   for (int j = 0; j < kSmallRegs; ++j) {
     if (!live(j)) break;
-    if (won & (1u << j)) st_pair(&sel[pos++], c[j]);
+    if (won & (1u << j)) out.put(pos++, c[j]);
     else r[c[j].idx] = c[j].val;
   }
   return th;
@@ -560,8 +582,8 @@ __device__ __forceinline__ void cluster_barrier() {
 
 // kPickSmall < C <= kPickCluster: the same with 8 CTAs that meet in the hardware barrier (0.2 us) and add
 // up their counts over distributed shared memory.  Every CTA of the first cluster calls this.
-__device__ __forceinline__ uint32_t pick_cluster(PickShared& s, float* r, const Pair* cand, Pair* sel, unsigned int k,
-                                                 unsigned int C, Level lv) {
+__device__ __forceinline__ uint32_t pick_cluster(PickShared& s, float* r, const Pair* cand, const Winners& out,
+                                                 unsigned int k, unsigned int C, Level lv) {
   namespace cg = cooperative_groups;
   const cg::cluster_group cluster = cg::this_cluster();
   const unsigned int rank = cluster.block_rank();
@@ -627,14 +649,14 @@ __device__ __forceinline__ uint32_t pick_cluster(PickShared& s, float* r, const 
 #pragma unroll
   for (int j = 0; j < kClusterRegs; ++j) {
     if (c[j].idx < 0) break;
-    if (won & (1u << j)) st_pair(&sel[pos++], c[j]);
+    if (won & (1u << j)) out.put(pos++, c[j]);
     else r[c[j].idx] = c[j].val;
   }
   return th;
 }
 
 __global__ void __cluster_dims__(kPickCtas, 1, 1) __launch_bounds__(kPickThreads, 1)
-k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Pair* sel, unsigned int k, K1State* st,
+k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Winners out, unsigned int k, K1State* st,
         Ctrl* ctrl_pair, int counted, float target_ratio, unsigned long long limit_ns) {
   __shared__ __align__(16) PickShared s;
   // what the cluster's CTAs add to in one another, ready before the stream pass has ended
@@ -669,10 +691,10 @@ k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Pair* sel, un
   if (!exact_mode && C <= kPickCluster) {
     if (C <= kPickSmall) {
       if (blockIdx.x != 0) return;
-      th = pick_small(s, r, cand, sel, k, C, lv, ahead);
+      th = pick_small(s, r, cand, out, k, C, lv, ahead);
     } else {
       if (blockIdx.x >= (unsigned int)kPickCtas) return;
-      th = pick_cluster(s, r, cand, sel, k, C, lv);
+      th = pick_cluster(s, r, cand, out, k, C, lv);
       if (blockIdx.x != 0) return;
     }
     trace_stamp(ctrl, 4);
@@ -739,7 +761,7 @@ k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Pair* sel, un
       for (int j = 0; j < 4; ++j) {
         if (c[j].idx < 0) break;
         if (won & (1u << j)) {
-          if (pos < k) st_pair(&sel[pos], c[j]);
+          if (pos < k) out.put(pos, c[j]);
           ++pos;
         } else {
           r[c[j].idx] = c[j].val;
@@ -857,7 +879,7 @@ k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Pair* sel, un
       Pair p;
       p.idx = (int32_t)i;
       p.val = x[e];
-      if (pos < k) st_pair(&sel[pos], p);
+      if (pos < k) out.put(pos, p);
       ++pos;
       r[i] = 0.f;
     }
@@ -876,8 +898,9 @@ using namespace gtk;
 extern "C" unsigned long long gtk_ctrl_bytes(void) { return sizeof(Ctrl); }
 
 namespace {
-int k1_launch(const float* g, float* r, const float* g_scale, long long d, unsigned int k,
-              Pair* cand, unsigned int cap, Pair* sel, K1State* st, Ctrl* ctrl_pair,
+// out.dense: g itself (then it is left sparsified) or nullptr (then g is only read).
+int k1_launch(const float* g_in, float* r, const float* g_scale, long long d, unsigned int k,
+              Pair* cand, unsigned int cap, Winners out, K1State* st, Ctrl* ctrl_pair,
               float target_ratio, unsigned long long limit_ns, cudaStream_t stream) {
   const DeviceInfo* di = gtk_device_info();
   if (!di) return GTK_ERR_CUDA;
@@ -892,33 +915,51 @@ int k1_launch(const float* g, float* r, const float* g_scale, long long d, unsig
   // The first level is counted on the fly where the candidates will be shared out by tickets; below, the CTAs
   // that pick count faster than the stream pass publishes.
   const int counted = k > kPickCluster / 2 ? 1 : 0;
-  auto stream_fn = dynamic ? (counted ? k1_stream<true, true> : k1_stream<false, true>)
-                           : (counted ? k1_stream<true, false> : k1_stream<false, false>);
-  cudaError_t e = launch_pdl(stream_fn, (int)grid, kK1Threads, stream, g, r, g_scale, d, cand, cap, st, ctrl_pair);
+  float* g = const_cast<float*>(g_in);
+  auto stream_pass = [&](auto zero) {
+    constexpr bool Z = decltype(zero)::value;
+    auto fn = dynamic ? (counted ? k1_stream<true, true, Z> : k1_stream<false, true, Z>)
+                      : (counted ? k1_stream<true, false, Z> : k1_stream<false, false, Z>);
+    return launch_pdl(fn, (int)grid, kK1Threads, stream, g, r, g_scale, d, cand, cap, st, ctrl_pair);
+  };
+  cudaError_t e = out.dense ? stream_pass(std::true_type{}) : stream_pass(std::false_type{});
   if (e != cudaSuccess) return GTK_ERR_CUDA;
   // k1_pick: as many clusters as exact mode can use
   long long pick = (d + kExactChunk - 1) / kExactChunk;
   if (pick > di->sms) pick = di->sms;
   pick = (pick + kPickCtas - 1) / kPickCtas * kPickCtas;
-  e = launch_pdl(k1_pick, (int)pick, kPickThreads, stream, r, d, cand, cap, sel, k, st, ctrl_pair, counted, target_ratio,
+  e = launch_pdl(k1_pick, (int)pick, kPickThreads, stream, r, d, cand, cap, out, k, st, ctrl_pair, counted, target_ratio,
                  limit_ns);
   gtk_count_launch(2);
   return e == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
 }
 }  // namespace
 
+static bool k1_args_ok(const float* g, const float* r, long long d, unsigned int k, unsigned int cap) {
+  if (d <= 0 || d >= (1ll << 31) || k == 0 || k > cap) return false;
+  // g and r must share their offset inside a 16-byte line (same flat layout)
+  return (reinterpret_cast<uintptr_t>(g) & 15u) == (reinterpret_cast<uintptr_t>(r) & 15u) &&
+         (reinterpret_cast<uintptr_t>(r) & 3u) == 0u;
+}
+
 // ctrl: TWO consecutive control blocks (2 * gtk_ctrl_bytes()), zero when first used.
 extern "C" int gtk_k1_select(const float* g, float* r, const float* g_scale, long long d,
                              unsigned int k, void* cand, unsigned int cap, void* sel, void* state,
                              void* ctrl, float target_ratio, unsigned long long limit_ns,
                              void* stream_) {
-  if (d <= 0 || d >= (1ll << 31) || k == 0 || k > cap) return GTK_ERR_ARG;
-  // g and r must share their offset inside a 16-byte line (same flat layout)
-  if ((reinterpret_cast<uintptr_t>(g) & 15u) != (reinterpret_cast<uintptr_t>(r) & 15u) ||
-      (reinterpret_cast<uintptr_t>(r) & 3u) != 0u)
-    return GTK_ERR_ARG;
-  return k1_launch(g, r, g_scale, d, k, (Pair*)cand, cap, (Pair*)sel, (K1State*)state, (Ctrl*)ctrl,
-                   target_ratio, limit_ns, (cudaStream_t)stream_);
+  if (!k1_args_ok(g, r, d, k, cap)) return GTK_ERR_ARG;
+  return k1_launch(g, r, g_scale, d, k, (Pair*)cand, cap, Winners{(Pair*)sel, nullptr, nullptr, nullptr}, (K1State*)state,
+                   (Ctrl*)ctrl, target_ratio, limit_ns, (cudaStream_t)stream_);
+}
+
+// The select, with g left sparsified (selected entries keep g + r, all others are 0) and the selection also
+// as int64 indices and fp32 values, min(k, d) of each.
+extern "C" int gtk_k1_compress(float* g, float* r, long long d, unsigned int k, void* cand, unsigned int cap, void* sel,
+                               void* state, void* ctrl, float target_ratio, unsigned long long limit_ns,
+                               long long* idx_out, float* val_out, void* stream_) {
+  if (!k1_args_ok(g, r, d, k, cap) || !idx_out || !val_out) return GTK_ERR_ARG;
+  return k1_launch(g, r, nullptr, d, k, (Pair*)cand, cap, Winners{(Pair*)sel, g, idx_out, val_out}, (K1State*)state,
+                   (Ctrl*)ctrl, target_ratio, limit_ns, (cudaStream_t)stream_);
 }
 
 // ---------------------------------------------------------------------------
@@ -1009,8 +1050,8 @@ extern "C" int gtk_k1_select_noalloc(const float* g, float* r, long long d, unsi
   }
   // What must start at zero -- the control block of this call -- was cleared by the previous call
   // (or is still in its initial zero state); the candidate list is overwritten before it is read.
-  const int code = k1_launch(g, r, nullptr, d, k, cand, kNoAllocCap, static_cast<Pair*>(sel_out), st,
-                             ctrl_pair, 3.0f, 2000000000ull, stream);
+  const int code = k1_launch(g, r, nullptr, d, k, cand, kNoAllocCap,
+                             Winners{static_cast<Pair*>(sel_out), nullptr, nullptr, nullptr}, st, ctrl_pair, 3.0f, 2000000000ull, stream);
   if (code != GTK_OK) return code;
   if (n_sel_out) {
     k1_noalloc_publish_count<<<1, 32, 0, stream>>>(st, n_sel_out);

@@ -62,7 +62,7 @@ struct Call<F> {
   {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&Call<name>::fast)), METH_FASTCALL, nullptr}
 
 PyMethodDef kMethods[] = {
-    GTK_METHOD(gtk_k1_select),        GTK_METHOD(gtk_k2_exchange),    GTK_METHOD(gtk_k2t_allgather),
+    GTK_METHOD(gtk_k1_select),        GTK_METHOD(gtk_k1_compress),    GTK_METHOD(gtk_k2_exchange),    GTK_METHOD(gtk_k2t_allgather),
     GTK_METHOD(gtk_k3_dense),         GTK_METHOD(gtk_k3_sparse),      GTK_METHOD(gtk_k3_scatter_dense),
     GTK_METHOD(gtk_k3_momentum_correct), GTK_METHOD(gtk_k4_sumsq_dense), GTK_METHOD(gtk_k4_sumsq_pairs),
     GTK_METHOD(gtk_k4_finalize),      {nullptr, nullptr, 0, nullptr}};

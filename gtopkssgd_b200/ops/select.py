@@ -129,6 +129,22 @@ class TopkSelector:
         if code:
             _lib.check(code, "gtk_k1_select")
 
+    def compress(self, g: torch.Tensor, r: torch.Tensor, k: int) -> Tuple[torch.Tensor, torch.Tensor]:
+        """``select`` that also leaves g sparsified (acc on the selection, 0 off
+        it) and returns the selection as (int64 indices, fp32 values).  Nothing
+        synchronises: the number of selected entries is min(k, numel)."""
+        assert g.numel() == self.numel and r.numel() == self.numel
+        assert g.dtype == torch.float32 and r.dtype == torch.float32
+        k = int(min(k, self.max_k))
+        self.last_k = k
+        idx = torch.empty(k, dtype=torch.int64, device=g.device)
+        val = torch.empty(k, dtype=torch.float32, device=g.device)
+        code = _lib.calls().gtk_k1_compress(g.data_ptr(), r.data_ptr(), self.numel, k, *self._buffers, idx.data_ptr(),
+                                            val.data_ptr(), current_stream_handle(self.device))
+        if code:
+            _lib.check(code, "gtk_k1_compress")
+        return idx, val
+
     def pairs(self) -> Tuple[torch.Tensor, torch.Tensor]:
         """(int64 indices, fp32 values) of the last selection (synchronises)."""
         n = int(self.state[1].item())

@@ -4,8 +4,8 @@ static ``compress / add_residuals / get_residuals / decompress`` and
 class-level state keyed by the merged-group name.
 
 ``compress`` is the stand-alone form of the operation: it runs the fused K1
-kernel (or the oracle on CPU) and then materialises the sparsified dense
-vector in ``tensor`` as the reference does.  The training engine does not go
+kernels in their form that leaves the sparsified dense vector in ``tensor``, as
+the reference does (or the oracle on CPU).  The training engine does not go
 through this materialising form; it keeps the k pairs sparse end to end.
 """
 from __future__ import annotations
@@ -71,18 +71,20 @@ class TopKCompressor:
 
     @staticmethod
     def compress(tensor, name=None, sigma_scale=2.5, ratio=0.05):
-        with torch.no_grad():
-            flat = tensor.data.view(-1)
-            k = num_selected(flat.numel(), ratio)
-            residual = TopKCompressor.get_residuals(name, flat)
-            sel = TopKCompressor._selector(name, flat, k)
+        flat = tensor.detach().view(-1)
+        k = num_selected(flat.numel(), ratio)
+        residual = TopKCompressor.get_residuals(name, flat)
+        sel = TopKCompressor._selector(name, flat, k)
+        if sel.is_cuda:
+            idx, val = sel.compress(flat, residual, k)
+        else:
             sel.select(flat, residual, k)
-            counts = sel.n_sel_tensor
-            scatter_dense(flat, sel.sel, counts, 1, sel.max_k, 1.0)
+            scatter_dense(flat, sel.sel, sel.n_sel_tensor, 1, sel.max_k, 1.0)
             idx, val = sel.pairs()
-            TopKCompressor.values[name] = val.clone()
-            TopKCompressor.indexes[name] = idx
-            return tensor, idx
+            val = val.clone()
+        TopKCompressor.values[name] = val
+        TopKCompressor.indexes[name] = idx
+        return tensor, idx
 
     @staticmethod
     def add_residuals(included_indexes, name):

@@ -444,3 +444,49 @@ def test_k2_bounded_wait_reports_timeout():
     assert all(r.status() == (0, 0) for r in ranks)
     assert [int(r.epoch.item()) for r in ranks] == [2, 2]
     assert int(ranks[1].n_global.item()) == k
+
+
+def _check_selection(idx, val, r, acc, k):
+    """k distinct entries of acc, none left out larger than any taken (which of
+    two equal ones is taken is free), residual = acc off them, 0 on them."""
+    assert idx.numel() == k and idx.unique().numel() == k and torch.equal(val, acc[idx])
+    assert torch.equal(val.abs().sort().values, torch.topk(acc.abs(), k).values.sort().values)
+    want = acc.clone()
+    want[idx] = 0.0
+    assert torch.equal(r, want)
+
+
+@pytest.mark.parametrize("d,k", [(1, 1), (5, 2), (4097, 4097), (300_001, 300), (2_000_003, 6000), (20_000_010, 20_000)])
+def test_k1_compress_leaves_g_sparsified(d, k):
+    """The compressor's form of K1: the vector keeps acc on the selection and 0
+    off it, indices and values come as separate lists (exact path on the first
+    call, predicted thresholds after it; static and dynamic stream pass)."""
+    torch.manual_seed(d + k)
+    sel = _selector(d, k)
+    r = torch.zeros(d, device=DEV)
+    for it in range(3):
+        g = torch.randn(d, device=DEV)
+        acc = g + r
+        idx, val = sel.compress(g, r, k)
+        assert sel.status() == (0, 0) and idx.dtype == torch.int64
+        _check_selection(idx, val, r, acc, k)
+        want = torch.zeros(d, device=DEV)
+        want[idx] = val
+        assert torch.equal(g, want)
+
+
+@pytest.mark.parametrize("d,k", [(60_000, 4000), (200_000, 4096), (400_000, 30_000), (3_000_000, 65_536), (4_000_000, 400_000)])
+@pytest.mark.parametrize("off", [0, 3])
+def test_k1_pick_in_one_cta_a_cluster_and_by_tickets(d, k, off):
+    """Candidate counts on both sides of the borders between the three forms of
+    k1_pick, on aligned and unaligned views."""
+    torch.manual_seed(k + off)
+    sel = _selector(d, k)
+    g, r = torch.empty(d + 4, device=DEV)[off:off + d], torch.zeros(d + 4, device=DEV)[off:off + d]
+    for it in range(4):
+        g.normal_()
+        acc = g + r
+        sel.select(g, r, k)
+        assert sel.status() == (0, 0)
+        _check_selection(*sel.pairs(), r, acc, k)
+    assert sel.stats()["n_fallbacks"] < 4
