@@ -89,6 +89,7 @@ class GroupEngine:
         if self.numel >= 2 ** 31:
             raise ValueError("merged group %d holds %d elements; the sparse pairs carry int32 indices, so a group must "
                              "stay below 2^31 elements: lower the merge threshold" % (g.index, self.numel))
+        self.param, self.momentum = fb.group_slice(fb.param, g), fb.group_slice(fb.momentum, g)
         self.last_k = 0
         self.select_done = None
         self.result: Optional[SparseResult] = None
@@ -131,10 +132,11 @@ class GroupEngine:
         t = o.timers
         t.start(self.g.key, "compression")
         self.selector.select(self.grad, self.resid, k, g_scale=g_scale)
-        if self.is_cuda:
+        if self.is_cuda and o.concurrent:
             # the dense part of the update streams the same HBM as the select: it is ordered behind this
             # event, so the select has the bandwidth to itself and the dense part overlaps the exchange
-            self.select_done = torch.cuda.Event()
+            if self.select_done is None:
+                self.select_done = torch.cuda.Event()
             self.select_done.record()
         t.stop(self.g.key, "compression")
         t.start(self.g.key, "allreduce")
@@ -235,6 +237,7 @@ class AllReducer:
                  threshold: Optional[int] = None, flat: Optional[FlatBuffers] = None,
                  wait_limit_ms: Optional[float] = None):
         self._running = False
+        self.concurrent = True     # reductions run on a stream of their own (the wrapping optimizer decides)
         self._msg_queue, self._msg_queue2 = msg_queue, msg_queue2
         self._writer = writer
         self._profiling = True

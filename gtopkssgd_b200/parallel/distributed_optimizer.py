@@ -11,11 +11,15 @@ the ``local`` switch for gradient accumulation and ``momentum_correction``;
 module-level ``rank()`` and ``size()``.
 
 Differences in mechanism, not in semantics:
-* per-parameter hooks only count arrivals; when the last gradient of a merged
-  group has been produced an event is recorded and the group's select +
-  exchange kernels are enqueued on a side stream (no device synchronisation,
-  no host thread, no queue);
-* ``synchronize()`` makes the compute stream wait for that side stream;
+* with several merged groups per-parameter hooks count arrivals; when the last
+  gradient of a group has been produced an event is recorded and the group's
+  select + exchange kernels are enqueued on a side stream (no device
+  synchronisation, no host thread, no queue).  With one group (the default
+  threshold) on a GPU there is nothing left of backward to overlap with when its
+  last gradient arrives, so there are no hooks (2.5 us of host time per
+  parameter) and the group is reduced by ``synchronize()`` / ``step()``;
+* ``synchronize()`` makes the compute stream wait for that side stream; one
+  group of a single worker needs none and stays on the compute stream;
 * ``step()`` is two launches over the flat buffers (dense part + k sparse
   pairs) instead of three launches per tensor; weight decay is applied after
   sparsification and the first momentum step is ``buf = d_p`` as in the
@@ -76,8 +80,12 @@ class _DistributedOptimizer(torch.optim.Optimizer):
                                          flat=self._flat, wait_limit_ms=wait_limit_ms)
         dev = self._flat.device
         self._is_cuda = dev.type == "cuda"
-        self._overlap = overlap and self._is_cuda
+        n_groups = len(self._flat.groups)
+        self._hooked = not self._is_cuda or n_groups > 1
+        self._overlap = overlap and self._is_cuda and (n_groups > 1 or comm.size() > 1)
+        self._allreducer.concurrent = self._overlap
         self._comm_stream = torch.cuda.Stream(device=dev) if self._is_cuda else None
+        self._ready = [torch.cuda.Event() for _ in range(n_groups)] if self._overlap else []
         self._arrived = [0] * len(self._flat.groups)
         self._launched = [False] * len(self._flat.groups)
         self._expected = [len(g.names) for g in self._flat.groups]
@@ -142,6 +150,8 @@ class _DistributedOptimizer(torch.optim.Optimizer):
 
     # -- hooks -----------------------------------------------------------------
     def _register_hooks(self):
+        if not self._hooked:
+            return
         for name, slot in self._flat.slots.items():
             self._hook_handles.append(slot.param.register_post_accumulate_grad_hook(self._make_hook(slot)))
 
@@ -165,14 +175,15 @@ class _DistributedOptimizer(torch.optim.Optimizer):
         updates parameter by parameter inside the hook; the result is the same).
         The factor is the wrapped optimizer's momentum, 0.9 if it has none."""
         eng = self._allreducer.engines[gi]
-        fb = self._flat
         m = float(self.param_groups[0].get("momentum", 0.0)) or 0.9
-        momentum_correct(fb.group_slice(fb.momentum, eng.g), eng.grad, m)
+        momentum_correct(eng.momentum, eng.grad, m)
 
     def _launch_group(self, gi: int) -> None:
         self._launched[gi] = True
-        if self._comm_stream is not None and self._overlap:
-            ev = torch.cuda.Event()
+        if not self._hooked and not self._flat.grads_attached():
+            self._flat.ensure_views()
+        if self._overlap:
+            ev = self._ready[gi]
             ev.record()
             self._comm_stream.wait_event(ev)
             with torch.cuda.stream(self._comm_stream):
@@ -295,7 +306,7 @@ class _DistributedOptimizer(torch.optim.Optimizer):
             for gi in range(len(self._launched)):
                 if not self._launched[gi]:  # parameters that got no gradient this iteration
                     self._launch_group(gi)
-            if self._comm_stream is not None and self._overlap:
+            if self._overlap:
                 torch.cuda.current_stream().wait_stream(self._comm_stream)
             self._synced = True
         if materialize and not self._materialized and self._allreducer.mode != "none":
@@ -362,7 +373,7 @@ class _DistributedOptimizer(torch.optim.Optimizer):
             h = SgdHyper(h.lr, 0.0, 0.0, h.weight_decay, False)
 
         def bufs(eng):
-            return (fb.group_slice(fb.param, eng.g), fb.group_slice(fb.momentum, eng.g) if use_buf else None)
+            return eng.param, eng.momentum if use_buf else None
 
         if self.local:
             # accumulation micro-step: plain local SGD on the raw gradient
@@ -377,7 +388,7 @@ class _DistributedOptimizer(torch.optim.Optimizer):
                 sgd_dense(p, buf, h, first, g=eng.grad, scale=scale, coef=self._post_coef, lr_dev=lr_dev)
         else:
             for eng in a.engines:
-                if eng.select_done is not None and self._is_cuda:
+                if eng.select_done is not None and self._overlap:
                     torch.cuda.current_stream().wait_event(eng.select_done)  # select first, then dense || exchange
                 p, buf = bufs(eng)
                 sgd_dense(p, buf, h, first, lr_dev=lr_dev)

@@ -117,6 +117,7 @@ class FlatBuffers:
                 view.copy_(p.data)
                 p.data = view
                 p.grad = self._view(self.grad, slot)
+        self._grad_slots = [(s.param, 4 * s.offset) for s in self.slots.values()]
 
     # -- views -----------------------------------------------------------------
     @staticmethod
@@ -141,6 +142,15 @@ class FlatBuffers:
 
     def residual_view(self, name: str) -> torch.Tensor:
         return self._view(self.residual, self.slots[name])
+
+    def grads_attached(self) -> bool:
+        """True when every ``p.grad`` is still the view that was set up here."""
+        base = self.grad.data_ptr()
+        for p, at in self._grad_slots:
+            g = p.grad
+            if g is None or g.data_ptr() != base + at:
+                return False
+        return True
 
     def ensure_views(self) -> int:
         """Re-attach any parameter whose ``.data`` or ``.grad`` was replaced

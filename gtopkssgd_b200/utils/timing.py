@@ -49,20 +49,22 @@ class CudaTimer:
         self._pending: List = []
         self._done: List[float] = []
         self._open = None
+        self._free: List = []   # events of resolved intervals, recorded again (a timing event costs 2 us to create)
+
+    def _mark(self):
+        ev = self._free.pop() if self._free else torch.cuda.Event(enable_timing=True)
+        ev.record()
+        return ev
 
     def start(self) -> None:
         if not self.enabled:
             return
-        ev = torch.cuda.Event(enable_timing=True)
-        ev.record()
-        self._open = ev
+        self._open = self._mark()
 
     def stop(self) -> None:
         if not self.enabled or self._open is None:
             return
-        ev = torch.cuda.Event(enable_timing=True)
-        ev.record()
-        self._pending.append((self._open, ev))
+        self._pending.append((self._open, self._mark()))
         self._open = None
 
     def resolve(self) -> List[float]:
@@ -71,6 +73,7 @@ class CudaTimer:
         for a, b in self._pending:
             if b.query():
                 self._done.append(a.elapsed_time(b) * 1e-3)
+                self._free += (a, b)
             else:
                 keep.append((a, b))
         self._pending = keep
