@@ -30,8 +30,8 @@ constexpr int kMaxRounds = 4;     // log2(16) recursive-doubling rounds
 constexpr int kMaxPeers = 16;
 constexpr int kTraceSlots = 64;
 
-// Per-rank control block.  The host clears it (one async memset) before every
-// launch that uses it, so every counter starts at zero.
+// Per-rank control block.  Its counters start at zero: every user owns two blocks, alternates between them
+// and clears the idle one.
 struct Ctrl {
   unsigned int bar;         // grid-barrier arrival counter
   unsigned int abort;       // non-zero: every wait returns at once
@@ -43,15 +43,14 @@ struct Ctrl {
   unsigned int scratch[9];
   unsigned int cursor[kMaxRounds + 2];        // one output cursor per round
   unsigned int tie[kMaxRounds + 2];           // one tie counter per round
-  unsigned int live[kMaxRounds + 2];
+  unsigned int live[kMaxRounds + 2];          // K2, K2t: keys in the threshold bin's list
   unsigned int ticket[8];                     // K1: work handed out per phase, and work completed
   unsigned int done[8];
   unsigned int pad[64 - 16 - 3 * (kMaxRounds + 2) - 16];
   unsigned long long trace[kTraceSlots];      // %globaltimer stamps of CTA 0 at phase boundaries
-  // Radix histograms, one set of four rows per tree round (K2) or per use (K1: sets 0-2, rows 0-2).
-  // K2 rows: 0 = first digit; 1 and 2[0..1023] = second digit of the entries whose first digit is one
-  // of three predicted ones (1024 bins each); 2[1024..] = second digit counted by a sweep when the
-  // prediction missed; 3 = third digit.
+  // Selection histograms, one set of four rows per tree round (K2; K2t uses set 0) or per use (K1: set 0
+  // candidate levels, set 1 exact mode).  K2 and K2t: row 0 = counts of the band, 1 = list of the threshold
+  // bin's keys, 2 and 3 = the counting sweeps of a missed prediction.
   unsigned int hist[kMaxRounds + 2][4][kHistBins];
 };
 
@@ -89,6 +88,11 @@ __device__ __forceinline__ void red_release_gpu_add(unsigned int* p, unsigned in
 // Phase stamp for the device-side trace: thread 0 of the rank's CTA 0 only.
 __device__ __forceinline__ void trace_stamp(Ctrl* c, int slot) {
   if (blockIdx.x == 0 && threadIdx.x == 0 && slot < kTraceSlots) c->trace[slot] = globaltimer_ns();
+}
+
+// The same for kernels whose every CTA serves a control block of its own.
+__device__ __forceinline__ void trace_stamp_of(Ctrl* c, int slot) {
+  if (threadIdx.x == 0 && slot < kTraceSlots) c->trace[slot] = globaltimer_ns();
 }
 
 // Pair <-> 64-bit word, so that a pair always moves with one 8-byte access.
@@ -186,8 +190,8 @@ __device__ __forceinline__ bool wait_flag(const uint64_t* flag, uint32_t epoch, 
       *payload = (uint32_t)(v & 0xffffffffull);
       return true;
     }
-    if (aborted(ctrl)) return false;
-    if ((++spins & 31u) == 0u) {
+    if ((++spins & 31u) == 0u) {  // (looking at the abort word each time doubles the polling period)
+      if (aborted(ctrl)) return false;
       if (globaltimer_ns() - t0 > limit_ns) {
         record_error(ctrl, ST_TIMEOUT_FLAG, where);
         return false;

@@ -20,9 +20,15 @@ namespace gtk {
 //   ag    : [2][kMaxPeers][kcap] pairs    all-gather slots, one per source rank (K2t only)
 //   gout  : [2][kcap] pairs               the global top-k set
 //   flags : [2][kFlagsPerParity] u64      (epoch << 32) | count
+//   ll    : [2][kMaxRounds + 1][kLLMaxK] 16-byte entries with their epoch (k2_tree_small.cu); the last
+//           row of a parity is the broadcast's
 constexpr int kFlagBcast = kMaxRounds;             // flag index of the broadcast
 constexpr int kFlagAg0 = kMaxRounds + 1;           // first all-gather flag (one per source)
 constexpr int kFlagsPerParity = kMaxRounds + 1 + kMaxPeers;
+constexpr unsigned int kLLMaxK = 2048;  // largest k of the small tree exchange (k2_tree_small.cu)
+__host__ __device__ constexpr size_t ll_off(unsigned int parity, unsigned int round) {
+  return ((size_t)parity * (kMaxRounds + 1) + round) * kLLMaxK;
+}
 
 struct K2Rank {
   const Pair* sel;        // local selection written by K1
@@ -34,8 +40,8 @@ struct K2Rank {
   Pair* ag;
   Pair* gout;
   uint64_t* flags;
-  Ctrl* ctrl;             // TWO control blocks.  K2 uses block (call & 1) and cleans the other one itself;
-                          // K2t uses block 0, cleared by the host before every launch
+  ulonglong2* ll;
+  Ctrl* ctrl;             // TWO control blocks: call e uses block (e & 1) and cleans the other one itself
   unsigned int* n_global; // kResWords device words: result of the last call, see kRes* below
   unsigned int* epoch;    // device word: call counter (starts at 1); the kernel reads it at entry and
                           // adds one after its last barrier, so a replayed CUDA graph needs no new argument
@@ -43,7 +49,13 @@ struct K2Rank {
   Pair* peer_ag[kMaxPeers];
   Pair* peer_gout[kMaxPeers];
   uint64_t* peer_flags[kMaxPeers];
+  ulonglong2* peer_ll[kMaxPeers];
 };
+
+// The tree exchange for small sets (k2_tree_small.cu).
+bool k2_small_serves(unsigned int nranks, unsigned int k, unsigned int nctas);
+int k2_small_launch(const K2Rank* ranks, unsigned int nranks, unsigned int rank_base, unsigned int P, unsigned int k,
+                    unsigned int kcap, unsigned int d, unsigned long long limit_ns, cudaStream_t stream);
 
 // Result words of an exchange (K2Rank::n_global).  kResCount is what the consumer (K3) reads: the
 // number of pairs in gout[parity], 0 after a failed call.  The other three are written once, by
@@ -118,14 +130,16 @@ __device__ __forceinline__ bool cta_wait_flag(ExchangeShared& sh, const uint64_t
   return sh.ok != 0;
 }
 
-// A <- copy of src, and map[idx] = position.
+// A <- copy of src, map[idx] = position, and tally(value, 1) for each.
+template <typename Tally>
 __device__ __forceinline__ void copy_and_map(Pair* A, const Pair* src, unsigned int n, int32_t* map,
                                              unsigned int d, unsigned int cta, unsigned int nct,
-                                             Ctrl* ctrl) {
+                                             Ctrl* ctrl, Tally tally) {
   const unsigned int stride = nct * kSelThreads;
   for (unsigned int i = cta * kSelThreads + threadIdx.x; i < n; i += stride) {
     const Pair e = ld_pair_cg(&src[i]);
     st_pair(&A[i], e);
+    tally(e.val, 1u);
     if ((unsigned int)e.idx < d) map[e.idx] = (int32_t)i;
     else record_error(ctrl, ST_BOUNDS, 300);
   }
@@ -139,31 +153,6 @@ __device__ __forceinline__ void build_map(const Pair* A, unsigned int n, int32_t
     const Pair e = ld_pair_cg(&A[i]);
     if ((unsigned int)e.idx < d) map[e.idx] = (int32_t)i;
     else record_error(ctrl, ST_BOUNDS, 301);
-  }
-}
-
-// Shared indices: A[p].val += B[j].val and B[j] is marked dead (idx = -1).
-// B lives in local memory.  Indices are unique inside A and inside B, so every
-// A[p] is touched by at most one thread.
-__device__ __forceinline__ void probe_merge(Pair* A, unsigned int n_a, Pair* B, unsigned int n_b,
-                                            const int32_t* map, unsigned int d, unsigned int cta,
-                                            unsigned int nct, Ctrl* ctrl) {
-  const unsigned int stride = nct * kSelThreads;
-  for (unsigned int j = cta * kSelThreads + threadIdx.x; j < n_b; j += stride) {
-    const Pair e = ld_pair_cg(&B[j]);
-    if ((unsigned int)e.idx >= d) {
-      record_error(ctrl, ST_BOUNDS, 302);
-      B[j].idx = -1;
-      continue;
-    }
-    const unsigned int p = (unsigned int)__ldcg(&map[e.idx]);
-    if (p < n_a) {
-      const Pair a = ld_pair_cg(&A[p]);
-      if (a.idx == e.idx) {
-        A[p].val = a.val + e.val;
-        B[j].idx = -1;
-      }
-    }
   }
 }
 

@@ -58,7 +58,7 @@ int gtk_k1_compress(float* g, float* r, long long d, unsigned int k, void* cand,
 int gtk_k2_exchange(const void* ranks_dev, unsigned int nranks, unsigned int rank_base, unsigned int P,
                     unsigned int k, unsigned int kcap, unsigned int d, unsigned int nctas,
                     unsigned long long limit_ns, int use_cluster, void* stream);
-int gtk_k2t_allgather(const void* ranks_dev, void* const* ctrl_dev, unsigned int nranks, unsigned int rank_base,
+int gtk_k2t_allgather(const void* ranks_dev, unsigned int nranks, unsigned int rank_base,
                       unsigned int P, unsigned int k, unsigned int kcap, unsigned int work_cap, unsigned int d,
                       int reselect, void* seg_counts, unsigned int nctas, unsigned long long limit_ns, void* stream);
 int gtk_k3_dense(float* p, float* buf, const float* g, const float* coef, float scale, long long d, float lr,

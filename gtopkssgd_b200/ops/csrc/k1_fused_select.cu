@@ -41,8 +41,7 @@
 #include <atomic>
 #include <cstddef>
 #include <type_traits>
-#include <cooperative_groups.h>
-#include "select_common.cuh"
+#include "pick_common.cuh"
 #include "host_api.h"
 #include "launch.cuh"
 
@@ -62,9 +61,7 @@ constexpr unsigned int kShards = 16;       // ticket counters of the dynamic str
 // SMs are too few for the scattered write-back.
 constexpr unsigned int kPickSmall = 4096;
 constexpr unsigned int kPickCluster = 65536;
-constexpr int kPickThreads = 1024;
 constexpr int kPickCtas = 8;               // CTAs per cluster
-constexpr int kBins = kHistBins;           // 2048
 
 // Bins of the first selection level: (key - lo) >> shift, the last bin open to the top.  lo is the candidate
 // threshold and shift puts the previous call's k-th magnitude into bins 256..511, so that the new one lies in
@@ -325,67 +322,13 @@ struct Winners {
   }
 };
 
-struct PickShared {
-  unsigned int hist[kBins];
-  unsigned int share[2][kBins / kPickCtas]; // cluster: the sums of bins b = rank (mod 8), for alternating levels
-  unsigned int warp_tot[kPickThreads / 32];
-  unsigned int warp_n[2][kPickThreads / 32];
-  unsigned int base[2];
-  unsigned int res_bin, res_krem;
+struct PickShared : WideShared {
+  unsigned int share[3][kBins / kPickCtas]; // cluster: the sums of bins b = rank (mod 8), a buffer per level in turn
   unsigned int chunk;
   unsigned int tie;
   unsigned int cta_n[kPickCtas];
   int ok;
 };
-
-// The keys that still matter: lo <= key <= hi, in bins of 2^shift.  An open level clamps everything
-// above its last bin into it.
-struct Level {
-  uint32_t lo, hi;
-  unsigned int shift;
-  bool open;
-  __device__ __forceinline__ bool has(uint32_t key) const { return key - lo <= hi - lo; }
-  __device__ __forceinline__ unsigned int bin(uint32_t key) const {
-    const unsigned int b = (key - lo) >> shift;
-    return b < (unsigned int)kBins ? b : (unsigned int)kBins - 1u;
-  }
-  // The level inside bin b; false when the bin is a single key (then lo is that key).
-  __device__ __forceinline__ bool narrow(unsigned int b) {
-    lo += b << shift;
-    if (!(open && b == (unsigned int)kBins - 1u)) {
-      if (shift == 0u) return false;
-      hi = lo + ((1u << shift) - 1u);
-    }
-    const uint32_t width = hi - lo;  // an open top is as wide as the keys go
-    const int bits = 32 - __clz(width);
-    shift = bits > 11 ? (unsigned int)(bits - 11) : 0u;
-    open = false;
-    return true;
-  }
-};
-
-// Finds the bin B with count(bins > B) < k_rem <= count(bins >= B): res_bin, and k_rem minus the count
-// above it: res_krem.  c: the complete counts of bins 2t and 2t + 1.
-__device__ __forceinline__ void find_bin(PickShared& s, uint2 c, unsigned int k_rem) {
-  const int t = threadIdx.x, w = t >> 5;
-  const unsigned int mine = c.x + c.y;
-  unsigned int suf = mine;  // inclusive suffix sum over the warp (higher lane = higher bins)
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned int v = __shfl_down_sync(0xffffffffu, suf, o);
-    if ((int)lane_id() + o < 32) suf += v;
-  }
-  if (lane_id() == 0) s.warp_tot[w] = suf;
-  __syncthreads();
-  const unsigned int v = s.warp_tot[lane_id()];
-  const unsigned int above = __reduce_add_sync(0xffffffffu, (int)lane_id() > w ? v : 0u) + (suf - mine);
-  if (above < k_rem && k_rem <= above + mine) {
-    const bool upper = k_rem <= above + c.y;
-    s.res_bin = 2u * t + (upper ? 1u : 0u);
-    s.res_krem = k_rem - above - (upper ? 0u : c.y);
-  }
-  __syncthreads();
-}
 
 __device__ __forceinline__ uint2 global_counts(const unsigned int* ghist) {
   return __ldcg(reinterpret_cast<const uint2*>(ghist) + threadIdx.x);
@@ -397,45 +340,6 @@ __device__ __forceinline__ void publish_hist(PickShared& s, unsigned int* ghist)
   const uint2 c = *my_bins(s);
   if (c.x) atomicAdd(&ghist[2 * threadIdx.x], c.x);
   if (c.y) atomicAdd(&ghist[2 * threadIdx.x + 1], c.y);
-}
-
-// Output position of the first of this thread's n entries.  cursor: global list cursor, or nullptr when
-// this CTA writes the whole list.  turn alternates between consecutive calls.
-__device__ __forceinline__ unsigned int place(PickShared& s, unsigned int n, unsigned int* cursor, unsigned int turn) {
-  const int w = threadIdx.x >> 5;
-  unsigned int pre = n;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned int v = __shfl_up_sync(0xffffffffu, pre, o);
-    if ((int)lane_id() >= o) pre += v;
-  }
-  if (lane_id() == 31) s.warp_n[turn & 1u][w] = pre;
-  __syncthreads();
-  const unsigned int v = s.warp_n[turn & 1u][lane_id()];
-  const unsigned int before = __reduce_add_sync(0xffffffffu, (int)lane_id() < w ? v : 0u);
-  unsigned int base = 0;
-  if (cursor) {
-    const unsigned int total = __reduce_add_sync(0xffffffffu, v);
-    if (threadIdx.x == 0) s.base[turn & 1u] = total ? atomicAdd(cursor, total) : 0u;
-    __syncthreads();
-    base = s.base[turn & 1u];
-  }
-  return base + before + pre - n;
-}
-
-// One entry against the threshold; called by whole warps.  Entries equal to it take tickets, the first
-// `quota` of which are selected.
-__device__ __forceinline__ bool passes(bool live, uint32_t key, uint32_t th, unsigned int quota, unsigned int* tie) {
-  const bool equal = live && key == th;
-  bool win = live && key > th;
-  const unsigned int m = __ballot_sync(0xffffffffu, equal);
-  if (m) {
-    unsigned int base = 0;
-    if (lane_id() == (unsigned int)(__ffs(m) - 1)) base = atomicAdd(tie, (unsigned int)__popc(m));
-    base = __shfl_sync(0xffffffffu, base, __ffs(m) - 1);
-    if (equal) win = base + __popc(m & lanemask_lt()) < quota;
-  }
-  return win;
 }
 
 // Calls f(chunk) for every chunk this CTA gets of phase ph; returns how many.
@@ -575,11 +479,6 @@ __device__ __forceinline__ uint32_t pick_small(PickShared& s, float* r, const Pa
   return th;
 }
 
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 // kPickSmall < C <= kPickCluster: the same with 8 CTAs that meet in the hardware barrier (0.2 us) and add
 // up their counts over distributed shared memory.  Every CTA of the first cluster calls this.
 __device__ __forceinline__ uint32_t pick_cluster(PickShared& s, float* r, const Pair* cand, const Winners& out,
@@ -612,13 +511,14 @@ __device__ __forceinline__ uint32_t pick_cluster(PickShared& s, float* r, const 
     }
     __syncthreads();
     // Bin b is summed up in CTA b mod 8.  (Reading all eight histograms in every CTA moves 64 KB per SM over
-    // the cluster network: 2 us per level.)  The next level's share is cleared here, which everybody is past
-    // reading since the barrier before.
+    // the cluster network: 2 us per level.)  The next level's buffer is cleared here: it was read two levels
+    // ago, before the barrier that this CTA has passed since, and is added to after the barrier below.
     const uint2 part = *my_bins(s);
     const unsigned int b0 = 2u * threadIdx.x;
     if (part.x) atomicAdd(cluster.map_shared_rank(&s.share[buf][b0 / kPickCtas], b0 % kPickCtas), part.x);
     if (part.y) atomicAdd(cluster.map_shared_rank(&s.share[buf][b0 / kPickCtas], b0 % kPickCtas + 1u), part.y);
-    if (threadIdx.x < (unsigned int)(kBins / kPickCtas)) s.share[buf ^ 1][threadIdx.x] = 0u;
+    const int next = buf == 2 ? 0 : buf + 1;
+    if (threadIdx.x < (unsigned int)(kBins / kPickCtas)) s.share[next][threadIdx.x] = 0u;
     cluster_barrier();
     uint2 sum;
     sum.x = *cluster.map_shared_rank(&s.share[buf][b0 / kPickCtas], b0 % kPickCtas);
@@ -626,7 +526,7 @@ __device__ __forceinline__ uint32_t pick_cluster(PickShared& s, float* r, const 
     find_bin(s, sum, k_rem);
     k_rem = s.res_krem;
     if (!lv.narrow(s.res_bin)) break;
-    buf ^= 1;
+    buf = next;
   }
   const uint32_t th = lv.lo;
   unsigned int* const tie = cluster.map_shared_rank(&s.tie, 0);

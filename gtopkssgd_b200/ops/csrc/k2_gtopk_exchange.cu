@@ -39,44 +39,29 @@ namespace gtk {
 // kK2Cache = union entries each thread keeps in registers across the phases of a round (template
 // parameter of the kernel: 4 by default, 8 when a 16-CTA cluster serves up to 64 K union entries).
 
-constexpr int kK2Pred = 3;  // second-digit histograms are built on the fly for this many predicted first digits
-
 struct K2Shared {
   ExchangeShared ex;
-  unsigned int hist0[kHistBins];  // this CTA's share of the first-digit histogram, built on the fly
-  unsigned int hist1[kK2Pred][1024];  // second digit of the entries whose first digit is pred, pred+1, pred+2
-  unsigned int cursor;            // single-CTA ranks: output cursor and tie tickets of the current round
-  unsigned int tie;               // live here instead of in global memory (two round trips less per round)
+  unsigned int band[kHistBins];   // this CTA's share of the first selection level, counted on the fly
 };
 
-__device__ __forceinline__ void hist0_clear(K2Shared& sh) {
-  for (int i = threadIdx.x; i < kHistBins; i += kSelThreads) sh.hist0[i] = 0u;
-  for (int i = threadIdx.x; i < kK2Pred * 1024; i += kSelThreads) (&sh.hist1[0][0])[i] = 0u;
+__device__ __forceinline__ void band_clear(K2Shared& sh) {
+  for (int i = threadIdx.x; i < kHistBins; i += kSelThreads) sh.band[i] = 0u;
   __syncthreads();
 }
-// Global home of the second-digit histogram of predicted first digit pred + off, inside one round's set.
-__device__ __forceinline__ unsigned int* pred_row(unsigned int (*set)[kHistBins], unsigned int off) {
-  return off < 2u ? set[1] + off * 1024u : set[2];
-}
-// Adds this CTA's (possibly "negative", i.e. wrapped) partial counts to a round's global histograms
-// (first digit, and second digit for the predicted first digits) and zeroes the shared copies.
-__device__ __forceinline__ void hist0_flush(K2Shared& sh, unsigned int (*set)[kHistBins]) {
+// Adds this CTA's (possibly "negative", i.e. wrapped) partial counts to a round's global ones and zeroes the
+// shared copy.
+__device__ __forceinline__ void band_flush(K2Shared& sh, unsigned int* ghist) {
   __syncthreads();
   for (int i = threadIdx.x; i < kHistBins; i += kSelThreads) {
-    const unsigned int c = sh.hist0[i];
-    if (c) atomicAdd(&set[0][i], c);
-    sh.hist0[i] = 0u;
-  }
-  for (int i = threadIdx.x; i < kK2Pred * 1024; i += kSelThreads) {
-    const unsigned int c = sh.hist1[i >> 10][i & 1023];
-    if (c) atomicAdd(&pred_row(set, (unsigned int)i >> 10)[i & 1023], c);
-    sh.hist1[i >> 10][i & 1023] = 0u;
+    const unsigned int c = sh.band[i];
+    if (c) atomicAdd(&ghist[i], c);
+    sh.band[i] = 0u;
   }
   __syncthreads();
 }
 
 template <int kK2Cache>
-__global__ void __launch_bounds__(kSelThreads, 1)
+__global__ void __launch_bounds__(kSelThreads, kK2Cache == 4 ? 2 : 1)
 k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsigned int P,
                   unsigned int k, unsigned int kcap, unsigned int d, unsigned long long limit_ns,
                   int use_cluster) {
@@ -89,7 +74,6 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
   const unsigned int parity = epoch & 1u;
   const unsigned int stride = nct * kSelThreads;
   const unsigned int lane0 = cta * kSelThreads + threadIdx.x;  // union index of this thread's trip 0
-  const bool single = nct == 1;  // the whole rank is this CTA: histograms never leave shared memory
   Ctrl* ctrl = R.ctrl + parity;
   int32_t* const map = R.map;
   RankBarrier bar{ctrl, nct, 0u, limit_ns, nullptr, use_cluster != 0};
@@ -118,20 +102,13 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
 
   unsigned int rounds = 0;
   while ((1u << rounds) < P) ++rounds;
-  hist0_clear(sh);
+  band_clear(sh);
+  if (cta == 0 && threadIdx.x == 0) ctrl->scratch[8] = 1u;  // this block's histograms will need clearing
   trace_stamp(ctrl, 0);
-  // Every live entry of a round's union is counted once by its first radix digit and, if that digit is
-  // pred0, pred0 + 1 or pred0 + 2, by its second digit as well (delta = 1 adds, 0xffffffff removes).  The
-  // union's k-th magnitude is at least this rank's own, and for heavy-tailed gradients about one first
-  // digit (a factor 2^(1/8)) above it, so the re-select usually finds both digits without a sweep.
-  unsigned int pred0 = mag_key(R.st->kth_mag) >> 20;  // round 0: first digit of K1's k-th magnitude
-  auto tally = [&](float v, unsigned int delta) {
-    const uint32_t key = mag_key(v);
-    const unsigned int fd = key >> 20;
-    atomicAdd(&sh.hist0[fd], delta);
-    const unsigned int off = fd - pred0;  // wraps for fd < pred0
-    if (off < (unsigned int)kK2Pred) atomicAdd(&sh.hist1[off][(key >> 10) & 1023u], delta);
-  };
+  // Every live entry of a round's union is counted once in the band above `pred` (delta = 1 adds, 0xffffffff
+  // removes): the union's k-th magnitude is at least this rank's own and for gradient tails a few per cent above.
+  uint32_t pred = mag_key(R.st->kth_mag);  // round 0: K1's k-th magnitude, then the previous round's threshold
+  auto tally = [&](float v, unsigned int delta) { atomicAdd(&sh.band[band_bin(mag_key(v), pred)], delta); };
 
   for (unsigned int r = 0; r < rounds; ++r) {
     const unsigned int bit = 1u << r;
@@ -141,7 +118,7 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
       const unsigned int partner = me - bit;
       Pair* dst = R.peer_slots[partner] + slot_off(parity, r, kcap);
       push_pairs(dst, cur, n_cur, cta, nct);
-      cta_fence_peer_stores(single);
+      cta_fence_peer_stores(nct == 1);
       if (!bar.sync(200 + r)) { fail(); return; }
       trace_stamp(ctrl, 1 + 8 * r + 6);
       if (cta == 0 && threadIdx.x == 0)
@@ -151,8 +128,8 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
     }
     if (low != 0u) break;  // already left the tree
 
-    // ---- receiver.  A = current set in a writable work buffer, with map[] and the first-digit
-    // histogram describing it (built here in round 0, by the previous compaction afterwards).
+    // ---- receiver.  A = current set in a writable work buffer, with map[] and the band counts
+    // describing it (built here in round 0, by the previous compaction afterwards).
     Pair* A;
     const bool copied = cur_buf < 0;
     if (copied) {
@@ -243,7 +220,7 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
         }
       }
     }
-    if (!single) hist0_flush(sh, ctrl->hist[r]);
+    band_flush(sh, ctrl->hist[r][0]);
     if (!bar.sync(240 + r)) { fail(); return; }  // sums and the on-the-fly histograms complete
     trace_stamp(ctrl, 1 + 8 * r + 3);
 
@@ -262,67 +239,19 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
       return e;
     };
 
-    // ---- re-select: the first digit is known from the histogram built on the fly
-    Threshold th;
-    th.select_all = false;
-    th.key = 0u;
-    th.quota = 0u;
-    find_digit_in<kHistBins>(ss, single ? sh.hist0 : ctrl->hist[r][0], k, single);
-    const bool all = ss.res_total <= k;
-    uint32_t prefix = ss.res_digit;
-    unsigned int k_rem = ss.res_krem;
-    __syncthreads();
-    const unsigned int first_digit = prefix;
-    const unsigned int pred_off = first_digit - pred0;  // wraps when the threshold digit is below the prediction
-    const bool predicted = !all && pred_off < (unsigned int)kK2Pred;
-    if (predicted) {
-      // second digit: counted on the fly, no sweep and no barrier
-      find_digit_in<1024>(ss, single ? sh.hist1[pred_off] : pred_row(ctrl->hist[r], pred_off), k_rem, single);
-      prefix = (prefix << 10) | ss.res_digit;
-      k_rem = ss.res_krem;
-      __syncthreads();
-    }
-    if (single) hist0_clear(sh);  // from here on the shared histograms collect the next round's digits
-    pred0 = all ? 0u : first_digit;  // the next union's threshold is at least this one
-    if (all) {
-      th.select_all = true;
-    } else {
-      if (!predicted) {
-        // pass 1: bits 19..10 of the entries whose first digit is the threshold digit
-        smem_hist_clear(ss);
-#pragma unroll
-        for (int t = 0; t < kK2Cache; ++t)
-          if (c[t].idx >= 0 && (mag_key(c[t].val) >> 20) == prefix)
-            atomicAdd(&ss.hist[(mag_key(c[t].val) >> 10) & 1023u], 1u);
-        for (unsigned int t = kK2Cache; t < trips; ++t) {
-          const Pair e = entry(t);
-          if (e.idx >= 0 && (mag_key(e.val) >> 20) == prefix)
-            atomicAdd(&ss.hist[(mag_key(e.val) >> 10) & 1023u], 1u);
-        }
-        if (!single) smem_hist_flush(ss, ctrl->hist[r][2] + 1024, 1024);
-        if (!bar.sync(250 + 10 * r)) { fail(); return; }
-        find_digit<1024>(ss, ctrl->hist[r][2] + 1024, k_rem, single);
-        prefix = (prefix << 10) | ss.res_digit;
-        k_rem = ss.res_krem;
-        __syncthreads();
-      }
-      // pass 2: bits 9..0
-      smem_hist_clear(ss);
+    // ---- re-select
+    auto visit = [&](auto f) {
 #pragma unroll
       for (int t = 0; t < kK2Cache; ++t)
-        if (c[t].idx >= 0 && (mag_key(c[t].val) >> 10) == prefix)
-          atomicAdd(&ss.hist[mag_key(c[t].val) & 1023u], 1u);
+        if (c[t].idx >= 0) f(mag_key(c[t].val));
       for (unsigned int t = kK2Cache; t < trips; ++t) {
         const Pair e = entry(t);
-        if (e.idx >= 0 && (mag_key(e.val) >> 10) == prefix) atomicAdd(&ss.hist[mag_key(e.val) & 1023u], 1u);
+        if (e.idx >= 0) f(mag_key(e.val));
       }
-      if (!single) smem_hist_flush(ss, ctrl->hist[r][3], 1024);
-      if (!bar.sync(251 + 10 * r)) { fail(); return; }
-      find_digit<1024>(ss, ctrl->hist[r][3], k_rem, single);
-      th.key = (prefix << 10) | ss.res_digit;
-      th.quota = ss.res_krem;
-      __syncthreads();
-    }
+    };
+    Threshold th;
+    if (!band_select_kth(ss, bar, k, pred, ctrl->hist[r], &ctrl->live[r], visit, &th, 250 + 10 * r)) { fail(); return; }
+    if (!th.select_all) pred = th.key;  // the next union's threshold is at least this one
     trace_stamp(ctrl, 1 + 8 * r + 4);
 
     // ---- compaction of the winners to where the next phase reads them
@@ -333,7 +262,7 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
     if (last) OUT = R.gout + (size_t)parity * kcap;
     else if (send_next) OUT = R.peer_slots[me - 2u * bit] + slot_off(parity, r + 1, kcap);
     else OUT = R.work[cur_buf ^ 1];
-    // keep: the table and (below) the first-digit histogram of the next round are built on the way;
+    // keep: the table and (below) the band counts of the next round are built on the way;
     // last: the table over the global set serves the residual put-back, and every peer gets its copy
     auto on_placed = [&](Pair e, unsigned int pos) {
       if (send_next) return;
@@ -341,14 +270,9 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
       if (last)
         for (unsigned int q = 1; q < P; ++q) st_pair(R.peer_gout[q] + (size_t)parity * kcap + pos, e);
     };
-    unsigned int* const cursor = single ? &sh.cursor : &ctrl->cursor[r];
-    unsigned int* const tie = single ? &sh.tie : &ctrl->tie[r];
-    if (single && threadIdx.x == 0) {
-      sh.cursor = 0u;
-      sh.tie = 0u;
-    }
-    StagedAppender app{&ss, OUT, cursor, kcap, ctrl};
-    app.begin();  // (a __syncthreads: the two words above are visible)
+    unsigned int* const tie = &ctrl->tie[r];
+    StagedAppender app{&ss, OUT, &ctrl->cursor[r], kcap, ctrl};
+    app.begin();
     auto consider = [&](const Pair& e) {
       if (e.idx >= 0 && passes_threshold(mag_key(e.val), th, tie)) {
         app.put(e);
@@ -367,11 +291,10 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
       app.end_tile(on_placed);
     }
     app.flush(on_placed);
-    if (!single && keep) hist0_flush(sh, ctrl->hist[r + 1]);
-    if (!keep) cta_fence_peer_stores(single);  // the winners went into other GPUs' memory
+    if (!keep) cta_fence_peer_stores(nct == 1);  // the winners went into other GPUs' memory
     if (!bar.sync(290 + r)) { fail(); return; }  // OUT and its cursor complete
     trace_stamp(ctrl, 1 + 8 * r + 5);
-    n_cur = single ? sh.cursor : __ldcg(&ctrl->cursor[r]);
+    n_cur = __ldcg(&ctrl->cursor[r]);
     if (n_cur > kcap) n_cur = kcap;
     if (send_next) {
       if (cta == 0 && threadIdx.x == 0)
@@ -434,6 +357,11 @@ using namespace gtk;
 
 extern "C" unsigned long long gtk_k2rank_bytes(void) { return sizeof(K2Rank); }
 
+// The small exchange's entries lie behind the flags.
+static unsigned long long ll_offset(unsigned long long flags) {
+  return (flags + 2ull * kFlagsPerParity * sizeof(uint64_t) + 255ull) & ~255ull;
+}
+
 // Symmetric-region geometry, in bytes, for a given kcap: offsets of slots, ag,
 // gout and flags, and the total size.  out[0..4] = {slots, ag, gout, flags, total}.
 extern "C" void gtk_symm_layout(unsigned int kcap, int with_allgather, unsigned long long* out) {
@@ -446,8 +374,8 @@ extern "C" void gtk_symm_layout(unsigned int kcap, int with_allgather, unsigned 
   off += 2ull * kcap * sizeof(Pair);
   off = (off + 255ull) & ~255ull;
   out[3] = off;
-  off += 2ull * kFlagsPerParity * sizeof(uint64_t);
-  off = (off + 255ull) & ~255ull;
+  off = ll_offset(off);
+  off += 2ull * (kMaxRounds + 1) * kLLMaxK * sizeof(ulonglong2);
   out[4] = off;
 }
 
@@ -471,6 +399,7 @@ extern "C" int gtk_k2rank_fill(void* desc_host, const void* sel, const void* st,
   r->ag = (Pair*)(base + lay[1]);
   r->gout = (Pair*)(base + lay[2]);
   r->flags = (uint64_t*)(base + lay[3]);
+  r->ll = (ulonglong2*)(base + ll_offset(lay[3]));
   r->ctrl = (Ctrl*)ctrl;
   r->n_global = (unsigned int*)n_global;
   r->epoch = (unsigned int*)epoch_word;
@@ -480,6 +409,7 @@ extern "C" int gtk_k2rank_fill(void* desc_host, const void* sel, const void* st,
     r->peer_ag[q] = pb ? (Pair*)(pb + lay[1]) : nullptr;
     r->peer_gout[q] = pb ? (Pair*)(pb + lay[2]) : nullptr;
     r->peer_flags[q] = pb ? (uint64_t*)(pb + lay[3]) : nullptr;
+    r->peer_ll[q] = pb ? (ulonglong2*)(pb + ll_offset(lay[3])) : nullptr;
   }
   return GTK_OK;
 }
@@ -558,6 +488,8 @@ extern "C" int gtk_k2_exchange(const void* ranks_dev, unsigned int nranks, unsig
   if (P < 2 || (P & (P - 1)) != 0 || P > (unsigned int)kMaxPeers) return GTK_ERR_ARG;
   if (k == 0 || k > kcap || nranks == 0 || nctas == 0) return GTK_ERR_ARG;
   const K2Rank* ranks = (const K2Rank*)ranks_dev;
+  if (k2_small_serves(nranks, k, nctas))
+    return k2_small_launch(ranks, nranks, rank_base, P, k, kcap, d, limit_ns, stream);
   int cluster = (use_cluster && k2_cluster_fits(nranks, nctas)) ? 1 : 0;
   const int depth = k2_cache_depth(k, nctas, cluster);
   const K2Kernel fn = k2_kernel(depth);

@@ -20,12 +20,14 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
                    int reselect, unsigned int* __restrict__ seg_counts_all,
                    unsigned long long limit_ns) {
   __shared__ ExchangeShared sh;
+  __shared__ unsigned int band[kHistBins];  // this CTA's share of the first selection level, counted on the fly
+  __shared__ unsigned int counts[kMaxPeers];
   const K2Rank& R = ranks[blockIdx.y];
   const unsigned int epoch = __ldcg(R.epoch);
   const unsigned int me = rank_base + blockIdx.y;
   const unsigned int cta = blockIdx.x, nct = gridDim.x;
   const unsigned int parity = epoch & 1u;
-  Ctrl* ctrl = R.ctrl;
+  Ctrl* ctrl = R.ctrl + parity;
   RankBarrier bar{ctrl, nct, 0u, limit_ns};
   unsigned int* seg_counts = seg_counts_all + (size_t)blockIdx.y * kMaxPeers;
 
@@ -62,24 +64,32 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
   if (!bar.sync(500)) { fail(); return; }
   if (cta == 0 && threadIdx.x < P && threadIdx.x != me)  // one releasing thread per destination
     release_flag(R.peer_flags[threadIdx.x] + flag_off(parity, kFlagAg0 + me), epoch, n_sel);
-  // wait for every source
-  unsigned int counts[kMaxPeers];
-  for (unsigned int q = 0; q < P; ++q) {
+  // wait for every source, one polling thread for each
+  if (threadIdx.x == 0) sh.ok = 1;
+  __syncthreads();
+  if (threadIdx.x < P) {
+    const unsigned int q = threadIdx.x;
     unsigned int c = n_sel;
-    if (q != me) {
-      if (!cta_wait_flag(sh, R.flags + flag_off(parity, kFlagAg0 + q), epoch, ctrl, limit_ns,
-                         510 + q, &c)) {
-        fail();
-        return;
-      }
-      if (c > kcap) {
-        record_error(ctrl, ST_CAPACITY, 530 + q);
-        c = kcap;
-      }
+    if (q != me && !wait_flag(R.flags + flag_off(parity, kFlagAg0 + q), epoch, ctrl, limit_ns, 510 + q, &c)) {
+      sh.ok = 0;
+      c = 0u;
+    }
+    if (c > kcap) {
+      record_error(ctrl, ST_CAPACITY, 530 + q);
+      c = kcap;
     }
     counts[q] = c;
+    if (cta == 0) seg_counts[q] = c;
   }
-  if (cta == 0 && threadIdx.x < P) seg_counts[threadIdx.x] = counts[threadIdx.x];
+  __syncthreads();
+  if (!sh.ok) { fail(); return; }
+  // The other control block, for the next call (what this form dirties of it: header, stamps, one histogram set).
+  {
+    uint4* other = reinterpret_cast<uint4*>(R.ctrl + (parity ^ 1u));
+    const size_t nvec16 = (offsetof(Ctrl, hist) + sizeof(((Ctrl*)0)->hist[0])) / 16;
+    for (size_t i = cta * kSelThreads + threadIdx.x; i < nvec16; i += (size_t)nct * kSelThreads)
+      other[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
   if (!reselect) {
     if (!bar.sync(535)) { fail(); return; }  // every CTA has read the epoch word
     if (cta == 0 && threadIdx.x == 0) {
@@ -90,9 +100,13 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
   }
 
   // ---- topk2: merge the P lists in rank order, then keep the k largest sums
+  const uint32_t pred = mag_key(R.st->kth_mag);  // no sum of P selections has its k-th magnitude below the own one
+  for (int i = threadIdx.x; i < kHistBins; i += kSelThreads) band[i] = 0u;
+  __syncthreads();
+  auto tally = [&](float v, unsigned int delta) { atomicAdd(&band[band_bin(mag_key(v), pred)], delta); };
   Pair* A = R.work[0];
   const Pair* L0 = R.ag + ag_off(parity, 0, kcap);
-  copy_and_map(A, L0, counts[0], R.map, d, cta, nct, ctrl);
+  copy_and_map(A, L0, counts[0], R.map, d, cta, nct, ctrl, tally);
   unsigned int n_a = counts[0];
   if (cta == 0 && threadIdx.x == 0) ctrl->n_live = n_a;
   if (!bar.sync(540)) { fail(); return; }
@@ -117,7 +131,10 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
           if (p < n_a) {
             const Pair a = ld_pair_cg(&A[p]);
             if (a.idx == e.idx) {
-              A[p].val = a.val + e.val;
+              const float sum = a.val + e.val;
+              A[p].val = sum;
+              tally(a.val, 0xffffffffu);
+              tally(sum, 1u);
               append = false;
             }
           }
@@ -133,19 +150,29 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
           if (pos < work_cap) {
             st_pair(&A[pos], e);
             R.map[e.idx] = (int32_t)pos;
+            tally(e.val, 1u);
           } else {
             record_error(ctrl, ST_CAPACITY, 551);
           }
         }
       }
     }
+    if (q + 1u == P) {  // the sums are final: publish this CTA's counts
+      __syncthreads();
+      for (int i = threadIdx.x; i < kHistBins; i += kSelThreads) {
+        const unsigned int n = band[i];
+        if (n) atomicAdd(&ctrl->hist[0][0][i], n);
+      }
+    }
     if (!bar.sync(560 + q)) { fail(); return; }
     n_a = __ldcg(&ctrl->n_live);
     if (n_a > work_cap) n_a = work_cap;
   }
-  auto key_at = [&](unsigned int i) -> uint32_t { return mag_key(ld_pair_cg(&A[i]).val); };
+  auto visit = [&](auto f) {
+    for (unsigned int i = cta * kSelThreads + threadIdx.x; i < n_a; i += stride) f(mag_key(ld_pair_cg(&A[i]).val));
+  };
   Threshold th;
-  if (!radix_select_kth(sh.sel, bar, cta, nct, n_a, k, ctrl->hist[0], key_at, &th, 580)) { fail(); return; }
+  if (!band_select_kth(sh.sel, bar, k, pred, ctrl->hist[0], &ctrl->live[0], visit, &th, 580)) { fail(); return; }
   Pair* G = R.gout + (size_t)parity * kcap;
   int32_t* map = R.map;
   auto on_placed = [&](Pair e, unsigned int pos) { map[e.idx] = (int32_t)pos; };
@@ -180,9 +207,9 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
 
 using namespace gtk;
 
-extern "C" int gtk_k2t_allgather(const void* ranks_dev, void* const* ctrl_dev, unsigned int nranks,
-                                 unsigned int rank_base, unsigned int P, unsigned int k,
-                                 unsigned int kcap, unsigned int work_cap, unsigned int d,
+// Nothing is cleared here: the kernel alternates between the two control blocks of each rank.
+extern "C" int gtk_k2t_allgather(const void* ranks_dev, unsigned int nranks, unsigned int rank_base, unsigned int P,
+                                 unsigned int k, unsigned int kcap, unsigned int work_cap, unsigned int d,
                                  int reselect, void* seg_counts,
                                  unsigned int nctas, unsigned long long limit_ns, void* stream_) {
   cudaStream_t stream = (cudaStream_t)stream_;
@@ -195,8 +222,6 @@ extern "C" int gtk_k2t_allgather(const void* ranks_dev, void* const* ctrl_dev, u
                                                             kSelThreads, 0) != cudaSuccess)
     return GTK_ERR_CUDA;
   if ((int)(nranks * nctas) > occ * di->sms) return GTK_ERR_ARG;
-  for (unsigned int i = 0; i < nranks; ++i)
-    if (cudaMemsetAsync(ctrl_dev[i], 0, sizeof(Ctrl), stream) != cudaSuccess) return GTK_ERR_CUDA;
   const K2Rank* ranks = (const K2Rank*)ranks_dev;
   unsigned int* segc = (unsigned int*)seg_counts;
   void* args[] = {&ranks, &rank_base, &P, &k, &kcap, &work_cap, &d, &reselect, &segc, &limit_ns};

@@ -22,8 +22,9 @@ __device__ __forceinline__ void pdl_begin(P*&... p) {
   ((void)([](P*& q) { asm volatile("" : "+l"(q)::"memory"); }(p)), ...);
 }
 
+// overlap = false: an ordinary launch of the same kernel.
 template <typename... K, typename... A>
-inline cudaError_t launch_pdl(void (*kernel)(K...), dim3 grid, dim3 block, cudaStream_t stream, A&&... args) {
+inline cudaError_t launch_pdl_if(bool overlap, void (*kernel)(K...), dim3 grid, dim3 block, cudaStream_t stream, A&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -32,8 +33,12 @@ inline cudaError_t launch_pdl(void (*kernel)(K...), dim3 grid, dim3 block, cudaS
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = overlap ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
+template <typename... K, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(K...), dim3 grid, dim3 block, cudaStream_t stream, A&&... args) {
+  return launch_pdl_if(true, kernel, grid, block, stream, static_cast<A&&>(args)...);
 }
 
 }  // namespace gtk

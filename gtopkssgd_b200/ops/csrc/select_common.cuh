@@ -1,7 +1,6 @@
-// Multi-CTA exact top-k-by-magnitude selection (3-pass radix select: 11+10+10
-// bits of the |value| bit pattern) and unordered compaction, shared by the
-// candidate select of K1, the dense fallback of K1 and the per-round re-select
-// of K2.  All CTAs of a rank run the same sequence and meet in RankBarrier.
+// Multi-CTA exact top-k-by-magnitude selection and unordered compaction, shared
+// by the re-selects of the two exchange kernels.  All CTAs of a rank run the same
+// sequence and meet in RankBarrier.
 #pragma once
 #include "common.cuh"
 
@@ -16,7 +15,6 @@ struct SelectShared {
   unsigned int res_digit;
   unsigned int res_krem;
   unsigned int res_total;
-  unsigned int res_equal;
   unsigned int stage_n;
   unsigned int stage_base;
   Pair stage[kStageCap];
@@ -44,12 +42,9 @@ __device__ __forceinline__ void smem_hist_flush(SelectShared& s, unsigned int* g
 // Every CTA scans the (complete) global histogram from the top bin downwards and
 // finds the digit D with count(bins > D) < k_rem <= count(bins >= D).
 // Results are left in shared memory: res_digit, res_krem (k_rem minus the count
-// above D), res_total (all entries), res_equal (count in bin D).
-// counts: the histogram to scan; in_smem says whether it is a shared-memory
-// array of this CTA (single-CTA ranks never touch a global copy) or a global one.
-template <int NBINS>
-__device__ __forceinline__ void find_digit_in(SelectShared& s, const unsigned int* counts,
-                                              unsigned int k_rem, bool in_smem) {
+// above D), res_total (all entries).  GLOBAL: counts lies in global memory, else in this CTA's shared memory.
+template <int NBINS, bool GLOBAL = true>
+__device__ __forceinline__ void find_digit_in(SelectShared& s, const unsigned int* counts, unsigned int k_rem) {
   constexpr int BPT = NBINS / kSelThreads;
   static_assert(BPT >= 1, "bins per thread");
   const int t = threadIdx.x;
@@ -57,7 +52,7 @@ __device__ __forceinline__ void find_digit_in(SelectShared& s, const unsigned in
   unsigned int mine = 0;
 #pragma unroll
   for (int j = 0; j < BPT; ++j) {
-    c[j] = in_smem ? counts[t * BPT + j] : __ldcg(&counts[t * BPT + j]);
+    c[j] = GLOBAL ? __ldcg(&counts[t * BPT + j]) : counts[t * BPT + j];
     mine += c[j];
   }
   // inclusive suffix sum over threads (higher thread = higher bins)
@@ -69,7 +64,7 @@ __device__ __forceinline__ void find_digit_in(SelectShared& s, const unsigned in
   }
   const int w = t >> 5;
   if (lane_id() == 0) s.warp_tot[w] = suf;
-  if (t == 0) { s.res_digit = 0u; s.res_krem = 0u; s.res_equal = 0u; }
+  if (t == 0) { s.res_digit = 0u; s.res_krem = 0u; }
   __syncthreads();
   unsigned int above_warps = 0, total = 0;
 #pragma unroll
@@ -87,7 +82,6 @@ __device__ __forceinline__ void find_digit_in(SelectShared& s, const unsigned in
       if (a < k_rem && k_rem <= a + c[j]) {
         s.res_digit = (unsigned int)(t * BPT + j);
         s.res_krem = k_rem - a;
-        s.res_equal = c[j];
       }
       a += c[j];
     }
@@ -95,84 +89,77 @@ __device__ __forceinline__ void find_digit_in(SelectShared& s, const unsigned in
   __syncthreads();
 }
 
-template <int NBINS>
-__device__ __forceinline__ void find_digit(SelectShared& s, const unsigned int* ghist,
-                                           unsigned int k_rem, bool local) {
-  find_digit_in<NBINS>(s, local ? s.hist : ghist, k_rem, local);
+// First selection level of a set whose k-th magnitude is expected at or a little above `lo`: bin 0 below lo,
+// bins of 2^kBandShift keys above it (together a quarter octave), the last bin open to the top.
+constexpr unsigned int kBandShift = 10u;
+__device__ __forceinline__ unsigned int band_bin(uint32_t key, uint32_t lo) {
+  if (key < lo) return 0u;
+  const unsigned int b = 1u + ((key - lo) >> kBandShift);
+  return b < (unsigned int)kHistBins ? b : (unsigned int)kHistBins - 1u;
 }
+constexpr unsigned int kBandList = kHistBins;  // entries of the threshold's bin that are looked at directly
 
-// Radix select of the k-th largest magnitude over `n` logical entries, where
-// key_at(i) returns the 31-bit magnitude key of entry i, or 0xffffffff for a dead
-// entry.  hist points to three zeroed global histograms [3][kHistBins].
-// have_pass0: hist[0] already holds the complete first-digit histogram of the
-// entries (an earlier phase built it), so the first sweep is skipped.
-// pre1 / pre1_lo / pre1_n: complete second-digit histograms (1024 bins each) of
-// the entries whose first digit is pre1_lo, pre1_lo + 1, ..., pre1_lo + pre1_n - 1;
-// if the threshold's first digit is one of them the second sweep is skipped too.
-// Returns false on abort.
-template <typename KeyAt>
-__device__ __forceinline__ bool radix_select_kth(SelectShared& s, RankBarrier& bar, unsigned int cta,
-                                                 unsigned int nctas, unsigned int n, unsigned int k,
-                                                 unsigned int (*hist)[kHistBins], KeyAt key_at,
-                                                 Threshold* out, uint32_t where,
-                                                 bool have_pass0 = false,
-                                                 unsigned int (*pre1)[kHistBins] = nullptr,
-                                                 unsigned int pre1_lo = 0u, unsigned int pre1_n = 0u) {
-  const unsigned int stride = nctas * kSelThreads;
+// The k-th largest magnitude of the entries that visit(f) calls f(key) for, each exactly once over all CTAs.
+// set: the rank's four zeroed global histogram rows for this selection, row 0 already holding the complete
+// counts of band_bin(key, lo).  list_n: a zeroed global word.  As a rule one sweep and one barrier: the entries of
+// the threshold's bin (a few hundred of 10^5) go into a list and every CTA counts their single keys.
+// When the prediction missed (bin 0 or the last one, or too many entries), three counting sweeps over bits
+// 30..20, 19..10 and 9..0.  Returns false on abort.
+template <typename Visit>
+__device__ __forceinline__ bool band_select_kth(SelectShared& s, RankBarrier& bar, unsigned int k, uint32_t lo,
+                                                unsigned int (*set)[kHistBins], unsigned int* list_n, Visit visit,
+                                                Threshold* out, uint32_t where) {
+  out->key = 0u;
+  out->quota = 0u;
+  find_digit_in<kHistBins>(s, set[0], k);
+  out->select_all = s.res_total <= k;  // not more live entries than k: keep them all
+  const unsigned int bin = s.res_digit;
+  unsigned int k_rem = s.res_krem;
+  __syncthreads();
+  if (out->select_all) return true;
+  if (bin != 0u && bin != (unsigned int)kHistBins - 1u) {
+    unsigned int* const list = set[1];
+    visit([&](uint32_t key) {
+      if (band_bin(key, lo) != bin) return;
+      const unsigned int at = atomicAdd(list_n, 1u);
+      if (at < kBandList) list[at] = key;
+    });
+    if (!bar.sync(where)) return false;
+    const unsigned int n = __ldcg(list_n);
+    if (n <= kBandList) {
+      constexpr uint32_t kWidth = 1u << kBandShift;
+      for (unsigned int i = threadIdx.x; i < kWidth; i += kSelThreads) s.hist[i] = 0u;
+      __syncthreads();
+      for (unsigned int i = threadIdx.x; i < n; i += kSelThreads)
+        atomicAdd(&s.hist[(__ldcg(&list[i]) - lo) & (kWidth - 1u)], 1u);
+      __syncthreads();
+      find_digit_in<(int)kWidth, false>(s, s.hist, k_rem);
+      out->key = lo + ((bin - 1u) << kBandShift) + s.res_digit;
+      out->quota = s.res_krem;
+      __syncthreads();
+      return true;
+    }
+  }
   uint32_t prefix = 0;
-  unsigned int k_rem = k;
-  const bool local = nctas == 1;
-  // pass 0: bits 30..20
-  if (!have_pass0) {
+  k_rem = k;
+  for (int pass = 0; pass < 3; ++pass) {
+    unsigned int* const ghist = pass == 0 ? set[2] : set[3] + (pass == 2 ? 1024 : 0);
+    const int shift = 20 - 10 * pass, nbins = pass == 0 ? kHistBins : 1024;
     smem_hist_clear(s);
-    for (unsigned int i = cta * kSelThreads + threadIdx.x; i < n; i += stride) {
-      const uint32_t key = key_at(i);
-      if (key != 0xffffffffu) atomicAdd(&s.hist[key >> 20], 1u);
-    }
-    if (!local) smem_hist_flush(s, hist[0], kHistBins);
-    if (!bar.sync(where + 0)) return false;
-  }
-  find_digit<kHistBins>(s, hist[0], k_rem, local && !have_pass0);
-  if (s.res_total <= k) {  // not more live entries than k: keep them all
-    out->key = 0u;
-    out->quota = 0u;
-    out->select_all = true;
+    visit([&](uint32_t key) {
+      if (pass == 0) atomicAdd(&s.hist[key >> 20], 1u);
+      else if ((key >> (shift + 10)) == prefix) atomicAdd(&s.hist[(key >> shift) & 1023u], 1u);
+    });
+    smem_hist_flush(s, ghist, nbins);
+    if (!bar.sync(where + 1 + pass)) return false;
+    if (pass == 0) find_digit_in<kHistBins>(s, ghist, k_rem);
+    else find_digit_in<1024>(s, ghist, k_rem);
+    prefix = pass == 0 ? s.res_digit : (prefix << 10) | s.res_digit;
+    k_rem = s.res_krem;
     __syncthreads();
-    return true;
   }
-  prefix = s.res_digit;
-  k_rem = s.res_krem;
-  __syncthreads();
-  // pass 1: bits 19..10
-  const unsigned int pre_off = prefix - pre1_lo;  // wraps when prefix < pre1_lo
-  if (pre1 != nullptr && pre_off < pre1_n) {
-    find_digit<1024>(s, pre1[pre_off], k_rem, false);  // built earlier: no sweep, no barrier
-  } else {
-    smem_hist_clear(s);
-    for (unsigned int i = cta * kSelThreads + threadIdx.x; i < n; i += stride) {
-      const uint32_t key = key_at(i);
-      if (key != 0xffffffffu && (key >> 20) == prefix) atomicAdd(&s.hist[(key >> 10) & 1023u], 1u);
-    }
-    if (!local) smem_hist_flush(s, hist[1], 1024);
-    if (!bar.sync(where + 1)) return false;
-    find_digit<1024>(s, hist[1], k_rem, local);
-  }
-  prefix = (prefix << 10) | s.res_digit;
-  k_rem = s.res_krem;
-  __syncthreads();
-  // pass 2: bits 9..0
-  smem_hist_clear(s);
-  for (unsigned int i = cta * kSelThreads + threadIdx.x; i < n; i += stride) {
-    const uint32_t key = key_at(i);
-    if (key != 0xffffffffu && (key >> 10) == prefix) atomicAdd(&s.hist[key & 1023u], 1u);
-  }
-  if (!local) smem_hist_flush(s, hist[2], 1024);
-  if (!bar.sync(where + 2)) return false;
-  find_digit<1024>(s, hist[2], k_rem, local);
-  out->key = (prefix << 10) | s.res_digit;
-  out->quota = s.res_krem;
-  out->select_all = false;
-  __syncthreads();
+  out->key = prefix;
+  out->quota = k_rem;
   return true;
 }
 

@@ -186,6 +186,7 @@ class ExchangeRank:
         self.result_words.zero_()
         self.result_host.zero_()
         self.ctrl.zero_()
+        self.region.tensor()[self.layout[3]:].zero_()   # flags and flagged entries that bear the failed call's number
 
     def last_ctrl(self) -> torch.Tensor:
         """Control block that the last completed gTop-k call used (synchronises)."""
@@ -216,18 +217,26 @@ def _desc_array(ranks: Sequence[ExchangeRank]) -> torch.Tensor:
     return torch.cat([r.desc for r in ranks])
 
 
+SMALL_MAX_K = 2048  # up to here the tree runs in one CTA with the set in shared memory (csrc/k2_tree_small.cu)
+
+
 def default_nctas(k: int, nranks: int = 1, sms: int = 148) -> int:
     """CTAs per rank for the exchange kernels, from sweeps on B200 (in-kernel
     time of one tree round + broadcast + put-back):
 
-    * up to 3 K union entries: one CTA (no inter-CTA barrier, histograms stay in
-      shared memory; about 10 us per round);
+    * up to 4 K union entries of the tree: one CTA, the set in shared memory
+      (whole call, two ranks: 10 us at k = 1 000 and 16 us at 2 000, against 23
+      and 25 us with a cluster; 26 against 25 us at 3 000);
     * up to 32 K union entries: a power-of-two cluster of 2..16 CTAs joined by
       the hardware cluster barrier, about 1024 entries per CTA (k = 4 000: 19 us
       against 25 us with the software barrier; k = 14 700: 23 us against 27 us);
     * above: one CTA per 768 entries (up to 128) with the software barrier
       (k = 25 600: 26 us with 64 CTAs against 33 us with a cluster of 16)."""
-    n_u = 2 * k
+    return 1 if k <= SMALL_MAX_K else _spread_nctas(2 * k, nranks, sms)
+
+
+def _spread_nctas(n_u: int, nranks: int, sms: int = 148) -> int:
+    """CTAs per rank for ``n_u`` entries shared out in global memory."""
     if n_u <= 3072:
         return 1
     if n_u <= 32768:
@@ -235,8 +244,7 @@ def default_nctas(k: int, nranks: int = 1, sms: int = 148) -> int:
         while n < 16 and n * 1024 < n_u:
             n *= 2
         return n
-    n = min(128, (n_u + 767) // 768)
-    return max(1, min(n, sms // max(nranks, 1)))
+    return max(1, min(128, (n_u + 767) // 768, sms // max(nranks, 1)))
 
 
 def launch_gtopk(ranks: Sequence[ExchangeRank], desc: torch.Tensor, rank_base: int, world: int, k: int,
@@ -261,9 +269,8 @@ def launch_allgather(ranks: Sequence[ExchangeRank], desc: torch.Tensor, seg_coun
     len(ranks) * 16 words receiving the per-source counts."""
     r0 = ranks[0]
     if nctas is None:
-        nctas = default_nctas(k * (world if reselect else 1) // 2 + 1, len(ranks))
-    ctrls = (C.c_void_p * len(ranks))(*[C.c_void_p(r.ctrl.data_ptr()) for r in ranks])
-    code = _lib.calls().gtk_k2t_allgather(desc.data_ptr(), C.addressof(ctrls), len(ranks), rank_base, world, k, r0.kcap,
+        nctas = _spread_nctas(k * (world if reselect else 1) + 2, len(ranks))
+    code = _lib.calls().gtk_k2t_allgather(desc.data_ptr(), len(ranks), rank_base, world, k, r0.kcap,
                                           r0.work_cap, r0.numel, int(reselect), seg_counts.data_ptr(), nctas,
                                           int(limit_ms * 1e6), current_stream_handle(r0.resid.device))
     if code:

@@ -490,3 +490,83 @@ def test_k1_pick_in_one_cta_a_cluster_and_by_tickets(d, k, off):
         assert sel.status() == (0, 0)
         _check_selection(*sel.pairs(), r, acc, k)
     assert sel.stats()["n_fallbacks"] < 4
+
+
+@pytest.mark.parametrize("P", [2, 8])
+@pytest.mark.parametrize("d,k", [(64, 1), (1500, 1024), (30_000, 1025), (3000, 2000), (400_000, 2048)])
+def test_k2_small_exchange_matches_oracle(P, d, k):
+    """One CTA per rank, set in shared memory, flags inside the data: k at the
+    edges of the CTA's 1024 threads, sets that overlap almost completely, scales
+    that put the threshold outside the predicted band, and the largest k."""
+    from gtopkssgd_b200.ops import exchange as ex
+    torch.manual_seed(7 * P + k)
+    ranks, desc = _emulated_world(P, d, k)
+    res_ref = [torch.zeros(d) for _ in range(P)]
+    for epoch, scales in enumerate(([1.0], [1.0, 1.0, 300.0, 1e-3], [1.0])):
+        grads = [torch.randn(d, device=DEV) * scales[r % len(scales)] for r in range(P)]
+        for r, g in zip(ranks, grads):
+            r.selector.select(g, r.resid, k)
+        ex.launch_gtopk(ranks, desc, 0, P, k, nctas=1, limit_ms=2000)
+        torch.cuda.synchronize()
+        assert all(r.status() == (0, 0) for r in ranks)
+        glob, _ = oracle.simulate_gtopk_step([g.cpu() for g in grads], res_ref, k)
+        ref = dict(zip(glob[0].tolist(), glob[1].tolist()))
+        for r in ranks:
+            gi, gv = _read_gout(r, r.last_parity())
+            got = dict(zip(gi.cpu().tolist(), gv.cpu().tolist()))
+            assert len(got) == gi.numel() and set(got) == set(ref), "rank %d epoch %d" % (r.rank, epoch)
+            for j in ref:
+                assert got[j] == pytest.approx(ref[j], rel=1e-5, abs=1e-9)
+            assert torch.allclose(r.resid.cpu(), res_ref[r.rank], rtol=1e-5, atol=1e-9)
+            assert r.region.guards_intact()
+
+
+def test_k2_small_bounded_wait_reports_timeout():
+    """The one-CTA form gives up like the other one when its partner never sends,
+    and works again after ``clear_failure``."""
+    from gtopkssgd_b200.ops import exchange as ex
+    d, k = 10000, 10
+    ranks, desc = _emulated_world(2, d, k)
+    ranks[0].selector.select(torch.randn(d, device=DEV), ranks[0].resid, k)
+    ex.launch_gtopk(ranks[:1], ranks[0].desc, 0, 2, k, nctas=1, limit_ms=50)
+    torch.cuda.synchronize()
+    status, where = ranks[0].status()
+    assert status == 1 and 210 <= where < 220
+    assert int(ranks[0].n_global.item()) == 0 and int(ranks[0].epoch.item()) == 1
+    ranks[0].clear_failure()
+    for r in ranks:
+        r.selector.select(torch.randn(d, device=DEV), r.resid, k)
+    ex.launch_gtopk(ranks, desc, 0, 2, k, nctas=1, limit_ms=2000)
+    torch.cuda.synchronize()
+    assert all(r.status() == (0, 0) for r in ranks) and int(ranks[1].n_global.item()) == k
+
+
+@pytest.mark.parametrize("P,d,k,nctas", [(2, 200_000, 3, 1), (5, 100_000, 4000, 3), (4, 3_000_000, 30_000, 16)])
+def test_k2t_reselect_in_and_outside_the_predicted_band(P, d, k, nctas):
+    """'topk2' with ranks of one scale (the threshold lies in the band above the
+    own k-th magnitude) and of very different scales (the counting sweeps), over
+    both control blocks."""
+    from gtopkssgd_b200.ops import exchange as ex
+    torch.manual_seed(P + k)
+    ranks, desc = _emulated_world(P, d, k, "topk2")
+    seg_counts = torch.zeros(P * ex.MAX_PEERS, dtype=torch.int32, device=DEV)
+    res_ref = [torch.zeros(d) for _ in range(P)]
+    for scales in ([1.0], [1.0], [1.0, 200.0, 1e-3], [1.0]):
+        grads = [torch.randn(d, device=DEV) * scales[r % len(scales)] for r in range(P)]
+        for r, g in zip(ranks, grads):
+            r.selector.select(g, r.resid, k)
+        ex.launch_allgather(ranks, desc, seg_counts, 0, P, k, reselect=True, nctas=nctas, limit_ms=2000)
+        torch.cuda.synchronize()
+        local = [oracle.compress(g.cpu(), rr, k) for g, rr in zip(grads, res_ref)]
+        gi_ref, gv_ref = oracle.topk2_reselect(local, k)
+        ref = dict(zip(gi_ref.tolist(), gv_ref.tolist()))
+        for rr, loc in zip(res_ref, local):
+            oracle.put_back(rr, loc, gi_ref)
+        for r in ranks:
+            assert r.status() == (0, 0)
+            gi, gv = _read_gout(r, r.last_parity())
+            got = dict(zip(gi.cpu().tolist(), gv.cpu().tolist()))
+            assert set(got) == set(ref)
+            for j in ref:
+                assert got[j] == pytest.approx(ref[j], rel=1e-5, abs=1e-6)
+            assert torch.allclose(r.resid.cpu(), res_ref[r.rank], rtol=1e-5, atol=1e-6)
