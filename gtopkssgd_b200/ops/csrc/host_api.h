@@ -40,6 +40,12 @@ typedef struct DeviceInfo {
   int cluster;
 } DeviceInfo;
 
+// A list of device addresses, in host memory.
+typedef struct gtk_addresses {
+  const unsigned long long* p;
+  unsigned int n;
+} gtk_addresses;
+
 const DeviceInfo* gtk_device_info(void);
 void gtk_count_launch(int n);
 long long gtk_launch_count(void);
@@ -52,6 +58,9 @@ const char* gtk_last_cuda_error(void);
 int gtk_k1_select(const float* g, float* r, const float* g_scale, long long d, unsigned int k,
                   void* cand, unsigned int cap, void* sel, void* state, void* ctrl,
                   float target_ratio, unsigned long long limit_ns, void* stream);
+int gtk_k1_select_segments(gtk_addresses grads, const unsigned int* segments, float* r, long long d, unsigned int k,
+                           void* cand, unsigned int cap, void* sel, void* state, void* ctrl, float target_ratio,
+                           unsigned long long limit_ns, void* stream);
 int gtk_k1_compress(float* g, float* r, long long d, unsigned int k, void* cand, unsigned int cap, void* sel,
                     void* state, void* ctrl, float target_ratio, unsigned long long limit_ns, long long* idx_out,
                     float* val_out, void* stream);

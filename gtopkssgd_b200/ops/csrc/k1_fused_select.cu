@@ -112,6 +112,47 @@ __device__ __forceinline__ void warp_flush(Pair* wbuf, unsigned int& wcnt, Pair*
   __syncwarp();
 }
 
+// Where the gradient of a float4 position comes from: one vector, or one tensor per parameter.
+struct FlatGrad {
+  float* g;        // behind the scalar head
+  __device__ __forceinline__ float4 vec(long long v) const { return __ldcs(reinterpret_cast<const float4*>(g) + v); }
+};
+// Segment s covers the float4 positions start[s] <= v < start[s + 1] of the flat layout (parameters begin at
+// multiples of four elements) and holds len[s] elements; g[s] is its gradient, nullptr for a parameter that got
+// none.  The segment is found by a search in shared memory that is the same for a whole warp (8 steps for 161
+// tensors, hidden behind the loads of r, which do not wait for it), then a lane moves on past what ends in between.
+template <int N>
+struct GradPointers {
+  const float* g[N];
+};
+struct SegmentedGrad {
+  const float* const* g;       // kernel parameters
+  const unsigned int* start;   // shared memory, n + 1 words
+  const unsigned int* len;     // shared memory
+  unsigned int n;
+  __device__ __forceinline__ float4 vec(long long v64) const {
+    const unsigned int v = (unsigned int)v64, row = v & ~31u;
+    unsigned int lo = 0, hi = n;
+    while (hi - lo > 1u) {
+      const unsigned int mid = (lo + hi) >> 1;
+      if (start[mid] <= row) lo = mid;
+      else hi = mid;
+    }
+    while (v >= start[lo + 1u]) ++lo;
+    const float* src = g[lo];
+    const unsigned int at = (v - start[lo]) * 4u, left = len[lo] - min(at, len[lo]);
+    float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (src == nullptr) return x;
+    src += at;
+    if (left >= 4u && (reinterpret_cast<uintptr_t>(src) & 15u) == 0u) return __ldcs(reinterpret_cast<const float4*>(src));
+    if (left > 0u) x.x = __ldcs(src);
+    if (left > 1u) x.y = __ldcs(src + 1);
+    if (left > 2u) x.z = __ldcs(src + 2);
+    if (left > 3u) x.w = __ldcs(src + 3);
+    return x;
+  }
+};
+
 // What a thread of the stream pass carries along.
 struct StreamCtx {
   float* r;
@@ -143,8 +184,8 @@ __device__ __forceinline__ void take_candidates(StreamShared& ss, StreamCtx& c, 
 
 // One tile of the stream pass: U float4 of g and of r per thread, STRIDE
 // float4 apart (the CTA's 512 threads or one warp's 32 lanes work side by side).
-template <int STRIDE, int U, bool HIST, bool ZERO>
-__device__ __forceinline__ void stream_tile(long long v0, long long nvec, long long head, float4* g4, float4* r4,
+template <int STRIDE, int U, bool HIST, bool ZERO, typename G>
+__device__ __forceinline__ void stream_tile(long long v0, long long nvec, long long head, const G& g, float4* r4,
                                             StreamShared& ss, StreamCtx& c) {
   // Candidates are decided on the bit pattern of |acc|, which orders like the magnitude for finite
   // values and puts +-Inf and NaN on top: a non-finite entry is a candidate on this path exactly as it
@@ -153,13 +194,12 @@ __device__ __forceinline__ void stream_tile(long long v0, long long nvec, long l
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const long long v = v0 + (long long)u * STRIDE;
-    if (v < nvec) {
-      gv[u] = __ldcs(&g4[v]);
-      rv[u] = r4[v];
-    } else {
-      gv[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-      rv[u] = gv[u];
-    }
+    rv[u] = v < nvec ? r4[v] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const long long v = v0 + (long long)u * STRIDE;
+    gv[u] = v < nvec ? g.vec(v) : make_float4(0.f, 0.f, 0.f, 0.f);
   }
 #pragma unroll
   for (int u = 0; u < U; ++u) {
@@ -180,7 +220,7 @@ __device__ __forceinline__ void stream_tile(long long v0, long long nvec, long l
       o.z = is[2] ? 0.f : a[2];
       o.w = is[3] ? 0.f : a[3];
       r4[v] = o;
-      if (ZERO) g4[v] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if constexpr (ZERO) reinterpret_cast<float4*>(g.g)[v] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (__any_sync(0xffffffffu, is[0] | is[1] | is[2] | is[3])) {
 #pragma unroll
@@ -190,15 +230,12 @@ __device__ __forceinline__ void stream_tile(long long v0, long long nvec, long l
 }
 
 // ZERO: g <- 0 on the way (a constant in a template, so that the training path has no store to g).
-template <bool HIST, bool DYNAMIC, bool ZERO>
-__global__ void __launch_bounds__(kK1Threads, 2)
-k1_stream(float* g, float* r, const float* g_scale, long long d, Pair* cand, unsigned int cap, K1State* st,
-          Ctrl* ctrl_pair) {
+// G: FlatGrad (its pointer still at the vector's beginning) or SegmentedGrad (r 16-byte aligned).
+template <bool HIST, bool DYNAMIC, bool ZERO, typename G>
+__device__ __forceinline__ void stream_pass(StreamShared& ss, G g, float* r, const float* g_scale, long long d, Pair* cand,
+                                            unsigned int cap, K1State* st, Ctrl* ctrl_pair) {
+  constexpr bool kFlat = std::is_same_v<G, FlatGrad>;
   constexpr int U = DYNAMIC ? 4 : 2;  // float4 loads of g and of r in flight per thread
-  __shared__ StreamShared ss;
-  if (HIST)
-    for (int i = threadIdx.x; i < kBins; i += kK1Threads) ss.hist[i] = 0u;
-  pdl_begin(g, r, g_scale, st, ctrl_pair);
   const unsigned int calls = st->n_calls;
   const float tau = st->tau;
   Ctrl* ctrl = ctrl_pair + (calls & 1u);
@@ -222,7 +259,7 @@ k1_stream(float* g, float* r, const float* g_scale, long long d, Pair* cand, uns
   if (head > d) head = d;
   const long long nvec = (d - head) >> 2;
   const long long tail0 = head + (nvec << 2);
-  float4* g4 = reinterpret_cast<float4*>(g + head);
+  if constexpr (kFlat) g.g += head;
   float4* r4 = reinterpret_cast<float4*>(r + head);
 
   if (!DYNAMIC) {
@@ -232,7 +269,7 @@ k1_stream(float* g, float* r, const float* g_scale, long long d, Pair* cand, uns
     constexpr long long kTileVec = (long long)kK1Threads * U;
     const long long ntiles = (nvec + kTileVec - 1) / kTileVec;
     for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-      stream_tile<kK1Threads, U, HIST, ZERO>(tile * kTileVec + threadIdx.x, nvec, head, g4, r4, ss, c);
+      stream_tile<kK1Threads, U, HIST, ZERO>(tile * kTileVec + threadIdx.x, nvec, head, g, r4, ss, c);
   } else {
     // Large vectors: SMs do not all see the same memory bandwidth, and with the static split the slowest
     // CTA ended up to 13 us (d = 64 M) after the first.  Here work is handed out per warp in tiles of 32 lanes
@@ -250,7 +287,7 @@ k1_stream(float* g, float* r, const float* g_scale, long long d, Pair* cand, uns
     for (long long tile = warp; tile < ntiles; tile = turn * kShards + shard) {
       unsigned int nxt = 0;
       if (lane_id() == 0) nxt = atomicAdd(ticket, 1u);  // consumed after this tile
-      stream_tile<32, U, HIST, ZERO>(tile * kWarpTileVec + lane_id(), nvec, head, g4, r4, ss, c);
+      stream_tile<32, U, HIST, ZERO>(tile * kWarpTileVec + lane_id(), nvec, head, g, r4, ss, c);
       turn = (long long)warps + __shfl_sync(0xffffffffu, nxt, 0);
     }
   }
@@ -263,10 +300,17 @@ k1_stream(float* g, float* r, const float* g_scale, long long d, Pair* cand, uns
     const long long j = lane_id();
     if (j < nscalar) {
       i = j < head ? j : tail0 + (j - head);
-      a = fmaf(g[i], c.scale, r[i]);
+      float gi;
+      if constexpr (kFlat) {
+        gi = g.g[i - head];
+      } else {  // (head is 0) the last float4 position, of which only some elements exist
+        const float4 x = g.vec(i >> 2);
+        gi = (i & 3) == 0 ? x.x : (i & 3) == 1 ? x.y : x.z;
+      }
+      a = fmaf(gi, c.scale, r[i]);
       is = mag_key(a) >= c.tau_key;
       r[i] = is ? 0.f : a;
-      if (ZERO) g[i] = 0.f;
+      if constexpr (ZERO) g.g[i - head] = 0.f;
     }
     take_candidates<HIST>(ss, c, is, i, a);
   }
@@ -301,6 +345,33 @@ k1_stream(float* g, float* r, const float* g_scale, long long d, Pair* cand, uns
     }
   }
   trace_stamp(ctrl, 1);  // CTA 0 finished its share
+}
+
+template <bool HIST, bool DYNAMIC, bool ZERO>
+__global__ void __launch_bounds__(kK1Threads, 2)
+k1_stream(float* g, float* r, const float* g_scale, long long d, Pair* cand, unsigned int cap, K1State* st,
+          Ctrl* ctrl_pair) {
+  __shared__ StreamShared ss;
+  if (HIST)
+    for (int i = threadIdx.x; i < kBins; i += kK1Threads) ss.hist[i] = 0u;
+  pdl_begin(g, r, g_scale, st, ctrl_pair);
+  stream_pass<HIST, DYNAMIC, ZERO>(ss, FlatGrad{g}, r, g_scale, d, cand, cap, st, ctrl_pair);
+}
+
+// segments: n + 1 start positions, then n lengths (written once at set-up, so they are read ahead of the wait).
+template <bool HIST, bool DYNAMIC, int N>
+__global__ void __launch_bounds__(kK1Threads, 2)
+k1_stream_segments(const __grid_constant__ GradPointers<N> g, const unsigned int* segments, unsigned int n, float* r,
+                   long long d, Pair* cand, unsigned int cap, K1State* st, Ctrl* ctrl_pair) {
+  __shared__ StreamShared ss;
+  __shared__ unsigned int seg[2 * N + 1];
+  if (HIST)
+    for (int i = threadIdx.x; i < kBins; i += kK1Threads) ss.hist[i] = 0u;
+  for (unsigned int i = threadIdx.x; i < 2u * n + 1u; i += kK1Threads) seg[i] = segments[i];
+  __syncthreads();
+  pdl_begin(r, st, ctrl_pair);
+  const float* no_scale = nullptr;
+  stream_pass<HIST, DYNAMIC, false>(ss, SegmentedGrad{g.g, seg, seg + n + 1, n}, r, no_scale, d, cand, cap, st, ctrl_pair);
 }
 
 // ---------------------------------------------------------------------------
@@ -798,10 +869,10 @@ using namespace gtk;
 extern "C" unsigned long long gtk_ctrl_bytes(void) { return sizeof(Ctrl); }
 
 namespace {
-// out.dense: g itself (then it is left sparsified) or nullptr (then g is only read).
-int k1_launch(const float* g_in, float* r, const float* g_scale, long long d, unsigned int k,
-              Pair* cand, unsigned int cap, Winners out, K1State* st, Ctrl* ctrl_pair,
-              float target_ratio, unsigned long long limit_ns, cudaStream_t stream) {
+// Launches the two kernels; `stream_pass(counted, dynamic, grid)` launches the first.
+template <typename Stream>
+int k1_launch_with(Stream stream_pass, float* r, long long d, unsigned int k, Pair* cand, unsigned int cap, Winners out,
+                   K1State* st, Ctrl* ctrl_pair, float target_ratio, unsigned long long limit_ns, cudaStream_t stream) {
   const DeviceInfo* di = gtk_device_info();
   if (!di) return GTK_ERR_CUDA;
   // Two float4 of each array per thread and tile in the static split (four: 2 % slower, a coarser last round),
@@ -814,24 +885,49 @@ int k1_launch(const float* g_in, float* r, const float* g_scale, long long d, un
   grid = grid < 1 ? 1 : (grid > full ? full : grid);
   // The first level is counted on the fly where the candidates will be shared out by tickets; below, the CTAs
   // that pick count faster than the stream pass publishes.
-  const int counted = k > kPickCluster / 2 ? 1 : 0;
-  float* g = const_cast<float*>(g_in);
-  auto stream_pass = [&](auto zero) {
-    constexpr bool Z = decltype(zero)::value;
-    auto fn = dynamic ? (counted ? k1_stream<true, true, Z> : k1_stream<false, true, Z>)
-                      : (counted ? k1_stream<true, false, Z> : k1_stream<false, false, Z>);
-    return launch_pdl(fn, (int)grid, kK1Threads, stream, g, r, g_scale, d, cand, cap, st, ctrl_pair);
-  };
-  cudaError_t e = out.dense ? stream_pass(std::true_type{}) : stream_pass(std::false_type{});
+  const bool counted = k > kPickCluster / 2;
+  cudaError_t e = stream_pass(counted, dynamic, (int)grid);
   if (e != cudaSuccess) return GTK_ERR_CUDA;
   // k1_pick: as many clusters as exact mode can use
   long long pick = (d + kExactChunk - 1) / kExactChunk;
   if (pick > di->sms) pick = di->sms;
   pick = (pick + kPickCtas - 1) / kPickCtas * kPickCtas;
-  e = launch_pdl(k1_pick, (int)pick, kPickThreads, stream, r, d, cand, cap, out, k, st, ctrl_pair, counted, target_ratio,
-                 limit_ns);
+  e = launch_pdl(k1_pick, (int)pick, kPickThreads, stream, r, d, cand, cap, out, k, st, ctrl_pair, counted ? 1 : 0,
+                 target_ratio, limit_ns);
   gtk_count_launch(2);
   return e == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
+}
+
+// out.dense: g itself (then it is left sparsified) or nullptr (then g is only read).
+int k1_launch(const float* g_in, float* r, const float* g_scale, long long d, unsigned int k,
+              Pair* cand, unsigned int cap, Winners out, K1State* st, Ctrl* ctrl_pair,
+              float target_ratio, unsigned long long limit_ns, cudaStream_t stream) {
+  float* g = const_cast<float*>(g_in);
+  auto stream_pass = [&](bool counted, bool dynamic, int grid) {
+    auto go = [&](auto zero) {
+      constexpr bool Z = decltype(zero)::value;
+      auto fn = dynamic ? (counted ? k1_stream<true, true, Z> : k1_stream<false, true, Z>)
+                        : (counted ? k1_stream<true, false, Z> : k1_stream<false, false, Z>);
+      return launch_pdl(fn, grid, kK1Threads, stream, g, r, g_scale, d, cand, cap, st, ctrl_pair);
+    };
+    return out.dense ? go(std::true_type{}) : go(std::false_type{});
+  };
+  return k1_launch_with(stream_pass, r, d, k, cand, cap, out, st, ctrl_pair, target_ratio, limit_ns, stream);
+}
+
+template <int N>
+int k1_launch_segments(const unsigned long long* grads, unsigned int n, const unsigned int* segments, float* r, long long d,
+                       unsigned int k, Pair* cand, unsigned int cap, Pair* sel, K1State* st, Ctrl* ctrl_pair,
+                       float target_ratio, unsigned long long limit_ns, cudaStream_t stream) {
+  GradPointers<N> g;
+  for (unsigned int i = 0; i < n; ++i) g.g[i] = reinterpret_cast<const float*>(static_cast<uintptr_t>(grads[i]));
+  auto stream_pass = [&](bool counted, bool dynamic, int grid) {
+    auto fn = dynamic ? (counted ? k1_stream_segments<true, true, N> : k1_stream_segments<false, true, N>)
+                      : (counted ? k1_stream_segments<true, false, N> : k1_stream_segments<false, false, N>);
+    return launch_pdl(fn, grid, kK1Threads, stream, g, segments, n, r, d, cand, cap, st, ctrl_pair);
+  };
+  return k1_launch_with(stream_pass, r, d, k, cand, cap, Winners{sel, nullptr, nullptr, nullptr}, st, ctrl_pair, target_ratio,
+                        limit_ns, stream);
 }
 }  // namespace
 
@@ -850,6 +946,25 @@ extern "C" int gtk_k1_select(const float* g, float* r, const float* g_scale, lon
   if (!k1_args_ok(g, r, d, k, cap)) return GTK_ERR_ARG;
   return k1_launch(g, r, g_scale, d, k, (Pair*)cand, cap, Winners{(Pair*)sel, nullptr, nullptr, nullptr}, (K1State*)state,
                    (Ctrl*)ctrl, target_ratio, limit_ns, (cudaStream_t)stream_);
+}
+
+// The select with the gradient in n tensors instead of one vector: grads[s] (device address, 0: no gradient) belongs
+// to the elements that segments (device memory: n + 1 start positions in float4, ascending from 0, the last one
+// ceil(d / 4); n lengths in elements) gives segment s.  r must be 16-byte aligned, n at most 1024.
+extern "C" int gtk_k1_select_segments(gtk_addresses grads, const unsigned int* segments, float* r, long long d,
+                                      unsigned int k, void* cand, unsigned int cap, void* sel, void* state, void* ctrl,
+                                      float target_ratio, unsigned long long limit_ns, void* stream_) {
+  if (!k1_args_ok(r, r, d, k, cap) || (reinterpret_cast<uintptr_t>(r) & 15u) || grads.n == 0) return GTK_ERR_ARG;
+  auto go = [&](auto n) {
+    return k1_launch_segments<decltype(n)::value>(grads.p, grads.n, segments, r, d, k, (Pair*)cand, cap, (Pair*)sel,
+                                                  (K1State*)state, (Ctrl*)ctrl, target_ratio, limit_ns,
+                                                  (cudaStream_t)stream_);
+  };
+  // (the pointers are kernel parameters, so that a captured launch carries them)
+  if (grads.n <= 64) return go(std::integral_constant<int, 64>{});
+  if (grads.n <= 256) return go(std::integral_constant<int, 256>{});
+  if (grads.n <= 1024) return go(std::integral_constant<int, 1024>{});
+  return GTK_ERR_ARG;
 }
 
 // The select, with g left sparsified (selected entries keep g + r, all others are 0) and the selection also

@@ -10,13 +10,24 @@
 #include <Python.h>
 #include <type_traits>
 #include <utility>
+#include <vector>
 #include "host_api.h"
 
 namespace {
 
 template <typename T>
 inline T convert(PyObject* o) {
-  if constexpr (std::is_pointer_v<T>) {
+  if constexpr (std::is_same_v<T, gtk_addresses>) {  // a list of int
+    static thread_local std::vector<unsigned long long> words;
+    if (!PyList_Check(o)) {
+      PyErr_SetString(PyExc_TypeError, "expected a list of addresses");
+      return gtk_addresses{nullptr, 0};
+    }
+    const Py_ssize_t n = PyList_GET_SIZE(o);
+    words.resize(n);
+    for (Py_ssize_t i = 0; i < n; ++i) words[i] = PyLong_AsUnsignedLongLong(PyList_GET_ITEM(o, i));
+    return gtk_addresses{words.data(), static_cast<unsigned int>(n)};
+  } else if constexpr (std::is_pointer_v<T>) {
     if (o == Py_None) return nullptr;
     return reinterpret_cast<T>(static_cast<uintptr_t>(PyLong_AsUnsignedLongLong(o)));
   } else if constexpr (std::is_floating_point_v<T>) {
@@ -62,7 +73,8 @@ struct Call<F> {
   {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&Call<name>::fast)), METH_FASTCALL, nullptr}
 
 PyMethodDef kMethods[] = {
-    GTK_METHOD(gtk_k1_select),        GTK_METHOD(gtk_k1_compress),    GTK_METHOD(gtk_k2_exchange),    GTK_METHOD(gtk_k2t_allgather),
+    GTK_METHOD(gtk_k1_select),        GTK_METHOD(gtk_k1_select_segments),
+    GTK_METHOD(gtk_k1_compress),      GTK_METHOD(gtk_k2_exchange),      GTK_METHOD(gtk_k2t_allgather),
     GTK_METHOD(gtk_k3_dense),         GTK_METHOD(gtk_k3_sparse),      GTK_METHOD(gtk_k3_scatter_dense),
     GTK_METHOD(gtk_k3_momentum_correct), GTK_METHOD(gtk_k4_sumsq_dense), GTK_METHOD(gtk_k4_sumsq_pairs),
     GTK_METHOD(gtk_k4_finalize),      {nullptr, nullptr, 0, nullptr}};

@@ -8,7 +8,7 @@ tensors it runs the PyTorch oracle instead, with the same outputs.
 from __future__ import annotations
 
 import math
-from typing import Optional, Tuple
+from typing import Optional, Sequence, Tuple
 
 import torch
 
@@ -58,6 +58,7 @@ class TopkSelector:
             self.ctrl_words = int(L.gtk_ctrl_bytes()) // 4
             self.ctrl = torch.zeros(2 * self.ctrl_words, dtype=torch.int32, device=self.device)
             self._select = _lib.calls().gtk_k1_select
+            self._select_segments = _lib.calls().gtk_k1_select_segments
             self._buffers = (self.cand.data_ptr(), self.cap, self.sel.data_ptr(), self.state.data_ptr(),
                              self.ctrl.data_ptr(), self.target_ratio, self.limit_ns)
         self.last_k = 0
@@ -129,6 +130,19 @@ class TopkSelector:
         if code:
             _lib.check(code, "gtk_k1_select")
 
+    def select_segments(self, addresses: Sequence[int], segments: torch.Tensor, r: torch.Tensor, k: int) -> None:
+        """``select`` (CUDA only) with the gradient in one tensor per parameter:
+        ``addresses`` are their device addresses (0: no gradient), ``segments`` an
+        int32 device tensor with the n + 1 start positions in float4 and the n
+        lengths in elements (see ``segment_table``)."""
+        assert r.numel() == self.numel and r.dtype == torch.float32
+        k = int(min(k, self.max_k))
+        self.last_k = k
+        code = self._select_segments(addresses, segments.data_ptr(), r.data_ptr(), self.numel, k, *self._buffers,
+                                     current_stream_handle(self.device))
+        if code:
+            _lib.check(code, "gtk_k1_select_segments")
+
     def compress(self, g: torch.Tensor, r: torch.Tensor, k: int) -> Tuple[torch.Tensor, torch.Tensor]:
         """``select`` that also leaves g sparsified (acc on the selection, 0 off
         it) and returns the selection as (int64 indices, fp32 values).  Nothing
@@ -150,6 +164,18 @@ class TopkSelector:
         n = int(self.state[1].item())
         p = self.sel[:n]
         return p[:, 0].to(torch.int64), p[:, 1].contiguous().view(torch.float32)
+
+
+MAX_SEGMENTS = 1024  # gradient tensors that one select can take
+
+
+def segment_table(offsets: Sequence[int], sizes: Sequence[int], numel: int, device: torch.device) -> torch.Tensor:
+    """The table that ``TopkSelector.select_segments`` reads, for parameters at
+    ``offsets`` (multiples of 4, without gaps of a whole float4) of a flat
+    vector of ``numel`` elements."""
+    assert all(o % 4 == 0 for o in offsets)
+    starts = [o // 4 for o in offsets] + [(numel + 3) // 4]
+    return torch.tensor(starts + list(sizes), dtype=torch.int32, device=device)
 
 
 def pairs_to_tensors(pairs: torch.Tensor, n: int) -> Tuple[torch.Tensor, torch.Tensor]:

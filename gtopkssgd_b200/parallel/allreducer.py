@@ -29,7 +29,7 @@ from .. import settings
 from ..ops import exchange as ex
 from ..ops import oracle
 from ..ops.clip import ClipNorm
-from ..ops.select import TopkSelector, pairs_to_tensors, tensors_to_pairs
+from ..ops.select import MAX_SEGMENTS, TopkSelector, pairs_to_tensors, segment_table, tensors_to_pairs
 from ..settings import logger
 from ..utils.timing import PhaseTimers
 from . import comm, fallback
@@ -82,7 +82,7 @@ class GroupEngine:
     def __init__(self, owner: "AllReducer", g: MergedGroup):
         self.owner, self.g = owner, g
         fb = owner.flat
-        self.grad = fb.group_slice(fb.grad, g)
+        self.attached_grad = fb.group_slice(fb.grad, g)   # the group's slice of the flat gradient buffer
         self.resid = fb.group_slice(fb.residual, g) if fb.residual is not None else None
         self.numel = g.numel                # span in the flat buffers: what the kernels run over
         self.param_numel = g.param_numel    # number of parameters: what the density applies to
@@ -102,6 +102,9 @@ class GroupEngine:
         dens = max(owner.densities()) if owner.densities() else owner._density
         self.max_k = oracle.num_selected(self.param_numel, dens)
         self.selector = TopkSelector(self.numel, self.max_k, dev, limit_ms=owner.wait_limit_ms)
+        self.segments = None
+        if self.is_cuda and len(g.names) <= MAX_SEGMENTS:
+            self.segments = segment_table(g.offsets, [fb.slots[n].numel for n in g.names], self.numel, dev)
         self.rank_ctx = None
         world = owner.size()
         # CUDA ranks that cannot reach each other's memory (several hosts, no peer access) stage their
@@ -121,9 +124,17 @@ class GroupEngine:
             self.host_pairs = torch.zeros((cap, 2), dtype=torch.int32, device=dev)
             self.host_counts = torch.zeros(ex.MAX_PEERS, dtype=torch.int32, device=dev)
 
+    @property
+    def grad(self) -> torch.Tensor:
+        """The group's gradient as one vector (filled first if the gradients are detached)."""
+        self.owner.flat.grad
+        return self.attached_grad
+
     # ------------------------------------------------------------------
-    def reduce(self, density: float, g_scale: Optional[torch.Tensor]) -> None:
-        """Enqueue select + exchange for this group on the current stream."""
+    def reduce(self, density: float, g_scale: Optional[torch.Tensor], detached: Optional[List[int]] = None) -> None:
+        """Enqueue select + exchange for this group on the current stream.
+        ``detached``: addresses of the group's gradients where they are not in
+        the flat buffer."""
         o = self.owner
         world, mode = o.size(), o.mode
         k = oracle.num_selected(self.param_numel, density)
@@ -131,7 +142,10 @@ class GroupEngine:
         self.last_k = k
         t = o.timers
         t.start(self.g.key, "compression")
-        self.selector.select(self.grad, self.resid, k, g_scale=g_scale)
+        if detached is not None:
+            self.selector.select_segments(detached, self.segments, self.resid, k)
+        else:
+            self.selector.select(self.grad, self.resid, k, g_scale=g_scale)
         if self.is_cuda and o.concurrent:
             # the dense part of the update streams the same HBM as the select: it is ordered behind this
             # event, so the select has the bandwidth to itself and the dense part overlaps the exchange
@@ -312,9 +326,15 @@ class AllReducer:
         return 3.0
 
     # -- reduction -----------------------------------------------------------
-    def reduce_group(self, gi: int) -> None:
+    def takes_detached(self) -> bool:
+        """Whether a group's reduction can read the gradients where backward left
+        them: the sparse modes on a GPU, nothing in between that needs the vector."""
+        return (self.mode != "none" and self._norm_clip is None and not settings.PROFILING_NORM
+                and len(self.engines) == 1 and self.engines[0].segments is not None)
+
+    def reduce_group(self, gi: int, detached: Optional[List[int]] = None) -> None:
         """Enqueue the reduction of group ``gi`` on the current CUDA stream (or
-        run it now on CPU)."""
+        run it now on CPU).  ``detached``: see ``GroupEngine.reduce``."""
         eng = self.engines[gi]
         key = eng.g.key
         if self.mode == "none":
@@ -331,7 +351,7 @@ class AllReducer:
         if self._norm_clip is not None:
             self.clip.add_dense(eng.grad)
             g_scale = self.clip.finalize(float(np.sqrt(1.0 / self.size()) * self._norm_clip))
-        eng.reduce(self.get_current_density(), g_scale)
+        eng.reduce(self.get_current_density(), g_scale, detached)
         if settings.PROFILING_NORM:
             self._profiling_after(eng, dense_ref)
         self.allreduce_count += 1

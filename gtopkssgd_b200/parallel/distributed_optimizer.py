@@ -180,7 +180,13 @@ class _DistributedOptimizer(torch.optim.Optimizer):
 
     def _launch_group(self, gi: int) -> None:
         self._launched[gi] = True
-        if not self._hooked and not self._flat.grads_attached():
+        detached = None
+        if self._flat.detached:
+            if self._allreducer.takes_detached() and not self.momentum_correction:
+                detached = self._flat.grad_addresses()
+            if detached is None:
+                self._flat.attach()
+        elif not self._hooked and not self._flat.grads_attached():
             self._flat.ensure_views()
         if self._overlap:
             ev = self._ready[gi]
@@ -189,11 +195,11 @@ class _DistributedOptimizer(torch.optim.Optimizer):
             with torch.cuda.stream(self._comm_stream):
                 if self.momentum_correction:
                     self._apply_momentum_correction(gi)
-                self._allreducer.reduce_group(gi)
+                self._allreducer.reduce_group(gi, detached)
         else:
             if self.momentum_correction:
                 self._apply_momentum_correction(gi)
-            self._allreducer.reduce_group(gi)
+            self._allreducer.reduce_group(gi, detached)
 
     # -- public API ---------------------------------------------------------------
     def pre_iteration(self) -> None:
@@ -297,6 +303,18 @@ class _DistributedOptimizer(torch.optim.Optimizer):
         self._flat.zero_grad()
         self._materialized = False
 
+    def begin_iteration(self):
+        """``zero_grad()`` for an iteration that the framework runs up to and
+        including ``step()``: where the reduction allows it, ``p.grad`` is None
+        until backward has produced it and is the tensor that backward computed
+        afterwards, not a view of the flat buffer."""
+        if self._hooked or self.local or self.momentum_correction or not self._allreducer.takes_detached():
+            self.zero_grad()
+            return
+        self.pre_iteration()
+        self._flat.begin_detached()
+        self._materialized = False
+
     def synchronize(self, materialize: bool = False):
         """Wait (on the stream, not on the host) until every group of this
         iteration has been reduced.  With ``materialize=True`` the dense
@@ -310,6 +328,7 @@ class _DistributedOptimizer(torch.optim.Optimizer):
                 torch.cuda.current_stream().wait_stream(self._comm_stream)
             self._synced = True
         if materialize and not self._materialized and self._allreducer.mode != "none":
+            self._flat.attach(keep=False)
             for eng in self._allreducer.engines:
                 r = eng.result
                 scatter_dense(eng.grad, r.pairs, r.counts, r.nseg, r.seg_stride, r.scale, r.use_atomics,

@@ -633,7 +633,7 @@ class DLTrainer:
     def _train_step(self, data, hidden, clip_norm, cuda_graph):
         use_graph = self.use_cuda_graph if cuda_graph is None else cuda_graph
         if not (use_graph and self.is_cuda and self.dnn != "lstman4"):
-            self.optimizer.zero_grad()
+            getattr(self.optimizer, "begin_iteration", self.optimizer.zero_grad)()
             if self.dnn == "lstm":
                 _, hidden = self.train(1, data=data, hidden=hidden)
             else:

@@ -37,7 +37,7 @@ class GraphedStep:
     def _iteration(self, x, y, hidden):
         t = self.t
         opt = t.optimizer
-        opt.zero_grad()
+        getattr(opt, "begin_iteration", opt.zero_grad)()
         if t.dnn == "lstm":
             outputs, hidden = t.net(x, hidden)
             loss = t.criterion(outputs.view(-1, t.net.vocab_size), y.reshape(-1))
@@ -91,6 +91,9 @@ class GraphedStep:
         finally:
             if hasattr(opt, "capturing"):
                 opt.capturing = False
+        flat = getattr(opt, "_flat", None)
+        # the graph's own gradients, refilled by every replay
+        st["grads"] = flat.current_grads() if flat is not None and flat.detached else None
         st["native_launches"] = _native.launch_count() - before  # kernels of the native library inside the graph
         _native.add_launches(-st["native_launches"])              # capture enqueued nothing yet
         if self.pool is None:
@@ -139,6 +142,8 @@ class GraphedStep:
         if hasattr(opt, "sync_lr"):
             opt.sync_lr()
         g.replay()
+        if st["grads"] is not None:
+            opt._flat.use_grads_of(st["grads"])
         if hasattr(opt, "post_iteration"):
             opt.post_iteration()
         _native.add_launches(st["native_launches"])

@@ -570,3 +570,32 @@ def test_k2t_reselect_in_and_outside_the_predicted_band(P, d, k, nctas):
             for j in ref:
                 assert got[j] == pytest.approx(ref[j], rel=1e-5, abs=1e-6)
             assert torch.allclose(r.resid.cpu(), res_ref[r.rank], rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("sizes,k", [([5], 2), ([1, 2, 3, 4, 5, 130], 9), ([64] * 300, 100), ([100_003, 7, 1_000_001, 10, 999], 1000),
+                                     ([20_000_001, 3, 4_000_000], 20_000)])
+def test_k1_select_reads_one_tensor_per_parameter(sizes, k):
+    """The gradient in one tensor per parameter, some of them at odd addresses
+    and one missing, equals the same select over one vector; static and dynamic
+    stream pass, tails of 1 to 3 elements, segments shorter than a warp's row."""
+    from gtopkssgd_b200.ops.select import segment_table
+    torch.manual_seed(sum(sizes))
+    offsets, at = [], 0
+    for n in sizes:
+        offsets.append(at)
+        at = (at + n + 3) // 4 * 4
+    d = offsets[-1] + sizes[-1]
+    sel = _selector(d, k)
+    table = segment_table(offsets, sizes, d, DEV)
+    r = torch.zeros(d, device=DEV)
+    for it in range(3):
+        grads = [torch.randn(n + 1, device=DEV)[i % 2:][:n] for i, n in enumerate(sizes)]
+        missing = 1 if len(sizes) > 1 and it == 2 else -1
+        g = torch.zeros(d, device=DEV)
+        for i, (o, t) in enumerate(zip(offsets, grads)):
+            if i != missing:
+                g[o:o + t.numel()] = t
+        acc = g + r
+        sel.select_segments([0 if i == missing else t.data_ptr() for i, t in enumerate(grads)], table, r, k)
+        assert sel.status() == (0, 0)
+        _check_selection(*sel.pairs(), r, acc, k)

@@ -160,6 +160,45 @@ def test_two_gpu_cuda_graph_step_matches_oracle(compressor, graphs):
     replay_and_check(traces, 0.001, compressor, rtol=1e-4, atol=1e-5)
 
 
+@pytest.mark.parametrize("graph", [False, True])
+def test_train_step_leaves_backwards_own_gradients(graph):
+    """An iteration that the trainer runs takes the gradients where backward left
+    them; ``zero_grad`` and the flat gradient buffer work as before around it."""
+    from gtopkssgd_b200 import settings
+    from gtopkssgd_b200.parallel.compression import compressors
+    from gtopkssgd_b200.parallel.distributed_optimizer import DistributedOptimizer
+    from gtopkssgd_b200.trainer.dl_trainer import DLTrainer
+    settings.PIN_DENSITY = True
+    torch.manual_seed(0)
+    dev = torch.device("cuda", 0)
+    t = DLTrainer(0, 1, dist=False, ngpus=1, batch_size=8, data_dir="synthetic", dataset="cifar10", dnn="resnet20", lr=0.1,
+                  nworkers=1, device=dev, synthetic_train_size=640, cuda_graph=graph)
+    opt = DistributedOptimizer(t.optimizer, t.net.named_parameters(), compression=compressors["gtopk"], is_sparse=True,
+                               density=0.01)
+    t.update_optimizer(opt)
+    fb = opt._flat
+    batch = (torch.randn(8, 3, 32, 32, device=dev), torch.randint(0, 10, (8,), device=dev))
+    for it in range(6):
+        before = fb.residual.clone()
+        t.train_step(data=batch)
+        assert not fb.grads_attached()
+        want = torch.cat([p.grad.flatten() for p in (s.param for s in fb.slots.values())])
+        got = torch.cat([fb.grad[s.offset:s.offset + s.numel] for s in fb.slots.values()])
+        assert torch.equal(want, got)
+        idx, val = opt._allreducer.engines[0].selector.pairs()
+        acc = (fb.grad + before)[:fb.numel]
+        assert torch.equal(val, acc[idx])
+        acc[idx] = 0.0
+        assert torch.equal(fb.residual[:fb.numel], acc)
+    opt.zero_grad()
+    assert fb.grads_attached() and float(fb.grad.abs().sum()) == 0.0
+    t.criterion(t.net(batch[0]), batch[1]).backward()   # an iteration of the user's own
+    assert fb.grads_attached() and float(fb.grad.abs().sum()) > 0.0
+    opt.step()
+    opt.check_status()
+    opt.stop()
+
+
 def test_graft_smoke():
     import __graft_entry__ as g
     g.smoke()
