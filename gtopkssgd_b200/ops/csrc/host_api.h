@@ -86,6 +86,8 @@ int gtk_k4_sumsq_dense(const float* x, long long d, void* state, void* stream);
 int gtk_k4_sumsq_pairs(const void* pairs, const unsigned int* counts, unsigned int nseg, unsigned int seg_stride,
                        void* state, const unsigned int* parity_word, unsigned int parity_stride, void* stream);
 int gtk_k4_finalize(void* state, float scale, float max_norm, float* coef_out, void* stream);
+int gtk_k5_top1(const float* logits, const long long* target, int rows, int classes, float scale, float* out,
+                void* stream);
 
 #ifdef __cplusplus
 }

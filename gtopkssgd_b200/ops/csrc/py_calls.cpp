@@ -77,7 +77,7 @@ PyMethodDef kMethods[] = {
     GTK_METHOD(gtk_k1_compress),      GTK_METHOD(gtk_k2_exchange),      GTK_METHOD(gtk_k2t_allgather),
     GTK_METHOD(gtk_k3_dense),         GTK_METHOD(gtk_k3_sparse),      GTK_METHOD(gtk_k3_scatter_dense),
     GTK_METHOD(gtk_k3_momentum_correct), GTK_METHOD(gtk_k4_sumsq_dense), GTK_METHOD(gtk_k4_sumsq_pairs),
-    GTK_METHOD(gtk_k4_finalize),      {nullptr, nullptr, 0, nullptr}};
+    GTK_METHOD(gtk_k4_finalize),      GTK_METHOD(gtk_k5_top1),          {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_gtk_calls", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 

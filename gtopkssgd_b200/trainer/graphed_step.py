@@ -42,7 +42,7 @@ class GraphedStep:
             outputs, hidden = t.net(x, hidden)
             loss = t.criterion(outputs.view(-1, t.net.vocab_size), y.reshape(-1))
         else:
-            outputs = t.net(x)
+            outputs = t.forward(x)
             loss = t.criterion(outputs, y)
         loss.backward()
         if self.clip_norm is not None and hasattr(opt, "clip_grad_norm"):

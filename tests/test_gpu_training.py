@@ -266,3 +266,32 @@ def test_two_gpu_planned_departure(leaver):
     assert [h[1] for h in o["hist"]] == [2] * at + [1] * (total - at)
     import torch
     assert torch.isfinite(o["params"]).all() and not torch.equal(o["params"], out[leaver]["params"])
+
+
+@pytest.mark.parametrize("rows,classes", [(1, 1), (33, 10), (128, 31), (64, 1000), (2000, 100)])
+def test_top1_accuracy_matches_library(rows, classes):
+    from gtopkssgd_b200.ops import accuracy
+    torch.manual_seed(rows)
+    x = torch.randn(rows, classes, device="cuda")
+    y = torch.randint(0, classes, (rows,), device="cuda")
+    x[0, classes - 1] = float("nan")
+    assert accuracy.takes(x, y)
+    want = 100.0 * x.topk(1, 1).indices[:, 0].eq(y).float().mean()
+    assert float(accuracy.top1_percent(x, y)) == pytest.approx(float(want), abs=1e-4)
+
+
+def test_batch_counters_advance_like_the_layers_do():
+    from gtopkssgd_b200.models import create_net
+    from gtopkssgd_b200.trainer.dl_trainer import BatchCounters
+    nets = []
+    for _ in range(2):
+        torch.manual_seed(0)
+        nets.append(create_net(10, "resnet20")[0].cuda())
+    frozen = [n.stage_2[0].bn_a.eval() for n in nets]
+    x = torch.randn(4, 3, 32, 32, device="cuda")
+    counters = BatchCounters(nets[0])
+    for _ in range(3):
+        a, b = counters.forward(nets[0], x), nets[1](x)
+    assert torch.allclose(a, b, atol=1e-5) and int(frozen[0].num_batches_tracked) == 0
+    for (k, u), v in zip(nets[0].state_dict().items(), nets[1].state_dict().values()):
+        assert torch.allclose(u, v, atol=1e-5) if u.is_floating_point() else torch.equal(u, v), k
