@@ -69,6 +69,58 @@ struct Call<F> {
   }
 };
 
+// ---- p.grad of many parameters -----------------------------------------------------------------------------
+// One iteration looks at every parameter's gradient; from Python that is 1 us each, here a quarter of that.
+PyObject *kGrad, *kDataPtr, *kDtype, *kIsContiguous;
+
+// clear_grads(params): p.grad = None
+PyObject* clear_grads(PyObject*, PyObject* params) {
+  PyObject* seq = PySequence_Fast(params, "expected a sequence of parameters");
+  if (!seq) return nullptr;
+  for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(seq); ++i)
+    if (PyObject_SetAttr(PySequence_Fast_GET_ITEM(seq, i), kGrad, Py_None) < 0) {
+      Py_DECREF(seq);
+      return nullptr;
+    }
+  Py_DECREF(seq);
+  Py_RETURN_NONE;
+}
+
+// grad_addresses(params, dtype): [p.grad.data_ptr() or 0 where there is none]; None if a gradient is not contiguous
+// or not of that dtype.
+PyObject* grad_addresses(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  if (nargs != 2) {
+    PyErr_SetString(PyExc_TypeError, "grad_addresses(params, dtype)");
+    return nullptr;
+  }
+  PyObject* seq = PySequence_Fast(args[0], "expected a sequence of parameters");
+  if (!seq) return nullptr;
+  const Py_ssize_t n = PySequence_Fast_GET_SIZE(seq);
+  PyObject* out = PyList_New(n);
+  bool usable = out != nullptr;
+  for (Py_ssize_t i = 0; usable && i < n; ++i) {
+    PyObject* g = PyObject_GetAttr(PySequence_Fast_GET_ITEM(seq, i), kGrad);
+    PyObject* at = nullptr;
+    if (g == Py_None) {
+      at = PyLong_FromLong(0);
+    } else if (g) {
+      PyObject* dtype = PyObject_GetAttr(g, kDtype);
+      PyObject* dense = dtype == args[1] ? PyObject_CallMethodNoArgs(g, kIsContiguous) : nullptr;
+      if (dense == Py_True) at = PyObject_CallMethodNoArgs(g, kDataPtr);
+      Py_XDECREF(dense);
+      Py_XDECREF(dtype);
+    }
+    Py_XDECREF(g);
+    if (at) PyList_SET_ITEM(out, i, at);
+    else usable = false;
+  }
+  Py_DECREF(seq);
+  if (usable) return out;
+  Py_XDECREF(out);
+  if (PyErr_Occurred()) return nullptr;
+  Py_RETURN_NONE;
+}
+
 #define GTK_METHOD(name) \
   {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&Call<name>::fast)), METH_FASTCALL, nullptr}
 
@@ -77,10 +129,19 @@ PyMethodDef kMethods[] = {
     GTK_METHOD(gtk_k1_compress),      GTK_METHOD(gtk_k2_exchange),      GTK_METHOD(gtk_k2t_allgather),
     GTK_METHOD(gtk_k3_dense),         GTK_METHOD(gtk_k3_sparse),      GTK_METHOD(gtk_k3_scatter_dense),
     GTK_METHOD(gtk_k3_momentum_correct), GTK_METHOD(gtk_k4_sumsq_dense), GTK_METHOD(gtk_k4_sumsq_pairs),
-    GTK_METHOD(gtk_k4_finalize),      GTK_METHOD(gtk_k5_top1),          {nullptr, nullptr, 0, nullptr}};
+    GTK_METHOD(gtk_k4_finalize),      GTK_METHOD(gtk_k5_top1),
+    {"clear_grads", clear_grads, METH_O, nullptr},
+    {"grad_addresses", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&grad_addresses)), METH_FASTCALL, nullptr},
+    {nullptr, nullptr, 0, nullptr}};
 
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_gtk_calls", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__gtk_calls(void) { return PyModule_Create(&kModule); }
+PyMODINIT_FUNC PyInit__gtk_calls(void) {
+  kGrad = PyUnicode_InternFromString("grad");
+  kDataPtr = PyUnicode_InternFromString("data_ptr");
+  kDtype = PyUnicode_InternFromString("dtype");
+  kIsContiguous = PyUnicode_InternFromString("is_contiguous");
+  return PyModule_Create(&kModule);
+}

@@ -31,7 +31,7 @@ from ..ops import oracle
 from ..ops.clip import ClipNorm
 from ..ops.select import MAX_SEGMENTS, TopkSelector, pairs_to_tensors, segment_table, tensors_to_pairs
 from ..settings import logger
-from ..utils.timing import PhaseTimers
+from ..utils.timing import PhaseTimers, current_stream
 from . import comm, fallback
 from .flat_buffer import FlatBuffers, MergedGroup
 
@@ -151,7 +151,7 @@ class GroupEngine:
             # event, so the select has the bandwidth to itself and the dense part overlaps the exchange
             if self.select_done is None:
                 self.select_done = torch.cuda.Event()
-            self.select_done.record()
+            self.select_done.record(current_stream())
         t.stop(self.g.key, "compression")
         t.start(self.g.key, "allreduce")
         if world == 1:

@@ -37,6 +37,7 @@ from .. import settings
 from ..ops.clip import ClipNorm
 from ..ops.sgd import SgdHyper, momentum_correct, scatter_dense, sgd_dense, sgd_sparse
 from ..settings import logger
+from ..utils.timing import current_stream
 from . import allreducer as ar
 from . import comm
 from .compression import NoneCompressor
@@ -190,7 +191,7 @@ class _DistributedOptimizer(torch.optim.Optimizer):
             self._flat.ensure_views()
         if self._overlap:
             ev = self._ready[gi]
-            ev.record()
+            ev.record(current_stream())
             self._comm_stream.wait_event(ev)
             with torch.cuda.stream(self._comm_stream):
                 if self.momentum_correction:
@@ -325,7 +326,7 @@ class _DistributedOptimizer(torch.optim.Optimizer):
                 if not self._launched[gi]:  # parameters that got no gradient this iteration
                     self._launch_group(gi)
             if self._overlap:
-                torch.cuda.current_stream().wait_stream(self._comm_stream)
+                current_stream().wait_stream(self._comm_stream)
             self._synced = True
         if materialize and not self._materialized and self._allreducer.mode != "none":
             self._flat.attach(keep=False)
@@ -408,7 +409,7 @@ class _DistributedOptimizer(torch.optim.Optimizer):
         else:
             for eng in a.engines:
                 if eng.select_done is not None and self._overlap:
-                    torch.cuda.current_stream().wait_event(eng.select_done)  # select first, then dense || exchange
+                    current_stream().wait_event(eng.select_done)  # select first, then dense || exchange
                 p, buf = bufs(eng)
                 sgd_dense(p, buf, h, first, lr_dev=lr_dev)
             self.synchronize()

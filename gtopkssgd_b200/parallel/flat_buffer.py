@@ -25,6 +25,8 @@ from typing import Dict, Iterable, List, Optional, Sequence, Tuple
 
 import torch
 
+from ..ops import lib as _native
+
 ALIGN = 64      # elements; every group starts on a 256-byte boundary
 SLOT_ALIGN = 4  # elements; every parameter starts on a 16-byte boundary.  Library kernels (cuDNN, cuBLAS)
                 # pick their vectorised and TMA-fed variants only for 16-byte aligned operands, and a
@@ -125,7 +127,9 @@ class FlatBuffers:
                 view.copy_(p.data)
                 p.data = view
                 p.grad = self._view(self._grad, slot)
-        self._grad_slots = [(s.param, 4 * s.offset) for s in self.slots.values()]
+        self._params = [s.param for s in self.slots.values()]
+        self._view_addresses = [self._grad.data_ptr() + 4 * s.offset for s in self.slots.values()]
+        self._channels_last = any(s.channels_last for s in self.slots.values())
 
     # -- views -----------------------------------------------------------------
     @staticmethod
@@ -153,12 +157,7 @@ class FlatBuffers:
 
     def grads_attached(self) -> bool:
         """True when every ``p.grad`` is still the view that was set up here."""
-        base = self._grad.data_ptr()
-        for p, at in self._grad_slots:
-            g = p.grad
-            if g is None or g.data_ptr() != base + at:
-                return False
-        return True
+        return self.grad_addresses() == self._view_addresses
 
     @property
     def grad(self) -> torch.Tensor:
@@ -182,21 +181,22 @@ class FlatBuffers:
 
     def begin_detached(self) -> None:
         """No gradients, and none attached: ``p.grad`` will be what backward produces."""
-        for p, _ in self._grad_slots:
-            p.grad = None
+        _native.calls().clear_grads(self._params)
         self._detached = "live"
 
     def current_grads(self) -> List[Optional[torch.Tensor]]:
-        return [p.grad for p, _ in self._grad_slots]
+        return [p.grad for p in self._params]
 
     def use_grads_of(self, grads: List[Optional[torch.Tensor]]) -> None:
         """A replayed graph has just refilled these."""
         self._detached = grads
 
     def grad_addresses(self) -> Optional[List[int]]:
-        """Device addresses of the detached gradients (0 where there is none), in
-        slot order; None when one of them is not laid out like its parameter and
-        has to be copied instead."""
+        """Device addresses of all ``p.grad`` (0 where there is none), in slot
+        order; None when one of them is not laid out like its parameter and has
+        to be copied instead."""
+        if not self._channels_last:
+            return _native.calls().grad_addresses(self._params, torch.float32)
         out = []
         for slot in self.slots.values():
             g = slot.param.grad

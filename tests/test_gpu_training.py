@@ -2,6 +2,8 @@
 fused sparse SGD step, side stream) replayed against the oracle, on one GPU
 and -- when the box has them -- on 2 and 4 GPUs through the peer-store
 exchange kernel over CUDA IPC."""
+import gc
+
 import pytest
 import torch
 
@@ -11,6 +13,14 @@ from gtopkssgd_b200.ops import oracle
 from gtopkssgd_b200.utils.launch import spawn_ranks
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(autouse=True)
+def _release_trainers():
+    """A trainer and its captured graphs form cycles; collected here, their memory
+    is not given back in the middle of a later test that watches the allocator."""
+    yield
+    gc.collect()
 
 
 @pytest.mark.parametrize("compressor", ["gtopk", "none"])
