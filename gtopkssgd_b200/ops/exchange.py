@@ -221,17 +221,20 @@ SMALL_MAX_K = 2048  # up to here the tree runs in one CTA with the set in shared
 
 
 def default_nctas(k: int, nranks: int = 1, sms: int = 148) -> int:
-    """CTAs per rank for the exchange kernels, from sweeps on B200 (in-kernel
-    time of one tree round + broadcast + put-back):
+    """CTAs per rank for the exchange kernels, from sweeps on B200 (whole call):
 
     * up to 4 K union entries of the tree: one CTA, the set in shared memory
-      (whole call, two ranks: 10 us at k = 1 000 and 16 us at 2 000, against 23
-      and 25 us with a cluster; 26 against 25 us at 3 000);
+      (two ranks: 10 us at k = 1 000 and 16 us at 2 000, against 23 and 25 us
+      with a cluster; 26 against 25 us at 3 000);
     * up to 32 K union entries: a power-of-two cluster of 2..16 CTAs joined by
-      the hardware cluster barrier, about 1024 entries per CTA (k = 4 000: 19 us
-      against 25 us with the software barrier; k = 14 700: 23 us against 27 us);
-    * above: one CTA per 768 entries (up to 128) with the software barrier
-      (k = 25 600: 26 us with 64 CTAs against 33 us with a cluster of 16)."""
+      the hardware cluster barrier, about 1024 entries per CTA (four ranks, k =
+      14 700: 41 us with 16 CTAs, 45 to 50 us with 24 to 74 and the software
+      barrier);
+    * above: one CTA per 768 entries with the software barrier, as many as the
+      device holds one per SM, and two per SM where each of those had more than
+      2 000 entries (eight ranks, k = 40 000: 112 us with 37 CTAs, 129 with 18;
+      two ranks, k = 255 570: 84 us with 148, 97 with 74; but k = 66 000: 45 us
+      with 148, 43 with 74)."""
     return 1 if k <= SMALL_MAX_K else _spread_nctas(2 * k, nranks, sms)
 
 
@@ -244,7 +247,9 @@ def _spread_nctas(n_u: int, nranks: int, sms: int = 148) -> int:
         while n < 16 and n * 1024 < n_u:
             n *= 2
         return n
-    return max(1, min(128, (n_u + 767) // 768, sms // max(nranks, 1)))
+    one = max(1, sms // max(nranks, 1))
+    per_sm = 1 if n_u <= 2000 * one else 2
+    return max(1, min(sms, per_sm * sms // max(nranks, 1), (n_u + 767) // 768))
 
 
 def launch_gtopk(ranks: Sequence[ExchangeRank], desc: torch.Tensor, rank_base: int, world: int, k: int,
