@@ -13,6 +13,8 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from . import direct
+
 
 class ZeroPadShortcut(nn.Module):
     """Option-A shortcut: stride-2 subsampling, new channels filled with zeros."""
@@ -40,10 +42,15 @@ class BasicBlock(nn.Module):
         self.downsample = downsample
 
     def forward(self, x):
-        y = F.relu(self.bn_a(self.conv_a(x)), inplace=True)
-        y = self.bn_b(self.conv_b(y))
+        if torch.jit.is_scripting():
+            y = F.relu(self.bn_a(self.conv_a(x)), inplace=True)
+            y = self.bn_b(self.conv_b(y))
+        else:
+            layers = self._modules
+            y = torch.relu_(direct.batch_norm(layers["bn_a"], direct.conv(layers["conv_a"], x)))
+            y = direct.batch_norm(layers["bn_b"], direct.conv(layers["conv_b"], y))
         skip = x if self.downsample is None else self.downsample(x)
-        return F.relu(skip + y, inplace=True)
+        return torch.relu_(skip + y)
 
 
 class CifarResNet(nn.Module):

@@ -305,3 +305,26 @@ def test_batch_counters_advance_like_the_layers_do():
     assert torch.allclose(a, b, atol=1e-5) and int(frozen[0].num_batches_tracked) == 0
     for (k, u), v in zip(nets[0].state_dict().items(), nets[1].state_dict().values()):
         assert torch.allclose(u, v, atol=1e-5) if u.is_floating_point() else torch.equal(u, v), k
+
+
+def test_direct_layer_calls_keep_hooks_and_results():
+    """The residual block's direct library calls give the layers' results bit for
+    bit, and a layer with a hook is called as a layer."""
+    from gtopkssgd_b200.models import create_net, direct
+    torch.manual_seed(0)
+    net = create_net(10, "resnet20")[0].cuda()
+    x = torch.randn(4, 16, 32, 32, device="cuda")
+    block = net.stage_1[0]
+    for conv, bn in ((block.conv_a, block.bn_a), (block.conv_b, block.bn_b)):
+        y = direct.conv(conv, x)
+        assert torch.equal(y, conv(x))
+        before = bn.running_mean.clone()
+        a = direct.batch_norm(bn, y)
+        moved, bn.running_mean[:] = bn.running_mean.clone(), before
+        assert torch.equal(a, bn(y)) and torch.equal(moved, bn.running_mean) and int(bn.num_batches_tracked) == 2
+    seen = []
+    handle = block.conv_a.register_forward_hook(lambda *a: seen.append(1))
+    block(x)
+    handle.remove()
+    block.eval()(x)
+    assert len(seen) == 1
