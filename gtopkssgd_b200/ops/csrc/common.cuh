@@ -30,6 +30,8 @@ constexpr int kMaxRounds = 4;     // log2(16) recursive-doubling rounds
 constexpr int kMaxPeers = 16;
 constexpr int kTraceSlots = 64;
 
+constexpr unsigned int kBarAbort = 0x80000000u;  // bit of Ctrl::bar: the rank has given up
+
 // Per-rank control block.  Its counters start at zero: every user owns two blocks, alternates between them
 // and clears the idle one.
 struct Ctrl {
@@ -81,6 +83,15 @@ __device__ __forceinline__ unsigned int ld_relaxed_gpu_u32(const unsigned int* p
   asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
   return v;
 }
+// One 8-byte access that no other agent of the system sees half of.
+__device__ __forceinline__ unsigned long long ld_relaxed_sys_u64(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.relaxed.sys.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_relaxed_sys_u64(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.relaxed.sys.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
 __device__ __forceinline__ void red_release_gpu_add(unsigned int* p, unsigned int v) {
   asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -118,6 +129,7 @@ __device__ __forceinline__ uint32_t mag_key(float v) { return __float_as_uint(v)
 __device__ __forceinline__ void record_error(Ctrl* c, uint32_t status, uint32_t where) {
   if (atomicCAS(&c->status, 0u, status) == 0u) c->where = where;
   atomicExch(&c->abort, 1u);
+  atomicOr(&c->bar, kBarAbort);  // what waits in RankBarrier sees it in the word that it polls
   __threadfence();
 }
 
@@ -128,53 +140,72 @@ __device__ __forceinline__ bool aborted(const Ctrl* c) {
 // Barrier over the `nctas` CTAs that serve one rank.  `gen` is a per-thread
 // running count of barriers passed (identical in all threads of all CTAs of the
 // rank).  Returns false if the rank aborted or the limit ran out.
+//
+// The software form costs an L2 round trip for the arrival and one for the poll that sees the last one.  The
+// abort bit therefore sits in the arrival word: looked up in a word of its own, in each poll and once more at
+// the end, it made that three to four round trips (two ranks, 74 CTAs each: 2.3 us a barrier).  The release
+// of the arrival covers what the CTA's other threads stored before the __syncthreads.
 struct RankBarrier {
   Ctrl* ctrl;
   unsigned int nctas;
   unsigned int gen;
   uint64_t limit_ns;
-  unsigned int* counter = nullptr;  // arrival counter; nullptr: ctrl->bar
   bool cluster = false;             // the rank's CTAs form one thread-block cluster: hardware barrier
 
-  __device__ __forceinline__ bool sync(uint32_t where) {
-    __shared__ int ok_s;
-    unsigned int* const arrivals = counter ? counter : &ctrl->bar;
-    if (nctas == 1) {  // a single CTA learns of its own failures through its shared flags
-      __syncthreads();
-      return true;
-    }
+  __device__ __forceinline__ void arrive() {
+    if (nctas == 1) return;
     if (cluster) {
       // Cluster-scope release/acquire: global and shared writes made before the barrier by any
       // CTA of the cluster are visible to all of them after it.  The hardware barrier waits only
       // for threads that have not exited, so a CTA that gave up on a flag wait does not block it.
       asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-      return true;
+      return;
     }
     gen += 1;
     __syncthreads();
+    if (threadIdx.x == 0) red_release_gpu_add(&ctrl->bar, 1u);
+  }
+  __device__ __forceinline__ bool wait(uint32_t where) {
+    __shared__ int ok_s;
+    if (nctas == 1) {  // a single CTA learns of its own failures through its shared flags
+      __syncthreads();
+      return true;
+    }
+    if (cluster) {
+      asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+      return true;
+    }
     if (threadIdx.x == 0) {
       int ok = 1;
-      __threadfence();
-      red_release_gpu_add(arrivals, 1u);
       const unsigned int target = gen * nctas;
       const uint64_t t0 = globaltimer_ns();
       unsigned int spins = 0;
-      while (ld_acquire_gpu_u32(arrivals) < target) {
-        if (aborted(ctrl)) { ok = 0; break; }
+      for (;;) {
+        const unsigned int v = ld_acquire_gpu_u32(&ctrl->bar);
+        if (v & kBarAbort) { ok = 0; break; }
+        if (v >= target) break;
         if ((++spins & 63u) == 0u && globaltimer_ns() - t0 > limit_ns) {
           record_error(ctrl, ST_TIMEOUT_BARRIER, where);
           ok = 0;
           break;
         }
       }
-      if (ok && aborted(ctrl)) ok = 0;
       ok_s = ok;
     }
     __syncthreads();
     const bool ok = ok_s != 0;
     __syncthreads();
     return ok;
+  }
+  __device__ __forceinline__ bool sync(uint32_t where) {
+    arrive();
+    return wait(where);
+  }
+  // Instead of a last barrier: true in one thread, the first of the CTA that gets here after all the others.
+  __device__ __forceinline__ bool last_arrival() {
+    __syncthreads();
+    if (threadIdx.x != 0) return false;
+    return nctas == 1 || (atomicAdd(&ctrl->bar, 1u) & ~kBarAbort) == gen * nctas + nctas - 1u;
   }
 };
 

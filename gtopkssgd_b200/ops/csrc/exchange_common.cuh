@@ -16,7 +16,7 @@ namespace gtk {
 // Layout of the symmetric (peer-visible) region of one rank, identical on all
 // ranks.  Two parities (epoch & 1) so that a fast sender of call e+1 never
 // overwrites what a slow reader of call e still needs.
-//   slots : [2][kMaxRounds][kcap] pairs   receive slot of each tree round
+//   slots : [2][kMaxRounds + 1][kcap] wire words   receive slot of each tree round and of the broadcast
 //   ag    : [2][kMaxPeers][kcap] pairs    all-gather slots, one per source rank (K2t only)
 //   gout  : [2][kcap] pairs               the global top-k set
 //   flags : [2][kFlagsPerParity] u64      (epoch << 32) | count
@@ -33,10 +33,10 @@ __host__ __device__ constexpr size_t ll_off(unsigned int parity, unsigned int ro
 struct K2Rank {
   const Pair* sel;        // local selection written by K1
   const K1State* st;      // st->n_sel = number of local pairs
-  Pair* work[2];          // [kcap_work] ping-pong merge buffers
+  Pair* work[2];          // [kcap_work] and [2 * kcap] merge buffers; the second half of work[1] holds received entries
   int32_t* map;           // [d] direct-address table
   float* resid;           // [d] residual
-  Pair* slots;            // local symmetric buffers
+  unsigned long long* slots;  // local symmetric buffers
   Pair* ag;
   Pair* gout;
   uint64_t* flags;
@@ -45,9 +45,8 @@ struct K2Rank {
   unsigned int* n_global; // kResWords device words: result of the last call, see kRes* below
   unsigned int* epoch;    // device word: call counter (starts at 1); the kernel reads it at entry and
                           // adds one after its last barrier, so a replayed CUDA graph needs no new argument
-  Pair* peer_slots[kMaxPeers];
+  unsigned long long* peer_slots[kMaxPeers];
   Pair* peer_ag[kMaxPeers];
-  Pair* peer_gout[kMaxPeers];
   uint64_t* peer_flags[kMaxPeers];
   ulonglong2* peer_ll[kMaxPeers];
 };
@@ -75,7 +74,51 @@ struct ExchangeShared {
 
 __device__ __forceinline__ size_t slot_off(unsigned int parity, unsigned int round,
                                            unsigned int kcap) {
-  return ((size_t)parity * kMaxRounds + round) * kcap;
+  return ((size_t)parity * (kMaxRounds + 1) + round) * kcap;
+}
+
+// The wire word of a slot: one pair in one 8-byte store that no reader sees half of, never 0 (an index has its
+// top bit clear, on the wire set), so that a word that has been cleared says whether its pair has arrived.  A
+// receiver polls the words themselves and clears what it has taken: a set crosses without a system-wide fence
+// in every CTA that stored, a barrier over them and a flag's release behind it, which took 6 us per hop.  The
+// slot's next use is two calls later, which its sender starts only after this receiver took part in the call
+// between (its set is in the one that the root sent round).
+__device__ __forceinline__ void wire_store(unsigned long long* slot, Pair e) {
+  e.idx ^= (int32_t)0x80000000;
+  st_relaxed_sys_u64(slot, pair_bits(e));
+}
+// Receives the words slot + at(j) of this thread, for the j of `want`, into e[j] (idx -1: not wanted, or an index
+// outside [0, d)) and clears them.  Returns false, the error recorded, when the limit runs out or the rank gives up.
+template <int N, typename At>
+__device__ __forceinline__ bool wire_receive(unsigned long long* slot, unsigned int want, At at, Pair (&e)[N],
+                                             unsigned int d, Ctrl* ctrl, uint64_t limit_ns, uint32_t where) {
+  const uint64_t t0 = want ? globaltimer_ns() : 0ull;
+  unsigned int spins = 0;
+  while (want) {
+    unsigned long long w[N];
+#pragma unroll
+    for (int j = 0; j < N; ++j) w[j] = (want & (1u << j)) ? ld_relaxed_sys_u64(slot + at(j)) : 0ull;
+#pragma unroll
+    for (int j = 0; j < N; ++j) {
+      if (w[j] == 0ull) continue;
+      slot[at(j)] = 0ull;
+      want &= ~(1u << j);
+      e[j] = bits_pair(w[j]);
+      e[j].idx ^= (int32_t)0x80000000;
+      if ((unsigned int)e[j].idx >= d) {
+        record_error(ctrl, ST_BOUNDS, where + 90u);
+        e[j].idx = -1;
+      }
+    }
+    if (want && (++spins & 63u) == 0u) {
+      if (aborted(ctrl)) return false;
+      if (globaltimer_ns() - t0 > limit_ns) {
+        record_error(ctrl, ST_TIMEOUT_FLAG, where);
+        return false;
+      }
+    }
+  }
+  return true;
 }
 __device__ __forceinline__ size_t ag_off(unsigned int parity, unsigned int src, unsigned int kcap) {
   return ((size_t)parity * kMaxPeers + src) * kcap;
@@ -142,17 +185,6 @@ __device__ __forceinline__ void copy_and_map(Pair* A, const Pair* src, unsigned 
     tally(e.val, 1u);
     if ((unsigned int)e.idx < d) map[e.idx] = (int32_t)i;
     else record_error(ctrl, ST_BOUNDS, 300);
-  }
-}
-
-__device__ __forceinline__ void build_map(const Pair* A, unsigned int n, int32_t* map,
-                                          unsigned int d, unsigned int cta, unsigned int nct,
-                                          Ctrl* ctrl) {
-  const unsigned int stride = nct * kSelThreads;
-  for (unsigned int i = cta * kSelThreads + threadIdx.x; i < n; i += stride) {
-    const Pair e = ld_pair_cg(&A[i]);
-    if ((unsigned int)e.idx < d) map[e.idx] = (int32_t)i;
-    else record_error(ctrl, ST_BOUNDS, 301);
   }
 }
 

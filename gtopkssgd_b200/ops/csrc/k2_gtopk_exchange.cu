@@ -7,10 +7,11 @@
 // broadcasts it; every rank returns "selected locally but not globally" values
 // to its residual (compression.py:66-75).
 //
-// Here every transfer is a plain NVLink peer store into the partner's receive
-// slot followed by a release store of an epoch-stamped flag in the partner's
-// memory; a receiver polls only its own memory.  No MPI, no NCCL, no host
-// staging, no per-round barrier between ranks.
+// Here every transfer is an NVLink peer store into the partner's receive slot,
+// one 8-byte word per pair that says by itself whether it has arrived; an
+// epoch-stamped word in the partner's memory says how many to expect.  A
+// receiver polls only its own memory.  No MPI, no NCCL, no host staging, no
+// per-round barrier between ranks, no fence between data and flag.
 //
 // One launch serves gridDim.y ranks: 1 in production (one process per GPU), P
 // when all ranks are emulated on one GPU for testing, in which case the launch
@@ -19,9 +20,16 @@
 //
 // A merged set is compacted straight to where the next phase reads it: into the
 // partner's receive slot when this rank sends in the next round, into every
-// rank's global-set buffer after the last round (rank 0), into the local work
+// rank's broadcast slot after the last round (rank 0), into the local work
 // buffer otherwise.  So only round 0 has a separate push, and there is no
 // separate broadcast copy.
+//
+// What bounds it: a chain of phases of 2 to 6 us, each a round of L2 or scattered
+// DRAM accesses (the table spans d) and a barrier; past k of about 200 000 the
+// scattered accesses themselves (45 a ns).  Two ranks, k = 66 034, whole call:
+// 44 us with flags behind fenced plain stores and the put-back at the end, 31 us
+// now (k = 255 570: 87 and 74; four ranks, k = 14 728: 41 and 35; eight ranks,
+// k = 40 000: 117 and 97).
 //
 // No host-side clearing: the rank owns two control blocks; call e uses block
 // (e & 1) and zeroes the other one for call e + 1 once its own work is done.
@@ -76,7 +84,12 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
   const unsigned int lane0 = cta * kSelThreads + threadIdx.x;  // union index of this thread's trip 0
   Ctrl* ctrl = R.ctrl + parity;
   int32_t* const map = R.map;
-  RankBarrier bar{ctrl, nct, 0u, limit_ns, nullptr, use_cluster != 0};
+  RankBarrier bar{ctrl, nct, 0u, limit_ns, use_cluster != 0};
+  // Says how many pairs a slot of rank q gets; they follow, or have come already, in no order.
+  auto announce = [&](unsigned int q, unsigned int which, unsigned int n) {
+    st_relaxed_sys_u64(reinterpret_cast<unsigned long long*>(R.peer_flags[q] + flag_off(parity, which)),
+                       ((unsigned long long)epoch << 32) | n);
+  };
   // Leaves an empty result and the sticky status behind; called by every CTA that gives up.
   auto fail = [&]() {
     if (threadIdx.x == 0) {
@@ -114,15 +127,12 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
     const unsigned int bit = 1u << r;
     const unsigned int low = me & (2u * bit - 1u);
     if (low == bit) {
-      // ---- sender: push the current set into the partner's slot, raise its flag
+      // ---- sender: push the current set into the partner's slot
       const unsigned int partner = me - bit;
-      Pair* dst = R.peer_slots[partner] + slot_off(parity, r, kcap);
-      push_pairs(dst, cur, n_cur, cta, nct);
-      cta_fence_peer_stores(nct == 1);
-      if (!bar.sync(200 + r)) { fail(); return; }
+      if (cta == 0 && threadIdx.x == 0) announce(partner, r, n_cur);
+      unsigned long long* const dst = R.peer_slots[partner] + slot_off(parity, r, kcap);
+      for (unsigned int i = lane0; i < n_cur; i += stride) wire_store(&dst[i], ld_pair_cg(&cur[i]));
       trace_stamp(ctrl, 1 + 8 * r + 6);
-      if (cta == 0 && threadIdx.x == 0)
-        release_flag(R.peer_flags[partner] + flag_off(parity, r), epoch, n_cur);
       trace_stamp(ctrl, 1 + 8 * r + 7);
       break;
     }
@@ -135,13 +145,18 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
     if (copied) {
       A = R.work[0];
       for (unsigned int i = lane0; i < n_cur; i += stride) {
-        const Pair e = ld_pair_cg(&cur[i]);
+        Pair e = ld_pair_cg(&cur[i]);
+        if ((unsigned int)e.idx < d) {
+          map[e.idx] = (int32_t)i;
+          tally(e.val, 1u);
+        } else {
+          record_error(ctrl, ST_BOUNDS, 300);
+          e.idx = -1;
+        }
         st_pair(&A[i], e);
-        if ((unsigned int)e.idx < d) map[e.idx] = (int32_t)i;
-        else record_error(ctrl, ST_BOUNDS, 300);
-        tally(e.val, 1u);
       }
       cur_buf = 0;
+      bar.arrive();
     } else {
       A = R.work[cur_buf];
     }
@@ -156,70 +171,71 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
       record_error(ctrl, ST_CAPACITY, 220 + r);
       n_b = kcap;
     }
-    Pair* B = R.slots + slot_off(parity, r, kcap);
+    unsigned long long* const slot = R.slots + slot_off(parity, r, kcap);
+    Pair* const B = R.work[1] + kcap;  // what is received beyond the register cache
     const unsigned int n_a = n_cur;
     const unsigned int n_u = n_a + n_b;
     const unsigned int trips = (n_u + stride - 1) / stride;
+
+    // ---- probe: every thread takes its B entries off the slot, joins them against A (sum on shared
+    // indices) and keeps them in registers; three dependent loads, issued level by level.
+    auto receive = [&](Pair (&e)[kK2Cache], unsigned int t0) {
+      unsigned int want = 0;
+#pragma unroll
+      for (int t = 0; t < kK2Cache; ++t) {
+        const unsigned int i = (t0 + t) * stride + lane0;
+        e[t].idx = -1;
+        e[t].val = 0.f;
+        if (t0 + t < trips && i >= n_a && i < n_u) want |= 1u << t;
+      }
+      return wire_receive(slot, want, [&](int t) { return (size_t)((t0 + t) * stride + lane0 - n_a); }, e, d, ctrl,
+                          limit_ns, 212 + r);
+    };
+    auto join = [&](Pair (&e)[kK2Cache]) {
+      unsigned int pm[kK2Cache];
+      Pair a[kK2Cache];
+#pragma unroll
+      for (int t = 0; t < kK2Cache; ++t) {
+        pm[t] = 0xffffffffu;
+        if (e[t].idx >= 0) pm[t] = (unsigned int)__ldcg(&map[e[t].idx]);
+      }
+#pragma unroll
+      for (int t = 0; t < kK2Cache; ++t) {
+        a[t].idx = -1;
+        if (pm[t] < n_a) a[t] = ld_pair_cg(&A[pm[t]]);
+      }
+#pragma unroll
+      for (int t = 0; t < kK2Cache; ++t) {
+        if (e[t].idx < 0) continue;
+        if (a[t].idx == e[t].idx) {
+          const float nv = a[t].val + e[t].val;
+          A[pm[t]].val = nv;  // A[p] belongs to another thread's sweep: goes through memory
+          tally(a[t].val, 0xffffffffu);
+          tally(nv, 1u);
+          e[t].idx = -1;
+        } else {
+          tally(e[t].val, 1u);
+        }
+      }
+    };
+    Pair c[kK2Cache];
+    bool ok = receive(c, 0);
     // A and map must be complete: after the copy above that needs a barrier, after a previous
     // round its closing barrier already gave it
-    if (copied && !bar.sync(230 + r)) { fail(); return; }
+    if (!__syncthreads_and(ok) || (copied && !bar.wait(230 + r))) { fail(); return; }
     trace_stamp(ctrl, 1 + 8 * r + 2);
-
-    // ---- probe: every thread joins its own B entries against A (sum on shared indices) and
-    // keeps them in registers; three dependent loads, issued level by level.
-    Pair c[kK2Cache];
-    unsigned int pm[kK2Cache];
-    auto join = [&](Pair& e, unsigned int p, unsigned int j) {
-      bool matched = false;
-      if (p < n_a) {
-        const Pair a = ld_pair_cg(&A[p]);
-        if (a.idx == e.idx) {
-          const float nv = a.val + e.val;
-          A[p].val = nv;  // A[p] belongs to another thread's sweep: goes through memory
-          tally(a.val, 0xffffffffu);
-          tally(nv, 1u);
-          B[j].idx = -1;
-          e.idx = -1;
-          matched = true;
-        }
-      }
-      if (!matched) tally(e.val, 1u);
-    };
+    join(c);
+    for (unsigned int t0 = kK2Cache; t0 < trips && ok; t0 += kK2Cache) {
+      Pair e[kK2Cache];
+      ok = receive(e, t0);
+      join(e);
 #pragma unroll
-    for (int t = 0; t < kK2Cache; ++t) {
-      const unsigned int i = (unsigned int)t * stride + lane0;
-      c[t].idx = -1;
-      c[t].val = 0.f;
-      if ((unsigned int)t < trips && i >= n_a && i < n_u) c[t] = ld_pair_cg(&B[i - n_a]);
-    }
-#pragma unroll
-    for (int t = 0; t < kK2Cache; ++t) {
-      pm[t] = 0xffffffffu;
-      if (c[t].idx >= 0) {
-        if ((unsigned int)c[t].idx < d) {
-          pm[t] = (unsigned int)__ldcg(&map[c[t].idx]);
-        } else {
-          record_error(ctrl, ST_BOUNDS, 302);
-          B[(unsigned int)t * stride + lane0 - n_a].idx = -1;
-          c[t].idx = -1;
-        }
+      for (int t = 0; t < kK2Cache; ++t) {
+        const unsigned int i = (t0 + t) * stride + lane0;
+        if (t0 + t < trips && i >= n_a && i < n_u) st_pair(&B[i - n_a], e[t]);
       }
     }
-#pragma unroll
-    for (int t = 0; t < kK2Cache; ++t)
-      if (c[t].idx >= 0) join(c[t], pm[t], (unsigned int)t * stride + lane0 - n_a);
-    for (unsigned int t = kK2Cache; t < trips; ++t) {  // entries beyond the register cache
-      const unsigned int i = t * stride + lane0;
-      if (i >= n_a && i < n_u) {
-        Pair e = ld_pair_cg(&B[i - n_a]);
-        if ((unsigned int)e.idx >= d) {
-          record_error(ctrl, ST_BOUNDS, 302);
-          B[i - n_a].idx = -1;
-        } else {
-          join(e, (unsigned int)__ldcg(&map[e.idx]), i - n_a);
-        }
-      }
-    }
+    if (!__syncthreads_and(ok)) { fail(); return; }
     band_flush(sh, ctrl->hist[r][0]);
     if (!bar.sync(240 + r)) { fail(); return; }  // sums and the on-the-fly histograms complete
     trace_stamp(ctrl, 1 + 8 * r + 3);
@@ -257,48 +273,69 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
     // ---- compaction of the winners to where the next phase reads them
     const bool last = r + 1 == rounds;                                  // then me == 0
     const bool send_next = !last && (me & (4u * bit - 1u)) == 2u * bit;  // sender of round r + 1
+    const bool only_round = last && copied;
     const bool keep = !last && !send_next;                              // receiver again in round r + 1
-    Pair* OUT;
-    if (last) OUT = R.gout + (size_t)parity * kcap;
-    else if (send_next) OUT = R.peer_slots[me - 2u * bit] + slot_off(parity, r + 1, kcap);
-    else OUT = R.work[cur_buf ^ 1];
+    Pair* const OUT = last ? R.gout + (size_t)parity * kcap : R.work[cur_buf ^ 1];
+    unsigned long long* const next = R.peer_slots[send_next ? me - 2u * bit : 0u] + slot_off(parity, r + 1, kcap);
+    n_cur = th.n < kcap ? th.n : kcap;
+    if (cta == 0 && send_next && threadIdx.x == 0) announce(me - 2u * bit, r + 1, n_cur);
+    if (cta == 0 && last && threadIdx.x < P && threadIdx.x > 0) announce(threadIdx.x, kFlagBcast, n_cur);
     // keep: the table and (below) the band counts of the next round are built on the way;
     // last: the table over the global set serves the residual put-back, and every peer gets its copy
     auto on_placed = [&](Pair e, unsigned int pos) {
-      if (send_next) return;
-      map[e.idx] = (int32_t)pos;
+      if (send_next) {
+        wire_store(&next[pos], e);
+        return;
+      }
       if (last)
-        for (unsigned int q = 1; q < P; ++q) st_pair(R.peer_gout[q] + (size_t)parity * kcap + pos, e);
+        for (unsigned int q = 1; q < P; ++q) wire_store(R.peer_slots[q] + slot_off(parity, kFlagBcast, kcap) + pos, e);
+      st_pair(&OUT[pos], e);
+      if (!only_round) map[e.idx] = (int32_t)pos;
     };
     unsigned int* const tie = &ctrl->tie[r];
-    StagedAppender app{&ss, OUT, &ctrl->cursor[r], kcap, ctrl};
+    StagedAppender app{&ss, &ctrl->cursor[r], kcap, ctrl};
     app.begin();
-    auto consider = [&](const Pair& e) {
-      if (e.idx >= 0 && passes_threshold(mag_key(e.val), th, tie)) {
-        app.put(e);
-        if (keep) tally(e.val, 1u);
-      }
-    };
+    auto sweep = [&](const Pair (&e)[kK2Cache], unsigned int t0) {
+      unsigned int lost = 0;
 #pragma unroll
-    for (int t = 0; t < kK2Cache; ++t) {
-      if ((unsigned int)t < trips) {
-        consider(c[t]);
+      for (int t = 0; t < kK2Cache; ++t) {
+        if (t0 + t >= trips) break;
+        if (e[t].idx >= 0) {
+          if (passes_threshold(mag_key(e[t].val), th, tie)) {
+            app.put(e[t]);
+            if (keep) tally(e[t].val, 1u);
+          } else {
+            lost |= 1u << t;
+          }
+        }
         app.end_tile(on_placed);
       }
+      if (t0 + kK2Cache >= trips) app.flush(on_placed);
+      if (!only_round) return;
+      // Two ranks: what drops out of A here is not in the global set, and A is this rank's selection.
+      float back[kK2Cache];
+#pragma unroll
+      for (int t = 0; t < kK2Cache; ++t) {
+        const unsigned int i = (t0 + t) * stride + lane0;
+        if (i >= n_a) lost &= ~(1u << t);
+        back[t] = 0.f;
+        if (lost & (1u << t)) back[t] = R.resid[e[t].idx] + R.sel[i].val;
+      }
+#pragma unroll
+      for (int t = 0; t < kK2Cache; ++t)
+        if (lost & (1u << t)) R.resid[e[t].idx] = back[t];
+    };
+    sweep(c, 0);
+    for (unsigned int t0 = kK2Cache; t0 < trips; t0 += kK2Cache) {
+      Pair e[kK2Cache];
+#pragma unroll
+      for (int t = 0; t < kK2Cache; ++t) e[t] = entry(t0 + t);
+      sweep(e, t0);
     }
-    for (unsigned int t = kK2Cache; t < trips; ++t) {
-      consider(entry(t));
-      app.end_tile(on_placed);
-    }
-    app.flush(on_placed);
-    if (!keep) cta_fence_peer_stores(nct == 1);  // the winners went into other GPUs' memory
-    if (!bar.sync(290 + r)) { fail(); return; }  // OUT and its cursor complete
+    // OUT and map complete; or, when this rank has sent, its work buffers and map free for other use
+    if (!bar.sync(290 + r)) { fail(); return; }
     trace_stamp(ctrl, 1 + 8 * r + 5);
-    n_cur = __ldcg(&ctrl->cursor[r]);
-    if (n_cur > kcap) n_cur = kcap;
     if (send_next) {
-      if (cta == 0 && threadIdx.x == 0)
-        release_flag(R.peer_flags[me - 2u * bit] + flag_off(parity, r + 1), epoch, n_cur);
       trace_stamp(ctrl, 1 + 8 * (r + 1) + 7);
       break;  // left the tree
     }
@@ -307,17 +344,29 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
     cur = R.work[cur_buf];
   }
 
-  // ---- the global set: rank 0 has just written it into every rank's buffer and only raises the
-  // flags; the others wait for theirs and build the table over it
-  Pair* G = R.gout + (size_t)parity * kcap;
+  // ---- the global set, and the residual put-back of S_local \ S_global
+  Pair* const G = R.gout + (size_t)parity * kcap;
   unsigned int n_g = 0;
-  if (me == 0u) {
+  if (me == 0u) {  // it has just been written, the table over it too
     n_g = n_cur;
-    if (cta == 0 && threadIdx.x < P && threadIdx.x > 0)  // one releasing thread per destination
-      release_flag(R.peer_flags[threadIdx.x] + flag_off(parity, kFlagBcast), epoch, n_cur);
     trace_stamp(ctrl, 40);
     trace_stamp(ctrl, 41);
+    if (rounds > 1u) put_back(R.sel, n_sel, G, n_g, map, R.resid, d, cta, nct);
   } else {
+    // While the root merges: all of the own selection goes back to the residual, what was there is kept, and
+    // the table is built over the selection.  What of it turns out to be in the global set is then undone as
+    // its entries come in, with no barrier behind them.  (Table over the global set, barrier, then the put-back:
+    // 10 us after the set was there at k = 66 000, 28 us at 255 000.)
+    float* const was = reinterpret_cast<float*>(R.work[0]);
+    for (unsigned int i = lane0; i < n_sel; i += stride) {
+      const Pair e = R.sel[i];
+      if ((unsigned int)e.idx >= d) continue;
+      map[e.idx] = (int32_t)i;
+      const float r0 = R.resid[e.idx];
+      was[i] = r0;
+      R.resid[e.idx] = r0 + e.val;
+    }
+    if (!bar.sync(420)) { fail(); return; }
     if (!cta_wait_flag(sh.ex, R.flags + flag_off(parity, kFlagBcast), epoch, ctrl, limit_ns, 410, &n_g)) {
       fail();
       return;
@@ -327,12 +376,33 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
       n_g = kcap;
     }
     trace_stamp(ctrl, 40);
-    build_map(G, n_g, map, d, cta, nct, ctrl);
-    if (!bar.sync(420)) { fail(); return; }
     trace_stamp(ctrl, 41);
+    unsigned long long* const slot = R.slots + slot_off(parity, kFlagBcast, kcap);
+    bool ok = true;
+    for (unsigned int i0 = lane0; i0 < n_g && ok; i0 += (unsigned int)kK2Cache * stride) {
+      Pair e[kK2Cache];
+      unsigned int p[kK2Cache];
+      unsigned int want = 0;
+#pragma unroll
+      for (int t = 0; t < kK2Cache; ++t) {
+        e[t].idx = -1;
+        e[t].val = 0.f;
+        if (i0 + t * stride < n_g) want |= 1u << t;
+      }
+      ok = wire_receive(slot, want, [&](int t) { return (size_t)(i0 + t * stride); }, e, d, ctrl, limit_ns, 412);
+#pragma unroll
+      for (int t = 0; t < kK2Cache; ++t) {
+        p[t] = 0xffffffffu;
+        if (e[t].idx < 0) continue;
+        st_pair(&G[i0 + t * stride], e[t]);
+        p[t] = (unsigned int)__ldcg(&map[e[t].idx]);
+      }
+#pragma unroll
+      for (int t = 0; t < kK2Cache; ++t)
+        if (p[t] < n_sel && R.sel[p[t]].idx == e[t].idx) R.resid[e[t].idx] = __ldcg(&was[p[t]]);
+    }
+    if (!__syncthreads_and(ok)) { fail(); return; }
   }
-  // ---- residual put-back of S_local \ S_global
-  put_back(R.sel, n_sel, G, n_g, map, R.resid, d, cta, nct);
   trace_stamp(ctrl, 42);
   // ---- the other control block, for the next call (nobody waits for this rank any more)
   {
@@ -340,8 +410,7 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
     const size_t nvec16 = (offsetof(Ctrl, hist) + (size_t)(rounds + 1) * sizeof(((Ctrl*)0)->hist[0])) / 16;
     for (size_t i = lane0; i < nvec16; i += stride) other[i] = make_uint4(0u, 0u, 0u, 0u);
   }
-  if (!bar.sync(430)) { fail(); return; }  // every CTA is past its last use of the call counter
-  if (cta == 0 && threadIdx.x == 0) {
+  if (bar.last_arrival()) {  // every CTA is past its last use of the call counter
     if (aborted(ctrl)) {  // a bounds or capacity error that no wait noticed
       fail();
     } else {
@@ -367,7 +436,7 @@ static unsigned long long ll_offset(unsigned long long flags) {
 extern "C" void gtk_symm_layout(unsigned int kcap, int with_allgather, unsigned long long* out) {
   unsigned long long off = 0;
   out[0] = off;
-  off += 2ull * kMaxRounds * kcap * sizeof(Pair);
+  off += 2ull * (kMaxRounds + 1) * kcap * sizeof(Pair);
   out[1] = off;
   if (with_allgather) off += 2ull * kMaxPeers * kcap * sizeof(Pair);
   out[2] = off;
@@ -395,7 +464,7 @@ extern "C" int gtk_k2rank_fill(void* desc_host, const void* sel, const void* st,
   r->map = (int32_t*)map;
   r->resid = (float*)resid;
   char* base = (char*)symm_local;
-  r->slots = (Pair*)(base + lay[0]);
+  r->slots = (unsigned long long*)(base + lay[0]);
   r->ag = (Pair*)(base + lay[1]);
   r->gout = (Pair*)(base + lay[2]);
   r->flags = (uint64_t*)(base + lay[3]);
@@ -405,9 +474,8 @@ extern "C" int gtk_k2rank_fill(void* desc_host, const void* sel, const void* st,
   r->epoch = (unsigned int*)epoch_word;
   for (unsigned int q = 0; q < (unsigned int)kMaxPeers; ++q) {
     char* pb = q < P ? (char*)symm_peers[q] : nullptr;
-    r->peer_slots[q] = pb ? (Pair*)(pb + lay[0]) : nullptr;
+    r->peer_slots[q] = pb ? (unsigned long long*)(pb + lay[0]) : nullptr;
     r->peer_ag[q] = pb ? (Pair*)(pb + lay[1]) : nullptr;
-    r->peer_gout[q] = pb ? (Pair*)(pb + lay[2]) : nullptr;
     r->peer_flags[q] = pb ? (uint64_t*)(pb + lay[3]) : nullptr;
     r->peer_ll[q] = pb ? (ulonglong2*)(pb + ll_offset(lay[3])) : nullptr;
   }

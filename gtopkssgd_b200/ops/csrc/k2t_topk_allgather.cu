@@ -36,8 +36,7 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
   auto fail = [&]() {
     if (threadIdx.x == 0) {
       atomicExch(&R.n_global[kResCount], 0u);
-      if (cta == 0)
-        for (unsigned int q = 0; q < (unsigned int)kMaxPeers; ++q) seg_counts[q] = 0u;
+      for (unsigned int q = 0; q < (unsigned int)kMaxPeers; ++q) seg_counts[q] = 0u;
       unsigned int st = ld_relaxed_gpu_u32(&ctrl->status);
       if (st == 0u) st = ST_TIMEOUT_BARRIER;
       if (atomicCAS(&R.n_global[kResStatus], 0u, st) == 0u) {
@@ -79,7 +78,6 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
       c = kcap;
     }
     counts[q] = c;
-    if (cta == 0) seg_counts[q] = c;
   }
   __syncthreads();
   if (!sh.ok) { fail(); return; }
@@ -91,10 +89,13 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
       other[i] = make_uint4(0u, 0u, 0u, 0u);
   }
   if (!reselect) {
-    if (!bar.sync(535)) { fail(); return; }  // every CTA has read the epoch word
-    if (cta == 0 && threadIdx.x == 0) {
-      if (aborted(ctrl)) fail();
-      else *R.epoch = epoch + 1u;
+    if (bar.last_arrival()) {  // every CTA has read the epoch word
+      if (aborted(ctrl)) {
+        fail();
+      } else {
+        for (unsigned int q = 0; q < P; ++q) seg_counts[q] = counts[q];
+        *R.epoch = epoch + 1u;
+      }
     }
     return;
   }
@@ -175,8 +176,11 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
   if (!band_select_kth(sh.sel, bar, k, pred, ctrl->hist[0], &ctrl->live[0], visit, &th, 580)) { fail(); return; }
   Pair* G = R.gout + (size_t)parity * kcap;
   int32_t* map = R.map;
-  auto on_placed = [&](Pair e, unsigned int pos) { map[e.idx] = (int32_t)pos; };
-  StagedAppender app{&sh.sel, G, &ctrl->cursor[0], kcap, ctrl};
+  auto on_placed = [&](Pair e, unsigned int pos) {
+    st_pair(&G[pos], e);
+    map[e.idx] = (int32_t)pos;
+  };
+  StagedAppender app{&sh.sel, &ctrl->cursor[0], kcap, ctrl};
   app.begin();
   const unsigned int trips = (n_a + stride - 1) / stride;
   for (unsigned int t = 0; t < trips; ++t) {
@@ -192,11 +196,11 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
   unsigned int n_g = __ldcg(&ctrl->cursor[0]);
   if (n_g > kcap) n_g = kcap;
   put_back(R.sel, n_sel, G, n_g, R.map, R.resid, d, cta, nct);
-  if (!bar.sync(595)) { fail(); return; }
-  if (cta == 0 && threadIdx.x == 0) {
+  if (bar.last_arrival()) {
     if (aborted(ctrl)) {
       fail();
     } else {
+      for (unsigned int q = 0; q < P; ++q) seg_counts[q] = counts[q];
       R.n_global[kResCount] = n_g;
       *R.epoch = epoch + 1u;
     }

@@ -24,6 +24,7 @@ struct Threshold {
   uint32_t key;        // bit pattern of the k-th largest magnitude
   uint32_t quota;      // how many entries equal to key are still selected
   bool select_all;     // fewer live entries than k: everything is selected
+  unsigned int n;      // how many entries are selected
 };
 
 __device__ __forceinline__ void smem_hist_clear(SelectShared& s) {
@@ -113,6 +114,7 @@ __device__ __forceinline__ bool band_select_kth(SelectShared& s, RankBarrier& ba
   out->quota = 0u;
   find_digit_in<kHistBins>(s, set[0], k);
   out->select_all = s.res_total <= k;  // not more live entries than k: keep them all
+  out->n = out->select_all ? s.res_total : k;
   const unsigned int bin = s.res_digit;
   unsigned int k_rem = s.res_krem;
   __syncthreads();
@@ -165,9 +167,9 @@ __device__ __forceinline__ bool band_select_kth(SelectShared& s, RankBarrier& ba
 
 // CTA-wide staged append.  Call put() from any thread, then end_tile() from all
 // threads once per loop trip (at most kSelThreads puts between two end_tile calls).
+// place(pair, position) stores an entry.
 struct StagedAppender {
   SelectShared* s;
-  Pair* out;             // may be peer memory
   unsigned int* cursor;  // global cursor (local memory)
   unsigned int cap;
   Ctrl* ctrl;
@@ -180,8 +182,8 @@ struct StagedAppender {
     const unsigned int pos = atomicAdd(&s->stage_n, 1u);
     s->stage[pos] = p;
   }
-  template <typename OnPlaced>
-  __device__ __forceinline__ void flush(OnPlaced on_placed) {
+  template <typename Place>
+  __device__ __forceinline__ void flush(Place place) {
     __syncthreads();
     const unsigned int n = s->stage_n;
     if (n) {
@@ -190,22 +192,18 @@ struct StagedAppender {
       const unsigned int base = s->stage_base;
       for (unsigned int i = threadIdx.x; i < n; i += kSelThreads) {
         const unsigned int pos = base + i;
-        if (pos < cap) {
-          st_pair(&out[pos], s->stage[i]);
-          on_placed(s->stage[i], pos);
-        } else {
-          record_error(ctrl, ST_CAPACITY, 900);
-        }
+        if (pos < cap) place(s->stage[i], pos);
+        else record_error(ctrl, ST_CAPACITY, 900);
       }
       __syncthreads();
       if (threadIdx.x == 0) s->stage_n = 0u;
     }
     __syncthreads();
   }
-  template <typename OnPlaced>
-  __device__ __forceinline__ void end_tile(OnPlaced on_placed) {
+  template <typename Place>
+  __device__ __forceinline__ void end_tile(Place place) {
     __syncthreads();
-    if (s->stage_n > (unsigned int)(kStageCap - kSelThreads)) flush(on_placed);
+    if (s->stage_n > (unsigned int)(kStageCap - kSelThreads)) flush(place);
   }
 };
 

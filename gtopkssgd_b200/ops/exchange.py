@@ -123,7 +123,7 @@ class ExchangeRank:
         self.with_allgather = with_allgather
         self.work_cap = self.kcap * (world if reselect else 1)
         self.work0 = torch.empty((self.work_cap, 2), dtype=torch.int32, device=dev)
-        self.work1 = torch.empty((self.kcap, 2), dtype=torch.int32, device=dev)
+        self.work1 = torch.empty((2 * self.kcap, 2), dtype=torch.int32, device=dev)
         self.map = torch.zeros(self.numel, dtype=torch.int32, device=dev)
         # two control blocks: the gTop-k kernel alternates between them and cleans the idle one itself
         self.ctrl_words = int(L.gtk_ctrl_bytes()) // 4
@@ -186,7 +186,7 @@ class ExchangeRank:
         self.result_words.zero_()
         self.result_host.zero_()
         self.ctrl.zero_()
-        self.region.tensor()[self.layout[3]:].zero_()   # flags and flagged entries that bear the failed call's number
+        self.region.tensor().zero_()   # entries, flags and flagged entries of the failed call
 
     def last_ctrl(self) -> torch.Tensor:
         """Control block that the last completed gTop-k call used (synchronises)."""
@@ -226,15 +226,15 @@ def default_nctas(k: int, nranks: int = 1, sms: int = 148) -> int:
     * up to 4 K union entries of the tree: one CTA, the set in shared memory
       (two ranks: 10 us at k = 1 000 and 16 us at 2 000, against 23 and 25 us
       with a cluster; 26 against 25 us at 3 000);
-    * up to 32 K union entries: a power-of-two cluster of 2..16 CTAs joined by
+    * up to 20 K union entries: a power-of-two cluster of 2..16 CTAs joined by
       the hardware cluster barrier, about 1024 entries per CTA (four ranks, k =
-      14 700: 41 us with 16 CTAs, 45 to 50 us with 24 to 74 and the software
-      barrier);
+      6 500: 27 us with 16 CTAs, 29 to 33 us with 24 to 74 and the software
+      barrier; k = 13 000: 34 and 32 us);
     * above: one CTA per 768 entries with the software barrier, as many as the
       device holds one per SM, and two per SM where each of those had more than
-      2 000 entries (eight ranks, k = 40 000: 112 us with 37 CTAs, 129 with 18;
-      two ranks, k = 255 570: 84 us with 148, 97 with 74; but k = 66 000: 45 us
-      with 148, 43 with 74)."""
+      2 000 entries (eight ranks, k = 40 000: 97 us with 37 CTAs, 115 with 18;
+      two ranks, k = 255 570: 74 us with 148, 82 with 74; k = 66 000: 31 us
+      with either)."""
     return 1 if k <= SMALL_MAX_K else _spread_nctas(2 * k, nranks, sms)
 
 
@@ -242,7 +242,7 @@ def _spread_nctas(n_u: int, nranks: int, sms: int = 148) -> int:
     """CTAs per rank for ``n_u`` entries shared out in global memory."""
     if n_u <= 3072:
         return 1
-    if n_u <= 32768:
+    if n_u <= 20480:
         n = 2
         while n < 16 and n * 1024 < n_u:
             n *= 2
@@ -285,10 +285,11 @@ def launch_allgather(ranks: Sequence[ExchangeRank], desc: torch.Tensor, seg_coun
 def decode_k2_trace(tr: dict, rank: int, world: int) -> dict:
     """Turns the %globaltimer stamps that CTA 0 of a rank leaves in its control block
     (slot 0: start; 1 + 8r + j for tree round r: j = 0 before / 1 after the wait for the
-    partner's flag, 2 table complete, 3 join done, 4 threshold known, 5 compaction done,
-    6 pushed (round-0 sender), 7 flag raised; 40 global set here, 41 its table built,
-    42 put-back done) into microseconds: ``total``, ``wait`` (time inside flag waits:
-    partner or root not there yet), ``work`` = total - wait, and per-phase entries."""
+    partner's count, 2 its first entries in and the table complete, 3 join done, 4 threshold
+    known, 5 compaction done, 6 pushed (round-0 sender), 7 the same; 40 and 41 the size of the
+    global set known, 42 set in and put-back done) into microseconds: ``total``, ``wait`` (time
+    until a partner's count is there, for the root's including the own put-back meanwhile),
+    ``work`` = total - wait, and per-phase entries."""
     if 42 not in tr:
         return {"complete": False}
     us = lambda a, b: (tr[b] - tr[a]) / 1e3 if a in tr and b in tr else 0.0
