@@ -1,5 +1,5 @@
 // Device-side pieces shared by the two sparse exchange kernels (K2: gTop-k tree,
-// K2t: Top-k all-gather): the per-rank descriptor, peer pushes with flags, the
+// K2t: Top-k all-gather): the per-rank descriptor, the wire words, flags, the
 // direct-address merge of two sparse sets, and the residual put-back.
 //
 // Merging without sorting: each rank owns an int32 table `map` of d entries.
@@ -18,6 +18,7 @@ namespace gtk {
 // overwrites what a slow reader of call e still needs.
 //   slots : [2][kMaxRounds + 1][kcap] wire words   receive slot of each tree round and of the broadcast
 //   ag    : [2][kMaxPeers][kcap] pairs    all-gather slots, one per source rank (K2t only)
+//   wire  : [2][kMaxPeers][kcap] wire words   the same for the re-selecting form (K2t only)
 //   gout  : [2][kcap] pairs               the global top-k set
 //   flags : [2][kFlagsPerParity] u64      (epoch << 32) | count
 //   ll    : [2][kMaxRounds + 1][kLLMaxK] 16-byte entries with their epoch (k2_tree_small.cu); the last
@@ -33,11 +34,14 @@ __host__ __device__ constexpr size_t ll_off(unsigned int parity, unsigned int ro
 struct K2Rank {
   const Pair* sel;        // local selection written by K1
   const K1State* st;      // st->n_sel = number of local pairs
-  Pair* work[2];          // [kcap_work] and [2 * kcap] merge buffers; the second half of work[1] holds received entries
+  // Merge buffers.  Tree: [kcap] and [2 * kcap] pairs, the second half of work[1] for received entries.  K2t:
+  // work[0] is the union [work_cap], work[1] holds a word per entry of it.
+  Pair* work[2];
   int32_t* map;           // [d] direct-address table
   float* resid;           // [d] residual
   unsigned long long* slots;  // local symmetric buffers
   Pair* ag;
+  unsigned long long* wire;
   Pair* gout;
   uint64_t* flags;
   ulonglong2* ll;
@@ -47,6 +51,7 @@ struct K2Rank {
                           // adds one after its last barrier, so a replayed CUDA graph needs no new argument
   unsigned long long* peer_slots[kMaxPeers];
   Pair* peer_ag[kMaxPeers];
+  unsigned long long* peer_wire[kMaxPeers];
   uint64_t* peer_flags[kMaxPeers];
   ulonglong2* peer_ll[kMaxPeers];
 };
@@ -127,16 +132,6 @@ __device__ __forceinline__ size_t flag_off(unsigned int parity, unsigned int whi
   return (size_t)parity * kFlagsPerParity + which;
 }
 
-// All CTAs of the rank copy n pairs to dst (peer or local memory).  The caller
-// then calls cta_fence_peer_stores(), passes the rank barrier, and one thread
-// publishes the data with release_flag().
-__device__ __forceinline__ void push_pairs(Pair* dst, const Pair* src, unsigned int n,
-                                           unsigned int cta, unsigned int nct) {
-  const unsigned int stride = nct * kSelThreads;
-  for (unsigned int i = cta * kSelThreads + threadIdx.x; i < n; i += stride)
-    st_pair(&dst[i], ld_pair_cg(&src[i]));
-}
-
 // Called by all threads of a CTA of a multi-CTA rank after its last store into peer memory of a phase
 // and before the rank's barrier: one thread issues a system-scope fence on behalf of the CTA (the
 // __syncthreads orders the other threads' stores before it).  By the PTX memory model the flag's own
@@ -171,21 +166,6 @@ __device__ __forceinline__ bool cta_wait_flag(ExchangeShared& sh, const uint64_t
   __syncthreads();
   *count = sh.payload;
   return sh.ok != 0;
-}
-
-// A <- copy of src, map[idx] = position, and tally(value, 1) for each.
-template <typename Tally>
-__device__ __forceinline__ void copy_and_map(Pair* A, const Pair* src, unsigned int n, int32_t* map,
-                                             unsigned int d, unsigned int cta, unsigned int nct,
-                                             Ctrl* ctrl, Tally tally) {
-  const unsigned int stride = nct * kSelThreads;
-  for (unsigned int i = cta * kSelThreads + threadIdx.x; i < n; i += stride) {
-    const Pair e = ld_pair_cg(&src[i]);
-    st_pair(&A[i], e);
-    tally(e.val, 1u);
-    if ((unsigned int)e.idx < d) map[e.idx] = (int32_t)i;
-    else record_error(ctrl, ST_BOUNDS, 300);
-  }
 }
 
 // Residual put-back (compression.py:66-75 in the reference): every locally

@@ -38,7 +38,8 @@
 // publish an EMPTY global set (n_global = 0, so the consumer applies nothing) and
 // a sticky status in the result words; the call counter is not advanced and every
 // later call returns at once with an empty set until the host has rebuilt the
-// exchange.
+// exchange.  A rank that has put its selection back by then keeps it in the
+// residual, as an empty global set asks for.
 #include <cstddef>
 #include "exchange_common.cuh"
 
@@ -431,14 +432,14 @@ static unsigned long long ll_offset(unsigned long long flags) {
   return (flags + 2ull * kFlagsPerParity * sizeof(uint64_t) + 255ull) & ~255ull;
 }
 
-// Symmetric-region geometry, in bytes, for a given kcap: offsets of slots, ag,
-// gout and flags, and the total size.  out[0..4] = {slots, ag, gout, flags, total}.
+// Symmetric-region geometry, in bytes, for a given kcap: offsets of slots, ag (the wire
+// words behind it), gout and flags, and the total size.  out[0..4] = {slots, ag, gout, flags, total}.
 extern "C" void gtk_symm_layout(unsigned int kcap, int with_allgather, unsigned long long* out) {
   unsigned long long off = 0;
   out[0] = off;
   off += 2ull * (kMaxRounds + 1) * kcap * sizeof(Pair);
   out[1] = off;
-  if (with_allgather) off += 2ull * kMaxPeers * kcap * sizeof(Pair);
+  if (with_allgather) off += 2ull * kMaxPeers * kcap * (sizeof(Pair) + sizeof(unsigned long long));
   out[2] = off;
   off += 2ull * kcap * sizeof(Pair);
   off = (off + 255ull) & ~255ull;
@@ -466,6 +467,8 @@ extern "C" int gtk_k2rank_fill(void* desc_host, const void* sel, const void* st,
   char* base = (char*)symm_local;
   r->slots = (unsigned long long*)(base + lay[0]);
   r->ag = (Pair*)(base + lay[1]);
+  const unsigned long long wire = lay[1] + 2ull * kMaxPeers * kcap * sizeof(Pair);
+  r->wire = (unsigned long long*)(base + wire);
   r->gout = (Pair*)(base + lay[2]);
   r->flags = (uint64_t*)(base + lay[3]);
   r->ll = (ulonglong2*)(base + ll_offset(lay[3]));
@@ -476,6 +479,7 @@ extern "C" int gtk_k2rank_fill(void* desc_host, const void* sel, const void* st,
     char* pb = q < P ? (char*)symm_peers[q] : nullptr;
     r->peer_slots[q] = pb ? (unsigned long long*)(pb + lay[0]) : nullptr;
     r->peer_ag[q] = pb ? (Pair*)(pb + lay[1]) : nullptr;
+    r->peer_wire[q] = pb ? (unsigned long long*)(pb + wire) : nullptr;
     r->peer_flags[q] = pb ? (uint64_t*)(pb + lay[3]) : nullptr;
     r->peer_ll[q] = pb ? (ulonglong2*)(pb + ll_offset(lay[3])) : nullptr;
   }

@@ -10,11 +10,23 @@
 //         return to the residual.  Here the P lists are merged in rank order
 //         (same arithmetic on every rank, so all ranks get the same set) with
 //         the direct-address table, then radix-selected.
+//
+// What bounds topk2: a barrier per merged list and three round trips between
+// them (table, entry, append).  The lists travel as the tree's 8-byte wire words,
+// so nobody fences or waits for a complete list, and a merged entry remembers
+// where in the own selection it comes from, so that dropping it is also its way
+// back to the residual.  Four ranks, k = 14 728: 41 us with flags behind fenced
+// stores, the put-back behind a table over the global set and one entry per thread
+// in flight, 35 now (eight ranks, k = 20 000: 113 and 97; two, k = 660 340: 256 and
+// 182).
 #include "exchange_common.cuh"
 
 namespace gtk {
 
-__global__ void __launch_bounds__(kSelThreads)
+constexpr int kBatch = 4;                         // entries per thread whose loads are in flight together
+constexpr unsigned int kNotOwn = 0xffffffffu;
+
+__global__ void __launch_bounds__(kSelThreads, 2)
 k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsigned int P,
                    unsigned int k, unsigned int kcap, unsigned int work_cap, unsigned int d,
                    int reselect, unsigned int* __restrict__ seg_counts_all,
@@ -54,15 +66,29 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
   unsigned int n_sel = R.st->n_sel;
   if (n_sel > kcap) n_sel = kcap;
 
-  // push my selection into slot[me] of every rank (my own included)
-  for (unsigned int q = 0; q < P; ++q) {
-    Pair* dst = (q == me ? R.ag : R.peer_ag[q]) + ag_off(parity, me, kcap);
-    push_pairs(dst, R.sel, n_sel, cta, nct);
+  const unsigned int stride = nct * kSelThreads;
+  const unsigned int lane0 = cta * kSelThreads + threadIdx.x;
+
+  // push my selection into slot[me] of every rank (topk: my own included)
+  if (reselect) {  // words that say themselves that they have arrived, in no order with the counts
+    if (cta == 0 && threadIdx.x < P && threadIdx.x != me)
+      st_relaxed_sys_u64(reinterpret_cast<unsigned long long*>(R.peer_flags[threadIdx.x] + flag_off(parity, kFlagAg0 + me)),
+                         ((unsigned long long)epoch << 32) | n_sel);
+    for (unsigned int i = lane0; i < n_sel; i += stride) {
+      const Pair e = ld_pair_cg(&R.sel[i]);
+      for (unsigned int q = 0; q < P; ++q)
+        if (q != me) wire_store(R.peer_wire[q] + ag_off(parity, me, kcap) + i, e);
+    }
+  } else {
+    for (unsigned int i = lane0; i < n_sel; i += stride) {
+      const Pair e = ld_pair_cg(&R.sel[i]);
+      for (unsigned int q = 0; q < P; ++q) st_pair(R.peer_ag[q] + ag_off(parity, me, kcap) + i, e);
+    }
+    cta_fence_peer_stores(nct == 1);
+    if (!bar.sync(500)) { fail(); return; }
+    if (cta == 0 && threadIdx.x < P && threadIdx.x != me)  // one releasing thread per destination
+      release_flag(R.peer_flags[threadIdx.x] + flag_off(parity, kFlagAg0 + me), epoch, n_sel);
   }
-  cta_fence_peer_stores(nct == 1);
-  if (!bar.sync(500)) { fail(); return; }
-  if (cta == 0 && threadIdx.x < P && threadIdx.x != me)  // one releasing thread per destination
-    release_flag(R.peer_flags[threadIdx.x] + flag_off(parity, kFlagAg0 + me), epoch, n_sel);
   // wait for every source, one polling thread for each
   if (threadIdx.x == 0) sh.ok = 1;
   __syncthreads();
@@ -105,57 +131,104 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
   for (int i = threadIdx.x; i < kHistBins; i += kSelThreads) band[i] = 0u;
   __syncthreads();
   auto tally = [&](float v, unsigned int delta) { atomicAdd(&band[band_bin(mag_key(v), pred)], delta); };
-  Pair* A = R.work[0];
-  const Pair* L0 = R.ag + ag_off(parity, 0, kcap);
-  copy_and_map(A, L0, counts[0], R.map, d, cta, nct, ctrl, tally);
-  unsigned int n_a = counts[0];
-  if (cta == 0 && threadIdx.x == 0) ctrl->n_live = n_a;
-  if (!bar.sync(540)) { fail(); return; }
-  const unsigned int stride = nct * kSelThreads;
-  for (unsigned int q = 1; q < P; ++q) {
-    const Pair* B = R.ag + ag_off(parity, q, kcap);
-    const unsigned int n_b = counts[q];
-    const unsigned int trips = (n_b + stride - 1) / stride;
-    for (unsigned int t = 0; t < trips; ++t) {
-      const unsigned int j = t * stride + cta * kSelThreads + threadIdx.x;
-      bool append = false;
-      Pair e;
-      e.idx = -1;
-      e.val = 0.f;
-      if (j < n_b) {
-        e = ld_pair_cg(&B[j]);
-        if ((unsigned int)e.idx >= d) {
+  Pair* const A = R.work[0];
+  int32_t* const map = R.map;
+  unsigned int* const own = reinterpret_cast<unsigned int*>(R.work[1]);  // A's entry i: where in the own selection, or kNotOwn
+  Pair c[kBatch];
+  // Takes trips t0 .. t0 + kBatch - 1 of list q into c[] (idx -1: none); slot q keeps them as in topk.
+  auto fetch = [&](unsigned int q, unsigned int t0) {
+    const unsigned int n = counts[q];
+    unsigned int want = 0;
+    bool ok = true;
+#pragma unroll
+    for (int t = 0; t < kBatch; ++t) {
+      const unsigned int j = (t0 + t) * stride + lane0;
+      c[t].idx = -1;
+      c[t].val = 0.f;
+      if (j < n) want |= 1u << t;
+    }
+    if (q != me) {
+      ok = wire_receive(R.wire + ag_off(parity, q, kcap), want,
+                        [&](int t) { return (size_t)((t0 + t) * stride + lane0); }, c, d, ctrl, limit_ns, 510 + q);
+    } else {
+#pragma unroll
+      for (int t = 0; t < kBatch; ++t) {
+        if (!(want & (1u << t))) continue;
+        c[t] = ld_pair_cg(&R.sel[(t0 + t) * stride + lane0]);
+        if ((unsigned int)c[t].idx >= d) {
           record_error(ctrl, ST_BOUNDS, 550);
-        } else {
-          append = true;
-          const unsigned int p = (unsigned int)__ldcg(&R.map[e.idx]);
-          if (p < n_a) {
-            const Pair a = ld_pair_cg(&A[p]);
-            if (a.idx == e.idx) {
-              const float sum = a.val + e.val;
-              A[p].val = sum;
-              tally(a.val, 0xffffffffu);
-              tally(sum, 1u);
-              append = false;
-            }
-          }
+          c[t].idx = -1;
         }
       }
-      const unsigned int m = __ballot_sync(0xffffffffu, append);
-      if (m) {
-        unsigned int base = 0;
-        if (lane_id() == (unsigned int)(__ffs(m) - 1)) base = atomicAdd(&ctrl->n_live, __popc(m));
-        base = __shfl_sync(0xffffffffu, base, __ffs(m) - 1);
-        if (append) {
-          const unsigned int pos = base + __popc(m & lanemask_lt());
+    }
+    Pair* const slot = R.ag + ag_off(parity, q, kcap);
+#pragma unroll
+    for (int t = 0; t < kBatch; ++t)
+      if (want & (1u << t)) st_pair(&slot[(t0 + t) * stride + lane0], c[t]);
+    return ok;
+  };
+  // Entries that list q adds are counted in scratch[q mod 3]: the union's size before the list must not move
+  // while slower CTAs read it, or a look-up could take an entry of an earlier call for one of this.  The word of
+  // list q + 1 was last read before the barrier behind list q - 1.
+  unsigned int n_a = 0;
+  for (unsigned int q = 0; q < P; ++q) {
+    unsigned int* const added = &ctrl->scratch[q % 3u];
+    const unsigned int trips = (counts[q] + stride - 1) / stride;
+    // a list's first entries come in while the one before is being completed
+    if (!__syncthreads_and(fetch(q, 0))) { fail(); return; }
+    if (q != 0u) {
+      if (!bar.wait(560 + q)) { fail(); return; }
+      n_a += __ldcg(&ctrl->scratch[(q - 1u) % 3u]);
+      if (n_a > work_cap) n_a = work_cap;
+    }
+    if (cta == 0 && threadIdx.x == 0) ctrl->scratch[(q + 1u) % 3u] = 0u;
+    for (unsigned int t0 = 0; t0 < trips; t0 += kBatch) {
+      if (t0 != 0u && !__syncthreads_and(fetch(q, t0))) { fail(); return; }
+      unsigned int pm[kBatch], fresh[kBatch];
+      Pair a[kBatch];
+#pragma unroll
+      for (int t = 0; t < kBatch; ++t) {
+        pm[t] = 0xffffffffu;
+        if (q != 0u && c[t].idx >= 0) pm[t] = (unsigned int)__ldcg(&map[c[t].idx]);
+      }
+#pragma unroll
+      for (int t = 0; t < kBatch; ++t) {
+        a[t].idx = -1;
+        a[t].val = 0.f;
+        if (pm[t] < n_a) a[t] = ld_pair_cg(&A[pm[t]]);
+      }
+      unsigned int n_fresh = 0;  // of this warp
+#pragma unroll
+      for (int t = 0; t < kBatch; ++t) {
+        const bool shared = c[t].idx >= 0 && a[t].idx == c[t].idx;
+        if (shared) {
+          const float sum = a[t].val + c[t].val;
+          A[pm[t]].val = sum;
+          if (q == me) own[pm[t]] = (t0 + t) * stride + lane0;
+          tally(a[t].val, 0xffffffffu);
+          tally(sum, 1u);
+          c[t].idx = -1;
+        }
+        fresh[t] = __ballot_sync(0xffffffffu, c[t].idx >= 0);
+        n_fresh += __popc(fresh[t]);
+      }
+      unsigned int base = 0;
+      if (n_fresh && lane_id() == 0) base = n_a + atomicAdd(added, n_fresh);
+      base = __shfl_sync(0xffffffffu, base, 0);
+#pragma unroll
+      for (int t = 0; t < kBatch; ++t) {
+        if (c[t].idx >= 0) {
+          const unsigned int pos = base + __popc(fresh[t] & lanemask_lt());
           if (pos < work_cap) {
-            st_pair(&A[pos], e);
-            R.map[e.idx] = (int32_t)pos;
-            tally(e.val, 1u);
+            st_pair(&A[pos], c[t]);
+            own[pos] = q == me ? (t0 + t) * stride + lane0 : kNotOwn;
+            map[c[t].idx] = (int32_t)pos;
+            tally(c[t].val, 1u);
           } else {
             record_error(ctrl, ST_CAPACITY, 551);
           }
         }
+        base += __popc(fresh[t]);
       }
     }
     if (q + 1u == P) {  // the sums are final: publish this CTA's counts
@@ -165,37 +238,70 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
         if (n) atomicAdd(&ctrl->hist[0][0][i], n);
       }
     }
-    if (!bar.sync(560 + q)) { fail(); return; }
-    n_a = __ldcg(&ctrl->n_live);
-    if (n_a > work_cap) n_a = work_cap;
+    bar.arrive();
   }
+  if (!bar.wait(560 + P)) { fail(); return; }
+  n_a += __ldcg(&ctrl->scratch[(P - 1u) % 3u]);
+  if (n_a > work_cap) n_a = work_cap;
+  const unsigned int trips = (n_a + stride - 1) / stride;
+  auto load = [&](Pair (&e)[kBatch], unsigned int t0) {
+#pragma unroll
+    for (int t = 0; t < kBatch; ++t) {
+      const unsigned int i = (t0 + t) * stride + lane0;
+      e[t].idx = -1;
+      e[t].val = 0.f;
+      if (i < n_a) e[t] = ld_pair_cg(&A[i]);
+    }
+  };
+  load(c, 0);  // kept in registers for both sweeps
   auto visit = [&](auto f) {
-    for (unsigned int i = cta * kSelThreads + threadIdx.x; i < n_a; i += stride) f(mag_key(ld_pair_cg(&A[i]).val));
+#pragma unroll
+    for (int t = 0; t < kBatch; ++t)
+      if (c[t].idx >= 0) f(mag_key(c[t].val));
+    for (unsigned int t0 = kBatch; t0 < trips; t0 += kBatch) {
+      Pair e[kBatch];
+      load(e, t0);
+#pragma unroll
+      for (int t = 0; t < kBatch; ++t)
+        if (e[t].idx >= 0) f(mag_key(e[t].val));
+    }
   };
   Threshold th;
   if (!band_select_kth(sh.sel, bar, k, pred, ctrl->hist[0], &ctrl->live[0], visit, &th, 580)) { fail(); return; }
-  Pair* G = R.gout + (size_t)parity * kcap;
-  int32_t* map = R.map;
-  auto on_placed = [&](Pair e, unsigned int pos) {
-    st_pair(&G[pos], e);
-    map[e.idx] = (int32_t)pos;
-  };
+  Pair* const G = R.gout + (size_t)parity * kcap;
+  auto on_placed = [&](Pair e, unsigned int pos) { st_pair(&G[pos], e); };
   StagedAppender app{&sh.sel, &ctrl->cursor[0], kcap, ctrl};
   app.begin();
-  const unsigned int trips = (n_a + stride - 1) / stride;
-  for (unsigned int t = 0; t < trips; ++t) {
-    const unsigned int i = t * stride + cta * kSelThreads + threadIdx.x;
-    if (i < n_a) {
-      const Pair e = ld_pair_cg(&A[i]);
-      if (passes_threshold(mag_key(e.val), th, &ctrl->tie[0])) app.put(e);
+  auto sweep = [&](const Pair (&e)[kBatch], unsigned int t0) {
+    unsigned int from[kBatch];
+    float back[kBatch];
+#pragma unroll
+    for (int t = 0; t < kBatch; ++t) {
+      from[t] = kNotOwn;
+      if (e[t].idx >= 0) {
+        if (passes_threshold(mag_key(e[t].val), th, &ctrl->tie[0])) app.put(e[t]);
+        else from[t] = __ldcg(&own[(t0 + t) * stride + lane0]);
+      }
+      if (t0 + t < trips) app.end_tile(on_placed);
     }
-    app.end_tile(on_placed);
+    // what drops out of the sum although this rank had selected it goes back to its residual
+#pragma unroll
+    for (int t = 0; t < kBatch; ++t) {
+      back[t] = 0.f;
+      if (from[t] != kNotOwn) back[t] = R.resid[e[t].idx] + R.sel[from[t]].val;
+    }
+#pragma unroll
+    for (int t = 0; t < kBatch; ++t)
+      if (from[t] != kNotOwn) R.resid[e[t].idx] = back[t];
+  };
+  sweep(c, 0);
+  for (unsigned int t0 = kBatch; t0 < trips; t0 += kBatch) {
+    Pair e[kBatch];
+    load(e, t0);
+    sweep(e, t0);
   }
   app.flush(on_placed);
-  if (!bar.sync(590)) { fail(); return; }
-  unsigned int n_g = __ldcg(&ctrl->cursor[0]);
-  if (n_g > kcap) n_g = kcap;
-  put_back(R.sel, n_sel, G, n_g, R.map, R.resid, d, cta, nct);
+  const unsigned int n_g = th.n < kcap ? th.n : kcap;
   if (bar.last_arrival()) {
     if (aborted(ctrl)) {
       fail();

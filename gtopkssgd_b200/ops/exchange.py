@@ -123,7 +123,7 @@ class ExchangeRank:
         self.with_allgather = with_allgather
         self.work_cap = self.kcap * (world if reselect else 1)
         self.work0 = torch.empty((self.work_cap, 2), dtype=torch.int32, device=dev)
-        self.work1 = torch.empty((2 * self.kcap, 2), dtype=torch.int32, device=dev)
+        self.work1 = torch.empty((max(2 * self.kcap, (self.work_cap + 1) // 2), 2), dtype=torch.int32, device=dev)
         self.map = torch.zeros(self.numel, dtype=torch.int32, device=dev)
         # two control blocks: the gTop-k kernel alternates between them and cleans the idle one itself
         self.ctrl_words = int(L.gtk_ctrl_bytes()) // 4

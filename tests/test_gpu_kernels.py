@@ -599,3 +599,44 @@ def test_k1_select_reads_one_tensor_per_parameter(sizes, k):
         sel.select_segments([0 if i == missing else t.data_ptr() for i, t in enumerate(grads)], table, r, k)
         assert sel.status() == (0, 0)
         _check_selection(*sel.pairs(), r, acc, k)
+
+
+@pytest.mark.parametrize("mode,P,k,nctas", [("topk2", 2, 9000, 2), ("topk2", 3, 4097, 1), ("topk2", 5, 2500, 4),
+                                            ("gtopk", 2, 4097, 2), ("gtopk", 2, 9000, 4), ("gtopk", 4, 9000, 3)])
+def test_exchange_of_the_same_indices_over_again(mode, P, k, nctas):
+    """More entries per thread than its registers hold, and call after call with
+    the same selections: received words, look-up tables and merge buffers still
+    carry the same indices from the calls before, at other positions."""
+    from gtopkssgd_b200.ops import exchange as ex
+    d = 40000
+    torch.manual_seed(P * k)
+    ranks, desc = _emulated_world(P, d, k, mode)
+    seg_counts = torch.zeros(P * ex.MAX_PEERS, dtype=torch.int32, device=DEV)
+    common = torch.randn(d, device=DEV)
+    grads = [common + torch.randn(d, device=DEV) for _ in range(P)]
+    res_ref = [torch.zeros(d) for _ in range(P)]
+    if mode == "topk2":
+        local = [oracle.compress(g.cpu(), rr, k) for g, rr in zip(grads, res_ref)]
+        gi, gv = oracle.topk2_reselect(local, k)
+        for rr, loc in zip(res_ref, local):
+            oracle.put_back(rr, loc, gi)
+    else:
+        (gi, gv), _ = oracle.simulate_gtopk_step([g.cpu() for g in grads], res_ref, k)
+    order = torch.argsort(gi)
+    for call in range(6):
+        for r, g in zip(ranks, grads):
+            r.resid.zero_()
+            r.selector.select(g, r.resid, k)
+        if mode == "topk2":
+            ex.launch_allgather(ranks, desc, seg_counts, 0, P, k, reselect=True, nctas=nctas, limit_ms=2000)
+        else:
+            ex.launch_gtopk(ranks, desc, 0, P, k, nctas=nctas, limit_ms=2000)
+        torch.cuda.synchronize()
+        for r in ranks:
+            assert r.status() == (0, 0)
+            qi, qv = _read_gout(r, r.last_parity())
+            o = torch.argsort(qi)
+            assert torch.equal(qi[o].cpu().long(), gi[order].long())
+            assert torch.allclose(qv[o].cpu(), gv[order], rtol=1e-5, atol=1e-6)
+            assert torch.allclose(r.resid.cpu(), res_ref[r.rank], rtol=1e-5, atol=1e-6)
+            assert r.region.guards_intact()
