@@ -45,8 +45,9 @@
 
 namespace gtk {
 
-// kK2Cache = union entries each thread keeps in registers across the phases of a round (template
-// parameter of the kernel: 4 by default, 8 when a 16-CTA cluster serves up to 64 K union entries).
+// Union entries that each thread keeps in registers across the phases of a round.  The default CTA counts leave
+// 2 to 4 per thread up to k of about 150 000; the rest is read again from memory, as many at a time.
+constexpr int kK2Cache = 4;
 
 struct K2Shared {
   ExchangeShared ex;
@@ -69,8 +70,7 @@ __device__ __forceinline__ void band_flush(K2Shared& sh, unsigned int* ghist) {
   __syncthreads();
 }
 
-template <int kK2Cache>
-__global__ void __launch_bounds__(kSelThreads, kK2Cache == 4 ? 2 : 1)
+__global__ void __launch_bounds__(kSelThreads, 2)
 k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsigned int P,
                   unsigned int k, unsigned int kcap, unsigned int d, unsigned long long limit_ns,
                   int use_cluster) {
@@ -486,29 +486,17 @@ extern "C" int gtk_k2rank_fill(void* desc_host, const void* sel, const void* st,
   return GTK_OK;
 }
 
-using K2Kernel = void (*)(const K2Rank*, unsigned int, unsigned int, unsigned int, unsigned int, unsigned int,
-                          unsigned long long, int);
-
-// Register-cache depth for a launch: 8 entries per thread when a cluster's threads would otherwise
-// have to re-read part of the union from memory in every phase, 4 otherwise.
-static int k2_cache_depth(unsigned int k, unsigned int nctas, int cluster) {
-  const unsigned long long per_thread4 = 4ull * nctas * kSelThreads;
-  return (cluster && 2ull * k > per_thread4) ? 8 : 4;
-}
-static K2Kernel k2_kernel(int depth) { return depth == 8 ? k2_gtopk_exchange<8> : k2_gtopk_exchange<4>; }
-
-static int k2_max_coresident(int depth) {
-  static int cached[2] = {0, 0};  // the occupancy query costs microseconds; the answer never changes
-  int& c = cached[depth == 8];
-  if (c) return c;
+static int k2_max_coresident() {
+  static int cached = 0;  // the occupancy query costs microseconds; the answer never changes
+  if (cached) return cached;
   const DeviceInfo* di = gtk_device_info();
   if (!di) return 0;
   int occ = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void*)k2_kernel(depth), kSelThreads, 0) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, (const void*)k2_gtopk_exchange, kSelThreads, 0) !=
       cudaSuccess)
     return 0;
-  c = occ * di->sms;
-  return c;
+  cached = occ * di->sms;
+  return cached;
 }
 
 // Largest cluster (CTAs of one rank joined by the hardware barrier) that `nranks` ranks can hold
@@ -521,29 +509,27 @@ static bool k2_cluster_fits(unsigned int nranks, unsigned int nctas) {
   c = 2;
   const DeviceInfo* di = gtk_device_info();
   if (!di || !di->cluster) return false;
-  for (int depth : {4, 8}) {
-    if (nctas > 8 && cudaFuncSetAttribute((const void*)k2_kernel(depth),
-                                          cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nctas, nranks);
-    cfg.blockDim = dim3(kSelThreads);
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = nctas;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int nclusters = 0;
-    if (cudaOccupancyMaxActiveClusters(&nclusters, (const void*)k2_kernel(depth), &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      return false;
-    }
-    if (nclusters < (int)nranks) return false;
+  if (nctas > 8 && cudaFuncSetAttribute((const void*)k2_gtopk_exchange,
+                                        cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
   }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(nctas, nranks);
+  cfg.blockDim = dim3(kSelThreads);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = nctas;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int nclusters = 0;
+  if (cudaOccupancyMaxActiveClusters(&nclusters, (const void*)k2_gtopk_exchange, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (nclusters < (int)nranks) return false;
   c = 1;
   return true;
 }
@@ -563,9 +549,8 @@ extern "C" int gtk_k2_exchange(const void* ranks_dev, unsigned int nranks, unsig
   if (k2_small_serves(nranks, k, nctas))
     return k2_small_launch(ranks, nranks, rank_base, P, k, kcap, d, limit_ns, stream);
   int cluster = (use_cluster && k2_cluster_fits(nranks, nctas)) ? 1 : 0;
-  const int depth = k2_cache_depth(k, nctas, cluster);
-  const K2Kernel fn = k2_kernel(depth);
-  if ((int)(nranks * nctas) > k2_max_coresident(depth)) return GTK_ERR_ARG;
+  const auto fn = k2_gtopk_exchange;
+  if ((int)(nranks * nctas) > k2_max_coresident()) return GTK_ERR_ARG;
   void* args[] = {&ranks, &rank_base, &P, &k, &kcap, &d, &limit_ns, &cluster};
   cudaError_t e;
   if (cluster) {
