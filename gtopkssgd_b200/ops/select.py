@@ -2,7 +2,7 @@
 
 ``TopkSelector`` owns the device buffers of one merged gradient group (the
 candidate list, the selected pairs, the persistent threshold state and the
-control block) and enqueues the K1 launch on the current stream.  On CPU
+control block) and enqueues the two K1 launches on the current stream.  On CPU
 tensors it runs the PyTorch oracle instead, with the same outputs.
 """
 from __future__ import annotations
@@ -93,9 +93,9 @@ class TopkSelector:
 
     def trace(self) -> dict:
         """Device-side phase stamps of the last select, in nanoseconds since its
-        start: slot 1 = CTA 0 finished its share of the stream pass, 2 = every CTA
-        did (grid barrier passed), 3 = k-th magnitude known, 4 = winners compacted
-        (3 and 4 only on the predicted-threshold path).  Synchronises."""
+        start: slot 1 = CTA 0 finished its share of the stream pass, 2 = the pick
+        began, 3 = k-th magnitude known (more than 64 K candidates), 4 = winners
+        compacted (2 to 4 only when the prediction held).  Synchronises."""
         if not self.is_cuda:
             return {}
         calls = int(self.state[5].item())
