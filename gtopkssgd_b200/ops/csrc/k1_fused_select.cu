@@ -55,12 +55,12 @@ constexpr int kWarpFlushAt = kWarpStage - 32;
 constexpr long long kDynamicMinVec = 5ll * 1000 * 1000;
 constexpr unsigned int kShards = 16;       // ticket counters of the dynamic stream pass
 // Up to kPickSmall candidates one CTA selects among them, up to kPickCluster one cluster of 8 CTAs, both from
-// registers; above, all CTAs share them out by tickets.  Measured at the borders (k1_pick alone): one CTA
-// 2.9 us at 2.6 K candidates and 2 us more than the cluster at 10 K; the cluster 9.3 us at 50 K as the tickets
-// at 100 K (whose phases cost 2 to 3 us of dependent global atomics and polls), but 27 us at 200 K, where 8
-// SMs are too few for the scattered write-back.
+// registers; above, all CTAs share them out by tickets.  Measured at the borders: one CTA 2.9 us at 2.6 K
+// candidates and 2 us more than the cluster at 10 K; the cluster as fast as the tickets at 35 K (9 us; whole call
+// at 14.7 M 31.3 and 31.5 us) and 3 us slower at 58 K (25.6 M: 60.8 and 58.2 us), where 8 SMs are too few for the
+// scattered write-back; the tickets 1 to 3.5 us slower at 8 K and 19 K.
 constexpr unsigned int kPickSmall = 4096;
-constexpr unsigned int kPickCluster = 65536;
+constexpr unsigned int kPickCluster = 32768;
 constexpr int kPickCtas = 8;               // CTAs per cluster
 
 // Bins of the first selection level: (key - lo) >> shift, the last bin open to the top.  lo is the candidate
@@ -396,6 +396,9 @@ struct Winners {
   float* dense;        // nullptr: pairs only
   long long* idx;
   float* val;
+  __device__ __forceinline__ Winners from(unsigned int pos) const {
+    return Winners{sel + pos, dense, idx ? idx + pos : nullptr, val ? val + pos : nullptr};
+  }
   __device__ __forceinline__ void put(unsigned int pos, Pair e) const {
     st_pair(&sel[pos], e);
     if (dense) {
@@ -689,11 +692,15 @@ k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Winners out, 
   int ph = 0;
   unsigned int k_rem = k;
   if (!exact_mode) {
-    // The candidates in chunks: the first level was counted by the stream pass (counted) or is counted here,
-    // the rest (one level of single keys, as a rule) and the compaction take a phase each.
+    // The candidates in chunks.  The first level was counted by the stream pass (counted) or is counted here.  As
+    // a rule the threshold's bin then holds few enough entries (300 to 1 400) to leave them to one CTA: a single
+    // sweep sends what lies above the bin to the list, returns what lies below to r, and puts what lies in it
+    // aside; the CTA that finishes the sweep picks among those (against a level and a sweep more: whole call
+    // at 25.6 M and 0.01 63.9 -> 60.6 us, 66 M and 0.01 148.6 -> 144.2, 138 M and 0.01 294 -> 288).
+    // A bin with more is counted by finer levels, a phase each.
     const unsigned int nchunks = (C + kPickChunk - 1u) / kPickChunk;
     unsigned int* level_hist = ctrl->hist[0][0];
-    bool have = counted != 0;
+    bool have = counted != 0, aside = false;
     int row = 0;
     for (;;) {
       if (!have) {
@@ -717,11 +724,18 @@ k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Winners out, 
       find_bin(s, global_counts(level_hist), k_rem);
       k_rem = s.res_krem;
       if (!lv.narrow(s.res_bin)) break;
+      if (s.res_n <= kPickSmall) {
+        aside = true;
+        break;
+      }
       level_hist = ctrl->hist[0][++row];
       __syncthreads();
     }
     th = lv.lo;
-    if (threadIdx.x == 0) ctrl->trace[3] = globaltimer_ns();  // k-th magnitude known
+    const uint32_t top = aside ? lv.hi : lv.lo;
+    Pair* const between = reinterpret_cast<Pair*>(ctrl->hist[2]);  // (rows that K1 has no other use for)
+    static_assert(sizeof(ctrl->hist[2]) >= kPickSmall * sizeof(Pair), "room for the entries put aside");
+    if (threadIdx.x == 0) ctrl->trace[3] = globaltimer_ns();  // k-th magnitude known, or its bin
     unsigned int turn = 0;
     const unsigned int mine = for_chunks(s, ctrl, ph, nchunks, [&](unsigned int chunk) {
       Pair c[4];
@@ -735,7 +749,19 @@ k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Winners out, 
       }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        if (passes(c[j].idx >= 0, mag_key(c[j].val), th, k_rem, &ctrl->tie[0])) {
+        const uint32_t key = mag_key(c[j].val);
+        bool win;
+        if (aside) {
+          win = c[j].idx >= 0 && key > top;
+          if (c[j].idx >= 0 && key >= th && !win) {
+            const unsigned int at = atomicAdd(&ctrl->live[0], 1u);
+            if (at < kPickSmall) st_pair(&between[at], c[j]);
+            c[j].idx = -1;
+          }
+        } else {
+          win = passes(c[j].idx >= 0, key, th, k_rem, &ctrl->tie[0]);
+        }
+        if (win) {
           won |= 1u << j;
           ++n;
         }
@@ -743,7 +769,7 @@ k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Winners out, 
       unsigned int pos = place(s, n, &ctrl->cursor[0], turn++);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        if (c[j].idx < 0) break;
+        if (c[j].idx < 0) continue;
         if (won & (1u << j)) {
           if (pos < k) out.put(pos, c[j]);
           ++pos;
@@ -752,7 +778,20 @@ k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Winners out, 
         }
       }
     });
-    if (report(ctrl, ph, mine, nchunks)) {
+    const bool last = report(ctrl, ph, mine, nchunks);
+    if (aside) {
+      if (threadIdx.x == 0) s.ok = last ? 1 : 0;
+      __syncthreads();
+      if (!s.ok) return;
+      __threadfence();
+      const unsigned int n = __ldcg(&ctrl->live[0]);
+      Pair front;
+      front.idx = 0;
+      front.val = 0.f;
+      if (threadIdx.x < n) front = ld_pair_cg(&between[threadIdx.x]);
+      th = pick_small(s, r, between, out.from(k - k_rem), k_rem, n, lv, front);
+    }
+    if (last) {
       finish_state(st, was, th, k, k, count, C, false, target_ratio);
       ctrl->trace[4] = globaltimer_ns();  // all winners compacted
     }
@@ -896,9 +935,10 @@ int k1_launch_with(Stream stream_pass, float* r, long long d, unsigned int k, Pa
   const long long tile = (long long)kK1Threads * (dynamic ? 4 : 2);
   long long grid = (nvec + tile - 1) / tile;
   grid = grid < 1 ? 1 : (grid > full ? full : grid);
-  // The first level is counted on the fly where the candidates will be shared out by tickets; below, the CTAs
-  // that pick count faster than the stream pass publishes.
-  const bool counted = k > kPickCluster / 2;
+  // The first level is counted on the fly where the candidates (up to 3 k, 2.3 k as a rule) will be shared out by
+  // tickets, which saves these a phase of 2 us; below, the CTAs that pick count faster than the stream pass
+  // publishes.
+  const bool counted = k > kPickCluster / 8 * 3;
   cudaError_t e = stream_pass(counted, dynamic, (int)grid);
   if (e != cudaSuccess) return GTK_ERR_CUDA;
   // k1_pick: as many clusters as exact mode can use

@@ -16,7 +16,7 @@ struct WideShared {
   unsigned int warp_tot[kPickThreads / 32];
   unsigned int warp_n[2][kPickThreads / 32];
   unsigned int base[2];
-  unsigned int res_bin, res_krem;
+  unsigned int res_bin, res_krem, res_n;
 };
 
 // The keys that still matter: lo <= key <= hi, in bins of 2^shift.  An open level clamps everything
@@ -46,7 +46,7 @@ struct Level {
 };
 
 // Finds the bin B with count(bins > B) < k_rem <= count(bins >= B): res_bin, and k_rem minus the count
-// above it: res_krem.  c: the complete counts of bins 2t and 2t + 1.  Returns the sum of all counts; when it
+// above it: res_krem, and its own count: res_n.  c: the complete counts of bins 2t and 2t + 1.  Returns the sum of all counts; when it
 // is below k_rem there is no such bin and the results are not set.
 __device__ __forceinline__ unsigned int find_bin(WideShared& s, uint2 c, unsigned int k_rem) {
   const int t = threadIdx.x, w = t >> 5;
@@ -65,6 +65,7 @@ __device__ __forceinline__ unsigned int find_bin(WideShared& s, uint2 c, unsigne
     const bool upper = k_rem <= above + c.y;
     s.res_bin = 2u * t + (upper ? 1u : 0u);
     s.res_krem = k_rem - above - (upper ? 0u : c.y);
+    s.res_n = upper ? c.y : c.x;
   }
   __syncthreads();
   return __reduce_add_sync(0xffffffffu, v);

@@ -640,3 +640,28 @@ def test_exchange_of_the_same_indices_over_again(mode, P, k, nctas):
             assert torch.allclose(qv[o].cpu(), gv[order], rtol=1e-5, atol=1e-6)
             assert torch.allclose(r.resid.cpu(), res_ref[r.rank], rtol=1e-5, atol=1e-6)
             assert r.region.guards_intact()
+
+
+@pytest.mark.parametrize("step", [0.0, 2.0 ** -12, 2.0 ** -6, 0.5])  # continuous; 4, 260 and 10 000s of equal entries
+@pytest.mark.parametrize("k,form", [(40_000, "select"), (200_000, "select"), (200_000, "compress")])
+def test_k1_pick_settles_the_thresholds_bin_apart(k, form, step):
+    """Many candidates: those in the threshold's bin are put aside and settled by
+    one CTA, unless they are too many, which equal magnitudes make them."""
+    d = 3_000_000
+    torch.manual_seed(k)
+    sel = _selector(d, k)
+    r = torch.zeros(d, device=DEV)
+    for it in range(4):
+        g = torch.randn(d, device=DEV)
+        if step:
+            g = (g / step).round() * step
+            r.copy_((r / step).round() * step)
+        acc = g + r
+        if form == "compress":
+            idx, val = sel.compress(g, r, k)
+        else:
+            sel.select(g, r, k)
+            idx, val = sel.pairs()
+            idx, val = idx.long(), val.clone()
+        assert sel.status() == (0, 0)
+        _check_selection(idx, val, r, acc, k)
