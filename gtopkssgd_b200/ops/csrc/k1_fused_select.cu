@@ -409,12 +409,18 @@ struct Winners {
   }
 };
 
+constexpr unsigned int kAside = 256;  // entries of the threshold's bin that one thread each ranks
 struct PickShared : WideShared {
   unsigned int share[3][kBins / kPickCtas]; // cluster: the sums of bins b = rank (mod 8), a buffer per level in turn
   unsigned int chunk;
   unsigned int tie;
   unsigned int cta_n[kPickCtas];
   int ok;
+  // Entries of the threshold's bin (one CTA, cluster: in CTA 0), their keys apart for the ranking.
+  __align__(16) uint32_t aside_key[kAside];
+  Pair aside[kAside];
+  unsigned int aside_n;
+  uint32_t kth;
 };
 
 __device__ __forceinline__ uint2 global_counts(const unsigned int* ghist) {
@@ -513,6 +519,30 @@ __device__ __forceinline__ void finish_state(K1State* st, const K1State& was, ui
   st->n_calls = was.stream_calls;
 }
 
+// Ranks the entries put aside, one per thread: the first k_rem go to the list from pos0 on, the others back to r.
+// Returns the k_rem-th key.  One CTA; the list is complete.
+__device__ __forceinline__ uint32_t settle_aside(PickShared& s, float* r, const Winners& out, unsigned int pos0,
+                                                 unsigned int k_rem) {
+  const unsigned int n = s.aside_n, t = threadIdx.x;
+  if (t < n) {
+    const uint32_t key = s.aside_key[t];
+    unsigned int rank = 0;
+    for (unsigned int u = 0; u < n; u += 4) {
+      const uint4 q = *reinterpret_cast<const uint4*>(&s.aside_key[u]);
+      rank += (u < n && (q.x > key || (q.x == key && u < t))) ? 1u : 0u;
+      rank += (u + 1 < n && (q.y > key || (q.y == key && u + 1 < t))) ? 1u : 0u;
+      rank += (u + 2 < n && (q.z > key || (q.z == key && u + 2 < t))) ? 1u : 0u;
+      rank += (u + 3 < n && (q.w > key || (q.w == key && u + 3 < t))) ? 1u : 0u;
+    }
+    const Pair e = s.aside[t];
+    if (rank < k_rem) out.put(pos0 + rank, e);
+    else r[e.idx] = e.val;
+    if (rank + 1u == k_rem) s.kth = key;
+  }
+  __syncthreads();
+  return s.kth;
+}
+
 constexpr int kSmallRegs = kPickSmall / kPickThreads;  // candidates per thread in registers: one CTA
 constexpr int kClusterRegs = kPickCluster / (kPickCtas * kPickThreads);  // and the cluster
 constexpr unsigned int kPickChunk = 4u * kPickThreads; // candidates per ticket above
@@ -534,9 +564,10 @@ __device__ __forceinline__ uint32_t pick_small(PickShared& s, float* r, const Pa
   }
   auto live = [&](int j) { return (unsigned int)j * kPickThreads + threadIdx.x < C; };
   unsigned int k_rem = k;
+  bool aside = false;  // the entries of the threshold's bin (5 to 50 after one level) are ranked directly
   for (;;) {
     *my_bins(s) = make_uint2(0u, 0u);
-    if (threadIdx.x == 0) s.tie = 0u;
+    if (threadIdx.x == 0) s.tie = s.aside_n = 0u;
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < kSmallRegs; ++j)
@@ -545,13 +576,30 @@ __device__ __forceinline__ uint32_t pick_small(PickShared& s, float* r, const Pa
     find_bin(s, *my_bins(s), k_rem);
     k_rem = s.res_krem;
     if (!lv.narrow(s.res_bin)) break;
+    if (s.res_n <= kAside) {
+      aside = true;
+      break;
+    }
   }
-  const uint32_t th = lv.lo;
-  unsigned int won = 0, n = 0;
+  const uint32_t th = lv.lo, top = lv.hi;
+  unsigned int won = 0, gone = 0, n = 0;
 #pragma unroll
   for (int j = 0; j < kSmallRegs; ++j) {
     if ((unsigned int)j * kPickThreads >= C) break;
-    if (passes(live(j), mag_key(c[j].val), th, k_rem, &s.tie)) {
+    const uint32_t key = mag_key(c[j].val);
+    bool win;
+    if (aside) {
+      win = live(j) && key > top;
+      if (live(j) && key >= th && !win) {
+        const unsigned int at = atomicAdd(&s.aside_n, 1u);
+        s.aside_key[at] = key;
+        s.aside[at] = c[j];
+        gone |= 1u << j;
+      }
+    } else {
+      win = passes(live(j), key, th, k_rem, &s.tie);
+    }
+    if (win) {
       won |= 1u << j;
       ++n;
     }
@@ -561,9 +609,9 @@ __device__ __forceinline__ uint32_t pick_small(PickShared& s, float* r, const Pa
   for (int j = 0; j < kSmallRegs; ++j) {
     if (!live(j)) break;
     if (won & (1u << j)) out.put(pos++, c[j]);
-    else r[c[j].idx] = c[j].val;
+    else if (!(gone & (1u << j))) r[c[j].idx] = c[j].val;
   }
-  return th;
+  return aside ? settle_aside(s, r, out, k - k_rem, k_rem) : th;
 }
 
 // kPickSmall < C <= kPickCluster: the same with 8 CTAs that meet in the hardware barrier (0.2 us) and add
@@ -586,6 +634,7 @@ __device__ __forceinline__ uint32_t pick_cluster(PickShared& s, float* r, const 
     if (i < C) c[j] = ld_pair_cg(&cand[i]);
   }
   unsigned int k_rem = k;
+  bool aside = false;  // as with one CTA; the list is in CTA 0, complete with the barrier that tells the totals
   int buf = 0;
   for (;;) {
     *my_bins(s) = make_uint2(0u, 0u);
@@ -613,15 +662,32 @@ __device__ __forceinline__ uint32_t pick_cluster(PickShared& s, float* r, const 
     find_bin(s, sum, k_rem);
     k_rem = s.res_krem;
     if (!lv.narrow(s.res_bin)) break;
+    if (s.res_n <= kAside) {
+      aside = true;
+      break;
+    }
     buf = next;
   }
-  const uint32_t th = lv.lo;
+  const uint32_t th = lv.lo, top = lv.hi;
   unsigned int* const tie = cluster.map_shared_rank(&s.tie, 0);
   unsigned int won = 0, n = 0;
 #pragma unroll
   for (int j = 0; j < kClusterRegs; ++j) {
     if ((unsigned int)j >= trips) break;
-    if (passes(c[j].idx >= 0, mag_key(c[j].val), th, k_rem, tie)) {
+    const uint32_t key = mag_key(c[j].val);
+    bool win;
+    if (aside) {
+      win = c[j].idx >= 0 && key > top;
+      if (c[j].idx >= 0 && key >= th && !win) {
+        const unsigned int at = atomicAdd(cluster.map_shared_rank(&s.aside_n, 0), 1u);
+        *cluster.map_shared_rank(&s.aside_key[at], 0) = key;
+        *cluster.map_shared_rank(&s.aside[at], 0) = c[j];
+        c[j].idx = -1;
+      }
+    } else {
+      win = passes(c[j].idx >= 0, key, th, k_rem, tie);
+    }
+    if (win) {
       won |= 1u << j;
       ++n;
     }
@@ -635,11 +701,11 @@ __device__ __forceinline__ uint32_t pick_cluster(PickShared& s, float* r, const 
   for (unsigned int q = 0; q < rank; ++q) pos += s.cta_n[q];
 #pragma unroll
   for (int j = 0; j < kClusterRegs; ++j) {
-    if (c[j].idx < 0) break;
+    if (c[j].idx < 0) continue;
     if (won & (1u << j)) out.put(pos++, c[j]);
     else r[c[j].idx] = c[j].val;
   }
-  return th;
+  return aside && rank == 0u ? settle_aside(s, r, out, k - k_rem, k_rem) : th;
 }
 
 __global__ void __cluster_dims__(kPickCtas, 1, 1) __launch_bounds__(kPickThreads, 1)
@@ -647,7 +713,7 @@ k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Winners out, 
         Ctrl* ctrl_pair, int counted, float target_ratio, unsigned long long limit_ns) {
   __shared__ __align__(16) PickShared s;
   // what the cluster's CTAs add to in one another, ready before the stream pass has ended
-  if (threadIdx.x == 0) s.tie = 0u;
+  if (threadIdx.x == 0) s.tie = s.aside_n = 0u;
   if (threadIdx.x < (unsigned int)(kBins / kPickCtas)) s.share[0][threadIdx.x] = 0u;
   cluster_barrier();
   pdl_begin(r, cand, st, ctrl_pair);
