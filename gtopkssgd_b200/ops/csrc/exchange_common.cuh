@@ -132,6 +132,21 @@ __device__ __forceinline__ size_t flag_off(unsigned int parity, unsigned int whi
   return (size_t)parity * kFlagsPerParity + which;
 }
 
+// Calls f(pair, i) for this thread's entries of a list, with the loads of four of them in flight.
+template <typename F>
+__device__ __forceinline__ void for_pairs(const Pair* list, unsigned int n, unsigned int lane0, unsigned int stride, F f) {
+  constexpr int N = 4;
+  for (unsigned int i0 = lane0; i0 < n; i0 += N * stride) {
+    Pair e[N];
+#pragma unroll
+    for (int t = 0; t < N; ++t)
+      if (i0 + t * stride < n) e[t] = ld_pair_cg(&list[i0 + t * stride]);
+#pragma unroll
+    for (int t = 0; t < N; ++t)
+      if (i0 + t * stride < n) f(e[t], i0 + t * stride);
+  }
+}
+
 // Called by all threads of a CTA of a multi-CTA rank after its last store into peer memory of a phase
 // and before the rank's barrier: one thread issues a system-scope fence on behalf of the CTA (the
 // __syncthreads orders the other threads' stores before it).  By the PTX memory model the flag's own
@@ -175,13 +190,28 @@ __device__ __forceinline__ void put_back(const Pair* sel, unsigned int n_sel, co
                                          unsigned int n_g, const int32_t* map, float* resid,
                                          unsigned int d, unsigned int cta, unsigned int nct) {
   const unsigned int stride = nct * kSelThreads;
-  for (unsigned int i = cta * kSelThreads + threadIdx.x; i < n_sel; i += stride) {
-    const Pair e = sel[i];
-    if ((unsigned int)e.idx >= d) continue;
-    const unsigned int p = (unsigned int)__ldcg(&map[e.idx]);
-    bool in_global = false;
-    if (p < n_g) in_global = ld_pair_cg(&G[p]).idx == e.idx;
-    if (!in_global) resid[e.idx] += e.val;
+  constexpr int N = 4;  // entries per thread whose four dependent loads go together
+  for (unsigned int i0 = cta * kSelThreads + threadIdx.x; i0 < n_sel; i0 += N * stride) {
+    Pair e[N];
+    unsigned int p[N];
+    float back[N];
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+      e[t].idx = -1;
+      e[t].val = 0.f;
+      if (i0 + t * stride < n_sel) e[t] = sel[i0 + t * stride];
+      if ((unsigned int)e[t].idx >= d) e[t].idx = -1;
+    }
+#pragma unroll
+    for (int t = 0; t < N; ++t) p[t] = e[t].idx >= 0 ? (unsigned int)__ldcg(&map[e[t].idx]) : 0xffffffffu;
+#pragma unroll
+    for (int t = 0; t < N; ++t)
+      if (p[t] < n_g && ld_pair_cg(&G[p[t]]).idx == e[t].idx) e[t].idx = -1;
+#pragma unroll
+    for (int t = 0; t < N; ++t) back[t] = e[t].idx >= 0 ? resid[e[t].idx] + e[t].val : 0.f;
+#pragma unroll
+    for (int t = 0; t < N; ++t)
+      if (e[t].idx >= 0) resid[e[t].idx] = back[t];
   }
 }
 

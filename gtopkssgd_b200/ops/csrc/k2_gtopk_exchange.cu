@@ -333,8 +333,9 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
       for (int t = 0; t < kK2Cache; ++t) e[t] = entry(t0 + t);
       sweep(e, t0);
     }
-    // OUT and map complete; or, when this rank has sent, its work buffers and map free for other use
-    if (!bar.sync(290 + r)) { fail(); return; }
+    // OUT and map complete; or, when this rank has sent, its work buffers and map free for other use (with two
+    // ranks the root has no more use for either)
+    if (!only_round && !bar.sync(290 + r)) { fail(); return; }
     trace_stamp(ctrl, 1 + 8 * r + 5);
     if (send_next) {
       trace_stamp(ctrl, 1 + 8 * (r + 1) + 7);
@@ -357,7 +358,8 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
     // While the root merges: all of the own selection goes back to the residual, what was there is kept, and
     // the table is built over the selection.  What of it turns out to be in the global set is then undone as
     // its entries come in, with no barrier behind them.  (Table over the global set, barrier, then the put-back:
-    // 10 us after the set was there at k = 66 000, 28 us at 255 000.)
+    // 10 us after the set was there at k = 66 000, 28 us at 255 000.)  One entry at a time: there is time enough, and
+    // four in flight take DRAM from the root where ranks share a GPU (k = 255 000: 74.6 -> 77.7 us).
     float* const was = reinterpret_cast<float*>(R.work[0]);
     for (unsigned int i = lane0; i < n_sel; i += stride) {
       const Pair e = R.sel[i];

@@ -74,16 +74,14 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
     if (cta == 0 && threadIdx.x < P && threadIdx.x != me)
       st_relaxed_sys_u64(reinterpret_cast<unsigned long long*>(R.peer_flags[threadIdx.x] + flag_off(parity, kFlagAg0 + me)),
                          ((unsigned long long)epoch << 32) | n_sel);
-    for (unsigned int i = lane0; i < n_sel; i += stride) {
-      const Pair e = ld_pair_cg(&R.sel[i]);
+    for_pairs(R.sel, n_sel, lane0, stride, [&](Pair e, unsigned int i) {
       for (unsigned int q = 0; q < P; ++q)
         if (q != me) wire_store(R.peer_wire[q] + ag_off(parity, me, kcap) + i, e);
-    }
+    });
   } else {
-    for (unsigned int i = lane0; i < n_sel; i += stride) {
-      const Pair e = ld_pair_cg(&R.sel[i]);
+    for_pairs(R.sel, n_sel, lane0, stride, [&](Pair e, unsigned int i) {
       for (unsigned int q = 0; q < P; ++q) st_pair(R.peer_ag[q] + ag_off(parity, me, kcap) + i, e);
-    }
+    });
     cta_fence_peer_stores(nct == 1);
     if (!bar.sync(500)) { fail(); return; }
     if (cta == 0 && threadIdx.x < P && threadIdx.x != me)  // one releasing thread per destination
