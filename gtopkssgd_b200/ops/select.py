@@ -16,6 +16,9 @@ from . import lib as _lib
 from . import oracle
 
 
+_FLOAT = torch.float32
+
+
 def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
     return None if t is None else t.data_ptr()
 
@@ -49,6 +52,7 @@ class TopkSelector:
         self.is_cuda = self.device.type == "cuda"
         self.sel = torch.zeros((self.max_k, 2), dtype=torch.int32, device=self.device)
         self.state = torch.zeros(16, dtype=torch.int32, device=self.device)
+        self._n_sel = self.state[1:2]   # (a view costs over 1 us to make)
         self.reset_threshold()
         if self.is_cuda:
             L = _lib.lib()
@@ -57,8 +61,10 @@ class TopkSelector:
             # two control blocks: call i uses block i & 1 and clears the other one for call i + 1
             self.ctrl_words = int(L.gtk_ctrl_bytes()) // 4
             self.ctrl = torch.zeros(2 * self.ctrl_words, dtype=torch.int32, device=self.device)
+            self._stream_index = self.sel.device.index
             self._select = _lib.calls().gtk_k1_select
             self._select_segments = _lib.calls().gtk_k1_select_segments
+            self._compress = _lib.calls().gtk_k1_compress
             self._buffers = (self.cand.data_ptr(), self.cap, self.sel.data_ptr(), self.state.data_ptr(),
                              self.ctrl.data_ptr(), self.target_ratio, self.limit_ns)
         self.last_k = 0
@@ -71,7 +77,7 @@ class TopkSelector:
     @property
     def n_sel_tensor(self) -> torch.Tensor:
         """Device word holding the number of selected pairs of the last call."""
-        return self.state[1:2]
+        return self._n_sel
 
     def stats(self) -> dict:
         """Host copy of the selection statistics (synchronises)."""
@@ -113,9 +119,10 @@ class TopkSelector:
     def select(self, g: torch.Tensor, r: torch.Tensor, k: int, g_scale: Optional[torch.Tensor] = None) -> None:
         """acc = g*scale + r; self.sel[:k] <- the k largest-magnitude (idx, acc)
         pairs; r <- acc off the selection, 0 on it.  g is not modified."""
-        assert g.numel() == self.numel and r.numel() == self.numel
-        assert g.dtype == torch.float32 and r.dtype == torch.float32
-        k = int(min(k, self.max_k))
+        numel = self.numel
+        assert g.numel() == numel and r.numel() == numel
+        assert g.dtype is _FLOAT and r.dtype is _FLOAT
+        k = int(k if k < self.max_k else self.max_k)
         self.last_k = k
         if not self.is_cuda:
             scale = float(g_scale) if g_scale is not None else 1.0
@@ -125,8 +132,8 @@ class TopkSelector:
             self.state[1] = k
             return
         assert g.is_contiguous() and r.is_contiguous()
-        code = self._select(g.data_ptr(), r.data_ptr(), _ptr(g_scale), self.numel, k, *self._buffers,
-                            current_stream_handle(self.device))
+        code = self._select(g.data_ptr(), r.data_ptr(), None if g_scale is None else g_scale.data_ptr(), numel, k,
+                            *self._buffers, _raw_stream(self._stream_index))
         if code:
             _lib.check(code, "gtk_k1_select")
 
@@ -139,7 +146,7 @@ class TopkSelector:
         k = int(min(k, self.max_k))
         self.last_k = k
         code = self._select_segments(addresses, segments.data_ptr(), r.data_ptr(), self.numel, k, *self._buffers,
-                                     current_stream_handle(self.device))
+                                     _raw_stream(self._stream_index))
         if code:
             _lib.check(code, "gtk_k1_select_segments")
 
@@ -153,8 +160,8 @@ class TopkSelector:
         self.last_k = k
         idx = torch.empty(k, dtype=torch.int64, device=g.device)
         val = torch.empty(k, dtype=torch.float32, device=g.device)
-        code = _lib.calls().gtk_k1_compress(g.data_ptr(), r.data_ptr(), self.numel, k, *self._buffers, idx.data_ptr(),
-                                            val.data_ptr(), current_stream_handle(self.device))
+        code = self._compress(g.data_ptr(), r.data_ptr(), self.numel, k, *self._buffers, idx.data_ptr(),
+                              val.data_ptr(), _raw_stream(self._stream_index))
         if code:
             _lib.check(code, "gtk_k1_compress")
         return idx, val

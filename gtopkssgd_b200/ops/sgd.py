@@ -16,7 +16,7 @@ import torch
 
 from . import lib as _lib
 from . import oracle
-from .select import _ptr, current_stream_handle, pairs_to_tensors
+from .select import _ptr, _raw_stream, current_stream_handle, pairs_to_tensors
 
 
 @dataclass
@@ -59,7 +59,7 @@ def sgd_sparse(p: torch.Tensor, buf: Optional[torch.Tensor], pairs: torch.Tensor
     overrides ``h.lr``; ``parity_word`` selects the half of a two-parity buffer
     on the device: base = pairs + ((word - 1) & 1) * parity_stride."""
     d = p.numel()
-    if p.device.type != "cuda":
+    if not p.is_cuda:
         if parity_word is not None:
             pairs = pairs[((int(parity_word) - 1) & 1) * parity_stride:]
         c = scale * (float(coef) if coef is not None else 1.0)
@@ -75,13 +75,15 @@ def sgd_sparse(p: torch.Tensor, buf: Optional[torch.Tensor], pairs: torch.Tensor
                 step = sv + h.momentum * sb if h.nesterov else sb
             p.index_add_(0, idx, step, alpha=-h.lr)
         return
-    if bad_index_count is None:
-        bad_index_count = _scratch_word(p.device)
-    code = _lib.calls().gtk_k3_sparse(p.data_ptr(), _ptr(buf), pairs.data_ptr(), counts.data_ptr(), nseg, seg_stride,
-                                      _ptr(coef), scale, d, h.lr, _ptr(lr_dev), h.momentum, h.dampening,
-                                      h.weight_decay, int(h.nesterov), int(first_step), int(use_atomics),
-                                      bad_index_count.data_ptr(), _ptr(parity_word), parity_stride,
-                                      current_stream_handle(p.device))
+    index = p.get_device()
+    bad = _scratch_address(index) if bad_index_count is None else bad_index_count.data_ptr()
+    code = _lib.calls().gtk_k3_sparse(p.data_ptr(), None if buf is None else buf.data_ptr(), pairs.data_ptr(),
+                                      counts.data_ptr(), nseg, seg_stride, None if coef is None else coef.data_ptr(),
+                                      scale, d, h.lr, None if lr_dev is None else lr_dev.data_ptr(), h.momentum,
+                                      h.dampening, h.weight_decay, 1 if h.nesterov else 0, 1 if first_step else 0,
+                                      1 if use_atomics else 0, bad,
+                                      None if parity_word is None else parity_word.data_ptr(), parity_stride,
+                                      _raw_stream(index))
     if code:
         _lib.check(code, "gtk_k3_sparse")
 
@@ -108,6 +110,7 @@ def scatter_dense(g: torch.Tensor, pairs: torch.Tensor, counts: torch.Tensor, ns
 
 
 _scratch = {}
+_scratch_addresses = {}
 
 
 def _scratch_word(device: torch.device) -> torch.Tensor:
@@ -115,6 +118,13 @@ def _scratch_word(device: torch.device) -> torch.Tensor:
     if word is None:
         word = _scratch[device] = torch.zeros(1, dtype=torch.int32, device=device)
     return word
+
+
+def _scratch_address(index: int) -> int:
+    at = _scratch_addresses.get(index)
+    if at is None:
+        at = _scratch_addresses[index] = _scratch_word(torch.device("cuda", index)).data_ptr()
+    return at
 
 
 def momentum_correct(v: torch.Tensor, g: torch.Tensor, momentum: float) -> None:
