@@ -77,7 +77,11 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
   __shared__ K2Shared sh;
   SelectShared& ss = sh.ex.sel;
   const K2Rank& R = ranks[blockIdx.y];
+  // One round of loads (a load behind the check of the status would be another round trip).
   const unsigned int epoch = __ldcg(R.epoch);  // every CTA reads it before its first barrier
+  const unsigned int status = __ldcg(&R.n_global[kResStatus]);
+  unsigned int n_sel = __ldcg(&R.st->n_sel);
+  const float kth_mag = __ldcg(&R.st->kth_mag);
   const unsigned int me = rank_base + blockIdx.y;
   const unsigned int cta = blockIdx.x, nct = gridDim.x;
   const unsigned int parity = epoch & 1u;
@@ -103,12 +107,11 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
       }
     }
   };
-  if (__ldcg(&R.n_global[kResStatus]) != 0u) {  // an earlier call failed: nothing is exchanged any more
+  if (status != 0u) {  // an earlier call failed: nothing is exchanged any more
     if (cta == 0 && threadIdx.x == 0) R.n_global[kResCount] = 0u;
     return;
   }
 
-  unsigned int n_sel = R.st->n_sel;
   if (n_sel > kcap) n_sel = kcap;
   const Pair* cur = R.sel;  // current set of this rank
   unsigned int n_cur = n_sel;
@@ -121,7 +124,7 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
   trace_stamp(ctrl, 0);
   // Every live entry of a round's union is counted once in the band above `pred` (delta = 1 adds, 0xffffffff
   // removes): the union's k-th magnitude is at least this rank's own and for gradient tails a few per cent above.
-  uint32_t pred = mag_key(R.st->kth_mag);  // round 0: K1's k-th magnitude, then the previous round's threshold
+  uint32_t pred = mag_key(kth_mag);  // round 0: K1's k-th magnitude, then the previous round's threshold
   auto tally = [&](float v, unsigned int delta) { atomicAdd(&sh.band[band_bin(mag_key(v), pred)], delta); };
 
   for (unsigned int r = 0; r < rounds; ++r) {

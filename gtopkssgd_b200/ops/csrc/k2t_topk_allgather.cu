@@ -35,7 +35,11 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
   __shared__ unsigned int band[kHistBins];  // this CTA's share of the first selection level, counted on the fly
   __shared__ unsigned int counts[kMaxPeers];
   const K2Rank& R = ranks[blockIdx.y];
+  // One round of loads (a load behind the check of the status would be another round trip).
   const unsigned int epoch = __ldcg(R.epoch);
+  const unsigned int status = __ldcg(&R.n_global[kResStatus]);
+  unsigned int n_sel = __ldcg(&R.st->n_sel);
+  const float kth_mag = __ldcg(&R.st->kth_mag);
   const unsigned int me = rank_base + blockIdx.y;
   const unsigned int cta = blockIdx.x, nct = gridDim.x;
   const unsigned int parity = epoch & 1u;
@@ -57,13 +61,12 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
       }
     }
   };
-  if (__ldcg(&R.n_global[kResStatus]) != 0u) {
+  if (status != 0u) {
     if (cta == 0 && threadIdx.x < (unsigned int)kMaxPeers) seg_counts[threadIdx.x] = 0u;
     if (cta == 0 && threadIdx.x == 0) R.n_global[kResCount] = 0u;
     return;
   }
 
-  unsigned int n_sel = R.st->n_sel;
   if (n_sel > kcap) n_sel = kcap;
 
   const unsigned int stride = nct * kSelThreads;
@@ -125,7 +128,7 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
   }
 
   // ---- topk2: merge the P lists in rank order, then keep the k largest sums
-  const uint32_t pred = mag_key(R.st->kth_mag);  // no sum of P selections has its k-th magnitude below the own one
+  const uint32_t pred = mag_key(kth_mag);  // no sum of P selections has its k-th magnitude below the own one
   for (int i = threadIdx.x; i < kHistBins; i += kSelThreads) band[i] = 0u;
   __syncthreads();
   auto tally = [&](float v, unsigned int delta) { atomicAdd(&band[band_bin(mag_key(v), pred)], delta); };
