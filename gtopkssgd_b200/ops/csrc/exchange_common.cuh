@@ -92,6 +92,12 @@ __device__ __forceinline__ void wire_store(unsigned long long* slot, Pair e) {
   e.idx ^= (int32_t)0x80000000;
   st_relaxed_sys_u64(slot, pair_bits(e));
 }
+// Brings the table's line for idx into L2, ahead of a look-up behind a barrier.  Tables of up to 2 M entries (8 MB a
+// rank) are there anyway: eight ranks of 4 M entries 95.0 -> 91.1 us ('topk2'), of 1 M 41.0 -> 42.1 without the rule.
+__device__ __forceinline__ void prefetch_entry(const int32_t* map, int32_t idx, unsigned int d) {
+  if (d > 2000000u && idx >= 0) asm volatile("prefetch.global.L2 [%0];" ::"l"(&map[idx]));
+}
+
 // Receives the words slot + at(j) of this thread, for the j of `want`, into e[j] (idx -1: not wanted, or an index
 // outside [0, d)) and clears them.  Returns false, the error recorded, when the limit runs out or the rank gives up.
 template <int N, typename At>

@@ -224,6 +224,8 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
     };
     Pair c[kK2Cache];
     bool ok = receive(c, 0);
+#pragma unroll
+    for (int t = 0; t < kK2Cache; ++t) prefetch_entry(map, c[t].idx, d);
     // A and map must be complete: after the copy above that needs a barrier, after a previous
     // round its closing barrier already gave it
     if (!__syncthreads_and(ok) || (copied && !bar.wait(230 + r))) { fail(); return; }

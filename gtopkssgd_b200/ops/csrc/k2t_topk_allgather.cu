@@ -178,8 +178,10 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
     // a list's first entries come in while the one before is being completed
     if (!__syncthreads_and(fetch(q, 0))) { fail(); return; }
     if (q != 0u) {
+#pragma unroll
+      for (int t = 0; t < kBatch; ++t) prefetch_entry(map, c[t].idx, d);
       if (!bar.wait(560 + q)) { fail(); return; }
-      n_a += __ldcg(&ctrl->scratch[(q - 1u) % 3u]);
+      n_a = q == 1u ? counts[0] : n_a + __ldcg(&ctrl->scratch[(q - 1u) % 3u]);
       if (n_a > work_cap) n_a = work_cap;
     }
     if (cta == 0 && threadIdx.x == 0) ctrl->scratch[(q + 1u) % 3u] = 0u;
@@ -214,12 +216,13 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
         n_fresh += __popc(fresh[t]);
       }
       unsigned int base = 0;
-      if (n_fresh && lane_id() == 0) base = n_a + atomicAdd(added, n_fresh);
+      if (q != 0u && n_fresh && lane_id() == 0) base = n_a + atomicAdd(added, n_fresh);
       base = __shfl_sync(0xffffffffu, base, 0);
 #pragma unroll
       for (int t = 0; t < kBatch; ++t) {
         if (c[t].idx >= 0) {
-          const unsigned int pos = base + __popc(fresh[t] & lanemask_lt());
+          // (the first list keeps its order: no counter, no round trip)
+          const unsigned int pos = q == 0u ? (t0 + t) * stride + lane0 : base + __popc(fresh[t] & lanemask_lt());
           if (pos < work_cap) {
             st_pair(&A[pos], c[t]);
             own[pos] = q == me ? (t0 + t) * stride + lane0 : kNotOwn;
@@ -242,7 +245,7 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
     bar.arrive();
   }
   if (!bar.wait(560 + P)) { fail(); return; }
-  n_a += __ldcg(&ctrl->scratch[(P - 1u) % 3u]);
+  n_a += __ldcg(&ctrl->scratch[(P - 1u) % 3u]);  // (two ranks at least)
   if (n_a > work_cap) n_a = work_cap;
   const unsigned int trips = (n_a + stride - 1) / stride;
   auto load = [&](Pair (&e)[kBatch], unsigned int t0) {
