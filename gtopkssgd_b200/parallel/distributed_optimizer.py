@@ -316,15 +316,21 @@ class _DistributedOptimizer(torch.optim.Optimizer):
         self._flat.begin_detached()
         self._materialized = False
 
+    def _launch_rest(self) -> None:
+        """Launch the groups that no hook has launched: those with a parameter
+        that got no gradient this iteration, and the only group where there are
+        no hooks."""
+        for gi, launched in enumerate(self._launched):
+            if not launched:
+                self._launch_group(gi)
+
     def synchronize(self, materialize: bool = False):
         """Wait (on the stream, not on the host) until every group of this
         iteration has been reduced.  With ``materialize=True`` the dense
         averaged gradient is also written into ``p.grad`` for callers that
         want to look at it (the fused step does not need it)."""
         if not self._synced:
-            for gi in range(len(self._launched)):
-                if not self._launched[gi]:  # parameters that got no gradient this iteration
-                    self._launch_group(gi)
+            self._launch_rest()
             if self._overlap:
                 current_stream().wait_stream(self._comm_stream)
             self._synced = True
@@ -380,8 +386,9 @@ class _DistributedOptimizer(torch.optim.Optimizer):
     def _step(self, closure=None):
         """Fused update over the flat buffers.  In the sparse modes the dense
         part (weight decay + momentum decay) does not depend on the exchange, so
-        it is enqueued before the compute stream waits for the side stream: it
-        runs while the exchange kernel is still waiting on its peers."""
+        it is enqueued behind the select, before the compute stream waits for the
+        side stream: it runs while the exchange kernel is still waiting on its
+        peers."""
         loss = closure() if closure is not None else None
         self.sync_lr()
         h = self._hyper()
@@ -407,8 +414,11 @@ class _DistributedOptimizer(torch.optim.Optimizer):
                 p, buf = bufs(eng)
                 sgd_dense(p, buf, h, first, g=eng.grad, scale=scale, coef=self._post_coef, lr_dev=lr_dev)
         else:
+            # Every select of this iteration is enqueued, and its event recorded, before anything waits for one: an
+            # event of an earlier iteration would order nothing, and a capture refuses one recorded outside of it.
+            self._launch_rest()
             for eng in a.engines:
-                if eng.select_done is not None and self._overlap:
+                if self._overlap:
                     current_stream().wait_event(eng.select_done)  # select first, then dense || exchange
                 p, buf = bufs(eng)
                 sgd_dense(p, buf, h, first, lr_dev=lr_dev)

@@ -328,3 +328,51 @@ def test_direct_layer_calls_keep_hooks_and_results():
     handle.remove()
     block.eval()(x)
     assert len(seen) == 1
+
+
+def _on_a_side_stream(opt):
+    """A single worker's optimizer reduces on the side stream, as those of several workers do."""
+    opt._overlap = opt._allreducer.concurrent = True
+    opt._ready = [torch.cuda.Event() for _ in opt._flat.groups]
+
+
+@pytest.mark.parametrize("graph", [False, True])
+def test_reduction_is_launched_before_the_dense_part(graph, monkeypatch):
+    """With one merged group nothing has launched the reduction when ``step``
+    begins: it goes out first, the dense part behind this iteration's select, in
+    eager iterations, in a captured one and in an eager one after it, with the
+    results of a reduction on the compute stream."""
+    from gtopkssgd_b200 import settings
+    from gtopkssgd_b200.parallel import distributed_optimizer as do
+    from gtopkssgd_b200.parallel.compression import compressors
+    from gtopkssgd_b200.trainer.dl_trainer import DLTrainer
+    monkeypatch.setattr(settings, "PIN_DENSITY", True)
+    monkeypatch.setattr(torch.backends.cudnn, "deterministic", True)
+    order = []
+    plain_dense = do.sgd_dense
+    monkeypatch.setattr(do, "sgd_dense", lambda *a, **kw: (order.append("dense"), plain_dense(*a, **kw)))
+    dev = torch.device("cuda", 0)
+    batches = [(torch.randn(8, 3, 32, 32, device=dev), torch.randint(0, 10, (8,), device=dev)) for _ in range(7)]
+    results = []
+    for side in (False, True):
+        torch.manual_seed(0)
+        t = DLTrainer(0, 1, dist=False, ngpus=1, batch_size=8, data_dir="synthetic", dataset="cifar10", dnn="resnet20",
+                      lr=0.1, nworkers=1, device=dev, synthetic_train_size=640, cuda_graph=graph)
+        opt = do.DistributedOptimizer(t.optimizer, t.net.named_parameters(), compression=compressors["gtopk"],
+                                      is_sparse=True, density=0.01)
+        t.update_optimizer(opt)
+        if side:
+            _on_a_side_stream(opt)
+        reduce_group = opt._allreducer.reduce_group
+        monkeypatch.setattr(opt._allreducer, "reduce_group",
+                            lambda *a, f=reduce_group: (order.append("reduce"), f(*a)))
+        del order[:]
+        for i, b in enumerate(batches):
+            t.train_step(data=b, cuda_graph=graph and i < 6)
+        if side:   # eager iterations, and the captured one once
+            assert order == ["reduce", "dense"] * (5 if graph else 7)
+        opt.check_status()
+        results.append([opt._flat.param.clone(), opt._flat.momentum.clone(), opt._flat.residual.clone()])
+        opt.stop()
+    for a, b in zip(*results):
+        assert torch.equal(a, b)
