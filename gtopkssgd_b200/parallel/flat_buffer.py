@@ -114,8 +114,7 @@ class FlatBuffers:
         self.param_numel = sum(g.param_numel for g in self.groups)
         self.param = torch.zeros(self.total, dtype=dtype, device=dev)
         self._grad = torch.zeros(self.total, dtype=dtype, device=dev)
-        # None: ``p.grad`` are the views; "live": they are backward's own tensors; a list: those of a captured graph
-        self._detached = None
+        self._detached = False   # ``p.grad`` are backward's own tensors (or None), not the views
         self.momentum = torch.zeros(self.total, dtype=dtype, device=dev)
         self.residual = torch.zeros(self.total, dtype=dtype, device=dev) if with_residual else None
         with torch.no_grad():
@@ -163,10 +162,9 @@ class FlatBuffers:
     def grad(self) -> torch.Tensor:
         """The flat gradient buffer.  After a detached iteration it is filled from
         the gradients first (which stay where they are)."""
-        if self._detached is not None:
-            grads = self.current_grads() if self._detached == "live" else self._detached
+        if self._detached:
             with torch.no_grad():
-                for slot, g in zip(self.slots.values(), grads):
+                for slot, g in zip(self.slots.values(), self.current_grads()):
                     view = self._view(self._grad, slot)
                     if g is None:
                         view.zero_()
@@ -177,19 +175,27 @@ class FlatBuffers:
     # -- detached iterations -------------------------------------------------------
     @property
     def detached(self) -> bool:
-        return self._detached is not None
+        return self._detached
 
     def begin_detached(self) -> None:
         """No gradients, and none attached: ``p.grad`` will be what backward produces."""
         _native.calls().clear_grads(self._params)
-        self._detached = "live"
+        self._detached = True
 
     def current_grads(self) -> List[Optional[torch.Tensor]]:
         return [p.grad for p in self._params]
 
-    def use_grads_of(self, grads: List[Optional[torch.Tensor]]) -> None:
-        """A replayed graph has just refilled these."""
-        self._detached = grads
+    def use_grads_of(self, grads: Optional[List[Optional[torch.Tensor]]]) -> None:
+        """A replayed graph has just refilled these (None: the views): they are
+        every ``p.grad``, whatever another graph, an eager iteration or the user
+        left there."""
+        if grads is None:
+            self.attach(keep=False)
+            return
+        for p, g in zip(self._params, grads):
+            if p.grad is not g:
+                p.grad = g
+        self._detached = True
 
     def grad_addresses(self) -> Optional[List[int]]:
         """Device addresses of all ``p.grad`` (0 where there is none), in slot
@@ -212,11 +218,11 @@ class FlatBuffers:
     def attach(self, keep: bool = True) -> None:
         """Back to ``p.grad`` as views of the flat buffer, with the values they
         had (``keep``) or with whatever the buffer holds."""
-        if self._detached is None:
+        if not self._detached:
             return
         if keep:
             self.grad
-        self._detached = None
+        self._detached = False
         for slot in self.slots.values():
             slot.param.grad = self._view(self._grad, slot)
 

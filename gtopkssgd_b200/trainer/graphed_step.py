@@ -92,7 +92,7 @@ class GraphedStep:
             if hasattr(opt, "capturing"):
                 opt.capturing = False
         flat = getattr(opt, "_flat", None)
-        # the graph's own gradients, refilled by every replay
+        # the graph's own gradients, refilled by every replay (kept for every signature, besides the flat buffer)
         st["grads"] = flat.current_grads() if flat is not None and flat.detached else None
         st["native_launches"] = _native.launch_count() - before  # kernels of the native library inside the graph
         _native.add_launches(-st["native_launches"])              # capture enqueued nothing yet
@@ -142,7 +142,7 @@ class GraphedStep:
         if hasattr(opt, "sync_lr"):
             opt.sync_lr()
         g.replay()
-        if st["grads"] is not None:
+        if hasattr(opt, "_flat"):
             opt._flat.use_grads_of(st["grads"])
         if hasattr(opt, "post_iteration"):
             opt.post_iteration()

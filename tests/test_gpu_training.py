@@ -376,3 +376,44 @@ def test_reduction_is_launched_before_the_dense_part(graph, monkeypatch):
         opt.stop()
     for a, b in zip(*results):
         assert torch.equal(a, b)
+
+
+def test_parameters_carry_the_gradient_of_the_last_replay():
+    """Two captured batch shapes in turn, with an iteration of the user's own in
+    between: ``p.grad`` is the gradient of the last iteration each time."""
+    from gtopkssgd_b200 import settings
+    from gtopkssgd_b200.parallel.compression import compressors
+    from gtopkssgd_b200.parallel.distributed_optimizer import DistributedOptimizer
+    from gtopkssgd_b200.trainer.dl_trainer import DLTrainer
+    settings.PIN_DENSITY = True
+    torch.manual_seed(0)
+    dev = torch.device("cuda", 0)
+    t = DLTrainer(0, 1, dist=False, ngpus=1, batch_size=8, data_dir="synthetic", dataset="cifar10", dnn="resnet20", lr=0.1,
+                  nworkers=1, device=dev, synthetic_train_size=640, cuda_graph=True)
+    opt = DistributedOptimizer(t.optimizer, t.net.named_parameters(), compression=compressors["gtopk"], is_sparse=True,
+                               density=0.01)
+    t.update_optimizer(opt)
+    fb = opt._flat
+    params = [s.param for s in fb.slots.values()]
+
+    def selected_from_gradients(before):
+        """What the step selected, against the sum of residual and ``p.grad``."""
+        idx, val = opt._allreducer.engines[0].selector.pairs()
+        g = torch.zeros_like(before)
+        for s in fb.slots.values():
+            assert s.param.grad is not None
+            g[s.offset:s.offset + s.numel] = s.param.grad.flatten()
+        assert torch.equal(val, (g + before)[idx]) and torch.equal(fb.grad, g)
+
+    for own, rows in ((0, 8), (0, 8), (0, 8), (0, 8), (0, 5), (0, 8), (0, 5), (1, 6), (0, 5), (0, 8), (2, 6), (0, 8)):
+        batch = (torch.randn(rows, 3, 32, 32, device=dev), torch.randint(0, 10, (rows,), device=dev))
+        before = fb.residual.clone()
+        if own:   # the user's own loop, with the optimizer's zero_grad or the network's
+            (opt if own == 1 else t.net).zero_grad()
+            t.criterion(t.net(batch[0]), batch[1]).backward()
+            opt.step()
+        else:
+            t.train_step(data=batch)
+        selected_from_gradients(before)
+    assert len(t._graphed.graphs) == 2
+    opt.stop()
