@@ -229,7 +229,9 @@ class FlatBuffers:
     def ensure_views(self) -> int:
         """Re-attach any parameter whose ``.data`` or ``.grad`` was replaced
         behind our back (``.cuda()``, ``zero_grad(set_to_none=True)``,
-        ``flatten_parameters``).  Returns how many were repaired."""
+        ``flatten_parameters``).  A gradient that is there is the whole gradient
+        and one that is not is zero: what the flat buffer holds in their place is
+        an earlier iteration's.  Returns how many were repaired."""
         fixed = 0
         with torch.no_grad():
             for s in self.slots.values():
@@ -241,10 +243,11 @@ class FlatBuffers:
                     fixed += 1
                 gwant = self._view(self._grad, s)
                 if p.grad is None:
+                    gwant.zero_()
                     p.grad = gwant
                     fixed += 1
                 elif p.grad.data_ptr() != gwant.data_ptr():
-                    gwant.add_(p.grad)
+                    gwant.copy_(p.grad)
                     p.grad = gwant
                     fixed += 1
         return fixed

@@ -639,3 +639,29 @@ def test_failed_exchange_seen_on_the_host_mirror_stops_the_next_iteration(monkey
     assert calls == [(1, 0)]
     d._allreducer.engines[0].rank_ctx = None
     d.stop()
+
+
+def check_replaced_gradients(device):
+    states = []
+    for own in (True, False):
+        torch.manual_seed(3)
+        params = [torch.nn.Parameter(torch.randn(n, device=device)) for n in (40, 7, 300)]
+        sgd = torch.optim.SGD(params, lr=0.1, momentum=0.9)
+        opt = DistributedOptimizer(sgd, [("p%d" % i, p) for i, p in enumerate(params)], compression=compressors["gtopk"],
+                                   is_sparse=True, density=0.05)
+        for it in range(4):
+            if own:
+                opt.zero_grad()
+            else:
+                sgd.zero_grad()   # set_to_none
+            used = params[:2] if it == 2 else params
+            torch.autograd.backward(used, [torch.randn(p.numel()).to(device) for p in used])
+            opt.step()
+        states.append([opt._flat.param.clone(), opt._flat.residual.clone()])
+        opt.stop()
+    for a, b in zip(*states):
+        assert torch.equal(a, b)
+
+
+def test_gradients_replaced_by_the_user_are_taken_as_they_are():
+    check_replaced_gradients("cpu")

@@ -417,3 +417,10 @@ def test_parameters_carry_the_gradient_of_the_last_replay():
         selected_from_gradients(before)
     assert len(t._graphed.graphs) == 2
     opt.stop()
+
+
+def test_gradients_replaced_by_the_user_are_taken_as_they_are():
+    """A loop with the network's own ``zero_grad`` (``p.grad`` None) gives what the
+    optimizer's gives, also for a parameter without a gradient in one iteration."""
+    import test_framework_cpu as cpu
+    cpu.check_replaced_gradients("cuda")
