@@ -142,6 +142,16 @@ class FlatBuffers:
             return flat.view(n, h, w, c).permute(0, 3, 1, 2)
         return flat.view(shape)
 
+    @staticmethod
+    def _fill(view: torch.Tensor, g: Optional[torch.Tensor]) -> None:
+        """``view`` <- a gradient of any layout (None: zero)."""
+        if g is None:
+            view.zero_()
+        elif g.layout is torch.strided:
+            view.copy_(g)
+        else:   # sparse, as ``nn.Embedding(sparse=True)`` leaves it: can be added but not copied
+            view.zero_().add_(g)
+
     def group_slice(self, buf: torch.Tensor, g: MergedGroup) -> torch.Tensor:
         return buf[g.start:g.start + g.numel]
 
@@ -165,11 +175,7 @@ class FlatBuffers:
         if self._detached:
             with torch.no_grad():
                 for slot, g in zip(self.slots.values(), self.current_grads()):
-                    view = self._view(self._grad, slot)
-                    if g is None:
-                        view.zero_()
-                    else:
-                        view.copy_(g)
+                    self._fill(self._view(self._grad, slot), g)
         return self._grad
 
     # -- detached iterations -------------------------------------------------------
@@ -242,12 +248,8 @@ class FlatBuffers:
                     p.data = want
                     fixed += 1
                 gwant = self._view(self._grad, s)
-                if p.grad is None:
-                    gwant.zero_()
-                    p.grad = gwant
-                    fixed += 1
-                elif p.grad.data_ptr() != gwant.data_ptr():
-                    gwant.copy_(p.grad)
+                if p.grad is None or p.grad.layout is not torch.strided or p.grad.data_ptr() != gwant.data_ptr():
+                    self._fill(gwant, p.grad)
                     p.grad = gwant
                     fixed += 1
         return fixed

@@ -665,3 +665,22 @@ def check_replaced_gradients(device):
 
 def test_gradients_replaced_by_the_user_are_taken_as_they_are():
     check_replaced_gradients("cpu")
+
+
+def test_detached_gradients_may_be_of_the_sparse_layout():
+    """What ``nn.Embedding(sparse=True)`` leaves in ``p.grad``: not laid out like
+    its parameter, so it is copied into the flat buffer."""
+    table, dense = torch.nn.Parameter(torch.randn(6, 3)), torch.nn.Parameter(torch.randn(5))
+    fb = FlatBuffers([("table", table), ("dense", dense)], 1000)
+    fb.grad.fill_(7.0)
+    fb.begin_detached()
+    (torch.nn.functional.embedding(torch.tensor([1, 4, 1]), table, sparse=True).sum() + dense.sum()).backward()
+    assert table.grad.is_sparse and fb.grad_addresses() is None
+    want = torch.zeros(6, 3)
+    want[1], want[4] = 2.0, 1.0
+    assert torch.equal(fb.grad_view("table"), want) and torch.equal(fb.grad_view("dense"), torch.ones(5))
+    fb.attach()
+    assert torch.equal(table.grad, want) and fb.grads_attached()
+    table.grad = torch.sparse_coo_tensor(torch.tensor([[2]]), torch.ones(1, 3), (6, 3))
+    fb.ensure_views()
+    assert fb.grads_attached() and float(table.grad.sum()) == 3.0
