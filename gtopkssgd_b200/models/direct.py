@@ -4,8 +4,10 @@ bound by host time.
 ``nn.Module.__call__`` and the layers' own Python cost 4 to 8 us per layer, a
 fifth of ResNet-20's forward pass on the host.  ``conv`` and ``batch_norm`` make
 the layer's one library call directly when nothing observes or replaces it: a
-plain layer without hooks (its own or global ones), called with a tensor, outside
-of scripting.  Otherwise they call the layer.
+plain layer without hooks (its own or global ones), whose forward is neither
+replaced (on the instance or for the class) nor compiled, called with a tensor
+outside of tracing.  Otherwise they call the layer.  (Code that is itself
+scripted or compiled calls the layers: the caller's check, once per block.)
 """
 from __future__ import annotations
 
@@ -13,26 +15,36 @@ import torch
 import torch.nn as nn
 from torch.nn.modules import module as _m
 
+_Module, _Conv2d, _BatchNorm2d = nn.Module, nn.Conv2d, nn.BatchNorm2d
+_call, _conv_forward, _bn_forward = nn.Module.__call__, nn.Conv2d.forward, nn.BatchNorm2d.forward
+_tracing = torch._C._get_tracing_state
+
 
 def _plain(layer: nn.Module) -> bool:
+    own = layer.__dict__
     return not (layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks
                 or _m._global_forward_hooks or _m._global_forward_pre_hooks or _m._global_backward_hooks
-                or _m._global_backward_pre_hooks)
+                or _m._global_backward_pre_hooks
+                or "forward" in own or "_conv_forward" in own or "_check_input_dim" in own
+                or own.get("_compiled_call_impl") is not None or _Module.__call__ is not _call or _tracing() is not None)
 
 
 def conv(layer: nn.Module, x):
-    if type(layer) is nn.Conv2d and isinstance(x, torch.Tensor) and layer.padding_mode == "zeros" and _plain(layer):
+    if type(layer) is _Conv2d and isinstance(x, torch.Tensor) and layer.padding_mode == "zeros" \
+            and _Conv2d.forward is _conv_forward and _plain(layer):
         p = layer._parameters
-        if "weight" in p:
+        if "weight" in p and "bias" in p:
             return torch.conv2d(x, p["weight"], p["bias"], layer.stride, layer.padding, layer.dilation, layer.groups)
     return layer(x)
 
 
 def batch_norm(layer: nn.Module, x):
-    if type(layer) is nn.BatchNorm2d and isinstance(x, torch.Tensor) and layer.training and layer.track_running_stats \
-            and layer.momentum is not None and x.dim() == 4 and x.numel() > x.size(1) and _plain(layer):
+    if type(layer) is _BatchNorm2d and isinstance(x, torch.Tensor) and layer.training and layer.track_running_stats \
+            and layer.momentum is not None and x.dim() == 4 and x.numel() > x.size(1) \
+            and _BatchNorm2d.forward is _bn_forward and _plain(layer):
         p, b = layer._parameters, layer._buffers
-        if "weight" in p and b.get("running_mean") is not None:
+        if "weight" in p and "bias" in p and "num_batches_tracked" in b and b.get("running_mean") is not None \
+                and b.get("running_var") is not None:
             counter = b["num_batches_tracked"]
             if counter is not None:
                 counter.add_(1)

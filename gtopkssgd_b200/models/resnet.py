@@ -42,7 +42,7 @@ class BasicBlock(nn.Module):
         self.downsample = downsample
 
     def forward(self, x):
-        if torch.jit.is_scripting():
+        if torch.jit.is_scripting() or torch.compiler.is_compiling():
             y = F.relu(self.bn_a(self.conv_a(x)), inplace=True)
             y = self.bn_b(self.conv_b(y))
         else:

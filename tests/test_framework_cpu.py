@@ -684,3 +684,42 @@ def test_detached_gradients_may_be_of_the_sparse_layout():
     table.grad = torch.sparse_coo_tensor(torch.tensor([[2]]), torch.ones(1, 3), (6, 3))
     fb.ensure_views()
     assert fb.grads_attached() and float(table.grad.sum()) == 3.0
+
+
+def test_direct_layer_calls_leave_replaced_layers_alone():
+    """A layer whose ``forward`` was replaced, on the instance or for the class, is
+    called as a layer; so is every layer while the network is traced."""
+    from gtopkssgd_b200.models import create_net, direct
+    net, _ = create_net(10, "resnet20")
+    block, x = net.stage_1[0], torch.randn(2, 16, 8, 8)
+    conv, bn = block.conv_a, block.bn_a
+    plain = conv(x)
+    conv.forward = lambda y: y + 1.0
+    assert torch.equal(direct.conv(conv, x), x + 1.0)
+    del conv.forward
+    conv._conv_forward = lambda y, w, b: y - 1.0
+    assert torch.equal(direct.conv(conv, x), x - 1.0)
+    del conv._conv_forward
+    assert torch.equal(direct.conv(conv, x), plain)
+    bn.forward = lambda y: y + 2.0
+    assert torch.equal(direct.batch_norm(bn, x), x + 2.0)
+    del bn.forward
+    for cls, layer, call in ((torch.nn.Conv2d, conv, direct.conv), (torch.nn.BatchNorm2d, bn, direct.batch_norm)):
+        owner = next(c for c in cls.__mro__ if "forward" in c.__dict__)
+        kept = owner.forward
+        owner.forward = lambda self, y: y * 3.0
+        try:
+            assert torch.equal(call(layer, x), x * 3.0)
+        finally:
+            owner.forward = kept
+    conv._compiled_call_impl = lambda y: y * 4.0   # what ``layer.compile()`` sets
+    assert torch.equal(direct.conv(conv, x), x * 4.0)
+    conv._compiled_call_impl = None
+    del conv._parameters["bias"]
+    conv.bias = None   # kept outside of the parameters
+    assert torch.equal(direct.conv(conv, x), plain)
+    scopes = {n.scopeName() for n in torch.jit.trace(block.eval(), x).inlined_graph.nodes()}
+    assert any("conv_a" in s for s in scopes)
+    block.train()
+    scopes = {n.scopeName() for n in torch.jit.trace(block, x, check_trace=False).inlined_graph.nodes()}
+    assert any("bn_a" in s for s in scopes)
