@@ -8,8 +8,12 @@ plain layer without hooks (its own or global ones), whose forward is neither
 replaced (on the instance or for the class) nor compiled, called with a tensor
 outside of tracing.  Otherwise they call the layer.  (Code that is itself
 scripted or compiled calls the layers: the caller's check, once per block.)
+``sequence`` does the same for the batch norms of an ``nn.Sequential``.
 """
 from __future__ import annotations
+
+import contextlib
+import threading
 
 import torch
 import torch.nn as nn
@@ -17,6 +21,7 @@ from torch.nn.modules import module as _m
 
 _Module, _Conv2d, _BatchNorm2d = nn.Module, nn.Conv2d, nn.BatchNorm2d
 _call, _conv_forward, _bn_forward = nn.Module.__call__, nn.Conv2d.forward, nn.BatchNorm2d.forward
+_sequence_forward = nn.Sequential.forward
 _tracing = torch._C._get_tracing_state
 
 
@@ -27,6 +32,33 @@ def _plain(layer: nn.Module) -> bool:
                 or _m._global_backward_pre_hooks
                 or "forward" in own or "_conv_forward" in own or "_check_input_dim" in own
                 or own.get("_compiled_call_impl") is not None or _Module.__call__ is not _call or _tracing() is not None)
+
+
+class _Gathered(threading.local):
+    counters = None   # of the batch-norm layers called so far, where this thread gathers them
+
+
+_gathered = _Gathered()
+
+
+@contextlib.contextmanager
+def gathered_counters():
+    """Within, the ``num_batches_tracked`` counters of the layers that
+    ``batch_norm`` calls directly are advanced by one launch at the end instead of
+    one per layer (8 us of host time each).  Each call counts once, as it would
+    have by itself; until the end the counters are behind by this pass."""
+    outer, mine = _gathered.counters, []
+    _gathered.counters = mine
+    try:
+        yield
+    finally:
+        _gathered.counters = outer
+        if len({c.data_ptr() for c in mine}) == len(mine):
+            if mine:
+                torch._foreach_add_(mine, 1)
+        else:   # a layer that ran twice, or two that share a counter: one launch would lose a count
+            for c in mine:
+                c.add_(1)
 
 
 def conv(layer: nn.Module, x):
@@ -47,7 +79,19 @@ def batch_norm(layer: nn.Module, x):
                 and b.get("running_var") is not None:
             counter = b["num_batches_tracked"]
             if counter is not None:
-                counter.add_(1)
+                if _gathered.counters is None:
+                    counter.add_(1)
+                else:
+                    _gathered.counters.append(counter)
             return torch.batch_norm(x, p["weight"], p["bias"], b["running_mean"], b["running_var"], True, layer.momentum,
                                     layer.eps, torch.backends.cudnn.enabled)
     return layer(x)
+
+
+def sequence(layers: nn.Module, x):
+    if type(layers) is nn.Sequential and isinstance(x, torch.Tensor) and nn.Sequential.forward is _sequence_forward \
+            and _plain(layers):
+        for layer in layers._modules.values():
+            x = batch_norm(layer, x) if type(layer) is _BatchNorm2d else layer(x)
+        return x
+    return layers(x)

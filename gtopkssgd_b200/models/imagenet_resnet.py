@@ -8,6 +8,8 @@ import math
 import torch
 import torch.nn as nn
 
+from . import direct
+
 
 class BasicBlock(nn.Module):
     expansion = 1
@@ -43,10 +45,16 @@ class Bottleneck(nn.Module):
         self.downsample, self.stride = downsample, stride
 
     def forward(self, x):
-        y = self.relu(self.bn1(self.conv1(x)))
-        y = self.relu(self.bn2(self.conv2(y)))
-        y = self.bn3(self.conv3(y))
-        skip = x if self.downsample is None else self.downsample(x)
+        if torch.jit.is_scripting() or torch.compiler.is_compiling():
+            y = self.relu(self.bn1(self.conv1(x)))
+            y = self.relu(self.bn2(self.conv2(y)))
+            y = self.bn3(self.conv3(y))
+            skip = x if self.downsample is None else self.downsample(x)
+        else:
+            y = self.relu(direct.batch_norm(self.bn1, self.conv1(x)))
+            y = self.relu(direct.batch_norm(self.bn2, self.conv2(y)))
+            y = direct.batch_norm(self.bn3, self.conv3(y))
+            skip = x if self.downsample is None else direct.sequence(self.downsample, x)
         return self.relu(y + skip)
 
 
@@ -82,7 +90,11 @@ class ResNet(nn.Module):
         return nn.Sequential(*blocks)
 
     def forward(self, x):
-        x = self.maxpool(self.relu(self.bn1(self.conv1(x))))
+        if torch.jit.is_scripting() or torch.compiler.is_compiling():
+            x = self.bn1(self.conv1(x))
+        else:
+            x = direct.batch_norm(self.bn1, self.conv1(x))
+        x = self.maxpool(self.relu(x))
         x = self.layer4(self.layer3(self.layer2(self.layer1(x))))
         return self.fc(torch.flatten(self.avgpool(x), 1))
 

@@ -90,7 +90,10 @@ class CifarResNet(nn.Module):
                 nn.init.zeros_(m.bias)
 
     def forward(self, x):
-        x = F.relu(self.bn_1(self.conv_1_3x3(x)), inplace=True)
+        if torch.jit.is_scripting() or torch.compiler.is_compiling():
+            x = F.relu(self.bn_1(self.conv_1_3x3(x)), inplace=True)
+        else:
+            x = torch.relu_(direct.batch_norm(self.bn_1, direct.conv(self.conv_1_3x3, x)))
         x = self.stage_3(self.stage_2(self.stage_1(x)))
         return self.classifier(torch.flatten(self.avgpool(x), 1))
 

@@ -6,6 +6,8 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
+from . import direct
+
 cfg = {
     "VGG11": [64, "M", 128, "M", 256, 256, "M", 512, 512, "M", 512, 512, "M"],
     "VGG13": [64, 64, "M", 128, 128, "M", 256, 256, "M", 512, 512, "M", 512, 512, "M"],
@@ -30,4 +32,8 @@ class VGG(nn.Module):
         self.fc = nn.Linear(512, num_classes)
 
     def forward(self, x):
-        return self.fc(torch.flatten(self.features(x), 1))
+        if torch.jit.is_scripting() or torch.compiler.is_compiling():
+            y = self.features(x)
+        else:
+            y = direct.sequence(self.features, x)
+        return self.fc(torch.flatten(y, 1))

@@ -26,6 +26,7 @@ import torch.utils.data.distributed
 from .. import models, settings
 from ..data import ptb_reader
 from ..data.synthetic import SyntheticAN4, SyntheticImages, SyntheticPTB
+from ..models import direct
 from ..models.lstm import repackage_hidden
 from ..ops import accuracy
 from ..settings import logger
@@ -34,7 +35,6 @@ from ..utils import create_path
 _support_datasets = ["imagenet", "cifar10", "an4", "ptb", "mnist"]
 _support_dnns = ["resnet50", "resnet20", "resnet56", "resnet110", "vgg19", "vgg16", "alexnet", "lstman4", "lstm",
                  "mnistnet"]
-_cnns = ("resnet50", "resnet20", "resnet56", "resnet110", "vgg19", "vgg16")   # batch norm, each layer once per pass
 NUM_CPU_THREADS = 1
 SYNTHETIC_SIZES = {"cifar10": (50000, 10000), "mnist": (60000, 10000), "imagenet": (1281167, 50000),
                    "ptb": (929589, 73760), "an4": (948, 130)}
@@ -67,29 +67,18 @@ class PrefetchedBatch:
 
 
 class BatchCounters:
-    """Runs a network with the ``num_batches_tracked`` counters of its batch-norm
-    layers advanced by one launch instead of one per layer (8 us of host time
-    each).  For networks that run every layer once per forward pass, as the CNNs
-    of the model zoo do.  The layers only count (their momentum is a constant), so
-    the counters are out of their sight while the network runs."""
+    """Runs a network with the ``num_batches_tracked`` counters of its directly
+    called batch-norm layers gathered into one launch
+    (``models.direct.gathered_counters``); all other layers count for themselves."""
 
     def __init__(self, net: nn.Module):
-        self.layers = [m for m in net.modules() if type(m) in (nn.BatchNorm1d, nn.BatchNorm2d, nn.BatchNorm3d)
-                       and m.track_running_stats and m.momentum is not None]
+        self.several = sum(type(m) is nn.BatchNorm2d for m in net.modules()) > 1
 
     def forward(self, net: nn.Module, x):
-        buffers = [m._buffers for m in self.layers if m.training]
-        if len(buffers) < 2:
+        if not self.several:
             return net(x)
-        counters = [b["num_batches_tracked"] for b in buffers]
-        torch._foreach_add_(counters, 1)
-        for b in buffers:
-            b["num_batches_tracked"] = None
-        try:
+        with direct.gathered_counters():
             return net(x)
-        finally:
-            for b, c in zip(buffers, counters):
-                b["num_batches_tracked"] = c
 
 
 class DLTrainer:
@@ -150,8 +139,7 @@ class DLTrainer:
                 self.net = torch.nn.DataParallel(self.net, device_ids=list(range(ngpus))).to(self.device)
             else:
                 self.net.to(self.device)
-        self._counters = BatchCounters(self.net) if isinstance(dnn, str) and dnn in _cnns and self.is_cuda and ngpus <= 1 \
-            else None
+        self._counters = BatchCounters(self.net) if self.is_cuda and ngpus <= 1 else None
         self.accuracy = 0
         self._loss_t: Optional[torch.Tensor] = None
         self.train_iter = 0

@@ -723,3 +723,57 @@ def test_direct_layer_calls_leave_replaced_layers_alone():
     block.train()
     scopes = {n.scopeName() for n in torch.jit.trace(block, x, check_trace=False).inlined_graph.nodes()}
     assert any("bn_a" in s for s in scopes)
+
+
+def test_batch_counters_follow_the_layers_of_the_network():
+    """Replaced layers that share the counters of the old ones, a layer that runs
+    twice, a hook that looks while the network runs: every pass counts each run
+    once and no counter is out of sight."""
+    from gtopkssgd_b200.models import create_net
+    from gtopkssgd_b200.trainer.dl_trainer import BatchCounters
+
+    class Counting(torch.nn.BatchNorm2d):
+        pass
+
+    net, _ = create_net(10, "resnet20")
+    counters = BatchCounters(net)
+    x = torch.randn(2, 3, 32, 32)
+    block, other = net.stage_2[1], net.stage_3[1]
+    bn = Counting(block.bn_a.num_features)
+    bn._buffers.update(block.bn_a._buffers)
+    block.bn_a = bn
+    other.bn_b = other.bn_a
+    seen = []
+    net.avgpool.register_forward_hook(lambda *a: seen.append([k for k in net.state_dict() if k.endswith("tracked")]))
+    counters.forward(net, x)
+    assert int(bn.num_batches_tracked) == 1 and int(other.bn_a.num_batches_tracked) == 2
+    assert int(block.bn_b.num_batches_tracked) == 1 and int(net.bn_1.num_batches_tracked) == 1
+    assert len(seen[0]) == 19
+
+    def stop(*a):
+        raise RuntimeError("stop")
+    net.stage_3.register_forward_pre_hook(stop)
+    with pytest.raises(RuntimeError):
+        counters.forward(net, x)
+    assert int(bn.num_batches_tracked) == 2 and int(other.bn_a.num_batches_tracked) == 2
+
+
+@pytest.mark.parametrize("dnn,side", [("vgg16", 32), ("resnet50", 224)])
+def test_batch_counters_of_other_networks(dnn, side):
+    from gtopkssgd_b200.models import create_net, direct
+    from gtopkssgd_b200.trainer.dl_trainer import BatchCounters
+    torch.manual_seed(0)
+    net, _ = create_net(10, dnn)
+    x = torch.randn(2, 3, side, side)
+    counted = [m for m in net.modules() if isinstance(m, torch.nn.BatchNorm2d)]
+    launches = []
+    kept = torch._foreach_add_
+    torch._foreach_add_ = lambda c, n: (launches.append(len(c)), kept(c, n))
+    try:
+        BatchCounters(net).forward(net, x)
+    finally:
+        torch._foreach_add_ = kept
+    assert launches == [len(counted)] and all(int(m.num_batches_tracked) == 1 for m in counted)
+    net(x)
+    assert all(int(m.num_batches_tracked) == 2 for m in counted)
+    torch.jit.script(net)
