@@ -142,7 +142,8 @@ class TopkSelector:
         ``addresses`` are their device addresses (0: no gradient), ``segments`` an
         int32 device tensor with the n + 1 start positions in float4 and the n
         lengths in elements (see ``segment_table``)."""
-        assert r.numel() == self.numel and r.dtype == torch.float32
+        assert r.numel() == self.numel and r.dtype is _FLOAT and r.is_contiguous()
+        assert segments.numel() == 2 * len(addresses) + 1 and segments.dtype is torch.int32 and segments.is_contiguous()
         k = int(min(k, self.max_k))
         self.last_k = k
         code = self._select_segments(addresses, segments.data_ptr(), r.data_ptr(), self.numel, k, *self._buffers,
@@ -155,7 +156,8 @@ class TopkSelector:
         it) and returns the selection as (int64 indices, fp32 values).  Nothing
         synchronises: the number of selected entries is min(k, numel)."""
         assert g.numel() == self.numel and r.numel() == self.numel
-        assert g.dtype == torch.float32 and r.dtype == torch.float32
+        assert g.dtype is _FLOAT and r.dtype is _FLOAT
+        assert g.is_contiguous() and r.is_contiguous()
         k = int(min(k, self.max_k))
         self.last_k = k
         idx = torch.empty(k, dtype=torch.int64, device=g.device)

@@ -665,3 +665,29 @@ def test_k1_pick_settles_the_thresholds_bin_apart(k, form, step):
             idx, val = idx.long(), val.clone()
         assert sel.status() == (0, 0)
         _check_selection(idx, val, r, acc, k)
+
+
+def test_selector_refuses_what_the_kernels_cannot_read():
+    """Strided vectors, which the kernels would take for contiguous ones, and a
+    segment table of another number of tensors."""
+    from gtopkssgd_b200.ops.select import segment_table
+    from gtopkssgd_b200.parallel.compression import TopKCompressor, compressors
+    d, k = 1000, 10
+    sel = _selector(d, k)
+    wide = torch.randn(2 * d, device=DEV)
+    kept, r = wide.clone(), torch.zeros(d, device=DEV)
+    for g, res in ((wide[::2], r), (torch.randn(d, device=DEV), wide[::2])):
+        with pytest.raises(AssertionError):
+            sel.compress(g, res, k)
+    TopKCompressor.clear()
+    with pytest.raises(AssertionError):
+        compressors["gtopk"].compress(wide[::2], "strided", ratio=0.01)
+    TopKCompressor.clear()
+    g = torch.randn(d, device=DEV)
+    table = segment_table([0, 500], [500, 500], d, DEV)
+    for addresses, t, res in (([g.data_ptr()] * 2, table, wide[::2]), ([g.data_ptr()] * 3, table, r),
+                              ([g.data_ptr()], table, r), ([g.data_ptr()] * 2, table.long(), r)):
+        with pytest.raises(AssertionError):
+            sel.select_segments(addresses, t, res, k)
+    torch.cuda.synchronize()
+    assert torch.equal(wide, kept)
