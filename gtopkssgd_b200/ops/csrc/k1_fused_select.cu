@@ -371,7 +371,7 @@ k1_stream(float* g, float* r, const float* g_scale, long long d, Pair* cand, uns
   stream_pass<HIST, DYNAMIC, ZERO>(ss, FlatGrad{g}, r, g_scale, d, cand, cap, st, ctrl_pair);
 }
 
-// segments: n + 1 start positions, then n lengths (written once at set-up, so they are read ahead of the wait).
+// segments: n + 1 start positions, then n lengths.
 template <bool HIST, bool DYNAMIC, int N>
 __global__ void __launch_bounds__(kK1Threads, 2)
 k1_stream_segments(const __grid_constant__ GradPointers<N> g, const unsigned int* segments, unsigned int n, float* r,
@@ -380,9 +380,9 @@ k1_stream_segments(const __grid_constant__ GradPointers<N> g, const unsigned int
   __shared__ unsigned int seg[2 * N + 1];
   if (HIST)
     for (int i = threadIdx.x; i < kBins; i += kK1Threads) ss.hist[i] = 0u;
+  pdl_begin(segments, r, st, ctrl_pair);
   for (unsigned int i = threadIdx.x; i < 2u * n + 1u; i += kK1Threads) seg[i] = segments[i];
   __syncthreads();
-  pdl_begin(r, st, ctrl_pair);
   const float* no_scale = nullptr;
   stream_pass<HIST, DYNAMIC, false>(ss, SegmentedGrad{g.g, seg, seg + n + 1, n}, r, no_scale, d, cand, cap, st, ctrl_pair);
 }

@@ -127,10 +127,9 @@ k2_tree_small(const K2Rank* ranks, unsigned int rank_base, unsigned int P, unsig
   const uint32_t bins_at = shared_address(s.hist);
   const unsigned int tid = threadIdx.x;
   const unsigned int me = rank_base + blockIdx.x;
-  const K2Rank& R = ranks[blockIdx.x];
   unsigned int* const bins = s.hist;
 
-  // ---- before the predecessor has ended: the table, and the descriptor (which no kernel writes)
+  // ---- before the predecessor has ended: the table
   auto clear_table = [&]() {
     for (unsigned int j = 4u * tid; j < slots; j += 4u * kPickThreads)
       *reinterpret_cast<uint4*>(&words[j]) = make_uint4(kEmpty, kEmpty, kEmpty, kEmpty);
@@ -144,16 +143,17 @@ k2_tree_small(const K2Rank* ranks, unsigned int rank_base, unsigned int P, unsig
     s.list_n = 0u;
     s.tie = 0u;
   }
-  const Pair* sel = R.sel;
-  const K1State* st = R.st;
-  unsigned int* epoch_word = R.epoch;
-  unsigned int* result = R.n_global;
-  Ctrl* ctrl_pair = R.ctrl;
-  float* resid = R.resid;
   __syncthreads();
-  pdl_begin(sel, st, epoch_word, result, ctrl_pair, resid);
+  pdl_begin(ranks);
 
-  // one round of loads
+  // the descriptor (several ranks' are put together by a kernel, possibly the one just before), then one round of loads
+  const K2Rank& R = ranks[blockIdx.x];
+  const Pair* const sel = R.sel;
+  const K1State* const st = R.st;
+  unsigned int* const epoch_word = R.epoch;
+  unsigned int* const result = R.n_global;
+  Ctrl* const ctrl_pair = R.ctrl;
+  float* const resid = R.resid;
   const unsigned int epoch = __ldcg(epoch_word);
   const unsigned int failed_before = __ldcg(&result[kResStatus]);
   const unsigned int heavy[2] = {__ldcg(&ctrl_pair[0].scratch[8]), __ldcg(&ctrl_pair[1].scratch[8])};

@@ -691,3 +691,42 @@ def test_selector_refuses_what_the_kernels_cannot_read():
             sel.select_segments(addresses, t, res, k)
     torch.cuda.synchronize()
     assert torch.equal(wide, kept)
+
+
+def test_tables_may_be_written_by_the_kernel_just_before():
+    """The rank descriptors of an exchange and the segment table of a select are
+    read behind the wait for the predecessor: it may be the kernel that wrote
+    them.  (Before, they hold another valid set.)"""
+    from gtopkssgd_b200.ops import exchange as ex
+    from gtopkssgd_b200.ops.select import segment_table
+    torch.manual_seed(2)
+    P, d, k = 4, 20_000, 500
+    worlds = [_emulated_world(P, d, k) for _ in range(2)]
+    desc = worlds[0][1].clone()
+    for it in range(6):
+        ranks, _ = worlds[it & 1]
+        grads = [torch.randn(d, device=DEV) for _ in range(P)]
+        for r, g in zip(ranks, grads):
+            r.resid.zero_()
+            r.selector.select(g, r.resid, k)
+        epochs = [int(r.epoch.item()) for w, _ in worlds for r in w]
+        torch.cat([r.desc for r in ranks], out=desc)
+        ex.launch_gtopk(ranks, desc, 0, P, k, nctas=1, limit_ms=2000)
+        torch.cuda.synchronize()
+        res = [torch.zeros(d) for _ in range(P)]
+        (gi, gv), _ = oracle.simulate_gtopk_step([g.cpu() for g in grads], res, k)
+        for r, want in zip(ranks, res):
+            assert r.status() == (0, 0) and set(_read_gout(r, r.last_parity())[0].tolist()) == set(gi.tolist())
+            assert torch.allclose(r.resid.cpu(), want, rtol=1e-5, atol=1e-9)
+        now = [int(r.epoch.item()) for w, _ in worlds for r in w]
+        assert [b - a for a, b in zip(epochs, now)] == [int(w == (it & 1)) for w in range(2) for _ in range(P)]
+    sizes = [[400, 1600], [1600, 400]]
+    tables = [segment_table([0, s[0]], s, 2000, DEV) for s in sizes]
+    table, sel, r = tables[0].clone(), _selector(2000, 20), torch.zeros(2000, device=DEV)
+    for it in range(6):
+        s = sizes[it & 1]
+        grads = [torch.randn(1600, device=DEV) for _ in s]
+        acc = torch.cat([g[:n] for g, n in zip(grads, s)]) + r
+        torch.add(tables[it & 1], 0, out=table)
+        sel.select_segments([g.data_ptr() for g in grads], table, r, 20)
+        _check_selection(*sel.pairs(), r, acc, 20)
