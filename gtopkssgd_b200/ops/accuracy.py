@@ -11,6 +11,7 @@ MAX_ELEMENTS = 1 << 18  # one CTA reads the logits; larger batches take the libr
 
 def takes(output: torch.Tensor, target: torch.Tensor) -> bool:
     return (output.is_cuda and output.dim() == 2 and output.dtype == torch.float32 and output.is_contiguous()
+            and output.get_device() == torch.cuda.current_device()  # a launch goes to the current device
             and 0 < output.numel() <= MAX_ELEMENTS and target.dtype == torch.int64 and target.is_contiguous()
             and target.numel() == output.size(0) and target.device == output.device)
 

@@ -424,3 +424,14 @@ def test_gradients_replaced_by_the_user_are_taken_as_they_are():
     optimizer's gives, also for a parameter without a gradient in one iteration."""
     import test_framework_cpu as cpu
     cpu.check_replaced_gradients("cuda")
+
+
+def test_top1_accuracy_of_another_device_takes_the_librarys_way(monkeypatch):
+    from gtopkssgd_b200.ops import accuracy
+    from gtopkssgd_b200.trainer.dl_trainer import DLTrainer
+    x, y = torch.randn(6, 4, device="cuda:0"), torch.randint(0, 4, (6,), device="cuda:0")
+    want = float(DLTrainer.cal_accuracy(x, y)[0])
+    assert accuracy.takes(x, y)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 1)
+    assert not accuracy.takes(x, y)
+    assert float(DLTrainer.cal_accuracy(x, y)[0]) == pytest.approx(want, abs=1e-4)
