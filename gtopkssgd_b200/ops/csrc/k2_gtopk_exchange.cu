@@ -123,7 +123,8 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
   if (cta == 0 && threadIdx.x == 0) ctrl->scratch[8] = 1u;  // this block's histograms will need clearing
   trace_stamp(ctrl, 0);
   // Every live entry of a round's union is counted once in the band above `pred` (delta = 1 adds, 0xffffffff
-  // removes): the union's k-th magnitude is at least this rank's own and for gradient tails a few per cent above.
+  // removes).  A prediction: for gradient tails the union's k-th magnitude is a few per cent above this rank's own,
+  // but where entries of opposite sign cancel it is below, at any distance (bin 0; the counting sweeps then).
   uint32_t pred = mag_key(kth_mag);  // round 0: K1's k-th magnitude, then the previous round's threshold
   auto tally = [&](float v, unsigned int delta) { atomicAdd(&sh.band[band_bin(mag_key(v), pred)], delta); };
 
@@ -273,7 +274,7 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
     };
     Threshold th;
     if (!band_select_kth(ss, bar, k, pred, ctrl->hist[r], &ctrl->live[r], visit, &th, 250 + 10 * r)) { fail(); return; }
-    if (!th.select_all) pred = th.key;  // the next union's threshold is at least this one
+    if (!th.select_all) pred = th.key;  // the prediction for the next union
     trace_stamp(ctrl, 1 + 8 * r + 4);
 
     // ---- compaction of the winners to where the next phase reads them

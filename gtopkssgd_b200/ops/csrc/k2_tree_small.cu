@@ -275,7 +275,7 @@ k2_tree_small(const K2Rank* ranks, unsigned int rank_base, unsigned int P, unsig
     Level lv{pred, 0x7fffffffu, kBandShift, true};
     unsigned int k_rem = k;
     for (bool direct = true;; direct = false) {
-      if (find_bin(s, counts, k_rem) < k_rem) {  // the threshold lies below the predicted band
+      if (find_bin(s, counts, k_rem) < k_rem) {  // the threshold lies below the predicted band: entries cancelled
         lv = Level{0u, 0x7fffffffu, 20u, false};
         direct = false;
       } else {

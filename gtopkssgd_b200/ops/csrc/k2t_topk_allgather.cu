@@ -128,7 +128,8 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
   }
 
   // ---- topk2: merge the P lists in rank order, then keep the k largest sums
-  const uint32_t pred = mag_key(kth_mag);  // no sum of P selections has its k-th magnitude below the own one
+  // A prediction, as in the tree: the sums' k-th magnitude lies below the own one where entries cancel.
+  const uint32_t pred = mag_key(kth_mag);
   for (int i = threadIdx.x; i < kHistBins; i += kSelThreads) band[i] = 0u;
   __syncthreads();
   auto tally = [&](float v, unsigned int delta) { atomicAdd(&band[band_bin(mag_key(v), pred)], delta); };

@@ -90,7 +90,7 @@ __device__ __forceinline__ void find_digit_in(SelectShared& s, const unsigned in
   __syncthreads();
 }
 
-// First selection level of a set whose k-th magnitude is expected at or a little above `lo`: bin 0 below lo,
+// First selection level of a set whose k-th magnitude is expected (not known) at or a little above `lo`: bin 0 below lo,
 // bins of 2^kBandShift keys above it (together a quarter octave), the last bin open to the top.
 constexpr unsigned int kBandShift = 10u;
 __device__ __forceinline__ unsigned int band_bin(uint32_t key, uint32_t lo) {

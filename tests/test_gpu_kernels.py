@@ -730,3 +730,54 @@ def test_tables_may_be_written_by_the_kernel_just_before():
         torch.add(tables[it & 1], 0, out=table)
         sel.select_segments([g.data_ptr() for g in grads], table, r, 20)
         _check_selection(*sel.pairs(), r, acc, 20)
+
+
+@pytest.mark.parametrize("mode,P,k,nctas", [("gtopk", 2, 1000, 1), ("gtopk", 4, 2000, 1), ("gtopk", 2, 6000, 4), ("gtopk", 4, 9000, 3),
+                                            ("gtopk", 2, 30_000, 40), ("topk2", 2, 1000, 1), ("topk2", 4, 6000, 4)])
+def test_exchange_of_gradients_that_cancel(mode, P, k, nctas):
+    """Ranks in pairs with almost opposite gradients: most of the largest entries
+    cancel, so that the sums' k-th magnitude lies far below every rank's own, the
+    bottom of the band that the re-select predicts.  (Sums of numbers of about 2
+    are multiples of 2^-23 or so: at 30 000 of them over a range of 0.2, two at
+    the k-th place may be equal, and either may be kept.)"""
+    from gtopkssgd_b200.ops import exchange as ex
+    d = 30 * k
+    torch.manual_seed(P + k)
+    ranks, desc = _emulated_world(P, d, k, mode)
+    seg_counts = torch.zeros(P * ex.MAX_PEERS, dtype=torch.int32, device=DEV)
+    for call in range(3):
+        res_ref = [torch.zeros(d) for _ in range(P)]
+        grads = []
+        for r in range(0, P, 2):
+            g = torch.randn(d, device=DEV)
+            grads += [g, -g + 0.2 * torch.randn(d, device=DEV)]
+        own = []
+        for r, g in zip(ranks, grads):
+            r.resid.zero_()
+            r.selector.select(g, r.resid, k)
+            own.append(float(r.selector.state[6:7].view(torch.float32)))
+        if mode == "topk2":
+            ex.launch_allgather(ranks, desc, seg_counts, 0, P, k, reselect=True, nctas=nctas, limit_ms=2000)
+            local = [oracle.compress(g.cpu(), rr, k) for g, rr in zip(grads, res_ref)]
+            gi, gv = oracle.topk2_reselect(local, k)
+            for rr, loc in zip(res_ref, local):
+                oracle.put_back(rr, loc, gi)
+        else:
+            ex.launch_gtopk(ranks, desc, 0, P, k, nctas=nctas, limit_ms=2000)
+            (gi, gv), _ = oracle.simulate_gtopk_step([g.cpu() for g in grads], res_ref, k)
+        torch.cuda.synchronize()
+        cut = float(gv.abs().min())
+        assert cut < 0.5 * min(own)
+        ref = dict(zip(gi.tolist(), gv.tolist()))
+        for r, want in zip(ranks, res_ref):
+            assert r.status() == (0, 0)
+            qi, qv = _read_gout(r, r.last_parity())
+            got = dict(zip(qi.cpu().tolist(), qv.cpu().tolist()))
+            assert len(got) == qi.numel() == len(ref)
+            swapped = set(got) ^ set(ref)
+            assert len(swapped) <= 2 and all(abs({**ref, **got}[j]) == pytest.approx(cut, rel=1e-6) for j in swapped)
+            for j in set(got) & set(ref):
+                assert got[j] == pytest.approx(ref[j], rel=1e-5, abs=1e-6)
+            same = torch.ones(d, dtype=torch.bool)
+            same[list(swapped)] = False
+            assert torch.allclose(r.resid.cpu()[same], want[same], rtol=1e-5, atol=1e-6)
