@@ -61,6 +61,15 @@ def gathered_counters():
                 c.add_(1)
 
 
+def layers_of(module: nn.Module, *names):
+    """The module's attributes of these names, without ``__getattr__`` where they are registered layers."""
+    registered = module._modules
+    try:
+        return [registered[n] for n in names]
+    except KeyError:
+        return [getattr(module, n) for n in names]
+
+
 def conv(layer: nn.Module, x):
     if type(layer) is _Conv2d and isinstance(x, torch.Tensor) and layer.padding_mode == "zeros" \
             and _Conv2d.forward is _conv_forward and _plain(layer):

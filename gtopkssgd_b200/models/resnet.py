@@ -46,9 +46,9 @@ class BasicBlock(nn.Module):
             y = F.relu(self.bn_a(self.conv_a(x)), inplace=True)
             y = self.bn_b(self.conv_b(y))
         else:
-            layers = self._modules
-            y = torch.relu_(direct.batch_norm(layers["bn_a"], direct.conv(layers["conv_a"], x)))
-            y = direct.batch_norm(layers["bn_b"], direct.conv(layers["conv_b"], y))
+            conv_a, bn_a, conv_b, bn_b = direct.layers_of(self, "conv_a", "bn_a", "conv_b", "bn_b")
+            y = torch.relu_(direct.batch_norm(bn_a, direct.conv(conv_a, x)))
+            y = direct.batch_norm(bn_b, direct.conv(conv_b, y))
         skip = x if self.downsample is None else self.downsample(x)
         return torch.relu_(skip + y)
 

@@ -777,3 +777,13 @@ def test_batch_counters_of_other_networks(dnn, side):
     net(x)
     assert all(int(m.num_batches_tracked) == 2 for m in counted)
     torch.jit.script(net)
+
+
+def test_block_layers_may_be_plain_callables():
+    """A batch norm that was folded away: deleted, a function in its place."""
+    from gtopkssgd_b200.models import create_net
+    block, x = create_net(10, "resnet20")[0].stage_1[0], torch.randn(2, 16, 8, 8)
+    del block.bn_a
+    block.bn_a = lambda y: 2.0 * y
+    want = torch.relu(x + block.bn_b(block.conv_b(torch.relu(2.0 * block.conv_a(x)))))
+    assert torch.allclose(block(x), want, atol=1e-6)
