@@ -26,10 +26,10 @@
 //
 // What bounds it: a chain of phases of 2 to 6 us, each a round of L2 or scattered
 // DRAM accesses (the table spans d) and a barrier; past k of about 200 000 the
-// scattered accesses themselves (45 a ns).  Two ranks, k = 66 034, whole call:
-// 44 us with flags behind fenced plain stores and the put-back at the end, 31 us
-// now (k = 255 570: 87 and 74; four ranks, k = 14 728: 41 and 35; eight ranks,
-// k = 40 000: 117 and 97).
+// scattered accesses themselves (45 a ns).  Two ranks, k = 66 034, the same
+// selection exchanged again and again: 40 us with flags behind fenced plain stores
+// and the put-back at the end, 23 us now (k = 255 570: 88 and 70; four ranks, k =
+// 14 728: 43 and 32; eight ranks, k = 40 000: 122 and 85).
 //
 // No host-side clearing: the rank owns two control blocks; call e uses block
 // (e & 1) and zeroes the other one for call e + 1 once its own work is done.

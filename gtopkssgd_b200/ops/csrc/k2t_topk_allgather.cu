@@ -15,10 +15,10 @@
 // them (table, entry, append).  The lists travel as the tree's 8-byte wire words,
 // so nobody fences or waits for a complete list, and a merged entry remembers
 // where in the own selection it comes from, so that dropping it is also its way
-// back to the residual.  Four ranks, k = 14 728: 41 us with flags behind fenced
-// stores, the put-back behind a table over the global set and one entry per thread
-// in flight, 35 now (eight ranks, k = 20 000: 113 and 97; two, k = 660 340: 256 and
-// 182).
+// back to the residual.  Four ranks, k = 14 728, the same selection again and again:
+// 53 us with flags behind fenced stores, the put-back behind a table over the global
+// set and one entry per thread in flight, 29 now (eight ranks, k = 20 000: 139 and
+// 76; two, k = 660 340: 312 and 176; 'topk', four ranks, k = 14 728: 23 and 10).
 #include "exchange_common.cuh"
 
 namespace gtk {

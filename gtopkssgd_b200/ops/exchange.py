@@ -221,20 +221,23 @@ SMALL_MAX_K = 2048  # up to here the tree runs in one CTA with the set in shared
 
 
 def default_nctas(k: int, nranks: int = 1, sms: int = 148) -> int:
-    """CTAs per rank for the exchange kernels, from sweeps on B200 (whole call):
+    """CTAs per rank for the exchange kernels, from sweeps on one B200 that holds
+    all ranks (whole call, the same selection again and again):
 
     * up to 4 K union entries of the tree: one CTA, the set in shared memory
-      (two ranks: 10 us at k = 1 000 and 16 us at 2 000, against 23 and 25 us
-      with a cluster; 26 against 25 us at 3 000);
+      (two ranks: 10 us at k = 1 000 and 15 us at 2 000, against 16.5 us with a
+      cluster; the shared arrays end there);
     * up to 20 K union entries: a power-of-two cluster of 2..16 CTAs joined by
       the hardware cluster barrier, about 1024 entries per CTA (four ranks, k =
-      6 500: 27 us with 16 CTAs, 29 to 33 us with 24 to 74 and the software
-      barrier; k = 13 000: 34 and 32 us);
-    * above: one CTA per 768 entries with the software barrier, as many as the
-      device holds one per SM, and two per SM where each of those had more than
-      2 000 entries (eight ranks, k = 40 000: 97 us with 37 CTAs, 115 with 18;
-      two ranks, k = 255 570: 74 us with 148, 82 with 74; k = 66 000: 31 us
-      with either)."""
+      6 500: 27.7 us with 16 CTAs, 28.7 with 24 and 37 and the software barrier,
+      34.9 with 74; k = 13 000: 33.2 with 16 and 31.8 with 33);
+    * above: one CTA per 768 entries with the software barrier, at most one per
+      SM over all ranks of the launch, and two per SM where each of those had
+      more than 2 000 entries (eight ranks, k = 40 000: 83 us with 37 CTAs each,
+      98 with 18; two ranks, k = 255 570: 69 us with 148, 78 with 74; k = 66 000:
+      22 and 23).  A rank gets at most ``sms`` CTAs in any case, so one that has
+      its GPU to itself stays at one per SM: two have not been measured there,
+      which takes a GPU for each rank."""
     return 1 if k <= SMALL_MAX_K else _spread_nctas(2 * k, nranks, sms)
 
 
