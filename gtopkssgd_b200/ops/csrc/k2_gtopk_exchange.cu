@@ -300,22 +300,24 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
       if (!only_round) map[e.idx] = (int32_t)pos;
     };
     unsigned int* const tie = &ctrl->tie[r];
-    StagedAppender app{&ss, &ctrl->cursor[r], kcap, ctrl};
+    StagedAppender app{&ss, &ctrl->cursor[r], kcap, ctrl, 0u};
     app.begin();
     auto sweep = [&](const Pair (&e)[kK2Cache], unsigned int t0) {
       unsigned int lost = 0;
 #pragma unroll
       for (int t = 0; t < kK2Cache; ++t) {
         if (t0 + t >= trips) break;
+        bool stays = false;
         if (e[t].idx >= 0) {
-          if (passes_threshold(mag_key(e[t].val), th, tie)) {
+          stays = passes_threshold(mag_key(e[t].val), th, tie);
+          if (stays) {
             app.put(e[t]);
             if (keep) tally(e[t].val, 1u);
           } else {
             lost |= 1u << t;
           }
         }
-        app.end_tile(on_placed);
+        app.end_tile(stays, on_placed);
       }
       if (t0 + kK2Cache >= trips) app.flush(on_placed);
       if (!only_round) return;

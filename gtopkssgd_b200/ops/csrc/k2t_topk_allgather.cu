@@ -275,7 +275,7 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
   if (!band_select_kth(sh.sel, bar, k, pred, ctrl->hist[0], &ctrl->live[0], visit, &th, 580)) { fail(); return; }
   Pair* const G = R.gout + (size_t)parity * kcap;
   auto on_placed = [&](Pair e, unsigned int pos) { st_pair(&G[pos], e); };
-  StagedAppender app{&sh.sel, &ctrl->cursor[0], kcap, ctrl};
+  StagedAppender app{&sh.sel, &ctrl->cursor[0], kcap, ctrl, 0u};
   app.begin();
   auto sweep = [&](const Pair (&e)[kBatch], unsigned int t0) {
     unsigned int from[kBatch];
@@ -283,11 +283,13 @@ k2t_topk_allgather(const K2Rank* __restrict__ ranks, unsigned int rank_base, uns
 #pragma unroll
     for (int t = 0; t < kBatch; ++t) {
       from[t] = kNotOwn;
+      bool stays = false;
       if (e[t].idx >= 0) {
-        if (passes_threshold(mag_key(e[t].val), th, &ctrl->tie[0])) app.put(e[t]);
+        stays = passes_threshold(mag_key(e[t].val), th, &ctrl->tie[0]);
+        if (stays) app.put(e[t]);
         else from[t] = __ldcg(&own[(t0 + t) * stride + lane0]);
       }
-      if (t0 + t < trips) app.end_tile(on_placed);
+      if (t0 + t < trips) app.end_tile(stays, on_placed);
     }
     // what drops out of the sum although this rank had selected it goes back to its residual
 #pragma unroll

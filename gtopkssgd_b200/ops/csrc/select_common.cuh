@@ -165,16 +165,19 @@ __device__ __forceinline__ bool band_select_kth(SelectShared& s, RankBarrier& ba
   return true;
 }
 
-// CTA-wide staged append.  Call put() from any thread, then end_tile() from all
-// threads once per loop trip (at most kSelThreads puts between two end_tile calls).
-// place(pair, position) stores an entry.
+// CTA-wide staged append.  Call put() from any thread, at most once, then end_tile(whether it has) from all threads,
+// once per loop trip; place(pair, position) stores an entry.  Whether the stage is full is decided from a count that every
+// thread of the CTA gets from the barrier: read from shared memory behind it, a fast thread's next put() could
+// reach a slow one's look at the counter, which then flushed alone.
 struct StagedAppender {
   SelectShared* s;
   unsigned int* cursor;  // global cursor (local memory)
   unsigned int cap;
   Ctrl* ctrl;
+  unsigned int staged;   // the same in all threads
 
   __device__ __forceinline__ void begin() {
+    staged = 0u;
     if (threadIdx.x == 0) s->stage_n = 0u;
     __syncthreads();
   }
@@ -184,26 +187,25 @@ struct StagedAppender {
   }
   template <typename Place>
   __device__ __forceinline__ void flush(Place place) {
-    __syncthreads();
-    const unsigned int n = s->stage_n;
-    if (n) {
-      if (threadIdx.x == 0) s->stage_base = atomicAdd(cursor, n);
-      __syncthreads();
-      const unsigned int base = s->stage_base;
-      for (unsigned int i = threadIdx.x; i < n; i += kSelThreads) {
-        const unsigned int pos = base + i;
-        if (pos < cap) place(s->stage[i], pos);
-        else record_error(ctrl, ST_CAPACITY, 900);
-      }
-      __syncthreads();
-      if (threadIdx.x == 0) s->stage_n = 0u;
+    if (staged == 0u) return;
+    if (threadIdx.x == 0) {
+      s->stage_base = atomicAdd(cursor, staged);
+      s->stage_n = 0u;
     }
+    __syncthreads();
+    const unsigned int base = s->stage_base;
+    for (unsigned int i = threadIdx.x; i < staged; i += kSelThreads) {
+      const unsigned int pos = base + i;
+      if (pos < cap) place(s->stage[i], pos);
+      else record_error(ctrl, ST_CAPACITY, 900);
+    }
+    staged = 0u;
     __syncthreads();
   }
   template <typename Place>
-  __device__ __forceinline__ void end_tile(Place place) {
-    __syncthreads();
-    if (s->stage_n > (unsigned int)(kStageCap - kSelThreads)) flush(place);
+  __device__ __forceinline__ void end_tile(bool has_put, Place place) {
+    staged += (unsigned int)__syncthreads_count(has_put);
+    if (staged > (unsigned int)(kStageCap - kSelThreads)) flush(place);
   }
 };
 

@@ -781,3 +781,35 @@ def test_exchange_of_gradients_that_cancel(mode, P, k, nctas):
             same = torch.ones(d, dtype=torch.bool)
             same[list(swapped)] = False
             assert torch.allclose(r.resid.cpu()[same], want[same], rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("mode,P,k", [("topk2", 8, 60_000), ("gtopk", 2, 200_000)])
+def test_exchange_stages_many_entries_per_cta(mode, P, k):
+    """Thousands of winners per CTA, so that the stage in shared memory fills and
+    empties several times in every call: all threads of a CTA have to agree on
+    when it is full (they did not always, and a call in a few hundred lost its
+    place in the output list)."""
+    from gtopkssgd_b200.ops import exchange as ex
+    d = 1_000_000
+    torch.manual_seed(P)
+    ranks, desc = _emulated_world(P, d, k, mode)
+    seg_counts = torch.zeros(P * ex.MAX_PEERS, dtype=torch.int32, device=DEV)
+    grads = [torch.randn(d, device=DEV) for _ in range(P)]
+    total = torch.zeros(d, device=DEV)
+    for r, g in zip(ranks, grads):
+        r.selector.select(g, r.resid, k)
+        idx, val = r.selector.pairs()
+        total[idx] += val
+    want = total.abs().topk(k).values[-1]
+    for call in range(60):
+        if mode == "topk2":
+            ex.launch_allgather(ranks, desc, seg_counts, 0, P, k, reselect=True, limit_ms=1000)
+        else:
+            ex.launch_gtopk(ranks, desc, 0, P, k, limit_ms=1000)
+    torch.cuda.synchronize()
+    for r in ranks:
+        assert r.status() == (0, 0)
+        gi, gv = _read_gout(r, r.last_parity())
+        assert gi.unique().numel() == k
+        assert torch.allclose(gv, total[gi], rtol=1e-5, atol=1e-6)
+        assert float(gv.abs().min()) == pytest.approx(float(want), rel=1e-5)
