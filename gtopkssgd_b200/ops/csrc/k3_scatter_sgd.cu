@@ -98,10 +98,17 @@ k3_dense(float* p, float* buf, const float* g,
 }
 
 // Sparse part.  `pairs` holds nseg segments of seg_stride pairs; segment s (one row of the grid) has
-// counts[s] live pairs.  use_atomics: indices may repeat across segments.  Bound by the latency of scattered
-// 4-byte accesses, so a thread has kSparseBatch entries' loads in flight before the first store.
-constexpr int kSparseBatch = 4;
-__global__ void __launch_bounds__(256)
+// counts[s] live pairs.  use_atomics: indices may repeat across segments.
+// What bounds it: scattered 4-byte accesses, each a 32-byte sector of DRAM read and written back (about 23 pairs a ns).
+// One entry per thread and as many CTAs as that takes: CTAs that have loaded and CTAs that store are then always
+// there side by side.  With four entries per thread in a grid that fills the chip once, all of it loads first and
+// stores afterwards: select + update of 138 M elements at 0.01 353 us against 337, with momentum 422 against 397
+// (60 M: 191 and 181; two entries per thread: 340, 408 and 188); the same up to 300 000 entries.
+// (The grid goes by the lists' capacity, of which there may be much more than entries: it ends at 16 times what the
+// chip holds, 4.8 M entries, and the threads loop from there on.)
+constexpr int kSparseThreads = 256;
+constexpr unsigned int kSparseMaxBlocks = 148u * 8u * 16u;
+__global__ void __launch_bounds__(kSparseThreads)
 k3_sparse(float* p, float* buf, const Pair* pairs,
           const unsigned int* counts, unsigned int seg_stride,
           const float* coef_ptr, float scale, unsigned int d, SgdHyper h,
@@ -113,47 +120,31 @@ k3_sparse(float* p, float* buf, const Pair* pairs,
   const float coef = coef_ptr ? (*coef_ptr) * scale : scale;
   const float f = h.first_step ? 1.0f : 1.0f - h.dampening;
   const bool has_buf = buf != nullptr && h.momentum != 0.f;
-  const Pair* seg = pairs + (size_t)blockIdx.y * seg_stride;
   unsigned int n = counts[blockIdx.y];
   if (n > seg_stride) n = seg_stride;
-  const unsigned int stride = gridDim.x * blockDim.x;
-  for (unsigned int i0 = blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += kSparseBatch * stride) {
-    Pair e[kSparseBatch];
-    float pv[kSparseBatch], bv[kSparseBatch];
-#pragma unroll
-    for (int u = 0; u < kSparseBatch; ++u) {
-      const unsigned int i = i0 + (unsigned int)u * stride;
-      e[u].idx = -1;
-      if (i >= n) continue;
-      e[u] = seg[i];
-      if ((unsigned int)e[u].idx >= d) {
-        atomicAdd(bad_index_count, 1u);
-        e[u].idx = -1;
-      }
+  const Pair* const seg = pairs + (size_t)blockIdx.y * seg_stride;
+  const unsigned int stride = gridDim.x * kSparseThreads;
+  for (unsigned int i = blockIdx.x * kSparseThreads + threadIdx.x; i < n; i += stride) {
+    const Pair e = seg[i];
+    if ((unsigned int)e.idx >= d) {
+      atomicAdd(bad_index_count, 1u);
+      continue;
     }
+    float pv = 0.f, bv = 0.f;
     if (!use_atomics) {
-#pragma unroll
-      for (int u = 0; u < kSparseBatch; ++u) {
-        pv[u] = bv[u] = 0.f;
-        if (e[u].idx < 0) continue;
-        pv[u] = p[e[u].idx];
-        if (has_buf) bv[u] = buf[e[u].idx];
-      }
+      pv = p[e.idx];
+      if (has_buf) bv = buf[e.idx];
     }
-#pragma unroll
-    for (int u = 0; u < kSparseBatch; ++u) {
-      if (e[u].idx < 0) continue;
-      const float sv = e[u].val * coef;
-      float step = sv;
-      if (has_buf) {
-        const float sb = f * sv;
-        if (use_atomics) atomicAdd(&buf[e[u].idx], sb);
-        else buf[e[u].idx] = bv[u] + sb;
-        step = h.nesterov ? fmaf(h.momentum, sb, sv) : sb;
-      }
-      if (use_atomics) atomicAdd(&p[e[u].idx], -h.lr * step);
-      else p[e[u].idx] = fmaf(-h.lr, step, pv[u]);
+    const float sv = e.val * coef;
+    float step = sv;
+    if (has_buf) {
+      const float sb = f * sv;
+      if (use_atomics) atomicAdd(&buf[e.idx], sb);
+      else buf[e.idx] = bv + sb;
+      step = h.nesterov ? fmaf(h.momentum, sb, sv) : sb;
     }
+    if (use_atomics) atomicAdd(&p[e.idx], -h.lr * step);
+    else p[e.idx] = fmaf(-h.lr, step, pv);
   }
 }
 
@@ -255,12 +246,12 @@ extern "C" int gtk_k3_sparse(float* p, float* buf, const void* pairs, const unsi
   cudaStream_t stream = (cudaStream_t)stream_;
   if (nseg == 0 || seg_stride == 0) return GTK_ERR_ARG;
   SgdHyper h{lr_ptr, lr, momentum, dampening, weight_decay, nesterov, first_step};
-  unsigned int blocks = (seg_stride + 255u) / 256u;
-  if (blocks > 1184u) blocks = 1184u;
+  unsigned int blocks = (seg_stride + kSparseThreads - 1u) / kSparseThreads;
+  if (blocks > kSparseMaxBlocks) blocks = kSparseMaxBlocks;
   // Behind a large exchange (a cooperative kernel, which cannot overlap) an ordinary launch: there the overlapped
   // one made the next exchange start 2 us later (57.3 against 55.4 us per exchange + update at 2 x 66 000).
   const bool overlap = parity_word == nullptr || seg_stride <= kLLMaxK;
-  const cudaError_t e = launch_pdl_if(overlap, k3_sparse, dim3(blocks, nseg), 256, stream, p, buf, (const Pair*)pairs, counts,
+  const cudaError_t e = launch_pdl_if(overlap, k3_sparse, dim3(blocks, nseg), kSparseThreads, stream, p, buf, (const Pair*)pairs, counts,
                                       seg_stride, coef, scale, d, h, use_atomics, bad_index_count, parity_word, parity_stride);
   gtk_count_launch(1);
   return e == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;

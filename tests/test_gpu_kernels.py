@@ -813,3 +813,32 @@ def test_exchange_stages_many_entries_per_cta(mode, P, k):
         assert gi.unique().numel() == k
         assert torch.allclose(gv, total[gi], rtol=1e-5, atol=1e-6)
         assert float(gv.abs().min()) == pytest.approx(float(want), rel=1e-5)
+
+
+@pytest.mark.parametrize("n,capacity,nseg", [(0, 5, 1), (1, 1, 1), (257, 300, 3), (256, 100_000, 2), (4_849_665, 4_900_000, 1)])
+@pytest.mark.parametrize("momentum", [0.0, 0.9])
+def test_k3_sparse_covers_lists_below_at_and_beyond_its_grid(n, capacity, nseg, momentum):
+    """List lengths at the edge of a CTA, capacities far above the length, and
+    more entries than the largest grid has threads; with the order of a list's
+    entries at random, distinct within a segment."""
+    from gtopkssgd_b200.ops.sgd import SgdHyper, sgd_sparse
+    d = max(4 * capacity, 64)
+    torch.manual_seed(n + nseg)
+    gen = torch.Generator(device=DEV).manual_seed(n)
+    p0 = torch.randn(d, device=DEV, generator=gen)
+    p, buf = p0.clone(), torch.zeros(d, device=DEV)
+    pairs = torch.zeros((nseg * capacity, 2), dtype=torch.int32, device=DEV)
+    want = torch.zeros(d, dtype=torch.float64, device=DEV)
+    for s in range(nseg):
+        idx = torch.randperm(d, device=DEV, generator=gen)[:n]
+        val = torch.randn(n, device=DEV, generator=gen)
+        pairs[s * capacity:s * capacity + n, 0] = idx.int()
+        pairs[s * capacity:s * capacity + n, 1] = val.view(torch.int32)
+        want.index_add_(0, idx, val.double())
+    counts = torch.full((nseg,), n, dtype=torch.int32, device=DEV)
+    h = SgdHyper(lr=0.1, momentum=momentum)
+    sgd_sparse(p, buf if momentum else None, pairs, counts, nseg, capacity, h, True, 0.5, use_atomics=nseg > 1)
+    # each addition rounds once to 24 bits: values below 8, at most 2 * nseg roundings
+    assert torch.allclose(p.double(), p0.double() - 0.05 * want, rtol=0, atol=2 * nseg * 8 * 2.0 ** -24)
+    if momentum:
+        assert torch.allclose(buf.double(), 0.5 * want, rtol=0, atol=2 * nseg * 8 * 2.0 ** -24)
