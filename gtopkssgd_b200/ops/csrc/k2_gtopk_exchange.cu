@@ -32,7 +32,8 @@
 // 14 728: 43 and 32; eight ranks, k = 40 000: 122 and 85).
 //
 // No host-side clearing: the rank owns two control blocks; call e uses block
-// (e & 1) and zeroes the other one for call e + 1 once its own work is done.
+// (e & 1) and zeroes the other one for call e + 1 at its beginning, where the stores
+// are gone long before anything waits for them.
 //
 // Failure: any wait that runs out, any capacity or bounds error makes the call
 // publish an EMPTY global set (n_global = 0, so the consumer applies nothing) and
@@ -48,6 +49,11 @@ namespace gtk {
 // Union entries that each thread keeps in registers across the phases of a round.  The default CTA counts leave
 // 2 to 4 per thread up to k of about 150 000; the rest is read again from memory, as many at a time.
 constexpr int kK2Cache = 4;
+// Entries of the own selection that each thread reads with the descriptor's first words, an L2 round trip (0.8 us)
+// before it knows how many there are (two: the default CTA counts leave 1 to 2).  With the control block cleared at the
+// beginning and old residual values kept beside their indices (one look-up less behind an arrival): three worlds of two
+// ranks and k = 66 034 in turn, with the update, 39.1 -> 37.75 us; four of k = 16 000 37.8 -> 37.1.
+constexpr int kK2Own = 2;
 
 struct K2Shared {
   ExchangeShared ex;
@@ -84,9 +90,17 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
   const float kth_mag = __ldcg(&R.st->kth_mag);
   const unsigned int me = rank_base + blockIdx.y;
   const unsigned int cta = blockIdx.x, nct = gridDim.x;
-  const unsigned int parity = epoch & 1u;
   const unsigned int stride = nct * kSelThreads;
   const unsigned int lane0 = cta * kSelThreads + threadIdx.x;  // union index of this thread's trip 0
+  const unsigned int n_ahead = k < d ? k : d;
+  Pair own[kK2Own];  // this thread's first entries of the selection (beyond n_sel: whatever is there, never looked at)
+#pragma unroll
+  for (int t = 0; t < kK2Own; ++t) {
+    own[t].idx = -1;
+    own[t].val = 0.f;
+    if (lane0 + t * stride < n_ahead) own[t] = ld_pair_cg(&R.sel[lane0 + t * stride]);
+  }
+  const unsigned int parity = epoch & 1u;
   Ctrl* ctrl = R.ctrl + parity;
   int32_t* const map = R.map;
   RankBarrier bar{ctrl, nct, 0u, limit_ns, use_cluster != 0};
@@ -94,6 +108,15 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
   auto announce = [&](unsigned int q, unsigned int which, unsigned int n) {
     st_relaxed_sys_u64(reinterpret_cast<unsigned long long*>(R.peer_flags[q] + flag_off(parity, which)),
                        ((unsigned long long)epoch << 32) | n);
+  };
+  // Calls f(entry, i) for this thread's entries of the own selection; behind the ones read ahead, four loads in flight.
+  auto for_own = [&](auto f) {
+#pragma unroll
+    for (int t = 0; t < kK2Own; ++t) {
+      const unsigned int i = lane0 + t * stride;
+      if (i < n_sel) f(i < n_ahead ? own[t] : ld_pair_cg(&R.sel[i]), i);
+    }
+    for_pairs(R.sel, n_sel, lane0 + kK2Own * stride, stride, f);
   };
   // Leaves an empty result and the sticky status behind; called by every CTA that gives up.
   auto fail = [&]() {
@@ -113,14 +136,16 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
   }
 
   if (n_sel > kcap) n_sel = kcap;
-  const Pair* cur = R.sel;  // current set of this rank
-  unsigned int n_cur = n_sel;
-  int cur_buf = -1;         // -1: cur is the read-only selection of K1; else index of the work buffer
-
   unsigned int rounds = 0;
   while ((1u << rounds) < P) ++rounds;
   band_clear(sh);
   if (cta == 0 && threadIdx.x == 0) ctrl->scratch[8] = 1u;  // this block's histograms will need clearing
+  // The other control block, for the next call (its last user was the call before).
+  {
+    uint4* other = reinterpret_cast<uint4*>(R.ctrl + (parity ^ 1u));
+    const size_t nvec16 = (offsetof(Ctrl, hist) + (size_t)(rounds + 1) * sizeof(((Ctrl*)0)->hist[0])) / 16;
+    for (size_t i = lane0; i < nvec16; i += stride) other[i] = make_uint4(0u, 0u, 0u, 0u);
+  }
   trace_stamp(ctrl, 0);
   // Every live entry of a round's union is counted once in the band above `pred` (delta = 1 adds, 0xffffffff
   // removes).  A prediction: for gradient tails the union's k-th magnitude is a few per cent above this rank's own,
@@ -128,43 +153,34 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
   uint32_t pred = mag_key(kth_mag);  // round 0: K1's k-th magnitude, then the previous round's threshold
   auto tally = [&](float v, unsigned int delta) { atomicAdd(&sh.band[band_bin(mag_key(v), pred)], delta); };
 
-  for (unsigned int r = 0; r < rounds; ++r) {
-    const unsigned int bit = 1u << r;
-    const unsigned int low = me & (2u * bit - 1u);
-    if (low == bit) {
-      // ---- sender: push the current set into the partner's slot
-      const unsigned int partner = me - bit;
-      if (cta == 0 && threadIdx.x == 0) announce(partner, r, n_cur);
-      unsigned long long* const dst = R.peer_slots[partner] + slot_off(parity, r, kcap);
-      for (unsigned int i = lane0; i < n_cur; i += stride) wire_store(&dst[i], ld_pair_cg(&cur[i]));
-      trace_stamp(ctrl, 1 + 8 * r + 6);
-      trace_stamp(ctrl, 1 + 8 * r + 7);
-      break;
-    }
-    if (low != 0u) break;  // already left the tree
-
+  if (me & 1u) {
+    // ---- sender of round 0: push the selection into the partner's slot
+    if (cta == 0 && threadIdx.x == 0) announce(me - 1u, 0, n_sel);
+    unsigned long long* const dst = R.peer_slots[me - 1u] + slot_off(parity, 0, kcap);
+    for_own([&](Pair e, unsigned int i) { wire_store(&dst[i], e); });
+    trace_stamp(ctrl, 1 + 6);
+    trace_stamp(ctrl, 1 + 7);
+  } else {
     // ---- receiver.  A = current set in a writable work buffer, with map[] and the band counts
-    // describing it (built here in round 0, by the previous compaction afterwards).
-    Pair* A;
-    const bool copied = cur_buf < 0;
-    if (copied) {
-      A = R.work[0];
-      for (unsigned int i = lane0; i < n_cur; i += stride) {
-        Pair e = ld_pair_cg(&cur[i]);
-        if ((unsigned int)e.idx < d) {
-          map[e.idx] = (int32_t)i;
-          tally(e.val, 1u);
-        } else {
-          record_error(ctrl, ST_BOUNDS, 300);
-          e.idx = -1;
-        }
-        st_pair(&A[i], e);
+    // describing it (built here before round 0, by the previous compaction afterwards).
+    for_own([&](Pair e, unsigned int i) {
+      if ((unsigned int)e.idx < d) {
+        map[e.idx] = (int32_t)i;
+        tally(e.val, 1u);
+      } else {
+        record_error(ctrl, ST_BOUNDS, 300);
+        e.idx = -1;
       }
-      cur_buf = 0;
-      bar.arrive();
-    } else {
-      A = R.work[cur_buf];
-    }
+      st_pair(&R.work[0][i], e);
+    });
+    bar.arrive();
+  }
+  unsigned int n_cur = n_sel;
+  int cur_buf = 0;  // of the two work buffers
+  for (unsigned int r = 0; (me & 1u) == 0u && r < rounds; ++r) {
+    const unsigned int bit = 1u << r;
+    const bool copied = r == 0u;
+    Pair* const A = R.work[cur_buf];
     unsigned int n_b = 0;
     trace_stamp(ctrl, 1 + 8 * r + 0);
     if (!cta_wait_flag(sh.ex, R.flags + flag_off(parity, r), epoch, ctrl, limit_ns, 210 + r, &n_b)) {
@@ -351,7 +367,6 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
     }
     if (last) break;
     cur_buf ^= 1;
-    cur = R.work[cur_buf];
   }
 
   // ---- the global set, and the residual put-back of S_local \ S_global
@@ -368,14 +383,16 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
     // its entries come in, with no barrier behind them.  (Table over the global set, barrier, then the put-back:
     // 10 us after the set was there at k = 66 000, 28 us at 255 000.)  One entry at a time: there is time enough, and
     // four in flight take DRAM from the root where ranks share a GPU (k = 255 000: 74.6 -> 77.7 us).
-    float* const was = reinterpret_cast<float*>(R.work[0]);
+    Pair* const was = R.work[0];
     for (unsigned int i = lane0; i < n_sel; i += stride) {
-      const Pair e = R.sel[i];
-      if ((unsigned int)e.idx >= d) continue;
-      map[e.idx] = (int32_t)i;
-      const float r0 = R.resid[e.idx];
-      was[i] = r0;
-      R.resid[e.idx] = r0 + e.val;
+      Pair e = R.sel[i];
+      if ((unsigned int)e.idx < d) {
+        map[e.idx] = (int32_t)i;
+        const float r0 = R.resid[e.idx];
+        R.resid[e.idx] = r0 + e.val;
+        e.val = r0;
+      }
+      st_pair(&was[i], e);
     }
     if (!bar.sync(420)) { fail(); return; }
     if (!cta_wait_flag(sh.ex, R.flags + flag_off(parity, kFlagBcast), epoch, ctrl, limit_ns, 410, &n_g)) {
@@ -408,19 +425,19 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
         st_pair(&G[i0 + t * stride], e[t]);
         p[t] = (unsigned int)__ldcg(&map[e[t].idx]);
       }
+      Pair w[kK2Cache];
+#pragma unroll
+      for (int t = 0; t < kK2Cache; ++t) {
+        w[t].idx = -1;
+        if (p[t] < n_sel) w[t] = ld_pair_cg(&was[p[t]]);
+      }
 #pragma unroll
       for (int t = 0; t < kK2Cache; ++t)
-        if (p[t] < n_sel && R.sel[p[t]].idx == e[t].idx) R.resid[e[t].idx] = __ldcg(&was[p[t]]);
+        if (e[t].idx >= 0 && w[t].idx == e[t].idx) R.resid[e[t].idx] = w[t].val;
     }
     if (!__syncthreads_and(ok)) { fail(); return; }
   }
   trace_stamp(ctrl, 42);
-  // ---- the other control block, for the next call (nobody waits for this rank any more)
-  {
-    uint4* other = reinterpret_cast<uint4*>(R.ctrl + (parity ^ 1u));
-    const size_t nvec16 = (offsetof(Ctrl, hist) + (size_t)(rounds + 1) * sizeof(((Ctrl*)0)->hist[0])) / 16;
-    for (size_t i = lane0; i < nvec16; i += stride) other[i] = make_uint4(0u, 0u, 0u, 0u);
-  }
   if (bar.last_arrival()) {  // every CTA is past its last use of the call counter
     if (aborted(ctrl)) {  // a bounds or capacity error that no wait noticed
       fail();
