@@ -83,7 +83,7 @@ def sgd_sparse(p: torch.Tensor, buf: Optional[torch.Tensor], pairs: torch.Tensor
                                       h.dampening, h.weight_decay, 1 if h.nesterov else 0, 1 if first_step else 0,
                                       1 if use_atomics else 0, bad,
                                       None if parity_word is None else parity_word.data_ptr(), parity_stride,
-                                      _raw_stream(index))
+                                      pairs.nbytes >> 3, _raw_stream(index))
     if code:
         _lib.check(code, "gtk_k3_sparse")
 
