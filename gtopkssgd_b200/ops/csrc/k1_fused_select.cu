@@ -29,9 +29,10 @@
 // about as much as the barrier did, and both now start in the shadow of the
 // kernel before them.
 //
-// No CTA waits for one that may not have started: within k1_pick work is handed
-// out by tickets, and a CTA only waits for tickets that running CTAs hold.  So no
-// co-residency is needed, whatever else runs on the device.
+// No CTA waits for one that may not have started: within k1_pick, work that others
+// wait for is handed out by tickets, and a CTA only waits for tickets that running
+// CTAs hold; fixed shares are for work that nobody waits for.  So no co-residency is
+// needed, whatever else runs on the device.
 //
 // No host-side clearing: the caller provides two control blocks; call i uses
 // block (i & 1) and the stream pass zeroes the other one for call i + 1 (i is
@@ -55,13 +56,13 @@ constexpr int kWarpFlushAt = kWarpStage - 32;
 constexpr long long kDynamicMinVec = 5ll * 1000 * 1000;
 constexpr unsigned int kShards = 16;       // ticket counters of the dynamic stream pass
 // Up to kPickSmall candidates one CTA selects among them, up to kPickCluster one cluster of 8 CTAs, both from
-// registers; above, all CTAs share them out by tickets.  Measured at the borders: one CTA 2.9 us at 2.6 K
-// candidates and 2 us more than the cluster at 10 K; the cluster as fast as the tickets at 35 K (9 us; whole call
-// at 14.7 M 31.3 and 31.5 us) and 3 us slower at 58 K (25.6 M: 60.8 and 58.2 us), where 8 SMs are too few for the
-// scattered write-back; the tickets 1 to 3.5 us slower at 8 K and 19 K.
+// registers; above, all CTAs share them out.  Measured at the borders: one CTA 2.9 us at 2.6 K candidates and 2 us more
+// than the cluster at 10 K; the cluster against the shares 31.85 and 31.3 us (select + update of 8 M at 0.003, 31 K
+// candidates, the cluster in launches that have one) or 1 us less than them (2.5 M at 0.01).
 constexpr unsigned int kPickSmall = 4096;
 constexpr unsigned int kPickCluster = 32768;
 constexpr int kPickCtas = 8;               // CTAs per cluster
+constexpr unsigned int kPickWide = 26000;  // largest k of a launch in clusters: of more, 1.25 k candidates are too many
 
 // Bins of the first selection level: (key - lo) >> shift, the last bin open to the top.  lo is the candidate
 // threshold and shift puts the previous call's k-th magnitude into bins 256..511, so that the new one lies in
@@ -544,6 +545,10 @@ __device__ __forceinline__ uint32_t settle_aside(PickShared& s, float* r, const 
 }
 
 constexpr int kSmallRegs = kPickSmall / kPickThreads;  // candidates per thread in registers: one CTA
+constexpr int kSweep = 8;  // candidates per thread and round of the sweep over all CTAs
+// Least share of a CTA in that sweep.  (1 024, 2 048 and 4 096: compress of 8 M at 0.005 34.4, 35.2 and 37.1 us, select
+// of 16 M at 0.001 45.8, 46.1 and 47.0; without a bound 8 M at 0.002 is 1 us slower.)
+constexpr unsigned int kMinShare = 1024u;
 constexpr int kClusterRegs = kPickCluster / (kPickCtas * kPickThreads);  // and the cluster
 constexpr unsigned int kPickChunk = 4u * kPickThreads; // candidates per ticket above
 constexpr int kExactVec = 4;                           // float4 of r per thread and ticket in exact mode
@@ -708,14 +713,18 @@ __device__ __forceinline__ uint32_t pick_cluster(PickShared& s, float* r, const 
   return aside && rank == 0u ? settle_aside(s, r, out, k - k_rem, k_rem) : th;
 }
 
-__global__ void __cluster_dims__(kPickCtas, 1, 1) __launch_bounds__(kPickThreads, 1)
-k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Winners out, unsigned int k, K1State* st,
-        Ctrl* ctrl_pair, int counted, float target_ratio, unsigned long long limit_ns) {
-  __shared__ __align__(16) PickShared s;
+// counted: the first level of the candidates has been counted by the stream pass.  WIDE: launched without clusters,
+// otherwise in clusters of kPickCtas.
+template <bool WIDE>
+__device__ __forceinline__ void pick(PickShared& s, float* r, long long d, const Pair* cand, unsigned int cap,
+                                     const Winners& out, unsigned int k, K1State* st, Ctrl* ctrl_pair, int counted,
+                                     float target_ratio, unsigned long long limit_ns) {
   // what the cluster's CTAs add to in one another, ready before the stream pass has ended
   if (threadIdx.x == 0) s.tie = s.aside_n = 0u;
-  if (threadIdx.x < (unsigned int)(kBins / kPickCtas)) s.share[0][threadIdx.x] = 0u;
-  cluster_barrier();
+  if (!WIDE) {
+    if (threadIdx.x < (unsigned int)(kBins / kPickCtas)) s.share[0][threadIdx.x] = 0u;
+    cluster_barrier();
+  }
   pdl_begin(r, cand, st, ctrl_pair);
   // one round of loads: the call's parity, both blocks' counts, and (unseen) the first candidates
   K1State was;
@@ -728,10 +737,15 @@ k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Winners out, 
   was.n_fallbacks = st->n_fallbacks;
   const unsigned int calls = was.stream_calls - 1u;
   const unsigned int n_out[2] = {__ldcg(&ctrl_pair[0].n_out), __ldcg(&ctrl_pair[1].n_out)};
+  uint2 level[2];  // WIDE (and so counted): the first level of either block
+  if (WIDE) {
+    level[0] = global_counts(ctrl_pair[0].hist[0][0]);
+    level[1] = global_counts(ctrl_pair[1].hist[0][0]);
+  }
   Pair ahead;
   ahead.idx = 0;
   ahead.val = 0.f;
-  if (blockIdx.x == 0 && threadIdx.x < cap) ahead = ld_pair_cg(&cand[threadIdx.x]);
+  if (!WIDE && blockIdx.x == 0 && threadIdx.x < cap) ahead = ld_pair_cg(&cand[threadIdx.x]);
   Ctrl* const ctrl = ctrl_pair + (calls & 1u);
   const unsigned int count = n_out[calls & 1u];
   const unsigned int C = count < cap ? count : cap;
@@ -741,7 +755,7 @@ k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Winners out, 
   Level lv{bands.lo, 0x7fffffffu, bands.shift, true};
   uint32_t th = 0u;
 
-  if (!exact_mode && C <= kPickCluster) {
+  if (!WIDE && !exact_mode && C <= kPickCluster) {
     if (C <= kPickSmall) {
       if (blockIdx.x != 0) return;
       th = pick_small(s, r, cand, out, k, C, lv, ahead);
@@ -758,12 +772,15 @@ k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Winners out, 
   int ph = 0;
   unsigned int k_rem = k;
   if (!exact_mode) {
-    // The candidates in chunks.  The first level was counted by the stream pass (counted) or is counted here.  As
-    // a rule the threshold's bin then holds few enough entries (300 to 1 400) to leave them to one CTA: a single
-    // sweep sends what lies above the bin to the list, returns what lies below to r, and puts what lies in it
-    // aside; the CTA that finishes the sweep picks among those (against a level and a sweep more: whole call
-    // at 25.6 M and 0.01 63.9 -> 60.6 us, 66 M and 0.01 148.6 -> 144.2, 138 M and 0.01 294 -> 288).
+    // The candidates shared out over all CTAs.  The first level was counted by the stream pass (counted) or is counted
+    // here, in chunks.  As a rule the threshold's bin then holds few enough entries (300 to 1 400) to leave them to
+    // one CTA: a single sweep sends what lies above the bin to the list, returns what lies below to r, and puts what
+    // lies in it aside; the CTA that finishes the sweep picks among those (against a level and a sweep more: whole
+    // call at 25.6 M and 0.01 63.9 -> 60.6 us, 66 M and 0.01 148.6 -> 144.2, 138 M and 0.01 294 -> 288).
     // A bin with more is counted by finer levels, a phase each.
+    const unsigned int share = max((C + gridDim.x - 1u) / gridDim.x, kMinShare), nshares = (C + share - 1u) / share;
+    const unsigned int begin = blockIdx.x * share, end = begin + share < C ? begin + share : C;
+    if (begin >= end) return;  // (from here on the call does not end without this CTA, however late it has started)
     const unsigned int nchunks = (C + kPickChunk - 1u) / kPickChunk;
     unsigned int* level_hist = ctrl->hist[0][0];
     bool have = counted != 0, aside = false;
@@ -780,14 +797,16 @@ k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Winners out, 
             if (lv.has(key)) atomicAdd(&s.hist[lv.bin(key)], 1u);
           }
         });
-        if (mine == 0u) return;  // those that hold chunks finish the call
-        publish_hist(s, level_hist);
+        if (mine) publish_hist(s, level_hist);
         report(ctrl, ph, mine, nchunks);
-        if (!wait_phase(s, ctrl, ph, nchunks, limit_ns, 100 + ph)) return;
+        if (!wait_phase(s, ctrl, ph, nchunks, limit_ns, 100 + ph)) return;  // (every CTA has a share of the sweep)
         ++ph;
       }
       have = false;
-      find_bin(s, global_counts(level_hist), k_rem);
+      uint2 counts;
+      if (WIDE && ph == 0) counts = (calls & 1u) ? level[1] : level[0];
+      else counts = global_counts(level_hist);
+      find_bin(s, counts, k_rem);
       k_rem = s.res_krem;
       if (!lv.narrow(s.res_bin)) break;
       if (s.res_n <= kPickSmall) {
@@ -802,19 +821,25 @@ k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Winners out, 
     Pair* const between = reinterpret_cast<Pair*>(ctrl->hist[2]);  // (rows that K1 has no other use for)
     static_assert(sizeof(ctrl->hist[2]) >= kPickSmall * sizeof(Pair), "room for the entries put aside");
     if (threadIdx.x == 0) ctrl->trace[3] = globaltimer_ns();  // k-th magnitude known, or its bin
+    // The sweep.  Every CTA has an equal share, up to kSweep entries per thread in flight, and one place in the list
+    // for all of a round's winners.  Nobody waits for anybody here, so the shares need no tickets.  (Chunks of 4 096
+    // by tickets were 9 us each, a chain of a ticket, a load, a place and the barriers between them; and in clusters,
+    // as the kernel was launched for every size, 112 of its 152 CTAs ran side by side.  select + update of 60 M at
+    // 0.007 153.9 -> 149.3 us, 16 M at 0.005 50.8 -> 49.0, 5 M at 0.01 26.6 -> 25.2; compress, which writes three
+    // lists, 4 M at 0.008 27.1 -> 22.7, 8 M at 0.005 38.7 -> 34.2, 30 M at 0.002 93.5 -> 88.6.)
     unsigned int turn = 0;
-    const unsigned int mine = for_chunks(s, ctrl, ph, nchunks, [&](unsigned int chunk) {
-      Pair c[4];
+    for (unsigned int base = begin; base < end; base += (unsigned int)kSweep * kPickThreads) {
+      Pair c[kSweep];
       unsigned int won = 0, n = 0;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const unsigned int i = chunk * kPickChunk + (unsigned int)j * kPickThreads + threadIdx.x;
+      for (int j = 0; j < kSweep; ++j) {
+        const unsigned int i = base + (unsigned int)j * kPickThreads + threadIdx.x;
         c[j].idx = -1;
         c[j].val = 0.f;
-        if (i < C) c[j] = ld_pair_cg(&cand[i]);
+        if (i < end) c[j] = ld_pair_cg(&cand[i]);
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < kSweep; ++j) {
         const uint32_t key = mag_key(c[j].val);
         bool win;
         if (aside) {
@@ -827,24 +852,24 @@ k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Winners out, 
         } else {
           win = passes(c[j].idx >= 0, key, th, k_rem, &ctrl->tie[0]);
         }
-        if (win) {
-          won |= 1u << j;
-          ++n;
-        }
+        if (win) won |= 1u << j;
+        n += (unsigned int)__popc(__ballot_sync(0xffffffffu, win));
       }
-      unsigned int pos = place(s, n, &ctrl->cursor[0], turn++);
+      unsigned int pos = place_warp(s, n, &ctrl->cursor[0], turn++);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (c[j].idx < 0) continue;
-        if (won & (1u << j)) {
-          if (pos < k) out.put(pos, c[j]);
-          ++pos;
-        } else {
+      for (int j = 0; j < kSweep; ++j) {
+        const bool win = (won & (1u << j)) != 0u;
+        const unsigned int m = __ballot_sync(0xffffffffu, win);
+        if (win) {
+          const unsigned int at = pos + __popc(m & lanemask_lt());
+          if (at < k) out.put(at, c[j]);
+        } else if (c[j].idx >= 0) {
           r[c[j].idx] = c[j].val;
         }
+        pos += (unsigned int)__popc(m);
       }
-    });
-    const bool last = report(ctrl, ph, mine, nchunks);
+    }
+    const bool last = report(ctrl, ph, 1u, nshares);
     if (aside) {
       if (threadIdx.x == 0) s.ok = last ? 1 : 0;
       __syncthreads();
@@ -980,6 +1005,19 @@ k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Winners out, 
   }
 }
 
+__global__ void __cluster_dims__(kPickCtas, 1, 1) __launch_bounds__(kPickThreads, 1)
+k1_pick(float* r, long long d, const Pair* cand, unsigned int cap, Winners out, unsigned int k, K1State* st,
+        Ctrl* ctrl_pair, int counted, float target_ratio, unsigned long long limit_ns) {
+  __shared__ __align__(16) PickShared s;
+  pick<false>(s, r, d, cand, cap, out, k, st, ctrl_pair, counted, target_ratio, limit_ns);
+}
+__global__ void __launch_bounds__(kPickThreads, 1)
+k1_pick_wide(float* r, long long d, const Pair* cand, unsigned int cap, Winners out, unsigned int k, K1State* st,
+             Ctrl* ctrl_pair, int counted, float target_ratio, unsigned long long limit_ns) {
+  __shared__ __align__(16) PickShared s;
+  pick<true>(s, r, d, cand, cap, out, k, st, ctrl_pair, counted, target_ratio, limit_ns);
+}
+
 }  // namespace gtk
 
 using namespace gtk;
@@ -1007,12 +1045,23 @@ int k1_launch_with(Stream stream_pass, float* r, long long d, unsigned int k, Pa
   const bool counted = k > kPickCluster / 8 * 3;
   cudaError_t e = stream_pass(counted, dynamic, (int)grid);
   if (e != cudaSuccess) return GTK_ERR_CUDA;
-  // k1_pick: as many clusters as exact mode can use
-  long long pick = (d + kExactChunk - 1) / kExactChunk;
-  if (pick > di->sms) pick = di->sms;
-  pick = (pick + kPickCtas - 1) / kPickCtas * kPickCtas;
-  e = launch_pdl(k1_pick, (int)pick, kPickThreads, stream, r, d, cand, cap, out, k, st, ctrl_pair, counted ? 1 : 0,
-                 target_ratio, limit_ns);
+  // The pick: as many CTAs as exact mode can use, or the sweep over many candidates.  Clusters only where a cluster may
+  // pick: 8 CTAs that each fill an SM find a place only inside one GPC, and not on every SM of it.  Without them fewer
+  // CTAs than SMs as long as the sweep is short, so that they start on the SMs whose share of the stream pass has
+  // ended, not on the last one too (with 64, 96, 111 and 148 CTAs: select + update of 5 M at 0.01 25.2, 25.2, 25.4 and
+  // 26.7 us, 30 M at 0.006 81.1, 80.8, 80.8 and 81.0, 138 M at 0.01 340, 337, 336 and 335; with fewer, exact mode would
+  // take longer).
+  const bool wide = k > kPickWide;
+  long long ctas = (d + kExactChunk - 1) / kExactChunk;
+  if (wide) {
+    const long long most = 96 + k / 16384;
+    if (ctas < (long long)k / kPickThreads) ctas = (long long)k / kPickThreads;
+    if (ctas > most) ctas = most;
+  }
+  if (ctas > di->sms) ctas = di->sms;
+  if (!wide) ctas = (ctas + kPickCtas - 1) / kPickCtas * kPickCtas;
+  e = launch_pdl(wide ? k1_pick_wide : k1_pick, (int)ctas, kPickThreads, stream, r, d, cand, cap, out, k, st, ctrl_pair,
+                 counted ? 1 : 0, target_ratio, limit_ns);
   gtk_count_launch(2);
   return e == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
 }

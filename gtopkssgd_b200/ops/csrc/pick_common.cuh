@@ -95,6 +95,19 @@ __device__ __forceinline__ unsigned int place(WideShared& s, unsigned int n, uns
   return base + before + pre - n;
 }
 
+// The same for a warp's n entries: the position of the first.  cursor: not nullptr.
+__device__ __forceinline__ unsigned int place_warp(WideShared& s, unsigned int n, unsigned int* cursor, unsigned int turn) {
+  const int w = threadIdx.x >> 5;
+  if (lane_id() == 0) s.warp_n[turn & 1u][w] = n;
+  __syncthreads();
+  const unsigned int v = s.warp_n[turn & 1u][lane_id()];
+  const unsigned int before = __reduce_add_sync(0xffffffffu, (int)lane_id() < w ? v : 0u);
+  const unsigned int total = __reduce_add_sync(0xffffffffu, v);
+  if (threadIdx.x == 0) s.base[turn & 1u] = total ? atomicAdd(cursor, total) : 0u;
+  __syncthreads();
+  return s.base[turn & 1u] + before;
+}
+
 // One entry against the threshold; called by whole warps.  Entries equal to it take tickets, the first
 // `quota` of which are selected.
 __device__ __forceinline__ bool passes(bool live, uint32_t key, uint32_t th, unsigned int quota, unsigned int* tie) {

@@ -842,3 +842,32 @@ def test_k3_sparse_covers_lists_below_at_and_beyond_its_grid(n, capacity, nseg, 
     assert torch.allclose(p.double(), p0.double() - 0.05 * want, rtol=0, atol=2 * nseg * 8 * 2.0 ** -24)
     if momentum:
         assert torch.allclose(buf.double(), 0.5 * want, rtol=0, atol=2 * nseg * 8 * 2.0 ** -24)
+
+
+@pytest.mark.parametrize("d,k", [(27_000, 26_001), (100_000, 26_000), (100_000, 26_001), (2_000_000, 27_500), (6_000_000, 130_000),
+                                 (5_000_000, 1_300_000)])
+@pytest.mark.parametrize("form", ["select", "compress", "ties"])
+def test_k1_pick_shares_many_candidates_out(d, k, form):
+    """The pick without clusters, from its smallest k on: nearly everything
+    selected, shares of less and of more than one round, few CTAs and all of
+    them, and candidates so often equal that the threshold's bin is counted by
+    finer levels or is a single magnitude."""
+    torch.manual_seed(k)
+    sel = _selector(d, k)
+    r = torch.zeros(d, device=DEV)
+    for it in range(4):
+        g = torch.randn(d, device=DEV)
+        if form == "ties":
+            g = (g * 8).round() / 8
+            r.zero_()
+        acc = g + r
+        if form == "compress":
+            idx, val = sel.compress(g, r, k)
+            want = torch.zeros(d, device=DEV)
+            want[idx] = val
+            assert torch.equal(g, want)
+        else:
+            sel.select(g, r, k)
+            idx, val = sel.pairs()
+        assert sel.status() == (0, 0)
+        _check_selection(idx, val, r, acc, k)
