@@ -62,7 +62,14 @@ constexpr unsigned int kShards = 16;       // ticket counters of the dynamic str
 constexpr unsigned int kPickSmall = 4096;
 constexpr unsigned int kPickCluster = 32768;
 constexpr int kPickCtas = 8;               // CTAs per cluster
-constexpr unsigned int kPickWide = 26000;  // largest k of a launch in clusters: of more, 1.25 k candidates are too many
+// Launches without clusters: from kCountFrom on, and from kPickWide on where the stream pass is short (2 M and less; the
+// start of more CTAs shows there).  select + update with and without clusters: 13 M at 0.001 40.4 and 40.0 us, 8 M at
+// 0.002 31.2 and 30.7, 25 M at 0.001 63.1 and 62.2, 1.6 M at 0.01 16.1 and 16.7, 2 M at 0.01 18.0 and 17.6.  Where
+// each winner goes to three places (gtk_k1_compress) 8 SMs are too few at any length: 8 M at 0.002 36.0 and 34.4,
+// 16 M at 0.0015 58.7 and 55.1; below kCountFrom 8 M at 0.001 32.5 and 34.1.
+constexpr unsigned int kCountFrom = kPickCluster / 8 * 3;
+constexpr unsigned int kPickWide = 18000;
+constexpr long long kWideShort = 3ll * 1000 * 1000;
 
 // Bins of the first selection level: (key - lo) >> shift, the last bin open to the top.  lo is the candidate
 // threshold and shift puts the previous call's k-th magnitude into bins 256..511, so that the new one lies in
@@ -1042,7 +1049,7 @@ int k1_launch_with(Stream stream_pass, float* r, long long d, unsigned int k, Pa
   // The first level is counted on the fly where the candidates (up to 3 k, 2.3 k as a rule) will be shared out by
   // tickets, which saves these a phase of 2 us; below, the CTAs that pick count faster than the stream pass
   // publishes.
-  const bool counted = k > kPickCluster / 8 * 3;
+  const bool counted = k > kCountFrom;
   cudaError_t e = stream_pass(counted, dynamic, (int)grid);
   if (e != cudaSuccess) return GTK_ERR_CUDA;
   // The pick: as many CTAs as exact mode can use, or the sweep over many candidates.  Clusters only where a cluster may
@@ -1051,7 +1058,7 @@ int k1_launch_with(Stream stream_pass, float* r, long long d, unsigned int k, Pa
   // ended, not on the last one too (with 64, 96, 111 and 148 CTAs: select + update of 5 M at 0.01 25.2, 25.2, 25.4 and
   // 26.7 us, 30 M at 0.006 81.1, 80.8, 80.8 and 81.0, 138 M at 0.01 340, 337, 336 and 335; with fewer, exact mode would
   // take longer).
-  const bool wide = k > kPickWide;
+  const bool wide = k > (out.dense || d >= kWideShort ? kCountFrom : kPickWide);
   long long ctas = (d + kExactChunk - 1) / kExactChunk;
   if (wide) {
     const long long most = 96 + k / 16384;
