@@ -33,6 +33,7 @@ __host__ __device__ constexpr size_t ll_off(unsigned int parity, unsigned int ro
 
 struct K2Rank {
   const Pair* sel;        // local selection written by K1
+  unsigned int sel_cap;   // pairs that its buffer holds
   const K1State* st;      // st->n_sel = number of local pairs
   // Merge buffers.  Tree: [kcap] and [2 * kcap] pairs, the second half of work[1] for received entries.  K2t:
   // work[0] is the union [work_cap], work[1] holds a word per entry of it.

@@ -92,7 +92,7 @@ k2_gtopk_exchange(const K2Rank* __restrict__ ranks, unsigned int rank_base, unsi
   const unsigned int cta = blockIdx.x, nct = gridDim.x;
   const unsigned int stride = nct * kSelThreads;
   const unsigned int lane0 = cta * kSelThreads + threadIdx.x;  // union index of this thread's trip 0
-  const unsigned int n_ahead = k < d ? k : d;
+  const unsigned int n_ahead = k < R.sel_cap ? k : R.sel_cap;
   Pair own[kK2Own];  // this thread's first entries of the selection (beyond n_sel: whatever is there, never looked at)
 #pragma unroll
   for (int t = 0; t < kK2Own; ++t) {
@@ -477,7 +477,7 @@ extern "C" void gtk_symm_layout(unsigned int kcap, int with_allgather, unsigned 
 }
 
 // Fill one K2Rank descriptor on the host (the caller copies it to the device).
-extern "C" int gtk_k2rank_fill(void* desc_host, const void* sel, const void* st, void* work0,
+extern "C" int gtk_k2rank_fill(void* desc_host, const void* sel, unsigned int sel_cap, const void* st, void* work0,
                                void* work1, void* map, void* resid, void* symm_local, void* ctrl,
                                void* n_global, void* epoch_word, unsigned int kcap,
                                int with_allgather, unsigned int P, void* const* symm_peers) {
@@ -486,6 +486,7 @@ extern "C" int gtk_k2rank_fill(void* desc_host, const void* sel, const void* st,
   gtk_symm_layout(kcap, with_allgather, lay);
   K2Rank* r = (K2Rank*)desc_host;
   r->sel = (const Pair*)sel;
+  r->sel_cap = sel_cap;
   r->st = (const K1State*)st;
   r->work[0] = (Pair*)work0;
   r->work[1] = (Pair*)work1;

@@ -149,6 +149,7 @@ k2_tree_small(const K2Rank* ranks, unsigned int rank_base, unsigned int P, unsig
   // the descriptor (several ranks' are put together by a kernel, possibly the one just before), then one round of loads
   const K2Rank& R = ranks[blockIdx.x];
   const Pair* const sel = R.sel;
+  const unsigned int n_ahead = k < R.sel_cap ? k : R.sel_cap;
   const K1State* const st = R.st;
   unsigned int* const epoch_word = R.epoch;
   unsigned int* const result = R.n_global;
@@ -165,7 +166,7 @@ k2_tree_small(const K2Rank* ranks, unsigned int rank_base, unsigned int P, unsig
     const unsigned int i = (unsigned int)u * kPickThreads + tid;
     own[u].idx = -1;
     own[u].val = 0.f;
-    if (i < k) own[u] = ld_pair_cg(&sel[i]);
+    if (i < n_ahead) own[u] = ld_pair_cg(&sel[i]);
   }
   const unsigned int parity = epoch & 1u;
   Ctrl* const ctrl = ctrl_pair + parity;

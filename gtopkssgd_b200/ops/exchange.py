@@ -147,7 +147,8 @@ class ExchangeRank:
         host = (C.c_char * nb)()
         peers = (C.c_void_p * MAX_PEERS)(*([C.c_void_p(p) for p in region.peer_ptrs] +
                                            [C.c_void_p(0)] * (MAX_PEERS - world)))
-        _lib.check(L.gtk_k2rank_fill(host, selector.sel.data_ptr(), selector.state.data_ptr(), self.work0.data_ptr(),
+        _lib.check(L.gtk_k2rank_fill(host, selector.sel.data_ptr(), selector.sel.shape[0],
+                                     selector.state.data_ptr(), self.work0.data_ptr(),
                                      self.work1.data_ptr(), self.map.data_ptr(), resid.data_ptr(), region.local_ptr,
                                      self.ctrl.data_ptr(), self.n_global.data_ptr(), self.epoch.data_ptr(), self.kcap,
                                      int(with_allgather), world, peers), "gtk_k2rank_fill")

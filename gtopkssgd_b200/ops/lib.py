@@ -64,7 +64,7 @@ def _declare(lib):
     lib.gtk_last_cuda_error.restype = C.c_char_p
     lib.gtk_symm_layout.argtypes = [u32, i32, C.POINTER(u64)]
     lib.gtk_symm_layout.restype = None
-    lib.gtk_k2rank_fill.argtypes = [vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, u32, i32, u32, C.POINTER(vp)]
+    lib.gtk_k2rank_fill.argtypes = [vp, vp, u32, vp, vp, vp, vp, vp, vp, vp, vp, vp, u32, i32, u32, C.POINTER(vp)]
     lib.gtk_k2rank_fill.restype = i32
     lib.gtk_p2p_alloc.argtypes = [u64, C.POINTER(vp)]
     lib.gtk_p2p_alloc.restype = i32

@@ -871,3 +871,29 @@ def test_k1_pick_shares_many_candidates_out(d, k, form):
             idx, val = sel.pairs()
         assert sel.status() == (0, 0)
         _check_selection(idx, val, r, acc, k)
+
+
+@pytest.mark.parametrize("d,max_k,kcap", [(20_000, 300, 1000), (400_000, 3000, 9000)])  # one CTA per rank, several
+def test_exchange_with_selections_shorter_than_its_k(d, max_k, kcap):
+    """The exchange may be set up for more entries than its selectors ever
+    deliver: nothing is read beyond a selection's buffer, and all entries stay."""
+    from gtopkssgd_b200.ops import exchange as ex
+    torch.manual_seed(d)
+    P = 2
+    regions = ex.SymmetricRegion.create_emulated(P, ex.region_bytes(kcap, False), DEV)
+    ranks, sels, grads = [], [], [torch.randn(d, device=DEV) for _ in range(P)]
+    for r in range(P):
+        sel, resid = _selector(d, max_k), torch.zeros(d, device=DEV)
+        ranks.append(ex.ExchangeRank(r, P, d, kcap, sel, resid, regions[r]))
+        sel.select(grads[r], resid, max_k)
+        sels.append(sel.pairs())
+    ex.launch_gtopk(ranks, torch.cat([r.desc for r in ranks]), 0, P, kcap, limit_ms=2000)
+    torch.cuda.synchronize()
+    total = torch.zeros(d, device=DEV)
+    for idx, val in sels:
+        total[idx] += val
+    for r in ranks:
+        assert r.status() == (0, 0)
+        gi, gv = _read_gout(r, r.last_parity())
+        assert sorted(gi.tolist()) == total.nonzero().view(-1).tolist()
+        assert torch.equal(gv, total[gi])
