@@ -832,8 +832,8 @@ __device__ __forceinline__ void pick(PickShared& s, float* r, long long d, const
     // for all of a round's winners.  Nobody waits for anybody here, so the shares need no tickets.  (Chunks of 4 096
     // by tickets were 9 us each, a chain of a ticket, a load, a place and the barriers between them; and in clusters,
     // as the kernel was launched for every size, 112 of its 152 CTAs ran side by side.  select + update of 60 M at
-    // 0.007 153.9 -> 149.3 us, 16 M at 0.005 50.8 -> 49.0, 5 M at 0.01 26.6 -> 25.2; compress, which writes three
-    // lists, 4 M at 0.008 27.1 -> 22.7, 8 M at 0.005 38.7 -> 34.2, 30 M at 0.002 93.5 -> 88.6.)
+    // 0.007 153.2 -> 149.2 us, 16 M at 0.005 51.0 -> 49.7, 5 M at 0.01 26.8 -> 25.9; compress, which writes three
+    // lists, 4 M at 0.008 27.1 -> 22.9, 8 M at 0.005 38.5 -> 34.5, 30 M at 0.002 93.3 -> 88.6.)
     unsigned int turn = 0;
     for (unsigned int base = begin; base < end; base += (unsigned int)kSweep * kPickThreads) {
       Pair c[kSweep];
@@ -1054,14 +1054,14 @@ int k1_launch_with(Stream stream_pass, float* r, long long d, unsigned int k, Pa
   if (e != cudaSuccess) return GTK_ERR_CUDA;
   // The pick: as many CTAs as exact mode can use, or the sweep over many candidates.  Clusters only where a cluster may
   // pick: 8 CTAs that each fill an SM find a place only inside one GPC, and not on every SM of it.  Without them fewer
-  // CTAs than SMs as long as the sweep is short, so that they start on the SMs whose share of the stream pass has
-  // ended, not on the last one too (with 64, 96, 111 and 148 CTAs: select + update of 5 M at 0.01 25.2, 25.2, 25.4 and
-  // 26.7 us, 30 M at 0.006 81.1, 80.8, 80.8 and 81.0, 138 M at 0.01 340, 337, 336 and 335; with fewer, exact mode would
-  // take longer).
+  // CTAs than SMs as long as the sweep is short, so that the call does not wait for CTAs on the SMs that end the stream
+  // pass last (with 96, 118 and 148 CTAs: select + update of 5 M at 0.01 25.2, 25.9 and 26.7 us, 16 M at 0.005 49.0,
+  // 49.7 and 50.0), and as many as make exact mode no slower than in clusters (8 M at 0.002, a first call: 68.9, 61.8
+  // and 57.7 us, in clusters 62.1; 30 M at 0.003 231, 203, 190 and 211).
   const bool wide = k > (out.dense || d >= kWideShort ? kCountFrom : kPickWide);
   long long ctas = (d + kExactChunk - 1) / kExactChunk;
   if (wide) {
-    const long long most = 96 + k / 16384;
+    const long long most = 118 + k / 8192;
     if (ctas < (long long)k / kPickThreads) ctas = (long long)k / kPickThreads;
     if (ctas > most) ctas = most;
   }
