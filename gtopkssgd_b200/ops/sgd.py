@@ -48,6 +48,12 @@ def sgd_dense(p: torch.Tensor, buf: Optional[torch.Tensor], h: SgdHyper, first_s
         _lib.check(code, "gtk_k3_dense")
 
 
+def _readable_pairs(pairs: torch.Tensor) -> int:
+    """How many pairs may be read from the tensor's address on, valid or not (0: not known).  An expanded view, or
+    another whose elements do not lie side by side, has more bytes than there is memory behind it."""
+    return pairs.nbytes >> 3 if pairs.is_contiguous() else 0
+
+
 def sgd_sparse(p: torch.Tensor, buf: Optional[torch.Tensor], pairs: torch.Tensor, counts: torch.Tensor,
                nseg: int, seg_stride: int, h: SgdHyper, first_step: bool, scale: float,
                coef: Optional[torch.Tensor] = None, use_atomics: bool = False,
@@ -83,7 +89,7 @@ def sgd_sparse(p: torch.Tensor, buf: Optional[torch.Tensor], pairs: torch.Tensor
                                       h.dampening, h.weight_decay, 1 if h.nesterov else 0, 1 if first_step else 0,
                                       1 if use_atomics else 0, bad,
                                       None if parity_word is None else parity_word.data_ptr(), parity_stride,
-                                      pairs.nbytes >> 3, _raw_stream(index))
+                                      _readable_pairs(pairs), _raw_stream(index))
     if code:
         _lib.check(code, "gtk_k3_sparse")
 

@@ -787,3 +787,44 @@ def test_block_layers_may_be_plain_callables():
     block.bn_a = lambda y: 2.0 * y
     want = torch.relu(x + block.bn_b(block.conv_b(torch.relu(2.0 * block.conv_a(x)))))
     assert torch.allclose(block(x), want, atol=1e-6)
+
+
+class _OnDevice:
+    """A parameter vector that says it is on a device, for looking at a launch's arguments."""
+    is_cuda = True
+
+    def __init__(self, d):
+        self.d = d
+
+    def numel(self):
+        return self.d
+
+    def get_device(self):
+        return 0
+
+    def data_ptr(self):
+        return 256
+
+
+def _sparse_launches(monkeypatch):
+    """Arguments of the sparse update's launches from here on, nothing launched."""
+    from types import SimpleNamespace
+    from gtopkssgd_b200.ops import sgd
+    launches = []
+    fake = SimpleNamespace(gtk_k3_sparse=lambda *a: launches.append(a) or 0)
+    monkeypatch.setattr(sgd._lib, "calls", lambda: fake)
+    monkeypatch.setattr(sgd, "_raw_stream", lambda index: 0)
+    monkeypatch.setattr(sgd, "_scratch_address", lambda index: 0)
+    return launches
+
+
+@pytest.mark.parametrize("view,readable", [(lambda t: t, 24), (lambda t: t[5:], 19), (lambda t: t[3:4], 1),
+                                           (lambda t: t[:1].expand(1 << 20, 2), 0), (lambda t: t[::2], 0),
+                                           (lambda t: t[:0], 0)])
+def test_sparse_update_reads_ahead_only_what_a_tensor_holds(monkeypatch, view, readable):
+    """The kernel may read pairs that are not valid, but none that no memory is behind."""
+    from gtopkssgd_b200.ops.sgd import SgdHyper, sgd_sparse
+    launches = _sparse_launches(monkeypatch)
+    pairs = torch.zeros((24, 2), dtype=torch.int32)
+    sgd_sparse(_OnDevice(100), None, view(pairs), torch.ones(1, dtype=torch.int32), 1, 8, SgdHyper(lr=0.1), False, 1.0)
+    assert launches[0][-2] == readable
