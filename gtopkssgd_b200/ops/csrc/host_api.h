@@ -77,7 +77,7 @@ int gtk_k3_sparse(float* p, float* buf, const void* pairs, const unsigned int* c
                   unsigned int seg_stride, const float* coef, float scale, unsigned int d, float lr,
                   const float* lr_ptr, float momentum, float dampening, float weight_decay, int nesterov,
                   int first_step, int use_atomics, unsigned int* bad_index_count, const unsigned int* parity_word,
-                  unsigned int parity_stride, unsigned long long n_pairs, void* stream);
+                  unsigned int parity_stride, unsigned long long n_pairs, unsigned int max_count, void* stream);
 int gtk_k3_scatter_dense(float* g, const void* pairs, const unsigned int* counts, unsigned int nseg,
                          unsigned int seg_stride, float scale, long long d, int use_atomics,
                          const unsigned int* parity_word, unsigned int parity_stride, void* stream);

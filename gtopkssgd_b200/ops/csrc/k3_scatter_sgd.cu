@@ -104,10 +104,16 @@ k3_dense(float* p, float* buf, const float* g,
 // there side by side.  With four entries per thread in a grid that fills the chip once, all of it loads first and
 // stores afterwards: select + update of 138 M elements at 0.01 353 us against 337, with momentum 422 against 397
 // (60 M: 191 and 181; two entries per thread: 340, 408 and 188); the same up to 300 000 entries.
-// (The grid goes by the lists' capacity, of which there may be much more than entries: it ends at 16 times what the
-// chip holds, 4.8 M entries, and the threads loop from there on.)
+// The lists may be far shorter than their buffers (four times after the first epoch of the default schedule), and then
+// reading up to the buffers' end, or CTAs without entries, are most of what there is to do.  So the grid goes by the
+// caller's count where there is one, it ends at four times what the chip holds (1.2 M entries over all lists; the threads
+// loop from there on), and entries are read ahead of the counts only where they are few.  Against a grid and a read-ahead
+// up to the buffers' size, without a count and with it: eight lists of 138 000 entries in four times the room 55.0, 43.5
+// and 43.5 us, eight of 13 800 in 40 times 22.7, 10.3 and 9.5, one of 345 000 in four times 9.5, 8.5 and 7.5; a full
+// one of 1.38 M 63.0 and 63.5, where two times what the chip holds takes 65.2.
 constexpr int kSparseThreads = 256;
-constexpr unsigned int kSparseMaxBlocks = 148u * 8u * 16u;
+constexpr unsigned int kSparseMaxBlocks = 4u * 148u * 8u;
+constexpr unsigned long long kSparseAhead = 1ull << 18;  // entries over all lists
 __global__ void __launch_bounds__(kSparseThreads)
 k3_sparse(float* p, float* buf, const Pair* pairs,
           const unsigned int* counts, unsigned int seg_stride,
@@ -252,23 +258,27 @@ extern "C" int gtk_k3_dense(float* p, float* buf, const float* g, const float* c
   return e == cudaSuccess ? GTK_OK : GTK_ERR_CUDA;
 }
 
-// n_pairs: how many pairs may be read from `pairs` on (0: only the valid ones).
+// n_pairs: how many pairs may be read from `pairs` on (0: only the valid ones).  max_count: as many of them as a list
+// has entries (0: not known); lists that are longer all the same are worked off too.
 extern "C" int gtk_k3_sparse(float* p, float* buf, const void* pairs, const unsigned int* counts,
                              unsigned int nseg, unsigned int seg_stride, const float* coef,
                              float scale, unsigned int d, float lr, const float* lr_ptr, float momentum,
                              float dampening, float weight_decay, int nesterov, int first_step,
                              int use_atomics, unsigned int* bad_index_count,
                              const unsigned int* parity_word, unsigned int parity_stride,
-                             unsigned long long n_pairs, void* stream_) {
+                             unsigned long long n_pairs, unsigned int max_count, void* stream_) {
   cudaStream_t stream = (cudaStream_t)stream_;
   if (nseg == 0 || seg_stride == 0) return GTK_ERR_ARG;
   SgdHyper h{lr_ptr, lr, momentum, dampening, weight_decay, nesterov, first_step};
-  unsigned int blocks = (seg_stride + kSparseThreads - 1u) / kSparseThreads;
-  if (blocks > kSparseMaxBlocks) blocks = kSparseMaxBlocks;
+  const unsigned int length = max_count && max_count < seg_stride ? max_count : seg_stride;
+  const unsigned int most = kSparseMaxBlocks / nseg;
+  unsigned int blocks = (length + kSparseThreads - 1u) / kSparseThreads;
+  if (blocks > most) blocks = most ? most : 1u;
   // Behind a large exchange (a cooperative kernel, which cannot overlap) an ordinary launch: there the overlapped
   // one made the next exchange start 2 us later (57.3 against 55.4 us per exchange + update at 2 x 66 000).
   const bool overlap = parity_word == nullptr || seg_stride <= kLLMaxK;
-  const int ahead = n_pairs >= (unsigned long long)nseg * seg_stride + (parity_word ? parity_stride : 0u);
+  const int ahead = (unsigned long long)nseg * length <= kSparseAhead &&
+                    n_pairs >= (unsigned long long)nseg * seg_stride + (parity_word ? parity_stride : 0u);
   const cudaError_t e = launch_pdl_if(overlap, k3_sparse, dim3(blocks, nseg), kSparseThreads, stream, p, buf, (const Pair*)pairs, counts,
                                       seg_stride, coef, scale, d, h, use_atomics, bad_index_count, parity_word, parity_stride, ahead);
   gtk_count_launch(1);

@@ -48,22 +48,19 @@ def sgd_dense(p: torch.Tensor, buf: Optional[torch.Tensor], h: SgdHyper, first_s
         _lib.check(code, "gtk_k3_dense")
 
 
-def _readable_pairs(pairs: torch.Tensor) -> int:
-    """How many pairs may be read from the tensor's address on, valid or not (0: not known).  An expanded view, or
-    another whose elements do not lie side by side, has more bytes than there is memory behind it."""
-    return pairs.nbytes >> 3 if pairs.is_contiguous() else 0
-
-
 def sgd_sparse(p: torch.Tensor, buf: Optional[torch.Tensor], pairs: torch.Tensor, counts: torch.Tensor,
                nseg: int, seg_stride: int, h: SgdHyper, first_step: bool, scale: float,
                coef: Optional[torch.Tensor] = None, use_atomics: bool = False,
                bad_index_count: Optional[torch.Tensor] = None, lr_dev: Optional[torch.Tensor] = None,
-               parity_word: Optional[torch.Tensor] = None, parity_stride: int = 0) -> None:
+               parity_word: Optional[torch.Tensor] = None, parity_stride: int = 0, max_count: int = 0) -> None:
     """Sparse part of the step: for every pair (j, v) of every segment add
     ``coef * scale * v`` as gradient of element j.  ``counts`` is a device
     tensor with the live length of each segment.  ``lr_dev`` (a device scalar)
     overrides ``h.lr``; ``parity_word`` selects the half of a two-parity buffer
-    on the device: base = pairs + ((word - 1) & 1) * parity_stride."""
+    on the device: base = pairs + ((word - 1) & 1) * parity_stride.
+    ``max_count``: how long a segment's list is expected to be at most, where
+    the caller knows it to be shorter than ``seg_stride`` (0: not known); it
+    decides how much is launched, not what is applied."""
     d = p.numel()
     if not p.is_cuda:
         if parity_word is not None:
@@ -82,14 +79,20 @@ def sgd_sparse(p: torch.Tensor, buf: Optional[torch.Tensor], pairs: torch.Tensor
             p.index_add_(0, idx, step, alpha=-h.lr)
         return
     index = p.get_device()
-    bad = _scratch_address(index) if bad_index_count is None else bad_index_count.data_ptr()
+    if bad_index_count is None:
+        bad = _scratch_addresses.get(index) or _scratch_address(index)
+    else:
+        bad = bad_index_count.data_ptr()
+    # how many pairs may be read, valid or not (0: not known): an expanded view, or another whose elements do not lie side
+    # by side, has more bytes than there is memory behind it
+    readable = pairs.nbytes >> 3 if pairs.is_contiguous() else 0
     code = _lib.calls().gtk_k3_sparse(p.data_ptr(), None if buf is None else buf.data_ptr(), pairs.data_ptr(),
                                       counts.data_ptr(), nseg, seg_stride, None if coef is None else coef.data_ptr(),
                                       scale, d, h.lr, None if lr_dev is None else lr_dev.data_ptr(), h.momentum,
                                       h.dampening, h.weight_decay, 1 if h.nesterov else 0, 1 if first_step else 0,
                                       1 if use_atomics else 0, bad,
                                       None if parity_word is None else parity_word.data_ptr(), parity_stride,
-                                      _readable_pairs(pairs), _raw_stream(index))
+                                      readable, max_count, _raw_stream(index))
     if code:
         _lib.check(code, "gtk_k3_sparse")
 

@@ -67,6 +67,8 @@ class SparseResult:
     # exchange's call counter, base = pairs + ((word - 1) & 1) * parity_stride (None: single buffer)
     parity_word: Optional[torch.Tensor] = None
     parity_stride: int = 0
+    # entries of a segment at most: seg_stride goes by the schedule's largest density (0: not known)
+    max_count: int = 0
 
     def live_pairs(self) -> torch.Tensor:
         """The live half as a tensor (reads the counter: synchronises)."""
@@ -155,22 +157,23 @@ class GroupEngine:
         t.stop(self.g.key, "compression")
         t.start(self.g.key, "allreduce")
         if world == 1:
-            self.result = SparseResult(self.selector.sel, self.selector.n_sel_tensor, 1, self.max_k, False, 1.0)
+            self.result = SparseResult(self.selector.sel, self.selector.n_sel_tensor, 1, self.max_k, False, 1.0,
+                                       max_count=k)
         elif self.is_cuda and not self.staged:
             rc = self.rank_ctx
             if mode == "gtopk":
                 ex.launch_gtopk([rc], rc.desc, o.rank(), world, k, limit_ms=o.wait_limit_ms)
                 self.result = SparseResult(self.gout, rc.n_global, 1, self.max_k, False, 1.0 / world,
-                                           rc.epoch, rc.parity_stride)
+                                           rc.epoch, rc.parity_stride, k)
             else:
                 ex.launch_allgather([rc], rc.desc, rc.seg_counts, o.rank(), world, k,
                                     reselect=(mode == "topk2"), limit_ms=o.wait_limit_ms)
                 if mode == "topk":
                     self.result = SparseResult(self.ag, rc.seg_counts, world, self.max_k, True, 1.0 / world,
-                                               rc.epoch, rc.ag_parity_stride)
+                                               rc.epoch, rc.ag_parity_stride, k)
                 else:
                     self.result = SparseResult(self.gout, rc.n_global, 1, self.max_k, False, 1.0 / world,
-                                               rc.epoch, rc.parity_stride)
+                                               rc.epoch, rc.parity_stride, k)
             rc.mirror_status()  # 16 bytes to pinned host memory, read by poll_failure() before the next iteration
         else:
             self._reduce_host(k, world, mode)
@@ -190,13 +193,13 @@ class GroupEngine:
                 n = tensors_to_pairs(gi, gv, self.host_pairs)
                 self.host_counts[0] = n
                 self.result = SparseResult(self.host_pairs, self.host_counts, 1, self.host_pairs.shape[0], False,
-                                           1.0 / world)
+                                           1.0 / world, max_count=n)
             elif mode == "topk":
                 ai, av = fallback.topk_allgather(idx, val, group=grp)
                 n = tensors_to_pairs(ai, av, self.host_pairs)
                 self.host_counts[0] = n
                 self.result = SparseResult(self.host_pairs, self.host_counts, 1, self.host_pairs.shape[0], True,
-                                           1.0 / world)
+                                           1.0 / world, max_count=n)
             else:  # topk2
                 ai, av = fallback.topk_allgather(idx, val, group=grp)
                 kk = idx.numel()
@@ -206,7 +209,7 @@ class GroupEngine:
                 n = tensors_to_pairs(gi, gv, self.host_pairs)
                 self.host_counts[0] = n
                 self.result = SparseResult(self.host_pairs, self.host_counts, 1, self.host_pairs.shape[0], False,
-                                           1.0 / world)
+                                           1.0 / world, max_count=n)
         except fallback.PeerTimeout as exc:
             o.report_failure(str(exc))
             raise GTopkTimeout(str(exc)) from exc

@@ -428,7 +428,7 @@ class _DistributedOptimizer(torch.optim.Optimizer):
                 r = eng.result
                 sgd_sparse(p, buf, r.pairs, r.counts, r.nseg, r.seg_stride, h, first, r.scale, coef=self._post_coef,
                            use_atomics=r.use_atomics, lr_dev=lr_dev, parity_word=r.parity_word,
-                           parity_stride=r.parity_stride)
+                           parity_stride=r.parity_stride, max_count=r.max_count)
         if use_buf and first:
             for name, slot in fb.slots.items():
                 self.state[slot.param]["momentum_buffer"] = fb.momentum_view(name)

@@ -827,4 +827,28 @@ def test_sparse_update_reads_ahead_only_what_a_tensor_holds(monkeypatch, view, r
     launches = _sparse_launches(monkeypatch)
     pairs = torch.zeros((24, 2), dtype=torch.int32)
     sgd_sparse(_OnDevice(100), None, view(pairs), torch.ones(1, dtype=torch.int32), 1, 8, SgdHyper(lr=0.1), False, 1.0)
-    assert launches[0][-2] == readable
+    assert launches[0][-3] == readable
+
+
+def test_sparse_update_is_told_how_many_entries_its_lists_have(monkeypatch):
+    """Under the default schedule the lists' buffers are sized for the first
+    epoch's density; what the update launches goes by the present one's."""
+    from gtopkssgd_b200.ops.sgd import SgdHyper, sgd_sparse
+    from gtopkssgd_b200.parallel import distributed_optimizer as do
+    counts, kept = [], do.sgd_sparse
+    monkeypatch.setattr(settings, "PIN_DENSITY", False)
+    monkeypatch.setattr(do, "sgd_sparse", lambda *a, **kw: counts.append((a[5], kw["max_count"])) or kept(*a, **kw))
+    model = torch.nn.Linear(100, 100)
+    opt = DistributedOptimizer(torch.optim.SGD(model.parameters(), lr=0.1), named_parameters=model.named_parameters(),
+                               compression=compressors["gtopk"], is_sparse=True, density=0.001)
+    for k in (40, 10):
+        opt.zero_grad()
+        model(torch.randn(4, 100)).sum().backward()
+        opt.step()
+        assert counts[-1] == (40, k)
+        opt.add_train_epoch()
+    opt.stop()
+    launches = _sparse_launches(monkeypatch)
+    sgd_sparse(_OnDevice(100), None, torch.zeros((40, 2), dtype=torch.int32), torch.ones(1, dtype=torch.int32), 1, 40,
+               SgdHyper(lr=0.1), False, 1.0, max_count=10)
+    assert launches[0][-2] == 10
