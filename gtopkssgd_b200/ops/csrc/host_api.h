@@ -55,6 +55,7 @@ unsigned long long gtk_k1state_bytes(void);
 const char* gtk_last_cuda_error(void);
 
 // ---- launches (each file documents its own) ----
+int gtk_k1_pick_is_wide(long long d, unsigned int k, int compress);
 int gtk_k1_select(const float* g, float* r, const float* g_scale, long long d, unsigned int k,
                   void* cand, unsigned int cap, void* sel, void* state, void* ctrl,
                   float target_ratio, unsigned long long limit_ns, void* stream);

@@ -62,14 +62,8 @@ constexpr unsigned int kShards = 16;       // ticket counters of the dynamic str
 constexpr unsigned int kPickSmall = 4096;
 constexpr unsigned int kPickCluster = 32768;
 constexpr int kPickCtas = 8;               // CTAs per cluster
-// Launches without clusters: from kCountFrom on, and from kPickWide on where the stream pass is short (2 M and less; the
-// start of more CTAs shows there).  select + update with and without clusters: 13 M at 0.001 40.4 and 40.0 us, 8 M at
-// 0.002 31.2 and 30.7, 25 M at 0.001 63.1 and 62.2, 1.6 M at 0.01 16.1 and 16.7, 2 M at 0.01 18.0 and 17.6.  Where
-// each winner goes to three places (gtk_k1_compress) 8 SMs are too few at any length: 8 M at 0.002 36.0 and 34.4,
-// 16 M at 0.0015 58.7 and 55.1; below kCountFrom 8 M at 0.001 32.5 and 34.1.
+// The first level is counted in the stream pass from here on: see k1_launch_with.
 constexpr unsigned int kCountFrom = kPickCluster / 8 * 3;
-constexpr unsigned int kPickWide = 18000;
-constexpr long long kWideShort = 3ll * 1000 * 1000;
 
 // Bins of the first selection level: (key - lo) >> shift, the last bin open to the top.  lo is the candidate
 // threshold and shift puts the previous call's k-th magnitude into bins 256..511, so that the new one lies in
@@ -1031,6 +1025,26 @@ using namespace gtk;
 
 extern "C" unsigned long long gtk_ctrl_bytes(void) { return sizeof(Ctrl); }
 
+// Whether a select (compress: gtk_k1_compress) of k out of d elements launches its pick without clusters.  The candidates
+// are 1.2 to 3 times k, and at most d.  One cluster picks from up to 32 K of them without a sweep over lists in memory;
+// without clusters more CTAs share that sweep.  So clusters for every vector most of which fits one, and up to the k where
+// the candidates of a short vector outgrow it; the longer the stream pass, the less the start of more CTAs shows behind
+// it, and where each winner goes to three places 8 SMs are soon too few.  In clusters and without, us:
+//   select + update   1.6 M at 0.01 16.1, 16.7   2 M at 0.01 18.0, 17.6   8 M at 0.002 31.2, 30.7
+//                     13 M at 0.001 40.4, 40.0   25 M at 0.001 63.1, 62.2
+//   select            25 K, k 18 001 12.9, 14.4   40 K, 27 000 14.1, 14.7; 36 000 14.8, 14.0
+//                     60 K, 16 000 13.1, 14.0; 24 000 14.6, 14.2   100 K, 18 001 12.85, 13.6; 24 000 15.15, 14.3
+//                     400 K, 18 001 13.3, 13.6; 24 000 14.0, 13.9   1 M, 13 000 13.7, 14.2; 18 001 14.55, 14.2
+//                     2.9 M, 13 000 16.1, 16.2; 16 000 16.95, 16.6
+//   compress          25 K, k 13 000 17.6, 18.5   60 K, 13 000 16.8, 18.0; 18 000 19.4, 18.6
+//                     100 K, 15 000 17.4, 17.7; 18 000 18.5, 17.8   200 K, 15 000 18.1, 17.7   1 M, 13 000 22.7, 21.1
+//                     8 M at 0.001 32.5, 34.1; at 0.002 36.0, 34.4   16 M at 0.0015 58.7, 55.1
+extern "C" int gtk_k1_pick_is_wide(long long d, unsigned int k, int compress) {
+  if (d < 3ll * kPickCluster / 2) return k > kPickCluster;
+  if (compress) return k > (d < 200 * 1000 ? 16000u : kCountFrom);
+  return k > (d < 800 * 1000 ? 22000u : d < 3 * 1000 * 1000 ? 18000u : kCountFrom);
+}
+
 namespace {
 // Launches the two kernels; `stream_pass(counted, dynamic, grid)` launches the first.
 template <typename Stream>
@@ -1058,7 +1072,7 @@ int k1_launch_with(Stream stream_pass, float* r, long long d, unsigned int k, Pa
   // pass last (with 96, 118 and 148 CTAs: select + update of 5 M at 0.01 25.2, 25.9 and 26.7 us, 16 M at 0.005 49.0,
   // 49.7 and 50.0), and as many as make exact mode no slower than in clusters (8 M at 0.002, a first call: 68.9, 61.8
   // and 57.7 us, in clusters 62.1; 30 M at 0.003 231, 203, 190 and 211).
-  const bool wide = k > (out.dense || d >= kWideShort ? kCountFrom : kPickWide);
+  const bool wide = gtk_k1_pick_is_wide(d, k, out.dense != nullptr) != 0;
   long long ctas = (d + kExactChunk - 1) / kExactChunk;
   if (wide) {
     const long long most = 118 + k / 8192;

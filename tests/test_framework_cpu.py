@@ -1,5 +1,6 @@
 """CPU tests of the framework layers: grouping, density schedule, compressor
 API, LR schedules, checkpoints + evaluate, log formats, models, data."""
+import ctypes
 import math
 import os
 import re
@@ -852,3 +853,15 @@ def test_sparse_update_is_told_how_many_entries_its_lists_have(monkeypatch):
     sgd_sparse(_OnDevice(100), None, torch.zeros((40, 2), dtype=torch.int32), torch.ones(1, dtype=torch.int32), 1, 40,
                SgdHyper(lr=0.1), False, 1.0, max_count=10)
     assert launches[0][-2] == 10
+
+
+@pytest.mark.parametrize("d,compress,border", [(20_000, 0, 32_768), (49_151, 0, 32_768), (49_152, 0, 22_000), (799_999, 0, 22_000),
+                                               (800_000, 0, 18_000), (2_999_999, 0, 18_000), (3_000_000, 0, 12_288),
+                                               (2_000_000_000, 0, 12_288), (49_151, 1, 32_768), (49_152, 1, 16_000),
+                                               (199_999, 1, 16_000), (200_000, 1, 12_288), (2_000_000_000, 1, 12_288)])
+def test_pick_without_clusters_is_for_more_candidates_than_one_cluster_takes(d, compress, border):
+    """Vectors whose candidates one cluster takes keep it, whatever their k."""
+    from gtopkssgd_b200.ops import lib
+    is_wide = lib.lib().gtk_k1_pick_is_wide
+    is_wide.argtypes = [ctypes.c_longlong, ctypes.c_uint, ctypes.c_int]
+    assert not is_wide(d, min(border, d), compress) and is_wide(d, border + 1, compress)

@@ -845,11 +845,12 @@ def test_k3_sparse_covers_lists_below_at_and_beyond_its_grid(n, capacity, nseg, 
 
 
 @pytest.mark.parametrize("d,k", [(19_000, 18_001), (100_000, 18_000), (100_000, 18_001), (3_000_000, 12_289), (6_000_000, 130_000),
-                                 (5_000_000, 1_300_000)])
+                                 (5_000_000, 1_300_000), (33_000, 32_769), (49_152, 16_001), (100_000, 22_001),
+                                 (200_000, 12_289), (800_000, 18_001)])
 @pytest.mark.parametrize("form", ["select", "compress", "ties"])
 def test_k1_pick_shares_many_candidates_out(d, k, form):
-    """The pick without clusters, from its smallest k on: nearly everything
-    selected, shares of less and of more than one round, few CTAs and all of
+    """The pick without clusters, from its smallest k on (compress's lies below
+    select's): nearly everything selected, shares of less and of more than one round, few CTAs and all of
     them, and candidates so often equal that the threshold's bin is counted by
     finer levels or is a single magnitude."""
     torch.manual_seed(k)
