@@ -865,3 +865,19 @@ def test_pick_without_clusters_is_for_more_candidates_than_one_cluster_takes(d, 
     is_wide = lib.lib().gtk_k1_pick_is_wide
     is_wide.argtypes = [ctypes.c_longlong, ctypes.c_uint, ctypes.c_int]
     assert not is_wide(d, min(border, d), compress) and is_wide(d, border + 1, compress)
+
+
+def test_exchange_descriptor_says_where_the_selection_ends():
+    """The kernels read a thread's first entries of the selection before they know
+    how many there are, up to the exchange's capacity or the end of the
+    selection's buffer, whichever comes first."""
+    from types import SimpleNamespace
+    from gtopkssgd_b200.ops import exchange as ex
+    from gtopkssgd_b200.ops.select import TopkSelector
+    region = SimpleNamespace(nbytes=ex.region_bytes(1000, False), local_ptr=1 << 20, peer_ptrs=[1 << 20, 1 << 24])
+    for max_k in (300, 1000):
+        sel = TopkSelector(20_000, max_k, torch.device("cpu"))
+        rank = ex.ExchangeRank(0, 2, 20_000, 1000, sel, torch.zeros(20_000), region)
+        # the descriptor's first two fields
+        assert int.from_bytes(rank.desc_host[:8], "little") == sel.sel.data_ptr()
+        assert int.from_bytes(rank.desc_host[8:12], "little") == sel.sel.shape[0] == max_k

@@ -477,9 +477,9 @@ def test_k1_compress_leaves_g_sparsified(d, k):
 
 @pytest.mark.parametrize("d,k", [(60_000, 4000), (200_000, 4096), (400_000, 30_000), (3_000_000, 65_536), (4_000_000, 400_000)])
 @pytest.mark.parametrize("off", [0, 3])
-def test_k1_pick_in_one_cta_a_cluster_and_by_tickets(d, k, off):
-    """Candidate counts on both sides of the borders between the three forms of
-    k1_pick, on aligned and unaligned views."""
+def test_k1_pick_in_one_cta_a_cluster_and_by_shares(d, k, off):
+    """Candidate counts on both sides of the borders between one CTA, a cluster and
+    shares over all CTAs, on aligned and unaligned views."""
     torch.manual_seed(k + off)
     sel = _selector(d, k)
     g, r = torch.empty(d + 4, device=DEV)[off:off + d], torch.zeros(d + 4, device=DEV)[off:off + d]
@@ -783,12 +783,15 @@ def test_exchange_of_gradients_that_cancel(mode, P, k, nctas):
             assert torch.allclose(r.resid.cpu()[same], want[same], rtol=1e-5, atol=1e-6)
 
 
-@pytest.mark.parametrize("mode,P,k", [("topk2", 8, 60_000), ("gtopk", 2, 200_000)])
-def test_exchange_stages_many_entries_per_cta(mode, P, k):
-    """Thousands of winners per CTA, so that the stage in shared memory fills and
-    empties several times in every call: all threads of a CTA have to agree on
-    when it is full (they did not always, and a call in a few hundred lost its
-    place in the output list)."""
+@pytest.mark.parametrize("mode,P,k,nctas", [("topk2", 8, 60_000, None), ("gtopk", 2, 200_000, None),
+                                            ("topk2", 8, 60_000, 4), ("gtopk", 2, 200_000, 3)])
+def test_exchange_stages_many_entries_per_cta(mode, P, k, nctas):
+    """1 300 to 1 650 winners per CTA with the CTA counts that the exchange takes
+    by itself, so that the stage in shared memory (emptied above 1 536) fills at the
+    end of a call if at all; 15 000 and 66 000 with few CTAs, where it fills and
+    empties 9 and 43 times in every call.  All threads of a CTA have to agree on when
+    it is full: where they did not, 8 ranks of 170 000 entries (4 600 winners per CTA)
+    lost their place in the output list in about one call of 50."""
     from gtopkssgd_b200.ops import exchange as ex
     d = 1_000_000
     torch.manual_seed(P)
@@ -803,9 +806,9 @@ def test_exchange_stages_many_entries_per_cta(mode, P, k):
     want = total.abs().topk(k).values[-1]
     for call in range(60):
         if mode == "topk2":
-            ex.launch_allgather(ranks, desc, seg_counts, 0, P, k, reselect=True, limit_ms=1000)
+            ex.launch_allgather(ranks, desc, seg_counts, 0, P, k, reselect=True, nctas=nctas, limit_ms=1000)
         else:
-            ex.launch_gtopk(ranks, desc, 0, P, k, limit_ms=1000)
+            ex.launch_gtopk(ranks, desc, 0, P, k, nctas=nctas, limit_ms=1000)
     torch.cuda.synchronize()
     for r in ranks:
         assert r.status() == (0, 0)
@@ -844,6 +847,44 @@ def test_k3_sparse_covers_lists_below_at_and_beyond_its_grid(n, capacity, nseg, 
         assert torch.allclose(buf.double(), 0.5 * want, rtol=0, atol=2 * nseg * 8 * 2.0 ** -24)
 
 
+@pytest.mark.parametrize("n,capacity,nseg,max_count", [(300, 300, 1, 0), (300, 300, 3, 0), (300, 1000, 3, 300), (2000, 2000, 3, 100),
+                                                       (100_000, 100_000, 3, 0), (1_300_000, 1_400_000, 1, 1_300_000)])
+@pytest.mark.parametrize("momentum", [0.0, 0.9])
+def test_k3_sparse_takes_the_live_half_of_two(n, capacity, nseg, max_count, momentum):
+    """Lists that alternate between two halves, as the exchanges leave them:
+    the half of the call counter is applied, whether entries are read ahead of it
+    (few, in a tensor that holds both halves), behind it (many, or a tensor that
+    ends before the second half's lists do), or in a loop (lists longer than
+    expected, or than the largest grid)."""
+    from gtopkssgd_b200.ops.sgd import SgdHyper, sgd_sparse
+    d, stride = 4 * capacity, 4 * capacity  # (room for four lists per half)
+    gen = torch.Generator(device=DEV).manual_seed(n + nseg)
+    p0 = torch.randn(d, device=DEV, generator=gen)
+    pairs = torch.zeros((2 * stride, 2), dtype=torch.int32, device=DEV)
+    want = torch.zeros((2, d), dtype=torch.float64, device=DEV)
+    for half in range(2):
+        for s in range(nseg):
+            at = half * stride + s * capacity
+            idx = torch.randperm(d, device=DEV, generator=gen)[:n]
+            val = torch.randn(n, device=DEV, generator=gen)
+            pairs[at:at + n, 0] = idx.int()
+            pairs[at:at + n, 1] = val.view(torch.int32)
+            want[half].index_add_(0, idx, val.double())
+    counts = torch.full((nseg,), n, dtype=torch.int32, device=DEV)
+    h = SgdHyper(lr=0.1, momentum=momentum)
+    for word in (1, 2, 3):
+        for given in (pairs, pairs[:nseg * capacity]):  # the second one's later half lies behind its end
+            p, buf = p0.clone(), torch.zeros(d, device=DEV)
+            sgd_sparse(p, buf if momentum else None, given, counts, nseg, capacity, h, True, 0.5, use_atomics=nseg > 1,
+                       parity_word=torch.tensor([word], dtype=torch.int32, device=DEV), parity_stride=stride,
+                       max_count=max_count)
+            step = 0.5 * want[(word - 1) & 1]
+            # each addition rounds once to 24 bits: values below 16, at most 2 * nseg roundings
+            assert torch.allclose(p.double(), p0.double() - 0.1 * step, rtol=0, atol=2 * nseg * 16 * 2.0 ** -24)
+            if momentum:
+                assert torch.allclose(buf.double(), step, rtol=0, atol=2 * nseg * 16 * 2.0 ** -24)
+
+
 @pytest.mark.parametrize("d,k", [(19_000, 18_001), (100_000, 18_000), (100_000, 18_001), (3_000_000, 12_289), (6_000_000, 130_000),
                                  (5_000_000, 1_300_000), (33_000, 32_769), (49_152, 16_001), (100_000, 22_001),
                                  (200_000, 12_289), (800_000, 18_001)])
@@ -874,10 +915,51 @@ def test_k1_pick_shares_many_candidates_out(d, k, form):
         _check_selection(idx, val, r, acc, k)
 
 
+@pytest.mark.parametrize("d,k,form", [(100_000, 22_001, "select"), (3_000_000, 12_289, "select"), (6_000_000, 130_000, "select"),
+                                      (200_000, 12_289, "compress"), (4_000_000, 20_000, "compress")])
+def test_k1_pick_without_clusters_predicts_and_recovers(d, k, form):
+    """Steady inputs take one exact pass, the first.  Too few candidates, or more
+    than their list holds, take another, which first puts back into the residual
+    what the stream pass took out of it."""
+    torch.manual_seed(d)
+    sel = _selector(d, k)
+    r = torch.zeros(d, device=DEV)
+
+    def call(g):
+        r.normal_().mul_(1e-3)
+        acc = g + r
+        if form == "compress":
+            idx, val = sel.compress(g, r, k)
+            want = torch.zeros(d, device=DEV)
+            want[idx] = val
+            assert torch.equal(g, want)
+        else:
+            sel.select(g, r, k)
+            idx, val = sel.pairs()
+        assert sel.status() == (0, 0)
+        _check_selection(idx, val, r, acc, k)
+        return sel.stats()
+
+    for it in range(6):
+        st = call(torch.randn(d, device=DEV))
+        assert st["n_fallbacks"] == 1 and (it == 0 or k <= st["n_cand"] <= sel.cap)
+    g = torch.randn(d, device=DEV) * 1e-3
+    g[torch.randperm(d, device=DEV)[:k // 2]] = 50.0
+    st = call(g)
+    assert st["n_cand"] == k // 2 and st["n_fallbacks"] == 2
+    call(torch.randn(d, device=DEV))
+    call(torch.randn(d, device=DEV))
+    before = sel.stats()["n_fallbacks"]
+    st = call(torch.randn(d, device=DEV) * 1000.0)
+    assert st["n_cand"] > 0.9 * d and st["n_fallbacks"] == before + (1 if st["n_cand"] > sel.cap else 0)
+    assert (st["n_cand"] > sel.cap) == (32 * k < 0.9 * d)
+
+
 @pytest.mark.parametrize("d,max_k,kcap", [(20_000, 300, 1000), (400_000, 3000, 9000)])  # one CTA per rank, several
 def test_exchange_with_selections_shorter_than_its_k(d, max_k, kcap):
     """The exchange may be set up for more entries than its selectors ever
-    deliver: nothing is read beyond a selection's buffer, and all entries stay."""
+    deliver: all of them stay, and nothing from behind them gets in.  (That the kernels
+    are told where a selection's buffer ends is checked on the host.)"""
     from gtopkssgd_b200.ops import exchange as ex
     torch.manual_seed(d)
     P = 2
