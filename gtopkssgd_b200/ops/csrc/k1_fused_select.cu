@@ -56,7 +56,7 @@ constexpr int kWarpFlushAt = kWarpStage - 32;
 constexpr long long kDynamicMinVec = 5ll * 1000 * 1000;
 constexpr unsigned int kShards = 16;       // ticket counters of the dynamic stream pass
 // Up to kPickSmall candidates one CTA selects among them, up to kPickCluster one cluster of 8 CTAs, both from
-// registers; above, all CTAs share them out.  Measured at the borders: one CTA 2.9 us at 2.6 K candidates and 2 us more
+// registers; above, and in a launch without clusters (gtk_k1_pick_is_wide), all CTAs share them out.  At the borders: one CTA 2.9 us at 2.6 K candidates and 2 us more
 // than the cluster at 10 K; the cluster against the shares 31.85 and 31.3 us (select + update of 8 M at 0.003, 31 K
 // candidates, the cluster in launches that have one) or 1 us less than them (2.5 M at 0.01).
 constexpr unsigned int kPickSmall = 4096;
@@ -551,7 +551,7 @@ constexpr int kSweep = 8;  // candidates per thread and round of the sweep over 
 // of 16 M at 0.001 45.8, 46.1 and 47.0; without a bound 8 M at 0.002 is 1 us slower.)
 constexpr unsigned int kMinShare = 1024u;
 constexpr int kClusterRegs = kPickCluster / (kPickCtas * kPickThreads);  // and the cluster
-constexpr unsigned int kPickChunk = 4u * kPickThreads; // candidates per ticket above
+constexpr unsigned int kPickChunk = 4u * kPickThreads; // candidates per ticket, where they are counted or put back
 constexpr int kExactVec = 4;                           // float4 of r per thread and ticket in exact mode
 constexpr unsigned int kExactChunk = kExactVec * 4u * kPickThreads;
 
@@ -1060,22 +1060,22 @@ int k1_launch_with(Stream stream_pass, float* r, long long d, unsigned int k, Pa
   const long long tile = (long long)kK1Threads * (dynamic ? 4 : 2);
   long long grid = (nvec + tile - 1) / tile;
   grid = grid < 1 ? 1 : (grid > full ? full : grid);
-  // The first level is counted on the fly where the candidates (up to 3 k, 2.3 k as a rule) will be shared out by
-  // tickets, which saves these a phase of 2 us; below, the CTAs that pick count faster than the stream pass
-  // publishes.
+  // The first level is counted on the fly where the candidates (1.2 to 3 times k) may be more than one cluster takes: it
+  // saves their sweep a phase of counting by tickets, 2 us; below, the CTAs that pick count faster than the stream
+  // pass publishes.
   const bool counted = k > kCountFrom;
   cudaError_t e = stream_pass(counted, dynamic, (int)grid);
   if (e != cudaSuccess) return GTK_ERR_CUDA;
   // The pick: as many CTAs as exact mode can use, or the sweep over many candidates.  Clusters only where a cluster may
   // pick: 8 CTAs that each fill an SM find a place only inside one GPC, and not on every SM of it.  Without them fewer
   // CTAs than SMs as long as the sweep is short, so that the call does not wait for CTAs on the SMs that end the stream
-  // pass last (with 96, 118 and 148 CTAs: select + update of 5 M at 0.01 25.2, 25.9 and 26.7 us, 16 M at 0.005 49.0,
+  // pass last (with 96, 118 and 148 of 148: select + update of 5 M at 0.01 25.2, 25.9 and 26.7 us, 16 M at 0.005 49.0,
   // 49.7 and 50.0), and as many as make exact mode no slower than in clusters (8 M at 0.002, a first call: 68.9, 61.8
   // and 57.7 us, in clusters 62.1; 30 M at 0.003 231, 203, 190 and 211).
   const bool wide = gtk_k1_pick_is_wide(d, k, out.dense != nullptr) != 0;
   long long ctas = (d + kExactChunk - 1) / kExactChunk;
   if (wide) {
-    const long long most = 118 + k / 8192;
+    const long long most = di->sms * 4 / 5 + k / 8192;
     if (ctas < (long long)k / kPickThreads) ctas = (long long)k / kPickThreads;
     if (ctas > most) ctas = most;
   }

@@ -50,7 +50,9 @@ namespace gtk {
 // 2 to 4 per thread up to k of about 150 000; the rest is read again from memory, as many at a time.
 constexpr int kK2Cache = 4;
 // Entries of the own selection that each thread reads with the descriptor's first words, an L2 round trip (0.8 us)
-// before it knows how many there are (two: the default CTA counts leave 1 to 2).  With the control block cleared at the
+// before it knows how many there are.  The default CTA counts leave at most two up to k of 150 000 where the GPU has one
+// or two ranks, 75 000 with four and 37 000 with eight; further ones (9 for eight ranks of 170 000) come behind, four
+// loads at a time.  With the control block cleared at the
 // beginning and old residual values kept beside their indices (one look-up less behind an arrival): three worlds of two
 // ranks and k = 66 034 in turn, with the update, 39.1 -> 37.75 us; four of k = 16 000 37.8 -> 37.1.
 constexpr int kK2Own = 2;

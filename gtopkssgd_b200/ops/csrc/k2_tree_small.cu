@@ -440,7 +440,7 @@ k2_tree_small(const K2Rank* ranks, unsigned int rank_base, unsigned int P, unsig
     }
   }
 
-  // ---- the global set: rank 0 sends it to every rank; the others put it into their buffer and their table
+  // ---- the global set: rank 0 has sent it to every rank; the others put it into their buffer
   float back[kPerThread];  // residual at the own entries: most of them get their value back
 #pragma unroll
   for (int u = 0; u < kPerThread; ++u) {

@@ -112,7 +112,7 @@ k3_dense(float* p, float* buf, const float* g,
 // and 43.5 us, eight of 13 800 in 40 times 22.7, 10.3 and 9.5, one of 345 000 in four times 9.5, 8.5 and 7.5; a full
 // one of 1.38 M 63.0 and 63.5, where two times what the chip holds takes 65.2.
 constexpr int kSparseThreads = 256;
-constexpr unsigned int kSparseMaxBlocks = 4u * 148u * 8u;
+constexpr unsigned int kSparseMaxBlocks = 4u * 148u * 8u;  // (148 SMs with 2 048 threads each)
 constexpr unsigned long long kSparseAhead = 1ull << 18;  // entries over all lists
 __global__ void __launch_bounds__(kSparseThreads)
 k3_sparse(float* p, float* buf, const Pair* pairs,

@@ -100,7 +100,7 @@ class TopkSelector:
     def trace(self) -> dict:
         """Device-side phase stamps of the last select, in nanoseconds since its
         start: slot 1 = CTA 0 finished its share of the stream pass, 2 = the pick
-        began, 3 = k-th magnitude or its bin known (more than 32 K candidates), 4 = winners
+        began, 3 = k-th magnitude or its bin known (where all CTAs share the candidates), 4 = winners
         compacted (2 to 4 only when the prediction held).  Synchronises."""
         if not self.is_cuda:
             return {}

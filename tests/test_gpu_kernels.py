@@ -53,8 +53,8 @@ def test_k1_select_matches_oracle(d, k):
 
 
 def test_k1_large_vector_dynamic_stream_pass():
-    """From 48 M elements on the stream pass hands its work out through a ticket
-    counter; compared here against the oracle computed on the device."""
+    """From 20 M elements on the stream pass hands its work out through ticket
+    counters; compared here against the oracle computed on the device."""
     d, k = 50_000_003, 50_000
     torch.manual_seed(7)
     sel = _selector(d, k)
